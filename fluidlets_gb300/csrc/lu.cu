@@ -8,9 +8,9 @@
 //                     published candidates per column (pivot search is a
 //                     grid-wide argmax, first index on ties as LAPACK's idamax),
 //                     with the next column's look-ahead overlapping it.
-//   laswp_kernel      the panel's row swaps on the other columns.
-//   trsm_f64_kernel   U12 = L11^-1 A12.
-//   dgemm_update      A22 -= L21 U12 (FP64 CUDA cores).
+//   swap_rows_kernel  the panel's row swaps on the columns left of it.
+//   swap_trsm_kernel  the swaps and U12 = L11^-1 A12 right of it, and U12's BF16 slices.
+//   slice_update      A22 -= L21 U12 in FP64 accuracy on the tensor cores (slice_gemm.cu).
 //
 // Low precision (preconditioner of FP64 GMRES-IR): blocked LU WITHOUT
 // pivoting in FP32 storage, block FLG_LU_LOWP_BLOCK = 128; the diagonal block
@@ -31,6 +31,7 @@
 #include <algorithm>
 
 #include "flg_common.cuh"
+#include "slices.cuh"
 #include "waits.cuh"
 
 namespace flg {
@@ -300,168 +301,135 @@ __global__ void __launch_bounds__(256) panel_f64_kernel(PanelArgs a) {
     }
 }
 
-// The panel's kb row interchanges (LAPACK laswp: for q = 0..kb-1 swap rows k0 + q and
-// ipiv[k0 + q]) applied to the columns [c0, c1), and with TRSM also U12 = L11^-1 A12 (the
-// unit lower L11 = A[k0:k0+kb, k0:k0+kb]) for the columns right of the panel.  Instead of
-// kb dependent read-modify-write swaps per column, each CTA first works out in shared
-// memory where every touched row's final content comes from (at most 2 kb rows: the panel
-// rows and the pivot rows below them); then each thread gathers its column's touched rows
-// with independent loads, solves, and writes them back.
-constexpr int kSwapThreads = 128;
-template <bool TRSM>
-__global__ void __launch_bounds__(kSwapThreads) swap_trsm_kernel(double *A, int64_t ld, const int32_t *ipiv,
-                                                                  int64_t k0, int kb, int64_t c0, int64_t c1) {
-    __shared__ double L[TRSM ? kPanel : 1][kPanel + 1];
-    __shared__ int64_t srow[2 * kPanel];   // slot -> row whose old content the slot's row receives
-    __shared__ int64_t xrow[kPanel];       // extra slot kb + e -> its row (a pivot row below the panel)
-    __shared__ int src[2 * kPanel];        // slot -> source slot, built by warp 0
-    __shared__ int s_ne;
-    extern __shared__ double E[];          // [extras][kSwapThreads]: old contents for the extra rows
-    const int t = threadIdx.x;
-    if (TRSM)
-        for (int e = t; e < kb * kb; e += blockDim.x) {
-            const int r = e / kb, q = e - r * kb;
-            L[r][q] = A[(k0 + r) * ld + k0 + q];
+// ---- row interchanges and U12 ---------------------------------------------------------
+// The net effect of a panel's kb <= 64 row interchanges (LAPACK laswp: for q = 0..kb-1 swap rows
+// k0 + q and ipiv[k0 + q]) on at most 2 kb rows: slot q < 64 is row k0 + q, slot 64 + q the pivot
+// row ipiv[k0 + q] where it lies below the panel and no earlier q named it.  dst[slot] is the
+// slot's row (-1: unused), src[slot] the row whose old content it receives, found by running
+// the interchanges backwards from the slot's row; one thread per slot, 64 dependent
+// compare-selects instead of 64 dependent swaps.
+__device__ __forceinline__ void swap_slots(const int32_t *ipiv, int64_t k0, int kb, int *piv, int *dst, int *src) {
+    for (int q = threadIdx.x; q < kPanel; q += blockDim.x) piv[q] = q < kb ? ipiv[k0 + q] : -1;
+    __syncthreads();
+    for (int s = threadIdx.x; s < 2 * kPanel; s += blockDim.x) {
+        const int q = s & (kPanel - 1);
+        int r = q < kb ? (int)k0 + q : -1;
+        if (s >= kPanel && q < kb) {
+            r = piv[q] >= (int)k0 + kb ? piv[q] : -1;
+            for (int p = 0; p < q; p++) r = piv[p] == r ? -1 : r;
         }
-    if (t < 32) {
-        // slots 0..kb-1: rows k0..k0+kb-1; kb.. : pivot rows below the panel, in order of appearance
-        for (int q = t; q < 2 * kPanel; q += 32) src[q] = q;
-        int ne = 0;
-        __syncwarp();
-        for (int q = 0; q < kb; q++) {
-            const int64_t p = ipiv[k0 + q];
-            int b;
-            if (p < k0 + kb) {
-                b = (int)(p - k0);
-            } else {
-                const bool hit0 = t < ne && xrow[t] == p, hit1 = t + 32 < ne && xrow[t + 32] == p;
-                const unsigned m0 = __ballot_sync(0xffffffffu, hit0), m1 = __ballot_sync(0xffffffffu, hit1);
-                if (m0) b = kb + __ffs(m0) - 1;
-                else if (m1) b = kb + 32 + __ffs(m1) - 1;
-                else {
-                    if (t == 0) xrow[ne] = p;
-                    b = kb + ne;
-                    ne++;
-                }
-            }
-            if (t == 0 && b != q) {
-                const int tmp = src[q];
-                src[q] = src[b];
-                src[b] = tmp;
-            }
-            __syncwarp();
+        dst[s] = r;
+        for (int p = kb - 1; p >= 0; p--) {
+            const int a = (int)k0 + p, b = piv[p];
+            r = r == a ? b : r == b ? a : r;
         }
-        if (t == 0) s_ne = ne;
-        __syncwarp();
-        for (int sl = t; sl < kb + ne; sl += 32) {
-            const int so = src[sl];
-            srow[sl] = so < kb ? k0 + so : xrow[so - kb];
-        }
+        src[s] = r;
     }
     __syncthreads();
-    const int ne = s_ne;
-    const int64_t c = c0 + (int64_t)blockIdx.x * blockDim.x + t;
-    if (c >= c1) return;
-    double x[kPanel];
-#pragma unroll
-    for (int q = 0; q < kPanel; q++)
-        if (q < kb) x[q] = A[srow[q] * ld + c];
-    for (int e = 0; e < ne; e++) E[e * kSwapThreads + t] = A[srow[kb + e] * ld + c];
-    if (TRSM) {
-#pragma unroll
-        for (int r = 0; r < kPanel; r++) {
-            double v = x[r];
-#pragma unroll
-            for (int q = 0; q < r; q++) v = fma(-L[r][q], x[q], v);
-            x[r] = v;
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < kPanel; q++)
-        if (q < kb) A[(k0 + q) * ld + c] = x[q];
-    for (int e = 0; e < ne; e++) A[xrow[e] * ld + c] = E[e * kSwapThreads + t];
 }
 
-// row swaps of rows k0 .. k0+kb-1 on columns [c0, c1)
-__global__ void laswp_kernel(double *A, int64_t ld, const int32_t *ipiv, int64_t k0, int kb, int64_t c0, int64_t c1) {
-    const int64_t c = c0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= c1) return;
-    for (int q = 0; q < kb; q++) {
-        const int64_t r = k0 + q, p = ipiv[r];
-        if (p != r) {
-            const double t = A[r * ld + c];
-            A[r * ld + c] = A[p * ld + c];
-            A[p * ld + c] = t;
-        }
+// the interchanges alone, on the columns [c0, c1): four lanes per column, each gathering its 32
+// slots with independent loads before any lane of the column writes
+constexpr int kSwapThreads = 128, kSwapCols = kSwapThreads / 4;
+__global__ void __launch_bounds__(kSwapThreads) swap_rows_kernel(double *A, int64_t ld, const int32_t *ipiv, int64_t k0,
+                                                                 int kb, int64_t c0, int64_t c1) {
+    __shared__ int piv[kPanel], dst[2 * kPanel], src[2 * kPanel];
+    swap_slots(ipiv, k0, kb, piv, dst, src);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 3;
+    const int64_t c = c0 + (int64_t)blockIdx.x * kSwapCols + warp * 8 + (lane & 7);
+    constexpr int R = 2 * kPanel / 4;
+    double x[R];
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const int s = 4 * i + g;
+        if (c < c1 && dst[s] >= 0 && dst[s] != src[s]) x[i] = A[src[s] * ld + c];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const int s = 4 * i + g;
+        if (c < c1 && dst[s] >= 0 && dst[s] != src[s]) A[dst[s] * ld + c] = x[i];
     }
 }
 
-// U12 = L11^-1 A12 (unit lower L11 = A[k0:k0+64, k0:k0+64]), thread per column;
-// the column lives in registers (the panel width is always kPanel here)
-__global__ void __launch_bounds__(128) trsm_f64_kernel(double *A, int64_t ld, int64_t k0, int64_t c0, int64_t c1) {
-    __shared__ double L[kPanel][kPanel + 1];
+// The interchanges and U12 = L11^-1 A12 (unit lower L11 = A[k0:k0+64, k0:k0+64]) on the columns
+// [c0, c1) right of a full panel, and the slices of U12's columns for the trailing update
+// (slices.cuh): SB [8][cap][64] BF16 with column c at row c - c0, exponents eb[c - c0].  Four lanes
+// per column, lane group g = lane / 8 holding rows 4 i + g: the substitution runs column by
+// column of L11 (every row's FMAs in the same order as row by row, but independent of one
+// another), and a warp's 504 FP64 instructions cover 8 columns, so that the few hundred
+// columns of a small system still spread over the SMs.
+constexpr int kTrsmCols = 8;                        // columns per warp
+constexpr int kTrsmStgLd = kPanel + 8;              // 16-bit words per staged slice row (no bank conflicts)
+constexpr int kTrsmStg = kSlices * kTrsmCols * kTrsmStgLd;
+constexpr size_t trsm_smem(int warps) { return sizeof(double) * kPanel * kPanel + sizeof(uint16_t) * kTrsmStg * warps; }
+__global__ void __launch_bounds__(128) swap_trsm_kernel(double *A, int64_t ld, const int32_t *ipiv, int64_t k0,
+                                                        int64_t c0, int64_t c1, uint16_t *SB, int64_t cap, int *eb) {
+    extern __shared__ __align__(16) double Lt[];  // [64][64]: Lt[q][r] = L11[r][q]; then the warps' staged slices
+    __shared__ int piv[kPanel], dst[2 * kPanel], src[2 * kPanel];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 3, cl = lane & 7;
     for (int e = threadIdx.x; e < kPanel * kPanel; e += blockDim.x) {
-        const int r = e / kPanel, q = e - r * kPanel;
-        L[r][q] = A[(k0 + r) * ld + k0 + q];
+        const int r = e / kPanel, q = e % kPanel;
+        Lt[q * kPanel + (r ^ (q & 15))] = A[(k0 + r) * ld + k0 + q];  // (swizzled rows: no bank conflicts either way)
     }
-    const int64_t c = c0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    __syncthreads();
-    if (c >= c1) return;
-    double x[kPanel];
+    swap_slots(ipiv, k0, kPanel, piv, dst, src);
+    const int64_t cw = c0 + ((int64_t)blockIdx.x * (blockDim.x >> 5) + warp) * kTrsmCols;
+    if (cw >= c1) return;
+    const bool live = cw + cl < c1;
+    const int64_t c = live ? cw + cl : c1 - 1;
+    constexpr int R = kPanel / 4;
+    double x[R], y[R];
 #pragma unroll
-    for (int r = 0; r < kPanel; r++) {
-        double v = A[(k0 + r) * ld + c];
+    for (int i = 0; i < R; i++) x[i] = A[src[4 * i + g] * ld + c];
 #pragma unroll
-        for (int q = 0; q < r; q++) v = fma(-L[r][q], x[q], v);
-        x[r] = v;
+    for (int i = 0; i < R; i++)
+        if (dst[kPanel + 4 * i + g] >= 0) y[i] = A[src[kPanel + 4 * i + g] * ld + c];
+    __syncwarp();  // every lane of a column has read before any writes
+#pragma unroll
+    for (int i = 0; i < R; i++)
+        if (live && dst[kPanel + 4 * i + g] >= 0) A[dst[kPanel + 4 * i + g] * ld + c] = y[i];
+#pragma unroll
+    for (int q = 0; q < kPanel - 1; q++) {
+        const double xq = __shfl_sync(0xffffffffu, x[q / 4], (q % 4) * 8 + cl);
+        const double *l = Lt + q * kPanel;
+#pragma unroll
+        for (int i = q / 4; i < R; i++) {
+            const double v = fma(-l[(4 * i + g) ^ (q & 15)], xq, x[i]);
+            x[i] = (i > q / 4 || g > q % 4) ? v : x[i];
+        }
     }
+    int exmax = 1;
 #pragma unroll
-    for (int r = 0; r < kPanel; r++) A[(k0 + r) * ld + c] = x[r];
+    for (int i = 0; i < R; i++) {
+        if (live) A[(k0 + 4 * i + g) * ld + c] = x[i];
+        exmax = max(exmax, slice_exponent(x[i]));
+    }
+    exmax = max(exmax, __shfl_xor_sync(0xffffffffu, exmax, 8));
+    exmax = max(exmax, __shfl_xor_sync(0xffffffffu, exmax, 16));
+    if (live && g == 0) eb[c - c0] = slice_scale(exmax);
+    uint16_t *stg = (uint16_t *)(Lt + kPanel * kPanel) + warp * kTrsmStg;
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const uint64_t w = slice_digits(x[i], exmax);
+#pragma unroll
+        for (int k = 0; k < kSlices; k++)
+            stg[(k * kTrsmCols + cl) * kTrsmStgLd + 4 * i + g] = (uint16_t)(slice_bf16_hi(w, k) >> 16);
+    }
+    __syncwarp();
+    // 64 staged rows (slice, column) of 128 bytes: eight lanes per row
+#pragma unroll
+    for (int it = 0; it < kSlices * kTrsmCols / 4; it++) {
+        const int row = it * 4 + g, k = row / kTrsmCols, col = row % kTrsmCols;
+        if (cw + col < c1)
+            *reinterpret_cast<uint4 *>(SB + ((int64_t)k * cap + (cw + col - c0)) * kSliceK + cl * 8) =
+                *reinterpret_cast<const uint4 *>(stg + row * kTrsmStgLd + cl * 8);
+    }
 }
 
-// C (m x nc) -= L (m x kb) * U (kb x nc); FP64, 64x64 tiles, 4x4 per thread,
-// K in chunks of 16
-constexpr int DG_BK = 16;
-__global__ void __launch_bounds__(256) dgemm_update_kernel(double *C, const double *Lp, const double *Up, int64_t ld,
-                                                           int64_t m, int64_t nc, int kb) {
-    __shared__ double As[DG_BK][64];  // As[k][row]
-    __shared__ double Bs[DG_BK][64];  // Bs[k][col]
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int64_t row0 = (int64_t)blockIdx.y * 64, col0 = (int64_t)blockIdx.x * 64;
-    double acc[4][4] = {};
-    for (int k0 = 0; k0 < kb; k0 += DG_BK) {
-        for (int e = threadIdx.x; e < 64 * DG_BK; e += 256) {
-            const int r = e / DG_BK, k = e - r * DG_BK;
-            As[k][r] = (row0 + r < m && k0 + k < kb) ? Lp[(row0 + r) * ld + k0 + k] : 0.0;
-            const int k2 = e >> 6, cc = e & 63;
-            Bs[k2][cc] = (col0 + cc < nc && k0 + k2 < kb) ? Up[(int64_t)(k0 + k2) * ld + col0 + cc] : 0.0;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < DG_BK; k++) {
-            double av[4], bv[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) av[i] = As[k][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) bv[j] = Bs[k][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int64_t r = row0 + ty * 4 + i;
-        if (r >= m) continue;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int64_t cc = col0 + tx * 4 + j;
-            if (cc < nc) C[r * ld + cc] -= acc[i][j];
-        }
-    }
-}
+// the trailing update on the tensor cores (slice_gemm.cu)
+int slice_rows(const double *A, int64_t lda, int64_t rows, int64_t cap, void *S, int *e, cudaStream_t st);
+int slice_update(double *C, int64_t ldc, int64_t m, int64_t nc, const void *SA, int64_t capA, int64_t a0, const int *ea,
+                 const void *SB, int64_t capB, int64_t b0, const int *eb, int *err, int max_ctas, cudaStream_t st);
 
 // ---- FP64 triangular solves (getrs) ------------------------------------------------
 // Row interchanges in LAPACK order (swap rows r and ipiv[r] for r = 0, 1, ...).
@@ -1381,6 +1349,23 @@ static int panel_geometry(int64_t m, int &nblk, int &rpc) {
     return rpc <= 384 ? FLG_OK : FLG_ERR_INVALID;
 }
 
+// operand slices of the trailing update: L21's rows (two buffers: the next panel's slices are
+// written while this panel's update still reads its own) and U12's columns, with their exponents
+struct SliceBufs {
+    uint16_t *A[2] = {}, *B = nullptr;
+    int *ea[2] = {}, *eb = nullptr;
+    template <class Ar>
+    void carve(Ar &ar, int64_t n) {
+        const size_t rows = n > kPanel ? (size_t)n : 0;
+        for (int k = 0; k < 2; k++) {
+            A[k] = ar.template take<uint16_t>(kSlices * rows * kSliceK);
+            ea[k] = ar.template take<int>(rows);
+        }
+        B = ar.template take<uint16_t>(kSlices * rows * kSliceK);
+        eb = ar.template take<int>(rows);
+    }
+};
+
 extern "C" size_t flg_lu_factor_f64_workspace(int64_t n) {
     CountingArena c;
     const int nblk = sm_count();
@@ -1388,7 +1373,8 @@ extern "C" size_t flg_lu_factor_f64_workspace(int64_t n) {
     c.take<unsigned long long>(2 * nblk);
     c.take<double>((size_t)2 * nblk * kRowBufLd);
     c.take<double>(2 * kPanel);
-    (void)n;
+    SliceBufs sb;
+    sb.carve(c, n);
     return c.bytes();
 }
 
@@ -1437,21 +1423,22 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
     unsigned long long *word = ar.take<unsigned long long>(2 * maxblk);
     double *rowbuf = ar.take<double>((size_t)2 * maxblk * kRowBufLd);
     double *diagbuf = ar.take<double>(2 * kPanel);
-    FLG_REQUIRE(diagbuf != nullptr, "workspace too small for LU (%zu bytes)", work_bytes);
+    SliceBufs sb;
+    sb.carve(ar, n);
+    FLG_REQUIRE(diagbuf != nullptr && (n <= kPanel || sb.eb != nullptr), "workspace too small for LU (%zu bytes)",
+                work_bytes);
     F64Streams *fs = nullptr;
     FLG_TRY(f64_streams(&fs));
     static bool attr_set = false;
     if (!attr_set) {
         FLG_CUDA(cudaFuncSetAttribute(panel_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       384 * kPanel * (int)sizeof(double)));
-        for (const void *k : {(const void *)swap_trsm_kernel<true>, (const void *)swap_trsm_kernel<false>})
-            FLG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          kPanel * kSwapThreads * (int)sizeof(double)));
+        FLG_CUDA(cudaFuncSetAttribute(swap_trsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)trsm_smem(4)));
         attr_set = true;
     }
-    const size_t swap_smem = (size_t)kPanel * kSwapThreads * sizeof(double);
     FLG_CUDA(cudaMemsetAsync(bar, 0, sizeof(GridBar), st));
-    // the panel of columns [k0, k0 + kb), rows k0.. on stream s
+    // the panel of columns [k0, k0 + kb), rows k0.. on stream s, and the slices of its L21
     auto panel = [&](int64_t k0, cudaStream_t s) -> int {
         const int kb = (int)std::min<int64_t>(kPanel, n - k0);
         const int64_t m = n - k0;
@@ -1469,7 +1456,8 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
         FLG_CUDA(cudaLaunchCooperativeKernel((void *)panel_f64_kernel, dim3(nblk), dim3(256), args, smem, s));
         count_launch();
         prof_end(FLG_SLOT_LU_PANEL, s);
-        return FLG_OK;
+        const int b = (int)(k0 / kPanel) & 1;
+        return slice_rows(A + (k0 + kb) * ld + k0, ld, n - k0 - kb, n, sb.A[b], sb.ea[b], s);
     };
     // Look-ahead: after each panel's trailing update has reached the next panel's 64 columns,
     // the next panel factors on the panel stream while the main stream updates the rest.
@@ -1484,31 +1472,32 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
         if (k0 > 0) {
             FLG_CUDA(cudaEventRecord(fs->factored, st));
             FLG_CUDA(cudaStreamWaitEvent(fs->left, fs->factored, 0));
-            swap_trsm_kernel<false><<<(unsigned)ceil_div(k0, kSwapThreads), kSwapThreads, swap_smem, fs->left>>>(
-                A, ld, ipiv, k0, kb, 0, k0);
+            swap_rows_kernel<<<(unsigned)ceil_div(k0, kSwapCols), kSwapThreads, 0, fs->left>>>(A, ld, ipiv, k0, kb,
+                                                                                                   0, k0);
             FLG_LAUNCH_CHECK();
         }
         const int64_t c0 = k0 + kb;
         ahead = false;
         if (c0 >= n) break;
         const int64_t nc = n - c0;
-        swap_trsm_kernel<true><<<(unsigned)ceil_div(nc, kSwapThreads), kSwapThreads, swap_smem, st>>>(A, ld, ipiv, k0,
-                                                                                                     kb, c0, n);
+        // as few warps per CTA as spread the columns over the SMs
+        const int tw = (int)std::min<int64_t>(4, ceil_div(nc, (int64_t)kTrsmCols * maxblk));
+        swap_trsm_kernel<<<(unsigned)ceil_div(nc, tw * kTrsmCols), tw * 32, trsm_smem(tw), st>>>(A, ld, ipiv, k0, c0, n,
+                                                                                              sb.B, n, sb.eb);
         FLG_LAUNCH_CHECK();
         prof_begin(FLG_SLOT_LU_UPDATE, st);
+        const int b = (int)(k0 / kPanel) & 1;
         const int64_t nn = std::min<int64_t>(kPanel, nc);  // the next panel's columns first
-        dgemm_update_kernel<<<dim3((unsigned)ceil_div(nn, 64), (unsigned)ceil_div(nc, 64)), 256, 0, st>>>(
-            A + c0 * ld + c0, A + c0 * ld + k0, A + k0 * ld + c0, ld, nc, nn, kb);
-        FLG_LAUNCH_CHECK();
+        FLG_TRY(slice_update(A + c0 * ld + c0, ld, nc, nn, sb.A[b], n, 0, sb.ea[b], sb.B, n, 0, sb.eb, &bar->err, maxblk,
+                             st));
         if (nc > nn) {
             FLG_CUDA(cudaEventRecord(fs->next_ready, st));
             FLG_CUDA(cudaStreamWaitEvent(fs->panel, fs->next_ready, 0));
             FLG_TRY(panel(c0, fs->panel));
             FLG_CUDA(cudaEventRecord(fs->panel_done, fs->panel));
             ahead = true;
-            dgemm_update_kernel<<<dim3((unsigned)ceil_div(nc - nn, 64), (unsigned)ceil_div(nc, 64)), 256, 0, st>>>(
-                A + c0 * ld + c0 + nn, A + c0 * ld + k0, A + k0 * ld + c0 + nn, ld, nc, nc - nn, kb);
-            FLG_LAUNCH_CHECK();
+            FLG_TRY(slice_update(A + c0 * ld + c0 + nn, ld, nc, nc - nn, sb.A[b], n, 0, sb.ea[b], sb.B, n, nn, sb.eb,
+                                 &bar->err, maxblk, st));
         }
         prof_end(FLG_SLOT_LU_UPDATE, st);
         if (!ahead) FLG_TRY(panel(c0, st));  // the last panel: nothing to overlap it with
@@ -1519,7 +1508,7 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
     FLG_CUDA(cudaMemcpyAsync(&hb, bar, sizeof(GridBar), cudaMemcpyDeviceToHost, st));
     FLG_CUDA(cudaStreamSynchronize(st));
     if (hb.err) {
-        set_error("a bounded device wait timed out (LU panel exchange)");
+        set_error("a bounded device wait timed out (LU panel exchange or tensor-core update)");
         return FLG_ERR_TIMEOUT;
     }
     *info = hb.info;

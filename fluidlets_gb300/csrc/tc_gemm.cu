@@ -31,11 +31,12 @@
 #include <mutex>
 
 #include "flg_common.cuh"
+#include "tc_common.cuh"
 #include "waits.cuh"
 
 namespace flg {
 
-constexpr int TC_BM = 128, TC_THREADS = 192, TC_EPI_WARPS = 4;
+constexpr int TC_THREADS = 192, TC_EPI_WARPS = 4;
 constexpr int TC_A_BYTES = TC_BM * 128;   // A tile of a K-block: 128 rows x 128 B
 constexpr int TC_STG_BYTES = 32 * 128;    // one 32 x 32 FP32 staging box
 
@@ -49,53 +50,6 @@ struct TcTile {
     static constexpr size_t SMEM = 1024 + STAGES * (TC_A_BYTES + B_BYTES) + TC_EPI_WARPS * 2 * TC_STG_BYTES;
     static_assert(SMEM <= 232448 - 256, "shared memory per CTA");
 };
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// 3-D tiles: x (innermost, 16-byte aligned), row y, system z
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y, int z) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], "
-        "[%2];" ::"r"(smem_u32(dst)),
-        "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
-        : "memory");
-}
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, const void *src, int x, int y, int z) {
-    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
-                     (uint64_t)map),
-                 "r"(smem_u32(src)), "r"(x), "r"(y), "r"(z)
-                 : "memory");
-}
-__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap *map, const void *src, int x, int y, int z) {
-    asm volatile(
-        "cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
-            (uint64_t)map),
-        "r"(smem_u32(src)), "r"(x), "r"(y), "r"(z)
-        : "memory");
-}
-
-// shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 B apart
-__device__ __forceinline__ uint64_t sw128_desc(const void *p) {
-    const uint64_t addr = smem_u32(p);
-    uint64_t d = 0;
-    d |= (addr >> 4) & 0x3FFFull;            // start address
-    d |= (uint64_t)1 << 16;                  // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;        // stride byte offset: next 8-row group
-    d |= (uint64_t)1 << 46;                  // descriptor version (tcgen05)
-    d |= (uint64_t)2 << 61;                  // swizzle mode: 128B
-    return d;
-}
-
-// instruction descriptor: D = F32, A/B format (TF32 = 2, BF16 = 1), K-major A and B, M = 128, N = bn
-__host__ __device__ constexpr uint32_t tc_idesc(uint32_t fmt, int bn) {
-    return (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
-}
 
 template <int MODE, int TC_BN>
 __global__ void __launch_bounds__(TC_THREADS, 1) tc_update_kernel(const __grid_constant__ CUtensorMap tmA,
@@ -305,9 +259,9 @@ static int64_t system_stride_bytes(int nb, int64_t stride_elems, int64_t rows, i
 }
 
 // operand map: nb systems (stride sb elements) of rows x K K-major elements (row stride
-// ld_elems), box box_rows x 128 bytes x 1 system, 128B swizzle
-static int make_operand_map(CUtensorMap *map, const void *base, int64_t rows, int64_t K, int64_t ld_elems, int mode,
-                            int box_rows, int nb = 1, int64_t sb = 0) {
+// ld_elems), box box_rows x 128 bytes x box_nb systems, 128B swizzle
+int make_operand_map(CUtensorMap *map, const void *base, int64_t rows, int64_t K, int64_t ld_elems, int mode,
+                     int box_rows, int nb, int64_t sb, int box_nb) {
     auto fn = encode_fn();
     FLG_REQUIRE(fn != nullptr, "cuTensorMapEncodeTiled unavailable");
     const bool bf = mode == FLG_LU_BF16;
@@ -317,7 +271,7 @@ static int make_operand_map(CUtensorMap *map, const void *base, int64_t rows, in
                 "TMA operand not 16-byte aligned");
     cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)nb};
     cuuint64_t strides[2] = {(cuuint64_t)(ld_elems * esz), (cuuint64_t)sbb};
-    cuuint32_t box[3] = {(cuuint32_t)(128 / esz), (cuuint32_t)box_rows, 1};
+    cuuint32_t box[3] = {(cuuint32_t)(128 / esz), (cuuint32_t)box_rows, (cuuint32_t)box_nb};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = fn(map, bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                     const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
