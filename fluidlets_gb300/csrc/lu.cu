@@ -31,6 +31,7 @@
 #include <algorithm>
 
 #include "flg_common.cuh"
+#include "panel.cuh"
 #include "slices.cuh"
 #include "waits.cuh"
 
@@ -354,76 +355,112 @@ __global__ void __launch_bounds__(kSwapThreads) swap_rows_kernel(double *A, int6
 
 // The interchanges and U12 = L11^-1 A12 (unit lower L11 = A[k0:k0+64, k0:k0+64]) on the columns
 // [c0, c1) right of a full panel, and the slices of U12's columns for the trailing update
-// (slices.cuh): SB [8][cap][64] BF16 with column c at row c - c0, exponents eb[c - c0].  Four lanes
-// per column, lane group g = lane / 8 holding rows 4 i + g: the substitution runs column by
-// column of L11 (every row's FMAs in the same order as row by row, but independent of one
-// another), and a warp's 504 FP64 instructions cover 8 columns, so that the few hundred
-// columns of a small system still spread over the SMs.
-constexpr int kTrsmCols = 8;                        // columns per warp
+// (slices.cuh): SB [8][cap][64] BF16 with column c at row c - c0, exponents eb[c - c0].  G lanes per
+// column, lane group g holding rows G i + g: the substitution runs column by column of L11
+// (every row's FMAs in the same order as row by row, but independent of one another).  An FP64
+// warp instruction takes 64 clocks of its scheduler, so a warp's 544 (G = 4) or 160 (G = 16) of them
+// are the kernel's time: 16 lanes per column spread the few hundred columns of a small system over all
+// schedulers, 4 waste fewer FMAs on rows already solved where there are columns for every
+// scheduler anyway.  `warps` of a CTA's eight have columns; all load L11 and work out the
+// interchanges.
+constexpr int kTrsmThreads = 256, kTrsmWarps = kTrsmThreads / 32;
 constexpr int kTrsmStgLd = kPanel + 8;              // 16-bit words per staged slice row (no bank conflicts)
-constexpr int kTrsmStg = kSlices * kTrsmCols * kTrsmStgLd;
-constexpr size_t trsm_smem(int warps) { return sizeof(double) * kPanel * kPanel + sizeof(uint16_t) * kTrsmStg * warps; }
-__global__ void __launch_bounds__(128) swap_trsm_kernel(double *A, int64_t ld, const int32_t *ipiv, int64_t k0,
-                                                        int64_t c0, int64_t c1, uint16_t *SB, int64_t cap, int *eb) {
+constexpr size_t trsm_smem(int G, int warps) {
+    return sizeof(double) * kPanel * kPanel + sizeof(uint16_t) * kSlices * (32 / G) * kTrsmStgLd * warps;
+}
+template <int G>
+__global__ void __launch_bounds__(kTrsmThreads) swap_trsm_kernel(double *A, int64_t ld, const int32_t *ipiv, int64_t k0,
+                                                                 int64_t c0, int64_t c1, int warps, uint16_t *SB,
+                                                                 int64_t cap, int *eb) {
     extern __shared__ __align__(16) double Lt[];  // [64][64]: Lt[q][r] = L11[r][q]; then the warps' staged slices
     __shared__ int piv[kPanel], dst[2 * kPanel], src[2 * kPanel];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 3, cl = lane & 7;
-    for (int e = threadIdx.x; e < kPanel * kPanel; e += blockDim.x) {
-        const int r = e / kPanel, q = e % kPanel;
-        Lt[q * kPanel + (r ^ (q & 15))] = A[(k0 + r) * ld + k0 + q];  // (swizzled rows: no bank conflicts either way)
+    constexpr int COLS = 32 / G, R = kPanel / G;  // columns per warp, rows per lane
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane / COLS, cl = lane % COLS;
+    {  // (swizzled rows: no bank conflicts either way)
+        double v[kPanel * kPanel / kTrsmThreads];
+#pragma unroll
+        for (int k = 0; k < kPanel * kPanel / kTrsmThreads; k++) {
+            const int e = threadIdx.x + k * kTrsmThreads;
+            v[k] = A[(k0 + e / kPanel) * ld + k0 + e % kPanel];
+        }
+#pragma unroll
+        for (int k = 0; k < kPanel * kPanel / kTrsmThreads; k++) {
+            const int e = threadIdx.x + k * kTrsmThreads, r = e / kPanel, q = e % kPanel;
+            Lt[q * kPanel + (r ^ (q & 15))] = v[k];
+        }
     }
     swap_slots(ipiv, k0, kPanel, piv, dst, src);
-    const int64_t cw = c0 + ((int64_t)blockIdx.x * (blockDim.x >> 5) + warp) * kTrsmCols;
-    if (cw >= c1) return;
+    const int64_t cw = c0 + ((int64_t)blockIdx.x * warps + warp) * COLS;
+    if (warp >= warps || cw >= c1) return;
     const bool live = cw + cl < c1;
     const int64_t c = live ? cw + cl : c1 - 1;
-    constexpr int R = kPanel / 4;
     double x[R], y[R];
 #pragma unroll
-    for (int i = 0; i < R; i++) x[i] = A[src[4 * i + g] * ld + c];
+    for (int i = 0; i < R; i++) x[i] = A[src[G * i + g] * ld + c];
 #pragma unroll
     for (int i = 0; i < R; i++)
-        if (dst[kPanel + 4 * i + g] >= 0) y[i] = A[src[kPanel + 4 * i + g] * ld + c];
+        if (dst[kPanel + G * i + g] >= 0) y[i] = A[src[kPanel + G * i + g] * ld + c];
     __syncwarp();  // every lane of a column has read before any writes
 #pragma unroll
     for (int i = 0; i < R; i++)
-        if (live && dst[kPanel + 4 * i + g] >= 0) A[dst[kPanel + 4 * i + g] * ld + c] = y[i];
+        if (live && dst[kPanel + G * i + g] >= 0) A[dst[kPanel + G * i + g] * ld + c] = y[i];
 #pragma unroll
     for (int q = 0; q < kPanel - 1; q++) {
-        const double xq = __shfl_sync(0xffffffffu, x[q / 4], (q % 4) * 8 + cl);
+        const double xq = __shfl_sync(0xffffffffu, x[q / G], (q % G) * COLS + cl);
         const double *l = Lt + q * kPanel;
 #pragma unroll
-        for (int i = q / 4; i < R; i++) {
-            const double v = fma(-l[(4 * i + g) ^ (q & 15)], xq, x[i]);
-            x[i] = (i > q / 4 || g > q % 4) ? v : x[i];
+        for (int i = q / G; i < R; i++) {
+            const double v = fma(-l[(G * i + g) ^ (q & 15)], xq, x[i]);
+            x[i] = (i > q / G || g > q % G) ? v : x[i];
         }
     }
     int exmax = 1;
 #pragma unroll
     for (int i = 0; i < R; i++) {
-        if (live) A[(k0 + 4 * i + g) * ld + c] = x[i];
+        if (live) A[(k0 + G * i + g) * ld + c] = x[i];
         exmax = max(exmax, slice_exponent(x[i]));
     }
-    exmax = max(exmax, __shfl_xor_sync(0xffffffffu, exmax, 8));
-    exmax = max(exmax, __shfl_xor_sync(0xffffffffu, exmax, 16));
+#pragma unroll
+    for (int o = COLS; o < 32; o <<= 1) exmax = max(exmax, __shfl_xor_sync(0xffffffffu, exmax, o));
     if (live && g == 0) eb[c - c0] = slice_scale(exmax);
-    uint16_t *stg = (uint16_t *)(Lt + kPanel * kPanel) + warp * kTrsmStg;
+    uint16_t *stg = (uint16_t *)(Lt + kPanel * kPanel) + warp * (kSlices * COLS * kTrsmStgLd);
 #pragma unroll
     for (int i = 0; i < R; i++) {
         const uint64_t w = slice_digits(x[i], exmax);
 #pragma unroll
         for (int k = 0; k < kSlices; k++)
-            stg[(k * kTrsmCols + cl) * kTrsmStgLd + 4 * i + g] = (uint16_t)(slice_bf16_hi(w, k) >> 16);
+            stg[(k * COLS + cl) * kTrsmStgLd + G * i + g] = (uint16_t)(slice_bf16_hi(w, k) >> 16);
     }
     __syncwarp();
-    // 64 staged rows (slice, column) of 128 bytes: eight lanes per row
+    // the staged rows (slice, column) of 128 bytes: eight lanes per row
 #pragma unroll
-    for (int it = 0; it < kSlices * kTrsmCols / 4; it++) {
-        const int row = it * 4 + g, k = row / kTrsmCols, col = row % kTrsmCols;
+    for (int it = 0; it < kSlices * COLS / 4; it++) {
+        const int row = it * 4 + (lane >> 3), k = row / COLS, col = row % COLS, ch = (lane & 7) * 8;
         if (cw + col < c1)
-            *reinterpret_cast<uint4 *>(SB + ((int64_t)k * cap + (cw + col - c0)) * kSliceK + cl * 8) =
-                *reinterpret_cast<const uint4 *>(stg + row * kTrsmStgLd + cl * 8);
+            *reinterpret_cast<uint4 *>(SB + ((int64_t)k * cap + (cw + col - c0)) * kSliceK + ch) =
+                *reinterpret_cast<const uint4 *>(stg + row * kTrsmStgLd + ch);
     }
+}
+static int swap_trsm(double *A, int64_t ld, const int32_t *ipiv, int64_t k0, int64_t c0, int64_t c1, uint16_t *SB,
+                     int64_t cap, int *eb, cudaStream_t st) {
+    const int64_t nc = c1 - c0;
+    static bool attr_set = false;
+    if (!attr_set) {
+        FLG_CUDA(cudaFuncSetAttribute(swap_trsm_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)trsm_smem(4, kTrsmWarps)));
+        FLG_CUDA(cudaFuncSetAttribute(swap_trsm_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)trsm_smem(16, kTrsmWarps)));
+        attr_set = true;
+    }
+    // G = 4 once its warps (8 columns each) fill half of the schedulers; below, G = 16's shorter chain
+    const bool wide = nc >= (int64_t)sm_count() * 2 * 8;
+    const int cols = wide ? 8 : 2;
+    const int w = (int)std::min<int64_t>(kTrsmWarps, ceil_div(nc, (int64_t)cols * sm_count()));
+    const unsigned grid = (unsigned)ceil_div(nc, (int64_t)w * cols);
+    if (wide) swap_trsm_kernel<4><<<grid, kTrsmThreads, trsm_smem(4, w), st>>>(A, ld, ipiv, k0, c0, c1, w, SB, cap, eb);
+    else swap_trsm_kernel<16><<<grid, kTrsmThreads, trsm_smem(16, w), st>>>(A, ld, ipiv, k0, c0, c1, w, SB, cap, eb);
+    FLG_LAUNCH_CHECK();
+    return FLG_OK;
 }
 
 // the trailing update on the tensor cores (slice_gemm.cu)
@@ -1384,7 +1421,7 @@ extern "C" size_t flg_lu_factor_f64_workspace(int64_t n) {
 struct F64Streams {
     int dev = -1;
     cudaStream_t panel = nullptr, left = nullptr;
-    cudaEvent_t next_ready = nullptr, panel_done = nullptr, factored = nullptr, left_done = nullptr;
+    cudaEvent_t next_ready = nullptr, panel_done = nullptr, panel_on = nullptr, factored = nullptr, left_done = nullptr;
 };
 constexpr int kF64StreamDevices = 64;
 static int f64_streams(F64Streams **out) {
@@ -1398,7 +1435,7 @@ static int f64_streams(F64Streams **out) {
         FLG_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
         FLG_CUDA(cudaStreamCreateWithPriority(&fs.panel, cudaStreamNonBlocking, hi));
         FLG_CUDA(cudaStreamCreateWithPriority(&fs.left, cudaStreamNonBlocking, lo));
-        for (cudaEvent_t *e : {&fs.next_ready, &fs.panel_done, &fs.factored, &fs.left_done})
+        for (cudaEvent_t *e : {&fs.next_ready, &fs.panel_done, &fs.panel_on, &fs.factored, &fs.left_done})
             FLG_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
         fs.dev = dev;
     }
@@ -1433,15 +1470,31 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
     if (!attr_set) {
         FLG_CUDA(cudaFuncSetAttribute(panel_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       384 * kPanel * (int)sizeof(double)));
-        FLG_CUDA(cudaFuncSetAttribute(swap_trsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)trsm_smem(4)));
         attr_set = true;
     }
     FLG_CUDA(cudaMemsetAsync(bar, 0, sizeof(GridBar), st));
-    // the panel of columns [k0, k0 + kb), rows k0.. on stream s, and the slices of its L21
-    auto panel = [&](int64_t k0, cudaStream_t s) -> int {
+    // the panel of columns [k0, k0 + kb), rows k0.. on stream s, and the slices of its L21;
+    // started (optional) completes once the panel's first kernel is resident
+    auto panel = [&](int64_t k0, cudaStream_t s, cudaEvent_t started) -> int {
         const int kb = (int)std::min<int64_t>(kPanel, n - k0);
         const int64_t m = n - k0;
+        const int b = (int)(k0 / kPanel) & 1;
+        if (m <= kClusterPanelRows) {
+            // two halves on a cluster, the second updated by the first in between
+            const int h0 = std::min(kHalf, kb), h1 = kb - h0;
+            prof_begin(FLG_SLOT_LU_PANEL, s);
+            FLG_TRY(cluster_panel({A, ld, n, k0, h0, ipiv, &bar->info, &bar->err, (int)k0 + h0,
+                                   (int)k0 + kb, 1, 0},
+                                  started, s));
+            if (h1 > 0) {
+                FLG_TRY(half_update(A, ld, k0 + kHalf, n, k0, h1, s));
+                FLG_TRY(cluster_panel({A, ld, n, k0 + kHalf, h1, ipiv, &bar->info, &bar->err, (int)k0,
+                                       (int)k0 + kHalf, 0, 0},
+                                      nullptr, s));
+            }
+            prof_end(FLG_SLOT_LU_PANEL, s);
+            return slice_rows(A + (k0 + kb) * ld + k0, ld, m - kb, n, sb.A[b], sb.ea[b], s);
+        }
         int nblk, rpc;
         panel_geometry(m, nblk, rpc);
         int per_sm = 0;
@@ -1456,15 +1509,14 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
         FLG_CUDA(cudaLaunchCooperativeKernel((void *)panel_f64_kernel, dim3(nblk), dim3(256), args, smem, s));
         count_launch();
         prof_end(FLG_SLOT_LU_PANEL, s);
-        const int b = (int)(k0 / kPanel) & 1;
-        return slice_rows(A + (k0 + kb) * ld + k0, ld, n - k0 - kb, n, sb.A[b], sb.ea[b], s);
+        return slice_rows(A + (k0 + kb) * ld + k0, ld, m - kb, n, sb.A[b], sb.ea[b], s);
     };
     // Look-ahead: after each panel's trailing update has reached the next panel's 64 columns,
     // the next panel factors on the panel stream while the main stream updates the rest.
     // The interchanges of the columns left of each panel go to the left stream, in order.
     FLG_CUDA(cudaEventRecord(fs->factored, st));
     FLG_CUDA(cudaStreamWaitEvent(fs->left, fs->factored, 0));  // the left stream starts after prior work
-    FLG_TRY(panel(0, st));
+    FLG_TRY(panel(0, st, nullptr));
     bool ahead = false;  // the current panel ran ahead on the panel stream
     for (int64_t k0 = 0; k0 < n; k0 += kPanel) {
         const int kb = (int)std::min<int64_t>(kPanel, n - k0);
@@ -1480,11 +1532,7 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
         ahead = false;
         if (c0 >= n) break;
         const int64_t nc = n - c0;
-        // as few warps per CTA as spread the columns over the SMs
-        const int tw = (int)std::min<int64_t>(4, ceil_div(nc, (int64_t)kTrsmCols * maxblk));
-        swap_trsm_kernel<<<(unsigned)ceil_div(nc, tw * kTrsmCols), tw * 32, trsm_smem(tw), st>>>(A, ld, ipiv, k0, c0, n,
-                                                                                              sb.B, n, sb.eb);
-        FLG_LAUNCH_CHECK();
+        FLG_TRY(swap_trsm(A, ld, ipiv, k0, c0, n, sb.B, n, sb.eb, st));
         prof_begin(FLG_SLOT_LU_UPDATE, st);
         const int b = (int)(k0 / kPanel) & 1;
         const int64_t nn = std::min<int64_t>(kPanel, nc);  // the next panel's columns first
@@ -1493,14 +1541,18 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
         if (nc > nn) {
             FLG_CUDA(cudaEventRecord(fs->next_ready, st));
             FLG_CUDA(cudaStreamWaitEvent(fs->panel, fs->next_ready, 0));
-            FLG_TRY(panel(c0, fs->panel));
+            // a cluster panel keeps its SMs out of the update's persistent grid, which waits until
+            // the cluster is resident (16 SMs of one GPC are never free at once under that grid)
+            const bool cluster = nc <= kClusterPanelRows;
+            FLG_TRY(panel(c0, fs->panel, cluster ? fs->panel_on : nullptr));
             FLG_CUDA(cudaEventRecord(fs->panel_done, fs->panel));
             ahead = true;
+            if (cluster) FLG_CUDA(cudaStreamWaitEvent(st, fs->panel_on, 0));
             FLG_TRY(slice_update(A + c0 * ld + c0 + nn, ld, nc, nc - nn, sb.A[b], n, 0, sb.ea[b], sb.B, n, nn, sb.eb,
-                                 &bar->err, maxblk, st));
+                                 &bar->err, cluster ? maxblk - kPanelCtas : maxblk, st));
         }
         prof_end(FLG_SLOT_LU_UPDATE, st);
-        if (!ahead) FLG_TRY(panel(c0, st));  // the last panel: nothing to overlap it with
+        if (!ahead) FLG_TRY(panel(c0, st, nullptr));  // the last panel: nothing to overlap it with
     }
     FLG_CUDA(cudaEventRecord(fs->left_done, fs->left));
     FLG_CUDA(cudaStreamWaitEvent(st, fs->left_done, 0));
