@@ -7,27 +7,28 @@
 // CTAs holds the whole panel, one thread per row, and a round is a few remote shared-memory
 // stores and one hardware cluster barrier.
 //
-// Thread lr of CTA c owns row k0 + c rpc + lr: the columns from the current one on live in its
-// registers, moved down by one with every column (the rank-1 update writes a[i - 1] from a[i]), the
-// finished multipliers in shared memory (Pm).  Column j:
-//   1. rows below pivot j - 1: multiplier, and column j's value; each warp's largest |x| (two
-//      32-bit reductions over the bits, which order like the value; NaN never wins), whose thread
-//      stages its remaining row;
-//   2. publisher warps, beside the row warps: four pick the CTA's candidate, complete its row
-//      (one FMA per lane) and send it to every CTA of the cluster, one sends the candidate's key
-//      and reciprocal, two do the same as the four for row k0 + j;
-//   3. the rest of the rank-1 update of column j - 1, beside the exchange;
-//   4. every warp picks the winner among the CTAs' candidates (ties: the smaller CTA, which owns
-//      the smaller rows); the winner's thread takes over row k0 + j, which the pivot row replaces.
+// CTA c owns rows k0 + c rpc ..., all kb columns of them in shared memory (Pm): finished multipliers
+// left of the current column, right of it the values as of the last full update.  Column j:
+//   1. warp w < W, rows 32 w ..: the interchange of column j - 1 on its rows, their multipliers, and
+//      column j's values; the warp's largest |x| (two 32-bit reductions over the bits, which order
+//      like the value; NaN never wins) and a copy of that row, and of row k0 + j;
+//   2. publisher warps: eight pick the CTA's candidate, complete its row (one FMA per lane) and
+//      send it to every CTA of the cluster, one sends the candidate's key, local row and
+//      reciprocal, two send row k0 + j like the eight;
+//   3. the row warps, beside the exchange: the rest of the rank-1 update of column j - 1;
+//   4. every row warp picks the winner among the CTAs' candidates (ties: the smaller CTA, which
+//      owns the smaller rows).
 // The exchange is st.async: the data's arrival completes the receiver's mbarrier, so a round has
-// no acknowledgement (measured with 16 CTAs: 490 clocks; plain remote stores and a cluster
-// barrier 1,215).  Received rows are buffered three deep: a CTA sends column j + 3's after it has
-// column j + 2's from every CTA, and those leave after every use of column j's.
+// no acknowledgement (measured with 16 CTAs: 490-700 clocks; plain remote stores and a cluster
+// barrier 1,215; bulk copies 1,700).  Received rows are buffered three deep: a CTA sends column
+// j + 3's after it has column j + 2's from every CTA, and those leave after every use of column j's.
 // FP64 is what a column costs otherwise: GB300 issues one FP64 warp instruction per 64 clocks and
 // scheduler whatever its active lanes (comparisons and reciprocals included), so tests run on
-// integer bits and the reciprocal is three FMAs on the 20-bit approximation.
+// integer bits, the reciprocal is three FMAs on the 20-bit approximation, and a panel of few rows
+// gives each row several warps (groups of columns) for the rank-1 update so that all four
+// schedulers have some.
 // Every element gets the same FMAs in the same column order as in the textbook loop, so factors
-// and pivots do not depend on the cluster size.
+// and pivots do not depend on the cluster size or the grouping.
 //
 // After the panel: its interchanges on a few companion columns (the other half of a 64-column
 // block), and with `trsm` also U12 = L11^-1 A12 on them, one warp per column.
@@ -39,22 +40,23 @@
 
 namespace flg {
 
-constexpr int kRowPubs = 4, kKeyPub = kRowPubs, kDiagPubs = 2;
-constexpr int kPubWarps = kRowPubs + 1 + kDiagPubs, kMaxRowWarps = 12;
+constexpr int kRowPubs = 8, kKeyPub = kRowPubs, kDiagPubs = 2;
+constexpr int kPubWarps = kRowPubs + 1 + kDiagPubs, kMaxRowWarps = 16;
 constexpr int kPmLd = kHalf + 1;
 constexpr int kRx = 3;  // buffers of received candidates
 
 struct PanelShared {
     double rx_row[kRx][kPanelCtas][kHalf];
-    double rx_diag[kRx][2 * kHalf];  // row k0 + j; the upper half stays unused padding for shifted reads
+    double rx_diag[kRx][kHalf];  // row k0 + j
     double rx_rcp[kRx][kPanelCtas];
     unsigned long long rx_key[kRx][kPanelCtas];
     unsigned long long rx_lrow[kRx][kPanelCtas];
     // candidates of this CTA, by column parity: a publisher may still read column j's while the row
-    // warps stage column j + 1's
-    double2 stage[2][kMaxRowWarps][kHalf / 2], dstage[2][kHalf / 2];
+    // warps copy column j + 1's
+    double stage[2][kMaxRowWarps][kHalf], dstage[2][kHalf];
     unsigned long long skey[2][kMaxRowWarps];
     int srow[2][kMaxRowWarps];
+    int swin[2];  // the last column's winner (-1: none), for the publishers
     int piv[kHalf], dst[2 * kHalf], src[2 * kHalf];
     double L11[kHalf][kPmLd];
     unsigned long long bar[kRx];
@@ -129,111 +131,133 @@ __device__ __forceinline__ int warp_argmax(unsigned long long key) {
     return (h | l) ? __ffs(who) - 1 : -1;
 }
 
-// MAXW: the most row warps of a launch; 9 (4,608 rows) leaves 128 registers per thread, 12 only 96
-template <int MAXW>
-__global__ void __launch_bounds__(32 * (MAXW + kPubWarps), 1) panel_cluster_kernel(ClusterPanelArgs a) {
+__global__ void __launch_bounds__(32 * (kMaxRowWarps + kPubWarps), 1) panel_cluster_kernel(ClusterPanelArgs a) {
     extern __shared__ __align__(16) uint8_t raw[];
     PanelShared &S = *reinterpret_cast<PanelShared *>(raw);
-    double *Pm = reinterpret_cast<double *>(raw + ((sizeof(PanelShared) + 15) & ~size_t(15)));  // [rpc][kPmLd]
+    double *Pm = reinterpret_cast<double *>(raw + ((sizeof(PanelShared) + 15) & ~size_t(15)));  // [32 W][kPmLd]
     const int c = blockIdx.x, ncta = gridDim.x, kb = a.kb, rpc = a.rpc;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, rw = (int)(blockDim.x >> 5) - kPubWarps;
-    const int pub = warp - rw;  // publisher warp, or negative: a row warp
+    const int pub = warp - rw;                 // publisher warp, or negative: a row warp
+    const int W = (rpc + 31) >> 5, CG = rw / W;  // row blocks of 32, column groups of the rank-1 update
+    const int rb = warp % W, cg = warp / W;    // row warps: row block, column group
     const int k0 = (int)a.k0, r0 = k0 + c * rpc;
     const int nr = max(0, min(rpc, (int)a.n - r0));
     if (t == 0) {
         for (int b = 0; b < kRx; b++) mbar_init((uint64_t *)&S.bar[b], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int lr = warp; lr < nr; lr += blockDim.x >> 5)
-        if (lane < kb) Pm[lr * kPmLd + lane] = a.A[(int64_t)(r0 + lr) * a.ld + k0 + lane];
-    __syncthreads();
-    const int row = r0 + t;  // row warps only
-    const bool have = pub < 0 && t < nr;
-    double x[kHalf];  // columns j, j + 1, ... of this thread's row
+    for (int l0 = warp; l0 < nr; l0 += 8 * (int)(blockDim.x >> 5)) {
+        double v[8];
 #pragma unroll
-    for (int i = 0; i < kHalf; i++) x[i] = have && i < kb ? Pm[t * kPmLd + i] : 0.0;
+        for (int k = 0; k < 8; k++) {
+            const int lr = l0 + k * (int)(blockDim.x >> 5);
+            v[k] = lr < nr && lane < kb ? a.A[(int64_t)(r0 + lr) * a.ld + k0 + lane] : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const int lr = l0 + k * (int)(blockDim.x >> 5);
+            if (lr < nr) Pm[lr * kPmLd + lane] = v[k];
+        }
+    }
+    __syncthreads();
+    const int lr = rb * 32 + lane, row = r0 + lr;  // row warps: this lane's row
+    double *mine = Pm + (size_t)lr * kPmLd;        // (inside the allocation for every lane of a row warp)
+    const bool have = pub < 0 && lr < nr;
     cluster_sync();  // every CTA's mbarriers are ready
 
     // what a CTA receives per column: a row, a key, a row index and a reciprocal from each CTA, and row k0 + j
     const uint32_t rx_bytes = (uint32_t)ncta * (8 * kHalf + 24) + 8 * kHalf;
+    int buf = 0, pbuf = 0, prow = -1;
+    uint32_t parity = 0;
     const double *pv = nullptr;  // the previous column's pivot row, by column
     double rcp = 0.0;
     bool ok = false;
-    int buf = 0;
-    uint32_t parity = 0;
     for (int j = 0; j < kb; j++) {
         const int g = k0 + j;
-        double l = 0.0, v = x[0];
-        if (pub < 0) {
+        double l = 0.0;
+        if (pub < 0 && cg == 0) {
+            if (j > 0) {  // column j - 1's interchange on this warp's rows (finished rows included)
+                const int gl = g - 1 - r0, pl = prow - r0;
+                if (prow != g - 1 && pl >= 0 && pl < nr && (pl >> 5) == rb) Pm[pl * kPmLd + lane] = S.rx_diag[pbuf][lane];
+                if (gl >= 0 && gl < nr && (gl >> 5) == rb) Pm[gl * kPmLd + lane] = pv[lane];
+                __syncwarp();
+            }
+            double v = mine[j];
             if (j > 0) {
-                l = ok ? x[0] * rcp : x[0];
-                v = ok ? fma(-l, pv[j], x[1]) : x[1];
-                if (have && row >= g) Pm[t * kPmLd + j - 1] = l;
+                l = mine[j - 1];
+                if (ok) {
+                    l *= rcp;
+                    v = fma(-l, pv[j], v);
+                }
+                if (have && row >= g) mine[j - 1] = l, mine[j] = v;
             }
             const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
             const unsigned long long key = have && row >= g && b <= 0x7ff0000000000000ull ? b + 1ull : 0ull;
             const int w = warp_argmax(key);
-            const bool diag = have && row == g;
-            if (lane == w || diag) {  // columns j, j + 1, ..., of which all but j lack column j - 1's update
-                double2 *st = lane == w ? S.stage[j & 1][warp] : S.dstage[j & 1];
-#pragma unroll
-                for (int i = 0; i < kHalf; i += 2)
-                    if (j + i < kb) {
-                        const double2 p = j > 0 ? make_double2(i ? x[i + 1 < kHalf ? i + 1 : kHalf - 1] : v,
-                                                               x[i + 2 < kHalf ? i + 2 : kHalf - 1])
-                                                : make_double2(x[i], x[i + 1]);
-                        st[i / 2] = p;
-                        if (diag) S.dstage[j & 1][i / 2] = p;
-                    }
-            }
+            __syncwarp();
+            // whole rows: multipliers, column j, and columns j + 1 ... without column j - 1's update
+            if (w >= 0) S.stage[j & 1][rb][lane] = Pm[(rb * 32 + w) * kPmLd + lane];
+            if ((g - r0) >> 5 == rb && g - r0 < nr) S.dstage[j & 1][lane] = Pm[(g - r0) * kPmLd + lane];
             if (lane == (w < 0 ? 0 : w)) {
-                S.skey[j & 1][warp] = key;
-                S.srow[j & 1][warp] = t;
+                S.skey[j & 1][rb] = key;
+                S.srow[j & 1][rb] = lr;
             }
         }
         __syncthreads();
         if (pub >= 0) {
             const void *bar = &S.bar[buf];
-            if (pub == kKeyPub && lane == 0) expect_tx(&S.bar[buf], rx_bytes);
+            if (j > 0) {
+                const int win = S.swin[(j - 1) & 1];
+                pv = win >= 0 ? S.rx_row[pbuf][win] : S.rx_diag[pbuf];
+                ok = finite_nonzero(pv[j - 1]);
+            }
             if (pub <= kKeyPub) {
-                const int w = warp_argmax(lane < rw ? S.skey[j & 1][lane] : 0ull);
-                const int lr = w >= 0 ? S.srow[j & 1][w] : 0;
-                const double *st = reinterpret_cast<const double *>(S.stage[j & 1][w < 0 ? 0 : w]);
+                if (pub == kKeyPub && lane == 0) expect_tx(bar, rx_bytes);
+                const unsigned long long key = lane < W ? S.skey[j & 1][lane] : 0ull;
+                const int w = warp_argmax(key);
+                const double *st = S.stage[j & 1][w < 0 ? 0 : w];
                 if (pub == kKeyPub) {
+                    const double p = w >= 0 ? st[j] : 0.0;
+                    const double rp = finite_nonzero(p) ? fast_rcp(p) : 0.0;
                     if (lane < ncta) {
                         send(&S.rx_key[buf][c], bar, lane, w >= 0 ? S.skey[j & 1][w] : 0ull);
-                        send(&S.rx_lrow[buf][c], bar, lane, (unsigned long long)lr);
+                        send(&S.rx_lrow[buf][c], bar, lane, (unsigned long long)(w >= 0 ? S.srow[j & 1][w] : 0));
+                        send(&S.rx_rcp[buf][c], bar, lane, rp);
                     }
-                    const double p = w >= 0 ? st[0] : 0.0;
-                    const double rp = finite_nonzero(p) ? fast_rcp(p) : 0.0;
-                    if (lane < ncta) send(&S.rx_rcp[buf][c], bar, lane, rp);
                 } else {
-                    double y = lane < j ? Pm[lr * kPmLd + lane] : st[lane - j];
-                    if (j > 0 && ok && lane > j) y = fma(-Pm[lr * kPmLd + j - 1], pv[lane], y);
+                    double y = st[lane];
+                    if (j > 0 && ok && lane > j) y = fma(-st[j - 1], pv[lane], y);
                     for (int d = pub; d < ncta; d += kRowPubs) send(&S.rx_row[buf][c][lane], bar, d, y);
                 }
             } else if (g >= r0 && g < r0 + nr) {
-                const int lr = g - r0;
-                double y = lane < j ? Pm[lr * kPmLd + lane] : reinterpret_cast<const double *>(S.dstage[j & 1])[lane - j];
-                if (j > 0 && ok && lane > j) y = fma(-Pm[lr * kPmLd + j - 1], pv[lane], y);
+                const double *st = S.dstage[j & 1];
+                double y = st[lane];
+                if (j > 0 && ok && lane > j) y = fma(-st[j - 1], pv[lane], y);
                 for (int d = pub - kKeyPub - 1; d < ncta; d += kDiagPubs) send(&S.rx_diag[buf][lane], bar, d, y);
             }
-            // no publisher still reads Pm when the pivot row and row g change places below
-            asm volatile("bar.sync 1, %0;" ::"n"(32 * kPubWarps) : "memory");
-        } else if (j > 0) {  // the rest of the previous column's rank-1 update, beside the exchange
-            x[0] = v;
-            if (ok) {
+            pbuf = buf;
+            if (++buf == kRx) buf = 0;
+            continue;
+        }
+        if (j > 0 && ok) {  // the rest of the previous column's rank-1 update, beside the exchange
+            if (cg > 0) l = mine[j - 1];
+            for (int q0 = j + 1 + cg; q0 < kb; q0 += 4 * CG) {
+                double y[4], u[4];
 #pragma unroll
-                for (int ib = 0; ib < kHalf; ib += 4)
-                    if (j + ib < kb)
+                for (int k = 0; k < 4; k++) {
+                    const int q = min(q0 + k * CG, kHalf - 1);
+                    y[k] = mine[q];
+                    u[k] = pv[q];
+                }
 #pragma unroll
-                        for (int i = ib; i < ib + 4; i++)
-                            if (i >= 1) x[i] = fma(-l, pv[min(j + i, kHalf - 1)], x[i + 1 < kHalf ? i + 1 : kHalf - 1]);
-            } else {
-#pragma unroll
-                for (int i = 1; i + 1 < kHalf; i++) x[i] = x[i + 1];
+                for (int k = 0; k < 4; k++)
+                    if (q0 + k * CG < kb) {
+                        const double z = fma(-l, u[k], y[k]);
+                        if (row >= g) mine[q0 + k * CG] = z;
+                    }
             }
         }
+        if (CG > 1) asm volatile("bar.sync 1, %0;" ::"r"(32 * rw) : "memory");  // the other groups' columns of this row
         cluster_wait((uint64_t *)&S.bar[buf], parity, a.err);
         __syncwarp();
         const int win = warp_argmax(lane < ncta ? S.rx_key[buf][lane] : 0ull);
@@ -241,28 +265,26 @@ __global__ void __launch_bounds__(32 * (MAXW + kPubWarps), 1) panel_cluster_kern
         pv = win >= 0 ? S.rx_row[buf][win] : S.rx_diag[buf];
         rcp = win >= 0 ? S.rx_rcp[buf][win] : 0.0;
         ok = finite_nonzero(pv[j]);
-        const int prow = win >= 0 ? k0 + win * rpc + (int)S.rx_lrow[buf][win] : g;
-        if (pub < 0) {
-            if (have && row == prow && prow != g) {  // the old row g moves here
-#pragma unroll
-                for (int i = 0; i < kHalf; i++) x[i] = S.rx_diag[buf][j + i];
-            }
-        } else if (pub == kKeyPub) {
-            const int pl = prow - r0, gl = g - r0;
-            if (pl >= 0 && pl < nr && prow != g && lane < j) Pm[pl * kPmLd + lane] = S.rx_diag[buf][lane];
-            if (gl >= 0 && gl < nr && lane < kb) Pm[gl * kPmLd + lane] = pv[lane];
-            if (lane == 0) {
-                S.piv[j] = prow;
-                if (c == 0) a.ipiv[g] = prow;
-                if (c == 0 && !ok) atomicCAS(a.info, 0, g + 1);
-            }
+        prow = win >= 0 ? k0 + win * rpc + (int)S.rx_lrow[buf][win] : g;
+        if (warp == 0 && lane == 0) {
+            S.swin[j & 1] = win;
+            S.piv[j] = prow;
+            if (c == 0) a.ipiv[g] = prow;
+            if (c == 0 && !ok) atomicCAS(a.info, 0, g + 1);
         }
+        pbuf = buf;
         if (++buf == kRx) buf = 0, parity ^= 1;
     }
-    if (have && row >= k0 + kb) Pm[t * kPmLd + kb - 1] = ok ? x[0] * rcp : x[0];
+    if (pub < 0 && cg == 0) {  // the last column's interchange and multipliers
+        const int gl = k0 + kb - 1 - r0, pl = prow - r0;
+        if (prow != k0 + kb - 1 && pl >= 0 && pl < nr && (pl >> 5) == rb) Pm[pl * kPmLd + lane] = S.rx_diag[pbuf][lane];
+        if (gl >= 0 && gl < nr && (gl >> 5) == rb) Pm[gl * kPmLd + lane] = pv[lane];
+        __syncwarp();
+        if (have && row >= k0 + kb && ok) mine[kb - 1] *= rcp;
+    }
     __syncthreads();
-    for (int lr = warp; lr < nr; lr += blockDim.x >> 5)
-        if (lane < kb) a.A[(int64_t)(r0 + lr) * a.ld + k0 + lane] = Pm[lr * kPmLd + lane];
+    for (int l0 = warp; l0 < nr; l0 += blockDim.x >> 5)
+        if (lane < kb) a.A[(int64_t)(r0 + l0) * a.ld + k0 + lane] = Pm[l0 * kPmLd + lane];
     // the panel's interchanges on the companion columns [cc0, cc1): slots as in lu.cu
     for (int s = t; s < 2 * kHalf; s += blockDim.x) {
         const int q = s & (kHalf - 1);
@@ -350,21 +372,20 @@ int cluster_panel(const ClusterPanelArgs &in, cudaEvent_t started, cudaStream_t 
     FLG_REQUIRE(a.kb >= 1 && a.kb <= kHalf && m <= kClusterPanelRows, "bad cluster panel");
     static bool attr_set = false;
     if (!attr_set) {
-        for (const void *k : {(const void *)panel_cluster_kernel<9>, (const void *)panel_cluster_kernel<kMaxRowWarps>}) {
-            FLG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            FLG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)panel_smem(32 * kMaxRowWarps)));
-        }
+        FLG_CUDA(cudaFuncSetAttribute(panel_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        FLG_CUDA(cudaFuncSetAttribute(panel_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)panel_smem(32 * kMaxRowWarps)));
         attr_set = true;
     }
     int ncta = 1;
     while (ncta < kPanelCtas && (int64_t)ncta * 32 < m) ncta *= 2;
     a.rpc = (int)ceil_div(m, ncta);
-    const int threads = (int)(ceil_div(a.rpc, 32) + kPubWarps) * 32;
+    const int W = (int)ceil_div(a.rpc, 32), CG = std::max(1, 8 / W);  // eight row warps where the rows fill fewer
+    const int threads = (W * CG + kPubWarps) * 32;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ncta);
     cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = panel_smem(a.rpc);
+    cfg.dynamicSmemBytes = panel_smem(32 * W);
     cfg.stream = st;
     cudaLaunchAttribute at[2] = {};
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -378,7 +399,7 @@ int cluster_panel(const ClusterPanelArgs &in, cudaEvent_t started, cudaStream_t 
         cfg.numAttrs = 2;
     }
     cfg.attrs = at;
-    FLG_CUDA(cudaLaunchKernelEx(&cfg, a.rpc <= 9 * 32 ? panel_cluster_kernel<9> : panel_cluster_kernel<kMaxRowWarps>, a));
+    FLG_CUDA(cudaLaunchKernelEx(&cfg, panel_cluster_kernel, a));
     count_launch();
     return FLG_OK;
 }

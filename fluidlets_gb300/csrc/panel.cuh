@@ -7,7 +7,7 @@ namespace flg {
 
 constexpr int kHalf = 32;        // panel width: half of a 64-column block
 constexpr int kPanelCtas = 16;   // CTAs of the cluster
-constexpr int64_t kClusterPanelRows = kPanelCtas * 32 * 12;  // one thread per row: 6,144 rows
+constexpr int64_t kClusterPanelRows = kPanelCtas * 32 * 16;  // 8,192 rows
 
 struct ClusterPanelArgs {
     double *A;
