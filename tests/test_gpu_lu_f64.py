@@ -101,3 +101,30 @@ def test_zero_rows_are_singular():
     A[130] = 0.0
     with pytest.raises(np.linalg.LinAlgError):
         factor(A)
+
+
+@pytest.mark.parametrize("n,nrhs", [(1, 1), (31, 1), (32, 2), (33, 1), (64, 3), (65, 1), (511, 1), (513, 2), (1030, 1),
+                                    (100, 33)])
+def test_triangular_solves_backward_error(n, nrhs):
+    """The library's solve with its own factors: componentwise backward error of two substitutions,
+    (2 n + 2) u |L| |U| |x|, taken as 3 n u for small n's constants."""
+    rng = np.random.default_rng(n + nrhs)
+    A = rng.normal(size=(n, n))
+    b = rng.normal(size=(n, nrhs))
+    L = _lib.load()
+    Ad = torch.tensor(A, device="cuda")
+    B = torch.full((n, nrhs + 2), 3.25, dtype=torch.float64, device="cuda")
+    B[:, :nrhs] = torch.tensor(b, device="cuda")
+    piv = torch.empty(n, dtype=torch.int32, device="cuda")
+    nb = L.flg_lu_factor_f64_workspace(n)
+    ws = dv.workspace(nb)
+    info = ctypes.c_int(0)
+    _lib.check(L.flg_lu_factor_f64(n, dv.ptr(Ad), n, dv.ptr(piv), ctypes.byref(info), dv.ptr(ws), nb, dv.stream()))
+    _lib.check(L.flg_lu_solve_f64(n, nrhs, dv.ptr(Ad), n, dv.ptr(piv), dv.ptr(B), nrhs + 2, dv.stream()))
+    assert torch.all(B[:, nrhs:] == 3.25)
+    F, p, x = Ad.cpu().numpy(), piv.cpu().numpy(), B[:, :nrhs].cpu().numpy()
+    for k in range(n):
+        b[[k, p[k]]] = b[[p[k], k]]
+    Lo, U = np.tril(F, -1) + np.eye(n), np.triu(F)
+    r = Lo.astype(np.longdouble) @ (U.astype(np.longdouble) @ x.astype(np.longdouble)) - b
+    assert np.all(np.abs(r) <= 3 * max(n, 4) * 2.0**-53 * (np.abs(Lo) @ (np.abs(U) @ np.abs(x)) + np.abs(b)))
