@@ -1,0 +1,311 @@
+// pair_fixed.cuh -- the FP64 pair kernels in 60-bit fixed point (fixed.cuh).
+//
+// The same formulas as pair_math.cuh's, written in bounded quantities.  With Q = |d|^2 + e^2 =
+// q 2^(2E), y = q^-1/2, the unit vector n = d / sqrt(Q) and w = e / sqrt(Q):
+//   Stokeslet     8 pi u = s [(1 + w^2) f + (f.n) n],                       s = y 2^-E
+//   Brinkmanlet   4 pi u = s [(f1 + w^2 f2) f + f2 (f.n) n]                 below z = 1/2 (series), and
+//                        = s^3 / alpha^2 [(F1 + w^2 F2) f + F2 (f.n) n],    F = z^2 f, above:
+//     F1 = E (1 + z + z^2) - 1, F2 = 3 - E (3 + 3 z + z^2), E = e^-z from 2^-n 2^(-i/64) e^-x with a table
+//     (P. T. P. Tang, "Table-driven implementation of the exponential function in IEEE
+//     floating-point arithmetic", ACM TOMS 15, 1989)
+//   wall          8 pi u = 2 t h sF s^2 [...] with rho = s / sF <= 1, nI = dp s and the bracket
+//     c f_j + n_j (Z3 (f.n) - 3 rho^2 B)           (j = x, y),  c = Z1 + w^2 Z3 - rho + 3 w^2 rho^3
+//     c' f_z + n_z Z3 (f.n) - 3 rho nI B,                       c' = Z1 + w^2 Z3 - rho - 3 w^2 rho^3
+//     Z1 = 2 / (1 + rho), Z3 = Z1 (1 + rho + rho^2) = 2 + ... , B = nI f_z - rho (n_x f_x + n_y f_y)
+//   (the bracket is the image form of pair_math.cuh divided by sF^3 rho^2, which keeps its
+//   precision where the wall is far: rho -> 0).
+// Displacements and Q stay in FP64 (their rounding is the FP64 kernel's own); everything after them
+// is an integer of 2^-59 absolute error in quantities of order one, where an FP64 chain of the
+// same length has several 2^-54 relative ones.  Pairs outside the ranges where this holds (Q
+// not a normal number far from the limits, strengths that are not finite, targets and sources on
+// opposite sides of the wall) go to the FP64 functions, pair by pair.
+#pragma once
+#include "fixed.cuh"
+
+namespace flg {
+
+// exponents of Q that the fixed-point path takes: every exponent sum stays far inside the range
+constexpr int kQExpMin = 1023 - 1000, kQExpMax = 1023 + 1000;
+FLG_HD bool q_in_range(double Q) {
+    const int ex = (int)(dbits(Q) >> 52);  // (a sign bit makes it too large)
+    return ex >= kQExpMin && ex <= kQExpMax;
+}
+
+// strengths of one source, f = F 2^e with the largest |F_k| in [1/4, 1/2); e = kFxBad: not finite
+constexpr int kFxBad = 1 << 28, kFxZero = -(1 << 20);
+FLG_HD int fx_strength(const double *f, int n, q60 *F) {
+    int em = 0;
+    for (int k = 0; k < n; k++) em = dexp(f[k]) > em ? dexp(f[k]) : em;
+    if (em == 0x7ff) return kFxBad;
+    for (int k = 0; k < n; k++) F[k] = q_of(f[k], em) >> 2;  // |f| 2^-em < 2: a quarter of it below 1/2
+    return em < 64 ? (em == 0 ? kFxZero : kFxBad) : em - 1023 + 2;
+}
+
+// what the pair kernels give: the coefficients of u = (A f + B (f.n) n) 2^x for a radial kernel
+struct FxRadial {
+    q60 A, B;  // A in [-1.8, 1.8], B in [0, 1.6]
+    int x;
+};
+struct FxDir {  // unit vector and w^2, with the root
+    q60 n[3], w2;
+    QRsqrt r;
+};
+FLG_HD FxDir fx_dir(double d0, double d1, double d2, double Q, double e) {
+    FxDir g;
+    g.r = q_rsqrt(Q);
+    const Qf y = qf(g.r.y);
+    g.n[0] = q_sign(qmul(qf(q_mag(d0, g.r.e)), y), d_neg(d0));
+    g.n[1] = q_sign(qmul(qf(q_mag(d1, g.r.e)), y), d_neg(d1));
+    g.n[2] = q_sign(qmul(qf(q_mag(d2, g.r.e)), y), d_neg(d2));
+    const Qf w = qf(qmul(qf(q_mag(e, g.r.e)), y));
+    g.w2 = qmul(w, w);
+    return g;
+}
+
+FLG_HD FxRadial fx_stokeslet(const FxDir &g) {
+    // (1 + w^2) / 2 and 1 / 2 of the root
+    FxRadial r;
+    r.A = qmul(qf((kQ1 + g.w2) >> 1), qf(g.r.y));
+    r.B = g.r.y >> 1;
+    r.x = 1 - (g.r.e - 1023);
+    return r;
+}
+
+// alpha = am 2^ae with am in [1/2, 1); 1 / alpha^2 = ia 2^iae with ia in [1/2, 1)
+struct FxAlpha {
+    q60 am, ia;
+    int ae, iae;
+};
+inline FxAlpha fx_alpha(double alpha) {
+    FxAlpha a;
+    int e;
+    const double m = std::frexp(alpha, &e);
+    a.am = (q60)std::ldexp(m, 60);
+    a.ae = e;
+    const long double i = 1.0L / ((long double)m * m);  // in (1, 4]
+    int ie;
+    const long double im = std::frexp(i, &ie);
+    a.ia = (q60)std::ldexp(im, 60);
+    a.iae = ie - 2 * e;
+    return a;
+}
+
+// 2^(-i / 64)
+#define FLG_EXP_TABLE \
+    0x1000000000000000ll, 0x0fd3e0c0cf486c17ll, 0x0fa83b2db722a034ll, 0x0f7d0df730ad13bcll, \
+    0x0f5257d152486cc3ll, 0x0f281773c59ffb14ll, 0x0efe4b99bdcdaf5dll, 0x0ed4f301ed9942b8ll, \
+    0x0eac0c6e7dd24393ll, 0x0e8396a503c4bdc7ll, 0x0e5b906e77c8348bll, 0x0e33f8972be8a5a5ll, \
+    0x0e0ccdeec2a94e11ll, 0x0de60f4825e0e912ll, 0x0dbfbb797daf2375ll, 0x0d99d15c278afd7bll, \
+    0x0d744fccad69d6afll, 0x0d4f35aabcfedfa2ll, 0x0d2a81d91f12ae46ll, 0x0d06333daef2b259ll, \
+    0x0ce248c151f8480ell, 0x0cbec14fef2727c6ll, 0x0c9b9bd866e2f27all, 0x0c78d74c8abb9b16ll, \
+    0x0c5672a115506daell, 0x0c346ccda2497640ll, 0x0c12c4cca6670945ll, 0x0bf1799b67a73108ll, \
+    0x0bd08a39f580c36cll, 0x0baff5ab2133e460ll, 0x0b8fbaf4762fb9efll, 0x0b6fd91e328d1779ll, \
+    0x0b504f333f9de648ll, 0x0b311c412a911249ll, 0x0b123f581d2ac259ll, 0x0af3b78ad690a437ll, \
+    0x0ad583eea42a14acll, 0x0ab7a39b5a93ed33ll, 0x0a9a15ab4ea7c0f0ll, 0x0a7cd93b4e965357ll, \
+    0x0a5fed6a9b15138fll, 0x0a43515ae09e680all, 0x0a27043030c49682ll, 0x0a0b0510fb9714fcll, \
+    0x09ef5326091a111bll, 0x09d3ed9a72cffb75ll, 0x09b8d39b9d54e554ll, 0x099e0459320b7fa6ll, \
+    0x09837f0518db8a97ll, 0x096942d3720185a0ll, 0x094f4efa8fef7096ll, 0x0935a2b2f13e6e93ll, \
+    0x091c3d373ab11c33ll, 0x09031dc431466b1ell, 0x08ea4398b45cd53cll, 0x08d1adf5b7e5ba9ell, \
+    0x08b95c1e3ea8bd6ell, 0x08a14d575496efdall, 0x088980e8092da852ll, 0x0871f61969e8d101ll, \
+    0x085aac367cc487b1ll, 0x0843a28c3acde404ll, 0x082cd8698ac2ba1dll, 0x08164d1f3bc03077ll
+// series coefficients of f1 and f2 (pair_math.cuh), 16 terms: the next is below 2^-60 at z = 1/2
+#define FLG_BR_Q1 \
+    576460752303423488ll, -768614336404564651ll, 432345564227567616ll, -153722867280912930ll, \
+    40031996687737742ll, -8235153604334621ll, 1401119884070821ll, -203337126032954ll, \
+    25734855013546ll, -2888311449332ll, 291238071141ll, -26661336455ll, \
+    2235002907ll, -172804959ll, 12398315ll, -829796ll
+#define FLG_BR_Q2 \
+    576460752303423488ll, 0ll, -144115188075855872ll, 76861433640456465ll, \
+    -24019198012642645ll, 5490102402889748ll, -1000799917193444ll, 152502844524715ll, \
+    -20015998343869ll, 2310649159465ll, -238285694570ll, 22217780379ll, \
+    -1891156306ll, 148118536ll, -10745206ll, 726071ll
+#if defined(__CUDACC__)
+static __constant__ q60 c_q_br1[16] = {FLG_BR_Q1};
+static __constant__ q60 c_q_br2[16] = {FLG_BR_Q2};
+static __device__ const q60 c_q_exp[64] = {FLG_EXP_TABLE};
+#endif
+static const q60 h_q_br1[16] = {FLG_BR_Q1};
+static const q60 h_q_br2[16] = {FLG_BR_Q2};
+static const q60 h_q_exp[64] = {FLG_EXP_TABLE};
+FLG_HD q60 q_br1(int i) {
+#if defined(__CUDA_ARCH__)
+    return c_q_br1[i];
+#else
+    return h_q_br1[i];
+#endif
+}
+FLG_HD q60 q_br2(int i) {
+#if defined(__CUDA_ARCH__)
+    return c_q_br2[i];
+#else
+    return h_q_br2[i];
+#endif
+}
+FLG_HD q60 q_exp_table(int i) {
+#if defined(__CUDA_ARCH__)
+    return c_q_exp[i];
+#else
+    return h_q_exp[i];
+#endif
+}
+
+// a b for b in Q36 below 2^30 (a factor below 1/64)
+FLG_HD q60 qmul36(q60 a, int b) {
+    const Qf f = qf(a);
+    return (((q60)f.h * b) >> 6) + (((q60)f.l * b) >> 36);
+}
+// e^-z = m 2^-n, m in (1/2, 1], for z = zm 2^kz with zm in [1/2, 1), 0 <= kz <= 6
+FLG_HD q60 q_expneg(q60 zm, int kz, int *n) {
+    const q60 v = qmul(qf(zm), qf(1663314137230540311ll));  // zm log2(e), in (0.7, 1.45)
+    const q60 frac = (q60)((uint64_t)v << kz) & (kQ1 - 1);
+    *n = (int)(v >> (60 - kz));
+    const int i = (int)(frac >> 54);
+    const q60 x = qmul(qf((frac << 6) & (kQ1 - 1)), qf(799144290325165979ll >> 6));  // remainder ln(2) / 64
+    const int xs = (int)(x >> 24);
+    const q60 v4 = (kQ1 / 24) - qmul36((kQ1 / 120) - qmul36((kQ1 / 720) - qmul36(kQ1 / 5040, xs), xs), xs);
+    const Qf xf = qf(x);
+    const q60 u = (kQ1 / 2) - qmul(xf, qf((kQ1 / 6) - qmul(xf, qf(v4))));
+    const q60 p = kQ1 - x + qmul(qf(qmul(xf, xf)), qf(u));
+    return qmul(qf(q_exp_table(i)), qf(p));
+}
+
+FLG_HD q60 q_shift(q60 x, int s) {  // x 2^-s
+    return s >= 0 ? x >> (s < 63 ? s : 63) : x << -s;
+}
+
+FLG_HD FxRadial fx_brinkman(const FxDir &g, const FxAlpha &al) {
+    const Qf y = qf(g.r.y);
+    const int E = g.r.e - 1023;
+    q60 zm = qmul(qf(al.am), qf(qmul(qf(g.r.qh), y)));  // in [1/4, 1)
+    const int low = zm < kQ1 / 2;
+    zm <<= low;
+    const int kz = al.ae + E + 1 - low;  // z = zm 2^kz, zm in [1/2, 1)
+    FxRadial r;
+    if (kz < 0) {
+        const Qf z = qf(q_shift(zm, -kz));
+        q60 f1 = q_br1(15), f2 = q_br2(15);
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+        for (int n = 14; n >= 0; n--) {
+            f1 = qmul(qf(f1), z) + q_br1(n);
+            f2 = qmul(qf(f2), z) + q_br2(n);
+        }
+        r.A = qmul(qf(f1 + qmul(qf(f2), qf(g.w2))), y);
+        r.B = qmul(qf(f2), y);
+        r.x = -E;
+        return r;
+    }
+    q60 F1 = -kQ1, F2h = kQ1 + kQ1 / 2;  // F1, F2 / 2 where E has vanished
+    if (kz < 6 || (kz == 6 && zm < kQ1 / 64 * 52)) {
+        int n;
+        const Qf em = qf(q_expneg(zm, kz, &n));
+        const q60 z2 = qmul(qf(zm), qf(zm)), z1 = zm >> kz, z0 = kQ1 >> (2 * kz);  // over 4^kz
+        const int h1 = kz == 0, h2 = kz < 2 ? 2 - kz : 0;  // so that the polynomials stay below 2
+        F1 += q_shift(qmul(em, qf((z2 + z1 + z0) >> h1)), n - 2 * kz - h1);
+        F2h -= q_shift(qmul(em, qf((z2 + 3 * (z1 + z0)) >> h2)), n - 2 * kz - h2 + 1);
+    }
+    // (small factors are scaled up: F1 and F2 of z < 1, y^3 / alpha^2 below 1/4)
+    q60 k = qmul(qf(qmul(qf(qmul(y, y)), y)), qf(al.ia));
+    const int sk = k < kQ1 / 4 ? 2 : 0, sf = kz == 0 ? 2 : 0;
+    const Qf kf = qf(k << sk), f2 = qf(F2h << sf);
+    r.A = qmul(qf(((F1 << sf) >> 1) + qmul(f2, qf(g.w2))), kf);
+    r.B = qmul(f2, kf);
+    r.x = 1 + al.iae - 3 * E - sk - sf;
+    return r;
+}
+
+// u / 2^x for strengths F; |u| < 2
+FLG_HD void fx_radial_apply(const FxDir &g, const FxRadial &r, const q60 *F, q60 *u) {
+    const Qf n0 = qf(g.n[0]), n1 = qf(g.n[1]), n2 = qf(g.n[2]), f0 = qf(F[0]), f1 = qf(F[1]), f2 = qf(F[2]);
+    const q60 t = qmul(f0, n0) + qmul(f1, n1) + qmul(f2, n2);
+    const Qf b = qf(qmul(qf(t), qf(r.B))), A = qf(r.A);
+    u[0] = qmul(A, f0) + qmul(b, n0);
+    u[1] = qmul(A, f1) + qmul(b, n1);
+    u[2] = qmul(A, f2) + qmul(b, n2);
+}
+
+// wall: everything that does not depend on the strengths
+struct FxWall {
+    q60 nx, ny, nm, nI, rho, rho2, Z3h, cq, czq, g;
+    int x;  // bracket / 8 . g . 2^x, without the factor t h
+};
+FLG_HD FxWall fx_wall(double d0, double d1, double dm, double dp, double QF, double QI, double e) {
+    const FxDir f = fx_dir(d0, d1, dm, QF, e);
+    const QRsqrt i = q_rsqrt(QI);
+    const Qf yI = qf(i.y);
+    FxWall w;
+    w.nx = f.n[0], w.ny = f.n[1], w.nm = f.n[2];
+    w.nI = q_sign(qmul(qf(q_mag(dp, i.e)), yI), d_neg(dp));
+    // rho = (yI / yF) 2^(EF - EI), 1 / yF = q yF
+    const q60 half = qmul(yI, qf(qmul(qf(f.r.qh), qf(f.r.y))));
+    w.rho = q_shift(half << 1, i.e - f.r.e);
+    if (w.rho > kQ1) w.rho = kQ1;
+    const Qf rho = qf(w.rho);
+    w.rho2 = qmul(rho, rho);
+    const q60 Z1h = q_rcp1p(w.rho);  // Z1 / 2
+    w.Z3h = kQ1 + qmul(qf(w.rho2), qf(Z1h));  // Z3 / 2 = 1 + rho^2 / (1 + rho)
+    const q60 w2r3 = qmul(qf(f.w2), qf(qmul(qf(w.rho2), rho)));
+    const q60 base = Z1h + qmul(qf(f.w2), qf(w.Z3h)) - qhalf(w.rho), i3 = w2r3 + qhalf(w2r3);
+    w.cq = qhalf(base + i3), w.czq = qhalf(base - i3);  // c / 4, c' / 4
+    w.g = qmul(qf(f.r.y), qf(qmul(yI, yI)));
+    w.x = 4 - (f.r.e - 1023) - 2 * (i.e - 1023);  // 8 from the bracket, 2 of 2 t h
+    return w;
+}
+// the exponent of u 2^x is returned: the bracket cancels near the wall and for far images, so it is
+// scaled up to [1/2, 1) before its last product
+FLG_HD int fx_wall_apply(const FxWall &w, const q60 *F, q60 *u) {
+    const Qf nx = qf(w.nx), ny = qf(w.ny), nm = qf(w.nm), nI = qf(w.nI), f0 = qf(F[0]), f1 = qf(F[1]), f2 = qf(F[2]);
+    const q60 D = qmul(f0, nx) + qmul(f1, ny);
+    const Qf B = qf(qmul(nI, f2) - qmul(qf(w.rho), qf(D)));
+    const q60 t1 = qmul(qf(w.Z3h), qf(D + qmul(f2, nm)));  // Z3 (f.n) / 2
+    const q60 r2B = qmul(qf(w.rho2), B), zB = qmul(qf(w.rho), qf(qmul(nI, B)));
+    const Qf b = qf(qhalf(t1 - r2B - qhalf(r2B))), cq = qf(w.cq), g = qf(w.g);
+    const q60 ux = qmul(cq, f0) + qmul(b, nx), uy = qmul(cq, f1) + qmul(b, ny);
+    const q60 uz = qmul(qf(w.czq), f2) + qhalf(qmul(nm, qf(t1)) - zB - qhalf(zB));
+    const uint64_t m = (uint64_t)((ux ^ (ux >> 63)) | (uy ^ (uy >> 63)) | (uz ^ (uz >> 63)));
+#if defined(__CUDA_ARCH__)
+    const int lz = __clz((int)(m >> 32));
+#else
+    const int lz = (m >> 32) ? __builtin_clz((unsigned)(m >> 32)) : 32;
+#endif
+    // |bracket| / 4 < 2.4: lz >= 2; one shift left of lz - 3 after the shift right that makes room
+    const int s = lz < 5 ? 0 : lz - 5;
+    u[0] = qmul(qf(qhalf(ux << s)), g);
+    u[1] = qmul(qf(qhalf(uy << s)), g);
+    u[2] = qmul(qf(qhalf(uz << s)), g);
+    return w.x - s;
+}
+
+// Sums of up to 16 terms u 2^x with |u| < 2: 64-bit integers of 57 fractional bits (a term is
+// rounded to 2^-58 of its unit, the sum stays below 2^62) relative to the largest exponent so far,
+// which outlives the 16 terms.
+constexpr int kFxSeg = 16;
+template <int NC>
+struct FxAcc {
+    q60 a[NC];
+    int x;
+    FLG_HD void init() {
+        clear();
+        x = -(1 << 24);
+    }
+    FLG_HD void clear() {
+        for (int k = 0; k < NC; k++) a[k] = 0;
+    }
+    // makes room for a term of exponent xt (rare once the first few pairs have passed)
+    FLG_HD void scale(int xt) {
+        if (xt > x) {
+            const int s = xt - x < 63 ? xt - x : 63;
+            for (int k = 0; k < NC; k++) a[k] = qshr(a[k], s);
+            x = xt;
+        }
+    }
+    // term u[0..3) of exponent xt at component c0 of the sum
+    FLG_HD void add(int c0, const q60 *u, int xt) {
+        const int s = x - xt + 3 < 63 ? x - xt + 3 : 63;
+        for (int k = 0; k < 3; k++) a[c0 + k] += qshr(u[k], s);
+    }
+    FLG_HD double value(int k) const { return q_to_double(a[k], x + 3); }
+};
+
+}  // namespace flg

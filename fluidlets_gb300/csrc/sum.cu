@@ -24,11 +24,15 @@
 #include <mutex>
 
 #include "flg_common.cuh"
+#include "pair_fixed.cuh"
 #include "pair_math.cuh"
 #include "sum_plan.cuh"
 
 namespace flg {
 
+#ifndef FLG_FX_MINB
+#define FLG_FX_MINB 4
+#endif
 constexpr int kF64Threads = 128;
 constexpr int kF64Tile = 128;
 constexpr int kF32Threads = 256;
@@ -150,6 +154,108 @@ __global__ void __launch_bounds__(kF64Threads) sum_f64_kernel(SumArgs a) {
 }
 
 // ---------------------------------------------------------------------------
+// The same sum for real kernels with the pairs in 60-bit fixed point (pair_fixed.cuh): the FP64
+// pipe (19 clocks per warp instruction and SM) keeps the displacements and squared distances, six
+// operations of a Stokeslet pair's 27 and eight of a wall pair's 56; the rest runs on the integer
+// pipe beside it.  Sums of 16 terms stay in 64-bit integers relative to their largest exponent.
+// A pair outside the fixed-point ranges takes the FP64 function.  The wall kernel's factor t is
+// applied once at the end, its factor h in the staged strengths.
+// ---------------------------------------------------------------------------
+constexpr int kFxThreads = 128, kFxTile = 64;
+struct FxSource {
+    double x, y, z, e2, e;
+    int ef;  // exponent of the strengths, or kFxBad
+};
+template <int KIND, int NF>
+__device__ __noinline__ void pair_f64_slow(double tx, double ty, double tz, const FxSource &s, const double *f,
+                                           int64_t j, double alpha, double *u) {
+    double fj[3 * NF];
+    load_strength<NF>(f, j, fj);
+    pair_f64<KIND, NF, false>(tx, ty, tz, 2.0, s.x, s.y, s.z, s.e2, fj, alpha, 0.0, u);
+}
+template <int KIND, int NF>
+__global__ void __launch_bounds__(kFxThreads, FLG_FX_MINB) sum_fx_kernel(SumArgs a, FxAlpha al) {
+    constexpr int NC = 3 * NF;
+    __shared__ FxSource s_src[kFxTile];
+    __shared__ q60 s_f[kFxTile][NC];
+    const int64_t i = (int64_t)blockIdx.x * kFxThreads + threadIdx.x;
+    const int64_t ii = i < a.M ? i : a.M - 1;
+    const double tx = a.tg[3 * ii], ty = a.tg[3 * ii + 1], tz = a.tg[3 * ii + 2];
+    double u[NC], us[NC];
+    FxAcc<NC> acc;
+    acc.init();
+#pragma unroll
+    for (int c = 0; c < NC; c++) u[c] = us[c] = 0.0;
+    const int64_t j0 = (int64_t)blockIdx.y * a.split_len;
+    const int64_t j1 = min(a.N, j0 + a.split_len);
+    for (int64_t jt = j0; jt < j1; jt += kFxTile) {
+        const int cnt = (int)(j1 - jt < kFxTile ? j1 - jt : kFxTile);
+        __syncthreads();
+        for (int k = threadIdx.x; k < cnt; k += kFxThreads) {
+            const int64_t j = jt + k;
+            FxSource s;
+            s.x = a.src[3 * j], s.y = a.src[3 * j + 1], s.z = a.src[3 * j + 2];
+            s.e = fabs(a.eps[j]);
+            s.e2 = s.e * s.e;
+            double f[NC];
+            load_strength<NF>(a.f, j, f);
+            if (KIND == FLG_WALL)
+#pragma unroll
+                for (int c = 0; c < NC; c++) f[c] *= s.z;
+            s.ef = fx_strength(f, NC, s_f[k]);
+            s_src[k] = s;
+        }
+        __syncthreads();
+        for (int k0 = 0; k0 < cnt; k0 += kFxSeg) {
+            acc.clear();
+            const int k1 = min(cnt, k0 + kFxSeg);
+#pragma unroll 1
+            for (int k = k0; k < k1; k++) {
+                const FxSource &s = s_src[k];
+                const double d0 = tx - s.x, d1 = ty - s.y, d2 = tz - s.z;
+                if constexpr (KIND == FLG_WALL) {
+                    const double dp = tz + s.z;
+                    const double rq = fma(d1, d1, fma(d0, d0, s.e2)), QF = fma(d2, d2, rq), QI = fma(dp, dp, rq);
+                    if (q_in_range(QF) && q_in_range(QI) && s.ef < kFxBad && !(d_neg(tz) ^ d_neg(s.z))) {
+                        const FxWall w = fx_wall(d0, d1, d2, dp, QF, QI, s.e);
+#pragma unroll
+                        for (int c = 0; c < NC; c += 3) {
+                            q60 t[3];
+                            const int x = fx_wall_apply(w, s_f[k] + c, t) + s.ef;
+                            acc.scale(x);
+                            acc.add(c, t, x);
+                        }
+                        continue;
+                    }
+                } else {
+                    const double Q = fma(d2, d2, fma(d1, d1, fma(d0, d0, s.e2)));
+                    if (q_in_range(Q) && s.ef < kFxBad) {
+                        const FxDir g = fx_dir(d0, d1, d2, Q, s.e);
+                        const FxRadial r = KIND == FLG_STOKESLET ? fx_stokeslet(g) : fx_brinkman(g, al);
+                        acc.scale(r.x + s.ef);
+#pragma unroll
+                        for (int c = 0; c < NC; c += 3) {
+                            q60 t[3];
+                            fx_radial_apply(g, r, s_f[k] + c, t);
+                            acc.add(c, t, r.x + s.ef);
+                        }
+                        continue;
+                    }
+                }
+                pair_f64_slow<KIND, NF>(tx, ty, tz, s, a.f, jt + k, a.alpha_re, us);
+            }
+#pragma unroll
+            for (int c = 0; c < NC; c++) u[c] += acc.value(c);
+        }
+    }
+    if (i < a.M) {
+        double *p = a.partial + ((int64_t)blockIdx.y * a.M + i) * NC;
+#pragma unroll
+        for (int c = 0; c < NC; c++) p[c] = KIND == FLG_WALL ? tz * (u[c] + us[c]) : u[c] + us[c];
+    }
+}
+
+// ---------------------------------------------------------------------------
 // finalize: out = (sum_s partial[s] + near) * scale / mu
 // ---------------------------------------------------------------------------
 struct FinalArgs {
@@ -157,7 +263,6 @@ struct FinalArgs {
     int S;
     int64_t M;
     int outw;
-    const double *near;  // [M][outw] or null
     double scale;
     int out_complex;
     int mu_complex;
@@ -193,16 +298,31 @@ __device__ __forceinline__ void final_store(const FinalArgs &a, int64_t i, const
     }
 }
 
+// u += the splits' partial sums of target i in split order, eight splits' loads in flight (one at a time
+// they cost an L2 round trip each: 17 of a 226 x 226 call's 27 us)
+template <int OUTW>
+__device__ __forceinline__ void sum_partials(const double *partial, int S, int64_t M, int64_t i, double *u) {
+    for (int s0 = 0; s0 < S; s0 += 8) {
+        double v[8][OUTW];
+#pragma unroll
+        for (int s = 0; s < 8; s++)
+#pragma unroll
+            for (int c = 0; c < OUTW; c++)
+                v[s][c] = s0 + s < S ? partial[((int64_t)(s0 + s) * M + i) * OUTW + c] : 0.0;
+#pragma unroll
+        for (int s = 0; s < 8; s++)
+            if (s0 + s < S)
+#pragma unroll
+                for (int c = 0; c < OUTW; c++) u[c] += v[s][c];
+    }
+}
+
 __global__ void finalize_kernel(FinalArgs a) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.M) return;
     double u[6] = {0, 0, 0, 0, 0, 0};
-    for (int s = 0; s < a.S; s++) {
-        const double *p = a.partial + ((int64_t)s * a.M + i) * a.outw;
-        for (int c = 0; c < a.outw; c++) u[c] += p[c];
-    }
-    if (a.near)
-        for (int c = 0; c < a.outw; c++) u[c] += a.near[i * a.outw + c];
+    if (a.outw == 3) sum_partials<3>(a.partial, a.S, a.M, i, u);
+    else sum_partials<6>(a.partial, a.S, a.M, i, u);
     final_store(a, i, u);
 }
 
@@ -682,12 +802,7 @@ __global__ void __launch_bounds__(128) near_f64_kernel(NearArgs a) {
     double u[OUTW];
 #pragma unroll
     for (int c = 0; c < OUTW; c++) u[c] = 0.0;
-    // far partials, summed in split order
-    for (int s = 0; s < a.fin.S; s++) {
-        const double *p = a.fin.partial + ((int64_t)s * a.M + kt) * OUTW;
-#pragma unroll
-        for (int c = 0; c < OUTW; c++) u[c] += p[c];
-    }
+    sum_partials<OUTW>(a.fin.partial, a.fin.S, a.M, kt, u);  // the far field
     const int cx = cell_coord(tx, G.ox, G.inv_h, G.nx);
     const int cy = cell_coord(ty, G.oy, G.inv_h, G.ny);
     const int cz = cell_coord(tz, G.oz, G.inv_h, G.nz);
@@ -739,7 +854,9 @@ static void mu_division(double mu_re, double mu_im, FinalArgs &f) {
     }
 }
 
-static void split_plan(int64_t M, int64_t N, int targets_per_cta, int tile, int ctas_per_sm, int64_t &S,
+// S source splits of split_len sources (a multiple of tile, or of `fine` where a split is shorter than a
+// tile): enough CTAs for four waves of ctas_per_sm, so that the last wave is a small part
+static void split_plan(int64_t M, int64_t N, int targets_per_cta, int tile, int fine, int ctas_per_sm, int64_t &S,
                        int64_t &split_len) {
     if (N <= 0) {
         S = 0;
@@ -749,9 +866,11 @@ static void split_plan(int64_t M, int64_t N, int targets_per_cta, int tile, int 
     const int64_t mblocks = ceil_div(M, targets_per_cta);
     const int64_t want = 4LL * sm_count() * ctas_per_sm;
     S = std::max<int64_t>(1, ceil_div(want, mblocks));
-    S = std::min<int64_t>(S, ceil_div(N, tile));
+    S = std::min<int64_t>(S, ceil_div(N, fine));
     S = std::min<int64_t>(S, 4096);
-    split_len = ceil_div(ceil_div(N, S), tile) * tile;
+    split_len = ceil_div(N, S);
+    const int64_t step = split_len < tile ? fine : tile;
+    split_len = ceil_div(split_len, step) * step;
     S = ceil_div(N, split_len);
 }
 
@@ -767,9 +886,12 @@ void sum_layout(int kind, int64_t M, int64_t N, int nf, bool ck, int precision, 
     L.outw = out_width(nf, ck);
     L.NQ = 1 + nf;
     if (precision == FLG_PREC_FP64) {
-        split_plan(M, N, kF64Threads, kF64Tile, 8, L.S, L.split_len);
+        // splits down to 8 sources: a pair is a chain of several hundred clocks, so a small call's time is
+        // the longest split (226 x 226: 112 us with whole tiles of 128, 9 us with 8)
+        split_plan(M, N, kF64Threads, kF64Tile, 8, 8, L.S, L.split_len);
     } else {
-        split_plan(M, N, kF32Threads * far_tpt(kind, nf, ck), kF32Tile, 4, L.S, L.split_len);
+        split_plan(M, N, kF32Threads * far_tpt(kind, nf, ck), kF32Tile, kF32Tile, 4, L.S,
+                   L.split_len);
     }
 }
 
@@ -890,13 +1012,20 @@ static int launch_sum(const SumRun &r, const SumLayout &L, int precision, const 
             SumArgs a{r.tg, r.M, r.src, r.eps, r.f, r.N, L.split_len, r.alpha_re, r.alpha_im, p->partial};
             dim3 grid((unsigned)ceil_div(r.M, kF64Threads), (unsigned)L.S);
             prof_begin(FLG_SLOT_SUM_F64, st);
-            sum_f64_kernel<KIND, NF, CK><<<grid, kF64Threads, 0, st>>>(a);
+            if constexpr (!CK) {
+                static_assert(kFxThreads == kF64Threads, "one grid for both");
+                FxAlpha al{};
+                if (KIND == FLG_BRINKMANLET) al = fx_alpha(r.alpha_re);
+                sum_fx_kernel<KIND, NF><<<grid, kFxThreads, 0, st>>>(a, al);
+            } else {
+                sum_f64_kernel<KIND, NF, CK><<<grid, kF64Threads, 0, st>>>(a);
+            }
             FLG_LAUNCH_CHECK();
             prof_end(FLG_SLOT_SUM_F64, st);
         } else {
             fin.S = 0;
         }
-        finalize_kernel<<<(unsigned)ceil_div(r.M, 256), 256, 0, st>>>(fin);
+        finalize_kernel<<<(unsigned)ceil_div(r.M, 64), 64, 0, st>>>(fin);
         FLG_LAUNCH_CHECK();
         return FLG_OK;
     }
@@ -941,6 +1070,10 @@ int sum_run(const SumRun &r, const SumLayout &L, int precision, const SumPlan *p
             return nf == 1 ? launch_sum<FLG_WALL, 1, false>(r, L, precision, p, st)
                            : launch_sum<FLG_WALL, 2, false>(r, L, precision, p, st);
         case FLG_BRINKMANLET:
+            // alpha = 0 is the Stokeslet (f1 = f2 = 1/2); the mixed path's FP32 far field keeps its own form
+            if (!ck && r.alpha_re == 0.0 && precision == FLG_PREC_FP64)
+                return nf == 1 ? launch_sum<FLG_STOKESLET, 1, false>(r, L, precision, p, st)
+                               : launch_sum<FLG_STOKESLET, 2, false>(r, L, precision, p, st);
             if (ck)
                 return nf == 1 ? launch_sum<FLG_BRINKMANLET, 1, true>(r, L, precision, p, st)
                                : launch_sum<FLG_BRINKMANLET, 2, true>(r, L, precision, p, st);

@@ -1,0 +1,112 @@
+"""FP64 sums whose pairs run in fixed point: short and ragged splits, the ranges that leave the
+fixed-point path, and scales far from one, against the oracle's FP64 loops."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import fluidlets_gb300 as fl  # noqa: E402
+import oracle as O  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+KERNELS = [(fl.Stokeslet3D(), "stokeslet", 0.0), (fl.WallStokeslet3D(), "wall", 0.0),
+           (fl.Brinkmanlet3D(0.0), "brinkman", 0.0), (fl.Brinkmanlet3D(2.5), "brinkman", 2.5),
+           (fl.Brinkmanlet3D(40.0), "brinkman", 40.0)]
+IDS = ["stokeslet", "wall", "alpha0", "alpha2.5", "alpha40"]
+
+
+def points(rng, m, n, scale=1.0):
+    X = np.c_[rng.uniform(-1, 1, (m, 2)), rng.uniform(0.0, 2.0, m)] * scale
+    Y = np.c_[rng.uniform(-1, 1, (n, 2)), rng.uniform(0.02, 2.0, n)] * scale
+    return X, Y
+
+
+def oracle_sum(name, alpha, *args):
+    return O.evaluate(name, *args, alpha=alpha) if name == "brinkman" else O.evaluate(name, *args)
+
+
+def check(kernel, name, alpha, X, Y, F, e, tol):
+    """Relative L2 against the oracle: n terms of a few roundings each on both sides."""
+    u = fl.evaluate(kernel, X, Y, F, e)
+    ref = oracle_sum(name, alpha, X, Y, F, e)
+    assert np.linalg.norm(u - ref) <= tol * np.linalg.norm(ref)
+    return u, ref
+
+
+@pytest.mark.parametrize("m,n", [(1, 1), (1, 7), (3, 8), (127, 15), (128, 16), (129, 17), (5, 63), (130, 65), (40, 1025)])
+@pytest.mark.parametrize("kernel,name,alpha", KERNELS, ids=IDS)
+def test_ragged_sizes(kernel, name, alpha, m, n):
+    rng = np.random.default_rng(m * 1000 + n)
+    X, Y = points(rng, m, n)
+    X[0] = Y[0]  # a pair at distance zero
+    F = rng.normal(size=(n, 3))
+    F[::5, 1] = 0.0
+    check(kernel, name, alpha, X, Y, F, 0.05 * rng.uniform(0.5, 2.0, n), 1e-13)
+
+
+@pytest.mark.parametrize("scale", [1e-90, 1e-12, 1e9, 1e85])
+@pytest.mark.parametrize("kernel,name,alpha", KERNELS[:3], ids=IDS[:3])
+def test_scales(kernel, name, alpha, scale):
+    rng = np.random.default_rng(3)
+    X, Y = points(rng, 40, 60, scale)
+    F = rng.normal(size=(60, 3)) * 10.0 ** rng.integers(-8, 8, (60, 1))
+    # the kernels are homogeneous of degree -1: the oracle runs at scale 1, where its s^5 cannot overflow
+    ref = oracle_sum(name, alpha, X / scale, Y / scale, F, 0.03) / scale
+    u = fl.evaluate(kernel, X, Y, F, 0.03 * scale)
+    assert np.linalg.norm(u * scale - ref * scale) <= 1e-13 * np.linalg.norm(ref * scale)
+
+
+@pytest.mark.parametrize("kernel,name,alpha", KERNELS[:2], ids=IDS[:2])
+def test_complex_strengths_and_tiny_blobs(kernel, name, alpha):
+    rng = np.random.default_rng(4)
+    X, Y = points(rng, 70, 90)
+    X[:30] = Y[:30] + 1e-7 * rng.normal(size=(30, 3))
+    X[:, 2] = np.abs(X[:, 2])
+    F = rng.normal(size=(90, 3)) + 1j * rng.normal(size=(90, 3))
+    check(kernel, name, alpha, X, Y, F, 1e-6, 1e-12)
+
+
+def test_targets_on_and_below_the_wall():
+    rng = np.random.default_rng(5)
+    X, Y = points(rng, 60, 50)
+    X[:20, 2] = 0.0
+    X[20:30, 2] *= -1.0
+    F = rng.normal(size=(50, 3))
+    u, ref = check(fl.WallStokeslet3D(), "wall", 0.0, X, Y, F, 0.05, 1e-12)
+    assert np.all(u[:20] == 0.0)
+
+
+def test_plane_problems_stay_in_the_plane():
+    rng = np.random.default_rng(6)
+    X, Y = points(rng, 50, 200)
+    X[:, 1] = Y[:, 1] = 0.25
+    F = rng.normal(size=(200, 3))
+    F[:, 1] = 0.0
+    for kernel, name, alpha in KERNELS:
+        u, _ = check(kernel, name, alpha, X, Y, F, 0.05, 1e-13)
+        assert np.all(u[:, 1] == 0.0)
+
+
+def test_non_finite_and_extreme_strengths():
+    rng = np.random.default_rng(7)
+    X, Y = points(rng, 20, 40)
+    F = rng.normal(size=(40, 3))
+    F[3] = 1e-305
+    F[4] = [1e300, -1e280, 0.0]
+    F[5] = 0.0
+    check(fl.Stokeslet3D(), "stokeslet", 0.0, X, Y, F, 0.05, 1e-13)
+    F[7, 1] = np.nan
+    assert np.all(np.isnan(fl.evaluate(fl.Stokeslet3D(), X, Y, F, 0.05)).any(axis=1))
+    F[7, 1] = np.inf
+    assert not np.isfinite(fl.evaluate(fl.Stokeslet3D(), X, Y, F, 0.05)).all(axis=1).any()
+    X[4] = np.nan
+    F[7] = 0.0
+    u = fl.evaluate(fl.WallStokeslet3D(), X, Y, F, 0.05)
+    assert np.all(np.isnan(u[4])) and np.isfinite(u[:4]).all()
+
+
+def test_zero_blob_on_a_source_is_not_finite():
+    X = np.array([[0.1, 0.2, 0.3], [0.4, 0.5, 0.6]])
+    u = fl.evaluate(fl.Stokeslet3D(), X, X[:1], np.ones((1, 3)), 0.0)
+    assert not np.isfinite(u[0]).any() and np.isfinite(u[1]).all()
