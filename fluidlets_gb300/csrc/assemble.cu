@@ -16,6 +16,7 @@
 #include <cuda_bf16.h>
 
 #include "flg_common.cuh"
+#include "pair_fixed.cuh"
 #include "pair_math.cuh"
 #include "sum_plan.cuh"
 
@@ -168,6 +169,188 @@ __device__ __forceinline__ void bucket_system(AsmArgs &a, const int64_t *&n_real
     a.out = (char *)a.out + z * a.sys_stride * (a.out_type == FLG_F64 ? 8 : 4);
     n_real_p += z;
 }
+
+// ---- real FP64 matrices in fixed point ---------------------------------------------------------
+// The block's coefficients (A, B of a radial kernel; five for the wall) come from pair_fixed.cuh with
+// the kernel's scale and 1 / mu in them; the entries are FP64 products of them with the displacement,
+// so each keeps its relative accuracy.  A wall block takes 25 operations of the FP64 pipe instead of
+// 108.  Pairs outside the fixed-point ranges take block_f64.
+struct FxAsm {
+    FxAlpha al;
+    FxConst c;      // scale / mu
+    double cd;      // the same as a number
+};
+template <int KIND>
+struct FxSrc {  // what a thread keeps of its source (or target) point
+    double x, y, z, e, e2;
+    FxConst h;      // wall: z times scale / mu
+    bool ok;
+};
+template <int KIND>
+__device__ __forceinline__ FxSrc<KIND> fx_src(double x, double y, double z, double e, const FxAsm &f) {
+    FxSrc<KIND> s{x, y, z, e, e * e, {0, 0}, true};
+    if (KIND == FLG_WALL) {
+        const double hc = z * f.cd;
+        s.ok = fx_const_ok(hc);
+        if (s.ok) s.h = fx_const(hc);
+    }
+    return s;
+}
+template <int KIND>
+__device__ __noinline__ void block_f64_slow(double tx, double ty, double tz, double sx, double sy, double sz, double e2,
+                                            double alpha, double c, double *G) {
+    double Gi[9];
+    block_f64<KIND, false>(tx, ty, tz, sx, sy, sz, e2, alpha, 0.0, G, Gi);
+    for (int k = 0; k < 9; k++) G[k] *= c;
+}
+// the scaled block G(t, s); cok: the constant is in range (else every pair takes the FP64 function)
+template <int KIND>
+__device__ __forceinline__ void block_fx(double tx, double ty, double tz, const FxSrc<KIND> &s, const FxAsm &f, bool cok,
+                                         double alpha, double (&G)[9]) {
+    const double d0 = tx - s.x, d1 = ty - s.y, d2 = tz - s.z;
+    if constexpr (KIND == FLG_WALL) {
+        const double dp = tz + s.z;
+        const double rq = fma(d1, d1, fma(d0, d0, s.e2)), QF = fma(d2, d2, rq), QI = fma(dp, dp, rq);
+        if (cok && s.ok && q_in_range(QF) && q_in_range(QI) && fx_const_ok(tz) && !(d_neg(tz) ^ d_neg(s.z))) {
+            const FxWallBlock w = fx_wall_block(d0, d1, d2, dp, QF, QI, s.e, fx_const(tz), s.h);
+            const double a0 = w.a * d0, a1 = w.a * d1;
+            G[0] = fma(a0, d0, w.c), G[1] = a0 * d1, G[2] = d0 * w.b1;
+            G[3] = G[1], G[4] = fma(a1, d1, w.c), G[5] = d1 * w.b1;
+            G[6] = d0 * w.b2, G[7] = d1 * w.b2, G[8] = w.z;
+            return;
+        }
+    } else {
+        const double Q = fma(d2, d2, fma(d1, d1, fma(d0, d0, s.e2)));
+        if (cok && q_in_range(Q)) {
+            const FxDir g = fx_dir(d0, d1, d2, Q, s.e);
+            double A, B;
+            fx_radial_block(g, KIND == FLG_STOKESLET ? fx_stokeslet(g) : fx_brinkman(g, f.al), f.c, &A, &B);
+            const double b0 = B * d0, b1 = B * d1, b2 = B * d2;
+            G[0] = fma(b0, d0, A), G[1] = b0 * d1, G[2] = b0 * d2;
+            G[3] = G[1], G[4] = fma(b1, d1, A), G[5] = b1 * d2;
+            G[6] = G[2], G[7] = G[5], G[8] = fma(b2, d2, A);
+            return;
+        }
+    }
+    double S[9];  // (an array of its own: G stays in registers on the usual path)
+    block_f64_slow<KIND>(tx, ty, tz, s.x, s.y, s.z, s.e2, alpha, f.cd, S);
+#pragma unroll
+    for (int k = 0; k < 9; k++) G[k] = S[k];
+}
+
+// A warp per 32 sources and every gridDim.y-th target: the 3 x 96 entries of a target go through shared
+// memory, so that a store covers 256 contiguous bytes (one 8-byte element per lane and 24 bytes
+// apart, the same entries took three times the L2 transactions)
+constexpr int kFxWarps = 4;
+template <int KIND>
+__global__ void __launch_bounds__(32 * kFxWarps) assemble_fx_kernel(AsmArgs a, FxAsm f, const int64_t *n_real) {
+    __shared__ double stg[kFxWarps][3][96];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (n_real) bucket_system(a, n_real);
+    const int64_t nr = n_real ? *n_real : INT64_MAX;  // rows and columns from nr on: the identity
+    const int64_t jw = ((int64_t)blockIdx.x * kFxWarps + warp) * 32, j = min(jw + lane, a.N - 1);
+    if (jw >= a.N) return;
+    const bool cok = fx_const_ok(f.cd);
+    const int64_t js = j < nr ? j : 0;
+    const FxSrc<KIND> s = fx_src<KIND>(a.src[3 * js], a.src[3 * js + 1], a.src[3 * js + 2], fabs(a.eps[js]), f);
+    const int ncol = (int)min((int64_t)96, 3 * (a.N - jw));
+    for (int64_t i = blockIdx.y; i < a.M; i += gridDim.y) {
+        double G[9];
+        if (i < nr && j < nr) {
+            block_fx<KIND>(a.tg[3 * i], a.tg[3 * i + 1], a.tg[3 * i + 2], s, f, cok, a.are, G);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 9; k++) G[k] = i == j && k % 4 == 0 ? 1.0 : 0.0;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) stg[warp][r][3 * lane + c] = G[3 * r + c];
+        __syncwarp();
+        double *o = (double *)a.out + 3 * i * a.ld + 3 * jw;
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                if (lane + 32 * k < ncol) o[r * a.ld + lane + 32 * k] = stg[warp][r][lane + 32 * k];
+    }
+}
+
+// The symmetric form (assemble_sym_kernel): a warp takes 32 sources j and tiles of kFxSymTile targets i,
+// writes the blocks (i, j), i <= j, as above and collects their mirrors (transposed for the wall kernel)
+// in shared memory: 96 rows of 3 kFxSymTile contiguous entries.  n_real (bucket plans): rows and
+// columns from *n_real on are those of the identity.
+constexpr int kFxSymTile = 4;
+template <int KIND, bool TRANSPOSE>
+__global__ void __launch_bounds__(32 * kFxWarps) assemble_fx_sym_kernel(AsmArgs a, FxAsm f, double eps,
+                                                                        const int64_t *n_real) {
+    constexpr int MC = 3 * kFxSymTile;
+    __shared__ double stg[kFxWarps][3][96], mir[kFxWarps][96][MC + 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (n_real) {
+        bucket_system(a, n_real);
+        eps = a.eps[0];
+    }
+    const int64_t nr = n_real ? *n_real : a.N;
+    const int64_t jw = ((int64_t)blockIdx.x * kFxWarps + warp) * 32, j = min(jw + lane, a.N - 1);
+    if (jw >= a.N) return;
+    const bool cok = fx_const_ok(f.cd);
+    const int64_t js = min(j, max(nr - 1, (int64_t)0));
+    const FxSrc<KIND> s = fx_src<KIND>(a.src[3 * js], a.src[3 * js + 1], a.src[3 * js + 2], fabs(eps), f);
+    const int64_t jn = min((int64_t)32, a.N - jw), last = jw + jn - 1;
+    double *out = (double *)a.out;
+    for (int64_t i0 = (int64_t)blockIdx.y * kFxSymTile; i0 <= last; i0 += (int64_t)gridDim.y * kFxSymTile) {
+        for (int t = 0; t < kFxSymTile; t++) {
+            const int64_t i = i0 + t;
+            if (i > last) break;
+            double G[9];
+            if (j < nr && i < nr) {
+                block_fx<KIND>(a.src[3 * i], a.src[3 * i + 1], a.src[3 * i + 2], s, f, cok, a.are, G);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 9; k++) G[k] = i == j && k % 4 == 0 ? 1.0 : 0.0;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < 3; r++)
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    stg[warp][r][3 * lane + c] = G[3 * r + c];
+                    mir[warp][3 * lane + r][3 * t + c] = TRANSPOSE ? G[3 * c + r] : G[3 * r + c];
+                }
+            __syncwarp();
+            double *o = out + 3 * i * a.ld + 3 * jw;
+            const int lo = i > jw ? 3 * (int)(i - jw) : 0;  // columns j >= i
+#pragma unroll
+            for (int r = 0; r < 3; r++)
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    const int c = lane + 32 * k;
+                    if (c >= lo && c < 3 * jn) o[r * a.ld + c] = stg[warp][r][c];
+                }
+        }
+        __syncwarp();
+        // mirrors: row 3 j + r, columns of the targets i < j
+        double *o = out + 3 * jw * a.ld + 3 * i0;
+#pragma unroll 4
+        for (int k = 0; k < 96 * MC / 32; k++) {
+            const int e = lane + 32 * k, row = e / MC, c = e % MC;
+            if (row < 3 * jn && i0 + c / 3 < jw + row / 3) o[row * a.ld + c] = mir[warp][row][c];
+        }
+        __syncwarp();
+    }
+}
+
+static FxAsm fx_asm(int kind, const AsmArgs &a) {
+    FxAsm f{};
+    if (kind == FLG_BRINKMANLET) f.al = fx_alpha(a.are);
+    f.cd = a.scale * a.imu_re;
+    if (fx_const_ok(f.cd)) f.c = fx_const(f.cd);
+    return f;
+}
+// the fixed-point kernels: real kernel and viscosity, FP64 output
+static bool fx_route(const AsmArgs &a) { return a.out_type == FLG_F64 && a.imu_im == 0.0 && a.aim == 0.0; }
 
 template <int KIND>
 __global__ void __launch_bounds__(128) assemble_bucket_kernel(AsmArgs a, const int64_t *n_real_p) {
@@ -577,12 +760,13 @@ __global__ void __launch_bounds__(256) convert2_f64_f32_kernel(int64_t nr, int64
 }
 
 // ---- host side ----------------------------------------------------------------
-static int prepare(int kind, double are, double aim, double mu_re, double mu_im, int out_type, AsmArgs &a) {
+static int prepare(int &kind, double are, double aim, double mu_re, double mu_im, int out_type, AsmArgs &a) {
     FLG_TRY(check_kernel_args(kind, are, aim));
     FLG_REQUIRE(!(mu_re == 0.0 && mu_im == 0.0), "mu must be non-zero");
     FLG_REQUIRE(out_type >= FLG_F64 && out_type <= FLG_BF16, "unknown out_type %d", out_type);
     const bool cplx = (kind == FLG_BRINKMANLET && aim != 0.0) || mu_im != 0.0;
     FLG_REQUIRE(!cplx || out_type == FLG_C128, "a complex kernel or viscosity needs out_type FLG_C128");
+    if (kind == FLG_BRINKMANLET && are == 0.0 && aim == 0.0) kind = FLG_STOKESLET;  // f1 = f2 = 1/2
     a.are = are;
     a.aim = aim;
     a.scale = kind == FLG_BRINKMANLET ? 1.0 / (4.0 * kPi) : 1.0 / (8.0 * kPi);
@@ -612,6 +796,28 @@ struct LaunchNearest {
     }
 };
 
+static void launch_fx(int kind, const AsmArgs &a, const int64_t *n_real, int nbat, cudaStream_t st) {
+    const FxAsm f = fx_asm(kind, a);
+    // eight targets per CTA: fewer leave the sources' loads and set-up uncovered
+    const dim3 grid((unsigned)ceil_div(a.N, 32 * kFxWarps), (unsigned)std::min<int64_t>(ceil_div(a.M, 8), 65535),
+                    (unsigned)nbat);
+    if (kind == FLG_STOKESLET) assemble_fx_kernel<FLG_STOKESLET><<<grid, 32 * kFxWarps, 0, st>>>(a, f, n_real);
+    else if (kind == FLG_WALL) assemble_fx_kernel<FLG_WALL><<<grid, 32 * kFxWarps, 0, st>>>(a, f, n_real);
+    else assemble_fx_kernel<FLG_BRINKMANLET><<<grid, 32 * kFxWarps, 0, st>>>(a, f, n_real);
+}
+static void launch_fx_sym(int kind, const AsmArgs &a, double eps, const int64_t *n_real, int nbat, cudaStream_t st) {
+    const FxAsm f = fx_asm(kind, a);
+    // four tiles of targets per CTA in the mean
+    const dim3 grid((unsigned)ceil_div(a.N, 32 * kFxWarps),
+                    (unsigned)std::min<int64_t>(ceil_div(a.N, 4 * kFxSymTile), 65535), (unsigned)nbat);
+    if (kind == FLG_STOKESLET)
+        assemble_fx_sym_kernel<FLG_STOKESLET, false><<<grid, 32 * kFxWarps, 0, st>>>(a, f, eps, n_real);
+    else if (kind == FLG_WALL)
+        assemble_fx_sym_kernel<FLG_WALL, true><<<grid, 32 * kFxWarps, 0, st>>>(a, f, eps, n_real);
+    else
+        assemble_fx_sym_kernel<FLG_BRINKMANLET, false><<<grid, 32 * kFxWarps, 0, st>>>(a, f, eps, n_real);
+}
+
 static dim3 asm_grid(int64_t M, int64_t N) {
     return dim3((unsigned)ceil_div(N, 128), (unsigned)std::min<int64_t>(M, 65535));
 }
@@ -639,7 +845,11 @@ extern "C" int flg_assemble(int kind, double alpha_re, double alpha_im, const do
     a.ld = ld;
     cudaStream_t st = as_stream(stream);
     prof_begin(FLG_SLOT_ASSEMBLE, st);
-    dispatch<LaunchAsm>(kind, kind == FLG_BRINKMANLET && alpha_im != 0.0, asm_grid(M, N), 128, st, a);
+    if (fx_route(a)) {
+        launch_fx(kind, a, nullptr, 1, st);
+    } else {
+        dispatch<LaunchAsm>(kind, kind == FLG_BRINKMANLET && alpha_im != 0.0, asm_grid(M, N), 128, st, a);
+    }
     FLG_LAUNCH_CHECK();
     prof_end(FLG_SLOT_ASSEMBLE, st);
     return FLG_OK;
@@ -666,7 +876,8 @@ extern "C" int flg_assemble_self_uniform(int kind, double alpha_re, double alpha
     const dim3 grid((unsigned)ceil_div(N, 128), (unsigned)std::min<int64_t>(ceil_div(N, kSymTile), 65535));
     const double e2 = eps * eps;
     prof_begin(FLG_SLOT_ASSEMBLE, st);
-    if (kind == FLG_STOKESLET) assemble_sym_kernel<FLG_STOKESLET, false, false><<<grid, 128, 0, st>>>(a, e2);
+    if (fx_route(a)) launch_fx_sym(kind, a, eps, nullptr, 1, st);
+    else if (kind == FLG_STOKESLET) assemble_sym_kernel<FLG_STOKESLET, false, false><<<grid, 128, 0, st>>>(a, e2);
     else if (kind == FLG_WALL) assemble_sym_kernel<FLG_WALL, false, true><<<grid, 128, 0, st>>>(a, e2);
     else if (alpha_im != 0.0) assemble_sym_kernel<FLG_BRINKMANLET, true, false><<<grid, 128, 0, st>>>(a, e2);
     else assemble_sym_kernel<FLG_BRINKMANLET, false, false><<<grid, 128, 0, st>>>(a, e2);
@@ -697,7 +908,10 @@ static int assemble_bucket_batch(int kind, double alpha_re, double alpha_im, con
     a.ld = ld;
     a.sys_stride = stride_out;
     prof_begin(FLG_SLOT_ASSEMBLE, st);
-    if (uniform) {
+    if (fx_route(a)) {
+        if (uniform) launch_fx_sym(kind, a, 0.0, n_real, nbat, st);
+        else launch_fx(kind, a, n_real, nbat, st);
+    } else if (uniform) {
         const dim3 grid((unsigned)ceil_div(n_cap, 128), (unsigned)std::min<int64_t>(ceil_div(n_cap, kSymTile), 65535),
                         (unsigned)nbat);
         if (kind == FLG_STOKESLET) assemble_bucket_sym_kernel<FLG_STOKESLET, false><<<grid, 128, 0, st>>>(a, n_real);

@@ -227,7 +227,8 @@ FLG_HD void fx_radial_apply(const FxDir &g, const FxRadial &r, const q60 *F, q60
 
 // wall: everything that does not depend on the strengths
 struct FxWall {
-    q60 nx, ny, nm, nI, rho, rho2, Z3h, cq, czq, g;
+    q60 nx, ny, nm, nI, rho, rho2, Z3h, cq, czq, g, yF;
+    int eF;  // sF = yF 2^-eF
     int x;  // bracket / 8 . g . 2^x, without the factor t h
 };
 FLG_HD FxWall fx_wall(double d0, double d1, double dm, double dp, double QF, double QI, double e) {
@@ -249,7 +250,8 @@ FLG_HD FxWall fx_wall(double d0, double d1, double dm, double dp, double QF, dou
     const q60 base = Z1h + qmul(qf(f.w2), qf(w.Z3h)) - qhalf(w.rho), i3 = w2r3 + qhalf(w2r3);
     w.cq = qhalf(base + i3), w.czq = qhalf(base - i3);  // c / 4, c' / 4
     w.g = qmul(qf(f.r.y), qf(qmul(yI, yI)));
-    w.x = 4 - (f.r.e - 1023) - 2 * (i.e - 1023);  // 8 from the bracket, 2 of 2 t h
+    w.yF = f.r.y, w.eF = f.r.e - 1023;
+    w.x = 4 - w.eF - 2 * (i.e - 1023);  // 8 from the bracket, 2 of 2 t h
     return w;
 }
 // the exponent of u 2^x is returned: the bracket cancels near the wall and for far images, so it is
@@ -275,6 +277,59 @@ FLG_HD int fx_wall_apply(const FxWall &w, const q60 *F, q60 *u) {
     u[1] = qmul(qf(qhalf(uy << s)), g);
     u[2] = qmul(qf(qhalf(uz << s)), g);
     return w.x - s;
+}
+
+// ---- matrix blocks ------------------------------------------------------------------------------
+// a real factor c = m 2^x with |m| in [1/2, 1) (0 for c = 0)
+struct FxConst {
+    q60 m;
+    int x;
+};
+FLG_HD FxConst fx_const(double c) {  // (not for denormals, infinities or NaN)
+    if (c == 0.0) return {0, 0};
+    const int e = dexp(c);
+    return {q_of(c, e) >> 1, e - 1022};
+}
+FLG_HD bool fx_const_ok(double c) { return c == 0.0 || (dexp(c) > 64 && dexp(c) < 1982); }
+
+// G = A I + B d d^T, both times c
+FLG_HD void fx_radial_block(const FxDir &g, const FxRadial &r, const FxConst &c, double *A, double *B) {
+    const Qf cm = qf(c.m), y = qf(g.r.y);
+    *A = q_to_double(qmul(qf(r.A), cm), r.x + c.x);
+    *B = q_to_double(qmul(qf(qmul(qf(r.B), qf(qmul(y, y)))), cm), r.x + c.x - 2 * (g.r.e - 1023));
+}
+// the wall block from d0, d1 and: G_jk = a d_j d_k + c delta_jk, G_jz = d_j b1, G_zj = d_j b2, G_zz = z
+// (j, k = x, y); th: t h times the constant
+struct FxWallBlock {
+    double a, b1, b2, c, z;
+};
+FLG_HD FxWallBlock fx_wall_block(double d0, double d1, double dm, double dp, double QF, double QI, double e,
+                                 const FxConst &t, const FxConst &h) {
+    const FxWall w = fx_wall(d0, d1, dm, dp, QF, QI, e);
+    // g t h, scaled up to [1/2, 1)
+    q60 k = qmul(qf(w.g), qf(qmul(qf(t.m), qf(h.m))));
+    const uint32_t hi = (uint32_t)((uint64_t)(k ^ (k >> 63)) >> 32);
+#if defined(__CUDA_ARCH__)
+    const int lz = __clz((int)hi);
+#else
+    const int lz = hi ? __builtin_clz(hi) : 32;
+#endif
+    const int s = lz < 12 ? lz - 4 : 0;  // |k| < 1: lz >= 4 (0: t = 0)
+    k <<= s;
+    const Qf kf = qf(k), yf = qf(w.yF), nm = qf(w.nm), nI = qf(w.nI), rho = qf(w.rho);
+    const q60 r2n = qmul(qf(w.rho2), nI), zn = qmul(qf(w.Z3h), nm), r3 = qmul(qf(w.rho2), rho);
+    const q60 i2n = r2n + qhalf(r2n);  // 3/2 rho^2 nI
+    const q60 a4 = qhalf(w.Z3h + r3 + qhalf(r3)), b14 = qhalf(zn - i2n), b24 = qhalf(zn + i2n);
+    const q60 rn2 = qmul(rho, qf(qmul(nI, nI)));
+    const q60 z4 = w.czq + qhalf(qmul(nm, qf(zn)) - rn2 - qhalf(rn2));
+    const int x = w.x - 1 - s + t.x + h.x;  // (the bracket over 4 here, over 8 in w.x)
+    FxWallBlock b;
+    b.a = q_to_double(qmul(qf(qmul(qf(a4), qf(qmul(yf, yf)))), kf), x - 2 * w.eF);
+    b.b1 = q_to_double(qmul(qf(qmul(qf(b14), yf)), kf), x - w.eF);
+    b.b2 = q_to_double(qmul(qf(qmul(qf(b24), yf)), kf), x - w.eF);
+    b.c = q_to_double(qmul(qf(w.cq), kf), x);
+    b.z = q_to_double(qmul(qf(z4), kf), x);
+    return b;
 }
 
 // Sums of up to 16 terms u 2^x with |u| < 2: 64-bit integers of 57 fractional bits (a term is

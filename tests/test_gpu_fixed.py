@@ -110,3 +110,49 @@ def test_zero_blob_on_a_source_is_not_finite():
     X = np.array([[0.1, 0.2, 0.3], [0.4, 0.5, 0.6]])
     u = fl.evaluate(fl.Stokeslet3D(), X, X[:1], np.ones((1, 3)), 0.0)
     assert not np.isfinite(u[0]).any() and np.isfinite(u[1]).all()
+
+
+# ---- matrices ---------------------------------------------------------------------------------
+def oracle_matrix(name, alpha, *args):
+    return O.assemble(name, *args, alpha=alpha) if name == "brinkman" else O.assemble(name, *args)
+
+
+@pytest.mark.parametrize("m,n", [(1, 1), (2, 31), (9, 32), (8, 33), (17, 127), (3, 128), (5, 129), (40, 161)])
+@pytest.mark.parametrize("kernel,name,alpha", KERNELS, ids=IDS)
+def test_matrix_ragged_sizes(kernel, name, alpha, m, n):
+    rng = np.random.default_rng(m * 100 + n)
+    X, Y = points(rng, m, n)
+    X[0] = Y[0]
+    e = 0.05 * rng.uniform(0.5, 2.0, n)
+    K, ref = fl.assemble(kernel, X, Y, e), oracle_matrix(name, alpha, X, Y, e)
+    B, R = (A.reshape(m, 3, n, 3).transpose(0, 2, 1, 3) for A in (K, ref))
+    # blocks of a few dozen roundings on each side; the wall's cancel towards z = 0
+    err = np.linalg.norm(B - R, axis=(2, 3)) / np.linalg.norm(R, axis=(2, 3))
+    assert np.median(err) < 1e-15 and err.max() < 1e-12
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 127, 130, 257])
+def test_symmetric_matrix_with_leading_dimension(n):
+    from fluidlets_gb300.core import _assemble_dev
+
+    rng = np.random.default_rng(n)
+    X = torch.tensor(np.c_[rng.uniform(-1, 1, (n, 2)), rng.uniform(0.05, 2.0, n)], device="cuda")
+    e = torch.full((n,), 0.06, dtype=torch.float64, device="cuda")
+    ld = 3 * n + 5
+    for kernel, name, alpha in KERNELS:
+        out = torch.full((3 * n, ld), 7.0, dtype=torch.float64, device="cuda")
+        _assemble_dev(kernel, X, X, e, 2.0, out=out, ld=ld, sym_eps=0.06, reciprocal=True)
+        full = _assemble_dev(kernel, X, X, e, 2.0)
+        assert torch.all(out[:, 3 * n:] == 7.0)
+        d = (out[:, :3 * n] - full).abs().max().item()
+        assert d == 0.0 if name != "wall" else d <= 1e-14 * full.abs().max().item()
+
+
+def test_matrix_on_and_below_the_wall():
+    rng = np.random.default_rng(8)
+    X, Y = points(rng, 12, 20)
+    X[:4, 2] = 0.0
+    X[4:8, 2] *= -1.0
+    K, ref = fl.assemble(fl.WallStokeslet3D(), X, Y, 0.05), O.assemble("wall", X, Y, 0.05)
+    assert np.all(K[:12] == 0.0)
+    assert np.abs(K - ref).max() <= 1e-13 * np.abs(ref).max()
