@@ -546,39 +546,41 @@ __device__ __forceinline__ void put(const SwimArgs &s, int64_t r, int64_t c, dou
     else ((float *)s.A)[r * s.ld + c] = (float)v;
 }
 
-// thread per force point m: its 3 rows of the [-I | r x] columns, and its
-// 3 columns of the net-force / net-torque rows
-__global__ void swimmer_kernel(SwimArgs s) {
-    const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// warp per force point m: its 3 rows of the [-I | r x] columns, and its 3 columns of the net-force /
+// net-torque rows, whose sums over the group's quadrature points run in ascending order (the lanes
+// look for members 32 at a time: alone, a thread walked all of nearest[], 150 us of a swimmer instant)
+__global__ void __launch_bounds__(128) swimmer_kernel(SwimArgs s) {
+    const int64_t m = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
     const int64_t n3 = 3 * s.N;
-    if (m < s.N) {
-        const double o0 = s.x0_dev ? s.x0_dev[0] : s.x0[0], o1 = s.x0_dev ? s.x0_dev[1] : s.x0[1],
-                     o2 = s.x0_dev ? s.x0_dev[2] : s.x0[2];
-        const double r0 = s.x[3 * m] - o0, r1 = s.x[3 * m + 1] - o1, r2 = s.x[3 * m + 2] - o2;
-        // cross matrix C(v): C @ w = v x w  (swimming.py:33-40)
-        const double C[9] = {0.0, -r2, r1, r2, 0.0, -r0, -r1, r0, 0.0};
-        for (int a = 0; a < 3; a++)
-            for (int b = 0; b < 3; b++) {
-                put(s, 3 * m + a, n3 + b, a == b ? -1.0 : 0.0);
-                put(s, 3 * m + a, n3 + 3 + b, C[3 * a + b]);
-            }
-        // count and sum of the quadrature points of group m, ascending k
-        double cnt = 0.0, X0 = 0.0, X1 = 0.0, X2 = 0.0;
-        for (int64_t k = 0; k < s.Q; k++)
-            if (s.nearest[k] == m) {
-                cnt += 1.0;
-                X0 += s.X[3 * k];
-                X1 += s.X[3 * k + 1];
-                X2 += s.X[3 * k + 2];
-            }
-        const double D[9] = {0.0, -X2, X1, X2, 0.0, -X0, -X1, X0, 0.0};
-        for (int a = 0; a < 3; a++)
-            for (int b = 0; b < 3; b++) {
-                put(s, n3 + a, 3 * m + b, a == b ? cnt : 0.0);
-                put(s, n3 + 3 + a, 3 * m + b, D[3 * a + b]);
-            }
+    if (blockIdx.x == 0 && threadIdx.x < 36) put(s, n3 + threadIdx.x / 6, n3 + threadIdx.x % 6, 0.0);
+    if (m >= s.N) return;
+    const double o0 = s.x0_dev ? s.x0_dev[0] : s.x0[0], o1 = s.x0_dev ? s.x0_dev[1] : s.x0[1],
+                 o2 = s.x0_dev ? s.x0_dev[2] : s.x0[2];
+    const double r0 = s.x[3 * m] - o0, r1 = s.x[3 * m + 1] - o1, r2 = s.x[3 * m + 2] - o2;
+    // count and sum of the quadrature points of group m, ascending k
+    double cnt = 0.0, X0 = 0.0, X1 = 0.0, X2 = 0.0;
+    for (int64_t k0 = 0; k0 < s.Q; k0 += 32) {
+        unsigned hit = __ballot_sync(0xffffffffu, k0 + lane < s.Q && s.nearest[k0 + lane] == m);
+        while (hit) {
+            const int64_t k = k0 + __ffs(hit) - 1;
+            hit &= hit - 1;
+            cnt += 1.0;
+            X0 += s.X[3 * k];
+            X1 += s.X[3 * k + 1];
+            X2 += s.X[3 * k + 2];
+        }
     }
-    if (m < 36) put(s, n3 + m / 6, n3 + m % 6, 0.0);
+    // cross matrices C(v): C @ w = v x w  (swimming.py:33-40), entry a, b on lane 3 a + b
+    if (lane < 9) {
+        const int a = lane / 3, b = lane % 3, c = 3 - a - b;  // the third axis
+        const double sg = (b - a + 3) % 3 == 1 ? -1.0 : 1.0;   // C[0][1] = -v2, C[1][2] = -v0, C[2][0] = -v1
+        const double rc = c == 0 ? r0 : c == 1 ? r1 : r2, Xc = c == 0 ? X0 : c == 1 ? X1 : X2;
+        put(s, 3 * m + a, n3 + b, a == b ? -1.0 : 0.0);
+        put(s, 3 * m + a, n3 + 3 + b, a == b ? 0.0 : sg * rc);
+        put(s, n3 + a, 3 * m + b, a == b ? cnt : 0.0);
+        put(s, n3 + 3 + a, 3 * m + b, a == b ? 0.0 : sg * Xc);
+    }
 }
 
 // ---- FP64 GEMV (row-major): warp per row ------------------------------------
@@ -1049,8 +1051,7 @@ extern "C" int flg_swimmer_constraints(const double *x, int64_t N, const double 
     FLG_REQUIRE(ld >= 3 * N + 6, "ld < 3N + 6");
     FLG_REQUIRE(x0_host && A && (N == 0 || x) && (Q == 0 || (X && nearest)), "null pointer");
     SwimArgs s{x, N, {x0_host[0], x0_host[1], x0_host[2]}, nullptr, X, nearest, Q, A, out_type, ld};
-    const int64_t threads = std::max<int64_t>(N, 36);
-    swimmer_kernel<<<(unsigned)ceil_div(threads, 128), 128, 0, as_stream(stream)>>>(s);
+    swimmer_kernel<<<(unsigned)std::max<int64_t>(1, ceil_div(N, 4)), 128, 0, as_stream(stream)>>>(s);
     FLG_LAUNCH_CHECK();
     return FLG_OK;
 }
@@ -1063,8 +1064,7 @@ extern "C" int flg_swimmer_constraints_dev(const double *x, int64_t N, const dou
     FLG_REQUIRE(ld >= 3 * N + 6, "ld < 3N + 6");
     FLG_REQUIRE(x0_dev && A && (N == 0 || x) && (Q == 0 || (X && nearest)), "null pointer");
     SwimArgs s{x, N, {0.0, 0.0, 0.0}, x0_dev, X, nearest, Q, A, out_type, ld};
-    const int64_t threads = std::max<int64_t>(N, 36);
-    swimmer_kernel<<<(unsigned)ceil_div(threads, 128), 128, 0, as_stream(stream)>>>(s);
+    swimmer_kernel<<<(unsigned)std::max<int64_t>(1, ceil_div(N, 4)), 128, 0, as_stream(stream)>>>(s);
     FLG_LAUNCH_CHECK();
     return FLG_OK;
 }
@@ -1115,36 +1115,38 @@ int gemv_f32_presplit(int64_t n_rows, int64_t n_cols, const float *A, int64_t ld
 }  // namespace flg
 
 // nearest force point of every quadrature point (the reference's k-d tree query,
-// core/assemble.py:61-65): exhaustive, FP64 squared distances, the first index
-// on ties; force points staged through shared memory in tiles of kNnTile
-constexpr int kNnTile = 1024;
+// core/assemble.py:61-65): exhaustive, FP64 squared distances, the first index on ties.  A warp per
+// query, each lane every 32nd force point, distances compared as integers (non-negative doubles order
+// like their bits; a NaN is above infinity and never taken): a thread per query walked all points
+// alone, seven FP64 instructions of 64 clocks each (896 x 226: 112 us, this form 7 us).
 __global__ void __launch_bounds__(256) nearest_kernel(const double *quad, int64_t Q, const double *force, int64_t N,
                                                       int64_t *out) {
-    __shared__ double fx[kNnTile], fy[kNnTile], fz[kNnTile];
-    const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    double px = 0.0, py = 0.0, pz = 0.0;
-    if (q < Q) px = quad[3 * q], py = quad[3 * q + 1], pz = quad[3 * q + 2];
-    double best = INFINITY;
-    int64_t bi = 0;
-    for (int64_t t0 = 0; t0 < N; t0 += kNnTile) {
-        const int nt = (int)min((int64_t)kNnTile, N - t0);
-        __syncthreads();
-        for (int k = threadIdx.x; k < nt; k += blockDim.x) {
-            fx[k] = force[3 * (t0 + k)];
-            fy[k] = force[3 * (t0 + k) + 1];
-            fz[k] = force[3 * (t0 + k) + 2];
-        }
-        __syncthreads();
-        for (int k = 0; k < nt; k++) {
-            const double dx = px - fx[k], dy = py - fy[k], dz = pz - fz[k];
-            const double d2 = dx * dx + dy * dy + dz * dz;
-            if (d2 < best) {
-                best = d2;
-                bi = t0 + k;
-            }
+    const int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (q >= Q) return;
+    const double px = quad[3 * q], py = quad[3 * q + 1], pz = quad[3 * q + 2];
+    unsigned long long best = 0x7ff0000000000000ull;  // infinity
+    long long bi = INT64_MAX;
+#pragma unroll 4
+    for (int64_t k = lane; k < N; k += 32) {
+        const double dx = px - force[3 * k], dy = py - force[3 * k + 1], dz = pz - force[3 * k + 2];
+        const double d2 = dx * dx + dy * dy + dz * dz;
+        const unsigned long long b = (unsigned long long)__double_as_longlong(d2);
+        if (b < best) {
+            best = b;
+            bi = k;
         }
     }
-    if (q < Q) out[q] = bi;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const long long oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (ob < best || (ob == best && oi < bi)) {
+            best = ob;
+            bi = oi;
+        }
+    }
+    if (lane == 0) out[q] = bi == INT64_MAX ? 0 : bi;
 }
 
 extern "C" int flg_nearest_neighbors(const double *quad, int64_t Q, const double *force, int64_t N, int64_t *out,
@@ -1154,7 +1156,7 @@ extern "C" int flg_nearest_neighbors(const double *quad, int64_t Q, const double
     if (Q == 0) return FLG_OK;
     FLG_REQUIRE(N > 0, "no force points to search");
     FLG_REQUIRE(quad && force && out, "null pointer");
-    nearest_kernel<<<(unsigned)ceil_div(Q, 256), 256, 0, as_stream(stream)>>>(quad, Q, force, N, out);
+    nearest_kernel<<<(unsigned)ceil_div(Q, 8), 256, 0, as_stream(stream)>>>(quad, Q, force, N, out);
     FLG_LAUNCH_CHECK();
     return FLG_OK;
 }
