@@ -538,7 +538,8 @@ static int gmres_run(int kind, double are, double aim, const double *X, const do
     opm.R = op64.R;
     T *d = ar.take<T>(n);
     FLG_REQUIRE(d != nullptr, "workspace too small");
-    FLG_TRY(sum_plan_geometry(X, eps, N, opm.L, &opm.P, st));
+    bool packed_f = false;
+    FLG_TRY(sum_plan_geometry(kind, X, eps, N, nullptr, opm.L, &opm.P, st, &packed_f));
     gi.A = [&](const T *v, T *out) { return opm.apply((const double *)v, (double *)out); };
     FLG_TRY(g.norm(b, &bn));
     if (bn == 0.0) {

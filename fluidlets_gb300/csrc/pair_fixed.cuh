@@ -78,8 +78,9 @@ struct FxAlpha {
 };
 inline FxAlpha fx_alpha(double alpha) {
     FxAlpha a;
+    if (alpha == 0.0) return {0, 0, -(1 << 20), 0};  // the series at z = 0
     int e;
-    const double m = std::frexp(alpha, &e);
+    const double m = std::frexp(alpha < 1.7e308 ? alpha : 1.7e308, &e);  // (an infinite alpha: u = 0)
     a.am = (q60)std::ldexp(m, 60);
     a.ae = e;
     const long double i = 1.0L / ((long double)m * m);  // in (1, 4]

@@ -40,6 +40,11 @@ constexpr int kF32Tile = 256;
 constexpr int kMaxCells = 1 << 20;
 constexpr int kBoundBlocks = 256;
 constexpr int kScanBlock = 1024;  // elements per scan block (one per thread)
+// source sets planned by one cluster; above, the separate kernels' spread over all SMs wins
+#ifndef FLG_PLAN_MAX
+#define FLG_PLAN_MAX 65536
+#endif
+constexpr int64_t kClusterPlanMax = FLG_PLAN_MAX;
 constexpr int64_t kSortTargetsMin = 32768;  // mixed sums bucket larger target sets by cell
 
 __host__ __device__ inline int out_width(int nf, bool ck) { return (nf == 2 || ck) ? 6 : 3; }
@@ -598,19 +603,10 @@ __global__ void __launch_bounds__(256) tile_box_kernel(const float4 *packed, int
     }
 }
 
-// slot k gets the strength of source order[k]; src (wall kernel only): the strengths are
-// scaled by the source height z_j, the factor of the wall pair that depends on the source
-// alone (see wall_far_geo)
-__global__ void pack_strengths_kernel(const double *f, const double *src, const int *order, int64_t N, int NF,
-                                      float4 *packed) {
-    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= N) return;
-    const int64_t j = order[k];
-    const int NQ = 1 + NF;
-    float4 *q = packed + k * NQ + 1;
-    const double *fj = f + (int64_t)3 * NF * j;
-    const double h = src ? src[3 * j + 2] : 1.0;
-    if (NF == 1) {
+// the strength of source j times h into its packed slot (q[0].w, the threshold, stays)
+__device__ __forceinline__ void pack_strength(const double *f, int64_t j, double h, int NQ, float4 *q) {
+    const double *fj = f + (int64_t)3 * (NQ - 1) * j;
+    if (NQ == 2) {
         q->x = __double2float_rn(h * fj[0]);
         q->y = __double2float_rn(h * fj[1]);
         q->z = __double2float_rn(h * fj[2]);
@@ -623,56 +619,92 @@ __global__ void pack_strengths_kernel(const double *f, const double *src, const 
     }
 }
 
+// slot k gets the strength of source order[k]; src (wall kernel only): the strengths are
+// scaled by the source height z_j, the factor of the wall pair that depends on the source
+// alone (see wall_far_geo)
+__global__ void pack_strengths_kernel(const double *f, const double *src, const int *order, int64_t N, int NF,
+                                      float4 *packed) {
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= N) return;
+    const int64_t j = order[k];
+    const int NQ = 1 + NF;
+    pack_strength(f, j, src ? src[3 * j + 2] : 1.0, NQ, packed + k * NQ + 1);
+}
+
 // ---------------------------------------------------------------------------
 // cell list for the near field
 // ---------------------------------------------------------------------------
-__global__ void cell_bounds_kernel(const double *src, const double *eps, int64_t N, double *blk) {
-    __shared__ double sm[7][256];
-    double v[7] = {1e300, 1e300, 1e300, -1e300, -1e300, -1e300, 0.0};
-    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < N; j += (int64_t)gridDim.x * blockDim.x) {
-        for (int c = 0; c < 3; c++) {
-            double x = src[3 * j + c];
-            v[c] = fmin(v[c], x);
-            v[3 + c] = fmax(v[3 + c], x);
-        }
-        v[6] = fmax(v[6], fabs(eps[j]));
+// order-preserving integers: FP64 comparisons run at a 64th of the integer rate
+__device__ __forceinline__ long long order_key(double x) {
+    const long long b = __double_as_longlong(x);
+    return b ^ (long long)((unsigned long long)(b >> 63) >> 1);
+}
+__device__ __forceinline__ double order_value(long long k) {
+    return __longlong_as_double(k ^ (long long)((unsigned long long)(k >> 63) >> 1));
+}
+// fmin / fmax semantics: a NaN loses against a number
+__device__ __forceinline__ bool is_nan_bits(double x) {
+    return ((unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull) > 0x7ff0000000000000ull;
+}
+// box[0..3) minima, box[3..6) maxima of the coordinates, box[6] largest |eps|
+struct BoxKeys {
+    long long v[7];
+    __device__ void init() {
+        for (int c = 0; c < 7; c++) v[c] = order_key(c < 3 ? 1e300 : c < 6 ? -1e300 : 0.0);
     }
-    for (int c = 0; c < 7; c++) sm[c][threadIdx.x] = v[c];
+    __device__ void add(double x, double y, double z, double e) {
+        const double p[3] = {x, y, z};
+        for (int c = 0; c < 3; c++)
+            if (!is_nan_bits(p[c])) {
+                const long long k = order_key(p[c]);
+                v[c] = min(v[c], k), v[3 + c] = max(v[3 + c], k);
+            }
+        if (!is_nan_bits(e)) v[6] = max(v[6], order_key(fabs(e)));
+    }
+    __device__ void join(const long long *o) {
+        for (int c = 0; c < 7; c++) v[c] = c < 3 ? min(v[c], o[c]) : max(v[c], o[c]);
+    }
+    __device__ void warp_reduce() {
+        for (int o = 16; o > 0; o >>= 1) {
+            long long w[7];
+            for (int c = 0; c < 7; c++) w[c] = __shfl_xor_sync(0xffffffffu, v[c], o);
+            join(w);
+        }
+    }
+};
+__global__ void __launch_bounds__(256) cell_bounds_kernel(const double *src, const double *eps, int64_t N,
+                                                          long long *blk) {
+    __shared__ long long sm[8][7];
+    BoxKeys b;
+    b.init();
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < N; j += (int64_t)gridDim.x * blockDim.x)
+        b.add(src[3 * j], src[3 * j + 1], src[3 * j + 2], eps[j]);
+    b.warp_reduce();
+    if ((threadIdx.x & 31) == 0)
+        for (int c = 0; c < 7; c++) sm[threadIdx.x >> 5][c] = b.v[c];
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) {
-            for (int c = 0; c < 3; c++) sm[c][threadIdx.x] = fmin(sm[c][threadIdx.x], sm[c][threadIdx.x + w]);
-            for (int c = 3; c < 7; c++) sm[c][threadIdx.x] = fmax(sm[c][threadIdx.x], sm[c][threadIdx.x + w]);
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int c = 0; c < 7; c++) blk[blockIdx.x * 7 + c] = sm[c][0];
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < 8; w++) b.join(sm[w]);
+    for (int c = 0; c < 7; c++) blk[blockIdx.x * 7 + c] = b.v[c];
 }
 
-__global__ void cell_setup_kernel(const double *blk, int nblk, CellGrid *g) {
-    if (threadIdx.x != 0) return;
-    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300}, emax = 0.0;
-    for (int b = 0; b < nblk; b++) {
-        for (int c = 0; c < 3; c++) {
-            lo[c] = fmin(lo[c], blk[b * 7 + c]);
-            hi[c] = fmax(hi[c], blk[b * 7 + 3 + c]);
-        }
-        emax = fmax(emax, blk[b * 7 + 6]);
-    }
+// the grid of a box (one thread)
+__device__ void make_grid(const long long *key, CellGrid *g) {
+    double lo[3], hi[3];
+    for (int c = 0; c < 3; c++) lo[c] = order_value(key[c]), hi[c] = order_value(key[3 + c]);
+    const double emax = order_value(key[6]);
     // cell edge >= 4.2 max eps: every pair with r < 4 eps (plus FP32 rounding)
     // lies in the 27-cell neighbourhood of the target's cell
     double h = fmax(4.2 * emax, 1e-300);
     double ext[3];
     for (int c = 0; c < 3; c++) ext[c] = fmax(hi[c] - lo[c], 0.0);
-    for (int it = 0; it < 64; it++) {
+    double n[3];
+    for (int it = 0; it <= 64; it++) {  // (the last pass only counts)
         double cells = 1.0;
-        for (int c = 0; c < 3; c++) cells *= floor(ext[c] / h) + 1.0;
-        if (cells <= (double)kMaxCells) break;
+        for (int c = 0; c < 3; c++) cells *= n[c] = floor(ext[c] / h) + 1.0;
+        if (cells <= (double)kMaxCells || it == 64) break;
         h *= fmax(1.01, cbrt(cells / (double)kMaxCells));
     }
-    double n[3];
-    for (int c = 0; c < 3; c++) n[c] = floor(ext[c] / h) + 1.0;
     const bool ok = n[0] >= 1.0 && n[1] >= 1.0 && n[2] >= 1.0 && n[0] * n[1] * n[2] <= (double)kMaxCells &&
                     h > 0.0 && h < 1e300 && lo[0] == lo[0] && lo[1] == lo[1] && lo[2] == lo[2];
     if (!ok) {  // non-finite input: one cell holding every source (still exact, only slower)
@@ -689,6 +721,18 @@ __global__ void cell_setup_kernel(const double *blk, int nblk, CellGrid *g) {
     g->ny = (int)n[1];
     g->nz = (int)n[2];
     g->ncell = g->nx * g->ny * g->nz;
+}
+__global__ void __launch_bounds__(kBoundBlocks) cell_setup_kernel(const long long *blk, CellGrid *g) {
+    __shared__ long long sm[kBoundBlocks / 32][7];
+    BoxKeys b;
+    for (int c = 0; c < 7; c++) b.v[c] = blk[threadIdx.x * 7 + c];
+    b.warp_reduce();
+    if ((threadIdx.x & 31) == 0)
+        for (int c = 0; c < 7; c++) sm[threadIdx.x >> 5][c] = b.v[c];
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < kBoundBlocks / 32; w++) b.join(sm[w]);
+    make_grid(b.v, g);
 }
 
 __device__ __forceinline__ int cell_coord(double x, double o, double inv_h, int n) {
@@ -773,6 +817,150 @@ __global__ void cell_sort_kernel(const int *offsets, const CellGrid *g, int *sor
     }
 }
 
+// ---------------------------------------------------------------------------
+// The whole plan of a small source set in one launch: box, cells, scan, order, packed sources (and
+// strengths) and tile boxes on one cluster of 16 CTAs, with cluster barriers between the steps
+// (ten-odd launches over the grid's 2^20 possible cells otherwise).  The same arrays as from the kernels above: a
+// source's place in its cell is the number of smaller source indices in it.
+// ---------------------------------------------------------------------------
+constexpr int kPlanCtas = 16, kPlanThreads = 1024, kPlanZero = 16384;
+struct PlanArgs {
+    const double *src, *eps, *f;  // f: null packs no strengths
+    int64_t N;
+    int NQ, scale_h;              // scale_h: strengths times the source height (wall kernel)
+    long long *bounds;
+    CellGrid *grid;
+    int *cell_of, *counts, *offsets, *block_sums, *slots, *sorted;
+    float4 *packed, *tile_box;
+};
+__device__ __forceinline__ void plan_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ int cell_index(const double *x, const CellGrid &G) {
+    const int cx = cell_coord(x[0], G.ox, G.inv_h, G.nx);
+    const int cy = cell_coord(x[1], G.oy, G.inv_h, G.ny);
+    const int cz = cell_coord(x[2], G.oz, G.inv_h, G.nz);
+    return (cz * G.ny + cy) * G.nx + cx;
+}
+__global__ void __launch_bounds__(kPlanThreads) plan_cluster_kernel(PlanArgs a) {
+    __shared__ long long sm[kPlanThreads / 32][7];
+    __shared__ CellGrid G;
+    __shared__ int ws[kPlanThreads / 32], s_base;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int gt = blockIdx.x * kPlanThreads + t, GT = kPlanCtas * kPlanThreads;
+    // box of the sources; the first counters cleared on the way
+    BoxKeys b;
+    b.init();
+    for (int64_t j = gt; j < a.N; j += GT) b.add(a.src[3 * j], a.src[3 * j + 1], a.src[3 * j + 2], a.eps[j]);
+    for (int c = gt; c < kPlanZero; c += GT) a.counts[c] = 0;
+    b.warp_reduce();
+    if (lane == 0)
+        for (int c = 0; c < 7; c++) sm[warp][c] = b.v[c];
+    __syncthreads();
+    if (warp == 0) {
+        for (int c = 0; c < 7; c++) b.v[c] = sm[lane][c];
+        b.warp_reduce();
+        if (lane == 0)
+            for (int c = 0; c < 7; c++) a.bounds[blockIdx.x * 7 + c] = b.v[c];
+    }
+    plan_sync();
+    if (warp == 0) {
+        for (int c = 0; c < 7; c++) b.v[c] = __ldcg(a.bounds + (lane & (kPlanCtas - 1)) * 7 + c);
+        b.warp_reduce();
+        if (lane == 0) {
+            make_grid(b.v, &G);
+            if (blockIdx.x == 0) *a.grid = G;
+        }
+    }
+    __syncthreads();
+    const int ncell = G.ncell;
+    if (ncell > kPlanZero) {
+        for (int c = kPlanZero + gt; c < ncell; c += GT) a.counts[c] = 0;
+        plan_sync();
+    }
+    // sources per cell; slots: a source's arrival number in its cell for now
+    for (int64_t j = gt; j < a.N; j += GT) {
+        const int c = cell_index(a.src + 3 * j, G);
+        a.cell_of[j] = c;
+        a.sorted[j] = atomicAdd(&a.counts[c], 1);
+    }
+    plan_sync();
+    // exclusive scan of the counts: a contiguous chunk per CTA, a contiguous piece of it per thread
+    const int chunk = (ncell + kPlanCtas - 1) / kPlanCtas, per = (chunk + kPlanThreads - 1) / kPlanThreads;
+    const int lo = min(ncell, blockIdx.x * chunk), hi = min(ncell, lo + chunk);
+    const int p0 = min(hi, lo + t * per), p1 = min(hi, p0 + per);
+    int sum = 0;
+    for (int c = p0; c < p1; c++) sum += __ldcg(a.counts + c);
+    int inc = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+    }
+    if (lane == 31) ws[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+        int w = ws[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += v;
+        }
+        ws[lane] = w;
+        if (lane == 31) a.block_sums[blockIdx.x] = w;
+    }
+    __syncthreads();
+    plan_sync();
+    if (t == 0) {
+        int base = 0;
+        for (int c = 0; c < (int)blockIdx.x; c++) base += __ldcg(a.block_sums + c);
+        s_base = base;
+    }
+    __syncthreads();
+    int run = s_base + (warp ? ws[warp - 1] : 0) + inc - sum;
+    for (int c = p0; c < p1; c++) {
+        a.offsets[c] = run;
+        run += __ldcg(a.counts + c);
+    }
+    if (gt == 0) a.offsets[ncell] = (int)a.N;
+    plan_sync();
+    // members of each cell in arrival order
+    for (int64_t j = gt; j < a.N; j += GT) a.slots[__ldcg(a.offsets + a.cell_of[j]) + a.sorted[j]] = (int)j;
+    plan_sync();
+    // ... and in ascending order, with the packed source in that place
+    for (int64_t j = gt; j < a.N; j += GT) {
+        const int c = a.cell_of[j], o0 = __ldcg(a.offsets + c), o1 = o0 + __ldcg(a.counts + c);
+        int pos = o0;
+        for (int k = o0; k < o1; k++) pos += __ldcg(a.slots + k) < (int)j;
+        a.sorted[pos] = (int)j;
+        const double e = a.eps[j], h = a.src[3 * j + 2];
+        const float e2 = __double2float_rn(e * e), thr = __fmul_rn(17.0f, e2);
+        float4 *q = a.packed + (int64_t)pos * a.NQ;
+        q[0] = make_float4(__double2float_rn(a.src[3 * j]), __double2float_rn(a.src[3 * j + 1]), __double2float_rn(h), e2);
+        q[1].w = thr;
+        if (a.f) pack_strength(a.f, j, a.scale_h ? h : 1.0, a.NQ, q + 1);
+    }
+    plan_sync();
+    // tile boxes, a warp per 256 sources
+    for (int64_t tile = blockIdx.x * (kPlanThreads / 32) + warp; tile * kF32Tile < a.N; tile += kPlanCtas * (kPlanThreads / 32)) {
+        float v[7] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY, 0.0f};
+        for (int64_t k = tile * kF32Tile + lane; k < min(a.N, (tile + 1) * kF32Tile); k += 32) {
+            const float4 p = __ldcg(a.packed + k * a.NQ);
+            v[0] = fminf(v[0], p.x), v[1] = fminf(v[1], p.y), v[2] = fminf(v[2], p.z);
+            v[3] = fmaxf(v[3], p.x), v[4] = fmaxf(v[4], p.y), v[5] = fmaxf(v[5], p.z);
+            v[6] = fmaxf(v[6], __fmul_rn(17.0f, p.w));
+        }
+        for (int o = 16; o > 0; o >>= 1)
+            for (int c = 0; c < 7; c++) {
+                const float w = __shfl_xor_sync(0xffffffffu, v[c], o);
+                v[c] = (c < 3) ? fminf(v[c], w) : fmaxf(v[c], w);
+            }
+        if (lane == 0) {
+            a.tile_box[2 * tile] = make_float4(v[0], v[1], v[2], v[6]);
+            a.tile_box[2 * tile + 1] = make_float4(v[3], v[4], v[5], 0.0f);
+        }
+    }
+}
+
 struct NearArgs {
     const double *tg;
     int64_t M;
@@ -790,19 +978,27 @@ struct NearArgs {
     FinalArgs fin;
 };
 
+// The near field in FP64 accuracy, and the split sums of the far field.  Eight lanes per target: they
+// walk the 27 cells' sources together (nine runs, the cells of a row being neighbours), collect the
+// near ones -- a seventh of them, so evaluating them as they are met would run the pair function for
+// one lane in eight -- in a short list, and share the list's pairs, real kernels in fixed point
+// (pair_fixed.cuh).  Measured against a thread per target with FP64 pairs: see sum_plan_geometry.
+constexpr int kNearThreads = 128, kNearLanes = 8, kNearTargets = kNearThreads / kNearLanes, kNearList = 64;
 template <int KIND, int NF, bool CK>
-__global__ void __launch_bounds__(128) near_f64_kernel(NearArgs a) {
+__global__ void __launch_bounds__(kNearThreads) near_f64_kernel(NearArgs a, FxAlpha al) {
     constexpr int OUTW = (NF == 2 || CK) ? 6 : 3;
-    const int64_t kt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;  // processing position
-    if (kt >= a.M) return;
-    const int64_t i = a.tperm ? a.tperm[kt] : kt;
+    __shared__ int list[kNearTargets][kNearList];
+    const int lane = threadIdx.x & 31, l = lane & (kNearLanes - 1), gs = lane & ~(kNearLanes - 1), grp = threadIdx.x / kNearLanes;
+    const int64_t kt = (int64_t)blockIdx.x * kNearTargets + grp;  // processing position
+    const bool live = kt < a.M;
+    const int64_t i = !live ? 0 : a.tperm ? a.tperm[kt] : kt;
     const CellGrid G = *a.grid;
-    const double tx = a.tg[3 * i], ty = a.tg[3 * i + 1], tz = a.tg[3 * i + 2], tz2 = 2.0 * tz;
+    const double tx = a.tg[3 * i], ty = a.tg[3 * i + 1], tz = a.tg[3 * i + 2];
     const float fx = __double2float_rn(tx), fy = __double2float_rn(ty), fz = __double2float_rn(tz);
-    double u[OUTW];
+    double u[OUTW], uf[OUTW];  // uf: fixed-point pairs (the wall's without their factor t)
 #pragma unroll
-    for (int c = 0; c < OUTW; c++) u[c] = 0.0;
-    sum_partials<OUTW>(a.fin.partial, a.fin.S, a.M, kt, u);  // the far field
+    for (int c = 0; c < OUTW; c++) u[c] = uf[c] = 0.0;
+    // the nine runs of candidates: run q is cell row (y, z) = (cy + q % 3 - 1, cz + q / 3 - 1)
     const int cx = cell_coord(tx, G.ox, G.inv_h, G.nx);
     const int cy = cell_coord(ty, G.oy, G.inv_h, G.ny);
     const int cz = cell_coord(tz, G.oz, G.inv_h, G.nz);
@@ -810,28 +1006,125 @@ __global__ void __launch_bounds__(128) near_f64_kernel(NearArgs a) {
     const bool outside = (tx - G.ox) * G.inv_h < -1.0 || (ty - G.oy) * G.inv_h < -1.0 ||
                          (tz - G.oz) * G.inv_h < -1.0 || (tx - G.ox) * G.inv_h > G.nx + 1.0 ||
                          (ty - G.oy) * G.inv_h > G.ny + 1.0 || (tz - G.oz) * G.inv_h > G.nz + 1.0;
-    if (!outside) {
-        for (int z = max(cz - 1, 0); z <= min(cz + 1, G.nz - 1); z++)
-            for (int y = max(cy - 1, 0); y <= min(cy + 1, G.ny - 1); y++)
-                for (int x = max(cx - 1, 0); x <= min(cx + 1, G.nx - 1); x++) {
-                    const int c = (z * G.ny + y) * G.nx + x;
-                    const int b = a.offsets[c], e = a.offsets[c + 1];
-                    for (int k = b; k < e; k++) {
-                        const int j = a.sorted[k];
-                        const float4 p = a.packed[(int64_t)k * a.NQ];  // packed in cell order
-                        const float thr = a.packed[(int64_t)k * a.NQ + 1].w;
-                        const float d0 = sub_rn(fx, p.x), d1 = sub_rn(fy, p.y), d2 = sub_rn(fz, p.z);
-                        if (free_Q_f32(d0, d1, d2, p.w) < thr) {
-                            const double ej = a.eps[j];
-                            double fj[3 * NF];
-                            load_strength<NF>(a.f, j, fj);
-                            pair_f64<KIND, NF, CK>(tx, ty, tz, tz2, a.src[3 * j], a.src[3 * j + 1], a.src[3 * j + 2],
-                                                   ej * ej, fj, a.alpha_re, a.alpha_im, u);
+    int rb[2] = {0, 0}, rn[2] = {0, 0};  // this lane's runs l and 8 + l (only run 8 exists)
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int q = l + kNearLanes * k, y = cy + q % 3 - 1, z = cz + q / 3 - 1;
+        if (q < 9 && live && !outside && y >= 0 && y < G.ny && z >= 0 && z < G.nz) {
+            const int row = (z * G.ny + y) * G.nx;
+            rb[k] = a.offsets[row + max(cx - 1, 0)];
+            rn[k] = a.offsets[row + min(cx + 1, G.nx - 1) + 1] - rb[k];
+        }
+    }
+    // far partials, each lane every eighth split
+    if (live)
+        for (int s = l; s < a.fin.S; s += kNearLanes) {
+            const double *p = a.fin.partial + ((int64_t)s * a.M + kt) * OUTW;
+#pragma unroll
+            for (int c = 0; c < OUTW; c++) u[c] += p[c];
+        }
+    int start[9], first[9], total = 0;
+#pragma unroll
+    for (int q = 0; q < 9; q++) {
+        start[q] = __shfl_sync(0xffffffffu, rb[q / kNearLanes], gs + q % kNearLanes);
+        first[q] = total;
+        total += __shfl_sync(0xffffffffu, rn[q / kNearLanes], gs + q % kNearLanes);
+    }
+    const int rounds = (int)(__reduce_max_sync(0xffffffffu, (unsigned)total) + kNearLanes - 1) / kNearLanes;
+    FxAcc<3 * NF> acc;
+    if constexpr (!CK) acc.init();
+    int terms = 0, cnt = 0;
+    auto evaluate = [&]() {
+        for (int q = l; q < cnt; q += kNearLanes) {
+            const int64_t j = a.sorted[list[grp][q]];
+            const double sx = a.src[3 * j], sy = a.src[3 * j + 1], sz = a.src[3 * j + 2], e = fabs(a.eps[j]);
+            double fj[3 * NF];
+            load_strength<NF>(a.f, j, fj);
+            if constexpr (!CK) {
+                const double d0 = tx - sx, d1 = ty - sy, d2 = tz - sz, e2 = e * e;
+                double fh[3 * NF];
+#pragma unroll
+                for (int c = 0; c < 3 * NF; c++) fh[c] = KIND == FLG_WALL ? fj[c] * sz : fj[c];
+                q60 F[3 * NF], t[3];
+                const int ef = fx_strength(fh, 3 * NF, F);
+                bool done = false;
+                if constexpr (KIND == FLG_WALL) {
+                    const double dp = tz + sz;
+                    const double rq = fma(d1, d1, fma(d0, d0, e2)), QF = fma(d2, d2, rq), QI = fma(dp, dp, rq);
+                    if (q_in_range(QF) && q_in_range(QI) && ef < kFxBad && !(d_neg(tz) ^ d_neg(sz))) {
+                        const FxWall w = fx_wall(d0, d1, d2, dp, QF, QI, e);
+#pragma unroll
+                        for (int c = 0; c < 3 * NF; c += 3) {
+                            const int x = fx_wall_apply(w, F + c, t) + ef;
+                            acc.scale(x);
+                            acc.add(c, t, x);
                         }
+                        done = true;
+                    }
+                } else {
+                    const double Q = fma(d2, d2, fma(d1, d1, fma(d0, d0, e2)));
+                    if (q_in_range(Q) && ef < kFxBad) {
+                        const FxDir g = fx_dir(d0, d1, d2, Q, e);
+                        const FxRadial r = KIND == FLG_STOKESLET ? fx_stokeslet(g) : fx_brinkman(g, al);
+                        acc.scale(r.x + ef);
+#pragma unroll
+                        for (int c = 0; c < 3 * NF; c += 3) {
+                            fx_radial_apply(g, r, F + c, t);
+                            acc.add(c, t, r.x + ef);
+                        }
+                        done = true;
                     }
                 }
+                if (done) {
+                    if (++terms == kFxSeg) {
+#pragma unroll
+                        for (int c = 0; c < 3 * NF; c++) uf[c] += acc.value(c);
+                        acc.clear();
+                        terms = 0;
+                    }
+                    continue;
+                }
+            }
+            pair_f64<KIND, NF, CK>(tx, ty, tz, 2.0 * tz, sx, sy, sz, e * e, fj, a.alpha_re, a.alpha_im, u);
+        }
+    };
+    for (int r = 0; r < rounds; r++) {
+        const int f = r * kNearLanes + l;
+        bool near = false;
+        int k = 0;
+        if (f < total) {
+#pragma unroll
+            for (int q = 0; q < 9; q++) k = f >= first[q] ? start[q] + f - first[q] : k;
+            const float4 p = a.packed[(int64_t)k * a.NQ];  // packed in cell order
+            const float thr = a.packed[(int64_t)k * a.NQ + 1].w;
+            const float d0 = sub_rn(fx, p.x), d1 = sub_rn(fy, p.y), d2 = sub_rn(fz, p.z);
+            near = free_Q_f32(d0, d1, d2, p.w) < thr;
+        }
+        const unsigned m = (__ballot_sync(0xffffffffu, near) >> gs) & ((1u << kNearLanes) - 1);
+        if (near) list[grp][cnt + __popc(m & ((1u << l) - 1))] = k;
+        cnt += __popc(m);
+        if (__any_sync(0xffffffffu, cnt > kNearList - kNearLanes)) {
+            __syncwarp();
+            evaluate();
+            __syncwarp();
+            cnt = 0;
+        }
     }
-    final_store(a.fin, i, u);
+    __syncwarp();
+    evaluate();
+    __syncwarp();
+    if constexpr (!CK) {
+#pragma unroll
+        for (int c = 0; c < 3 * NF; c++) {
+            uf[c] += acc.value(c);
+            u[c] += KIND == FLG_WALL ? tz * uf[c] : uf[c];
+        }
+    }
+#pragma unroll
+    for (int o = 1; o < kNearLanes; o <<= 1)
+#pragma unroll
+        for (int c = 0; c < OUTW; c++) u[c] += __shfl_xor_sync(0xffffffffu, u[c], o);
+    if (live && l == 0) final_store(a.fin, i, u);
 }
 
 // ---------------------------------------------------------------------------
@@ -902,12 +1195,13 @@ static void carve_plan(A &ar, int64_t M, int64_t N, const SumLayout &L, int prec
         p->packed = ar.template take<float4>((size_t)N * L.NQ);
         p->tile_box = ar.template take<float4>(2 * (size_t)ceil_div(std::max<int64_t>(N, 1), kF32Tile));
         p->grid = ar.template take<CellGrid>(1);
-        p->bounds = ar.template take<double>(kBoundBlocks * 7);
+        p->bounds = ar.template take<long long>(kBoundBlocks * 7);
         p->cell_of = ar.template take<int>(N);
         p->counts = ar.template take<int>(kMaxCells);
         p->offsets = ar.template take<int>(kMaxCells + 1);
         p->block_sums = ar.template take<int>(kMaxCells / kScanBlock + 1);
         p->sorted = ar.template take<int>(N);
+        p->slots = ar.template take<int>(N <= kClusterPlanMax ? N : 0);
         p->tcell = p->toffsets = p->tperm = nullptr;
         if (M >= kSortTargetsMin) {
             p->tcell = ar.template take<int>(M);
@@ -931,7 +1225,7 @@ int sum_plan_carve(void *work, size_t work_bytes, int64_t M, int64_t N, const Su
     if (M == 0 || N == 0) return FLG_OK;
     Arena ar(work, work_bytes);
     carve_plan(ar, M, N, L, precision, p);
-    const bool ok = p->partial != nullptr && (precision != FLG_PREC_MIXED || p->sorted != nullptr) &&
+    const bool ok = p->partial != nullptr && (precision != FLG_PREC_MIXED || p->slots != nullptr) &&
                     (precision != FLG_PREC_MIXED || M < kSortTargetsMin || p->tperm != nullptr);
     FLG_REQUIRE(ok, "workspace too small: %zu bytes given, %zu needed", work_bytes,
                 sum_workspace_bytes(0, M, N, L.nf, L.ck, precision));
@@ -940,13 +1234,39 @@ int sum_plan_carve(void *work, size_t work_bytes, int64_t M, int64_t N, const Su
 
 // Geometry part of the mixed plan (sources and eps only): packed FP32
 // coordinates and the sorted cell list.  Reusable while the sources stay put.
-int sum_plan_geometry(const double *src, const double *eps, int64_t N, const SumLayout &L, SumPlan *p,
-                      cudaStream_t st) {
+// f (optional): the strengths of the first sum, packed along where that costs no launch; *packed_f
+// tells whether they were.
+int sum_plan_geometry(int kind, const double *src, const double *eps, int64_t N, const double *f, const SumLayout &L,
+                      SumPlan *p, cudaStream_t st, bool *packed_f) {
+    *packed_f = false;
     if (N == 0) return FLG_OK;
+    if (N <= kClusterPlanMax) {
+        PlanArgs a{src, eps, f, N, L.NQ, kind == FLG_WALL ? 1 : 0, p->bounds, p->grid, p->cell_of, p->counts, p->offsets,
+                   p->block_sums, p->slots, p->sorted, p->packed, p->tile_box};
+        static bool attr_set = false;
+        if (!attr_set) {
+            FLG_CUDA(cudaFuncSetAttribute(plan_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            attr_set = true;
+        }
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kPlanCtas);
+        cfg.blockDim = dim3(kPlanThreads);
+        cfg.stream = st;
+        cudaLaunchAttribute at[1] = {};
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kPlanCtas;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        FLG_CUDA(cudaLaunchKernelEx(&cfg, plan_cluster_kernel, a));
+        count_launch();
+        *packed_f = f != nullptr;
+        return FLG_OK;
+    }
     const int tb = 256;
     cell_bounds_kernel<<<kBoundBlocks, 256, 0, st>>>(src, eps, N, p->bounds);
     FLG_LAUNCH_CHECK();
-    cell_setup_kernel<<<1, 32, 0, st>>>(p->bounds, kBoundBlocks, p->grid);
+    cell_setup_kernel<<<1, kBoundBlocks, 0, st>>>(p->bounds, p->grid);
     FLG_LAUNCH_CHECK();
     FLG_CUDA(cudaMemsetAsync(p->counts, 0, sizeof(int) * kMaxCells, st));
     cell_count_kernel<<<(unsigned)ceil_div(N, tb), tb, 0, st>>>(src, N, p->grid, p->cell_of, p->counts);
@@ -1030,9 +1350,11 @@ static int launch_sum(const SumRun &r, const SumLayout &L, int precision, const 
         return FLG_OK;
     }
     // mixed: strengths into the packed slots, FP32 far field, FP64 near field + combine
-    pack_strengths_kernel<<<(unsigned)ceil_div(r.N, 256), 256, 0, st>>>(r.f, KIND == FLG_WALL ? r.src : nullptr,
-                                                                       p->sorted, r.N, NF, p->packed);
-    FLG_LAUNCH_CHECK();
+    if (!r.packed_f) {
+        pack_strengths_kernel<<<(unsigned)ceil_div(r.N, 256), 256, 0, st>>>(r.f, KIND == FLG_WALL ? r.src : nullptr,
+                                                                           p->sorted, r.N, NF, p->packed);
+        FLG_LAUNCH_CHECK();
+    }
     // targets in cell order: the sources' own order when the targets are the sources, a
     // bucket sort for other large target sets, the given order for small ones
     const int *tperm = nullptr;
@@ -1053,7 +1375,9 @@ static int launch_sum(const SumRun &r, const SumLayout &L, int precision, const 
     NearArgs na{r.tg, r.M, tperm, r.src, r.eps, r.f, r.N, p->packed, L.NQ, p->grid, p->offsets, p->sorted,
                 r.alpha_re, r.alpha_im, fin};
     prof_begin(FLG_SLOT_NEAR_F64, st);
-    near_f64_kernel<KIND, NF, CK><<<(unsigned)ceil_div(r.M, 128), 128, 0, st>>>(na);
+    FxAlpha al{};
+    if (KIND == FLG_BRINKMANLET && !CK) al = fx_alpha(r.alpha_re);
+    near_f64_kernel<KIND, NF, CK><<<(unsigned)ceil_div(r.M, kNearTargets), kNearThreads, 0, st>>>(na, al);
     FLG_LAUNCH_CHECK();
     prof_end(FLG_SLOT_NEAR_F64, st);
     return FLG_OK;
@@ -1124,8 +1448,11 @@ extern "C" int flg_evaluate(int kind, double alpha_re, double alpha_im, const do
     SumPlan p{};
     FLG_TRY(sum_plan_carve(work, work_bytes, M, N, L, precision, &p));
     cudaStream_t st = as_stream(stream);
-    if (precision == FLG_PREC_MIXED && M > 0 && N > 0) FLG_TRY(sum_plan_geometry(sources, eps, N, L, &p, st));
+    bool packed_f = false;
+    if (precision == FLG_PREC_MIXED && M > 0 && N > 0)
+        FLG_TRY(sum_plan_geometry(kind, sources, eps, N, strengths, L, &p, st, &packed_f));
     SumRun r{};
+    r.packed_f = packed_f;
     r.kind = kind;
     r.tg = targets;
     r.M = M;

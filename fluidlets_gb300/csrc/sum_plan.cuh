@@ -27,8 +27,9 @@ struct SumPlan {
     float4 *packed;   // [N][NQ] FP32 sources in cell order (mixed only)
     float4 *tile_box; // [ceil(N / 256)][2]: lo x, y, z, max threshold | hi x, y, z
     CellGrid *grid;
-    double *bounds;
+    long long *bounds;  // the boxes of the blocks of cell_bounds_kernel
     int *cell_of, *counts, *offsets, *block_sums, *sorted;
+    int *slots;  // scratch of the one-launch plan (small source sets)
     int *tcell, *toffsets, *tperm;  // targets bucketed by source cell (large target sets)
 };
 
@@ -41,6 +42,7 @@ struct SumRun {
     double alpha_re, alpha_im, mu_re, mu_im;
     double *out;
     int out_complex;
+    bool packed_f;  // the plan already holds the strengths f
 };
 
 int check_kernel_args(int kind, double alpha_re, double alpha_im);
@@ -48,8 +50,8 @@ void sum_layout(int kind, int64_t M, int64_t N, int nf, bool ck, int precision, 
 size_t sum_workspace_bytes(int kind, int64_t M, int64_t N, int nf, bool ck, int precision);
 int sum_plan_carve(void *work, size_t work_bytes, int64_t M, int64_t N, const SumLayout &L, int precision,
                    SumPlan *p);
-int sum_plan_geometry(const double *src, const double *eps, int64_t N, const SumLayout &L, SumPlan *p,
-                      cudaStream_t st);
+int sum_plan_geometry(int kind, const double *src, const double *eps, int64_t N, const double *f, const SumLayout &L,
+                      SumPlan *p, cudaStream_t st, bool *packed_f);
 int sum_run(const SumRun &r, const SumLayout &L, int precision, const SumPlan *p, cudaStream_t st);
 
 }  // namespace flg

@@ -156,3 +156,28 @@ def test_matrix_on_and_below_the_wall():
     K, ref = fl.assemble(fl.WallStokeslet3D(), X, Y, 0.05), O.assemble("wall", X, Y, 0.05)
     assert np.all(K[:12] == 0.0)
     assert np.abs(K - ref).max() <= 1e-13 * np.abs(ref).max()
+
+
+# ---- the mixed sum's plan and near field ------------------------------------------------------------
+@pytest.mark.parametrize("n", [1, 5, 255, 257, 1024, 16385, 65536, 65537])
+@pytest.mark.parametrize("kernel", [fl.Stokeslet3D(), fl.WallStokeslet3D(), fl.Brinkmanlet3D(2.5),
+                                    fl.Brinkmanlet3D(1 + 2j)], ids=["stokeslet", "wall", "alpha2.5", "complex"])
+def test_mixed_sum_of_source_counts(kernel, n):
+    """Both plans (one launch up to 65,536 sources), ragged tiles; uneven blob widths, a cluster of
+    sources in one cell, targets far outside the box."""
+    rng = np.random.default_rng(n)
+    m = 333
+    X, Y = points(rng, m, n)
+    X[:40] = Y[rng.integers(0, n, 40)]
+    X[40:50] = [50.0, -30.0, 40.0]
+    Y[: n // 50] = Y[0] + 1e-3 * rng.normal(size=(n // 50, 3))
+    Y[:, 2] = np.abs(Y[:, 2]) + 1e-3
+    e = 0.4 * (8.0 / max(n, 8)) ** (1 / 3) * rng.uniform(0.3, 1.0, n)
+    F = rng.normal(size=(n, 3)) + (1j * rng.normal(size=(n, 3)) if n % 2 else 0)
+    u, ref = fl.evaluate(kernel, X, Y, F, e, precision="mixed"), fl.evaluate(kernel, X, Y, F, e)
+    assert np.linalg.norm(u - ref) <= 2e-6 * np.linalg.norm(ref)
+    # where every source is near a target the mixed sum is the FP64 one
+    if n <= 257:
+        big = np.full(n, 60.0)
+        u, ref = (fl.evaluate(kernel, X, Y, F, big, precision=p) for p in ("mixed", "fp64"))
+        assert np.linalg.norm(u - ref) <= 1e-13 * np.linalg.norm(ref)
