@@ -557,372 +557,374 @@ __global__ void trsv_update_kernel(const double *LU, int64_t ld, double *B, int6
 }
 
 // ---- low precision (FP32) no-pivot LU ----------------------------------------------
-// One CTA (16 warps) factors the nb x nb diagonal block (nb <= 128, padded with
-// the identity to 128) in shared memory, in 32 x 32 sub-blocks, and builds the
-// inverses of its L and U factors alongside (they precondition the panels and
-// the solves).  With X = inv(L) and Y = inv(U) started at zero, step s:
-//   warp 0:  D[s][s] = L_ss U_ss (lane = row, the pivot row broadcast by warp
-//            shuffles); the same sweep solves Y[s][s] U_ss = I row by row with
-//            the broadcast pivot rows, and publishes each column of L_ss;
-//   warp 4:  X[s][s] = inv(L_ss) column by column (lane = column), following
-//            warp 0's published columns (bounded waits);
-//   stage 1: U panel D[s][t] = X[s][s] D[s][t], L panel D[t][s] = D[t][s] Y[s][s]
-//            (t > s); X[s][q] = X[s][s] X[s][q], Y[q][s] = Y[q][s] Y[s][s] (q < s);
-//   stage 2: D[t][u] -= D[t][s] D[s][u] (t, u > s);
-//            X[t][q] -= D[t][s] X[s][q] (t > s, q <= s);
-//            Y[q][u] -= Y[q][s] D[s][u] (q <= s, u > s).
-// Stage 2 looks ahead: warps 0 and 4 update D[s+1][s+1] alone and go on to step
-// s + 1, while the 12 warps of the other three schedulers do the rest of stage 2
-// and store the block row s of D and X and the block column s of Y (no later step
-// changes them).  Warps 0 and 4 share scheduler 0 (warp w issues on scheduler
-// w % 4): the latency-bound 32 x 32 factorization keeps a scheduler without
-// block products.  The block products are bound by shared-memory bandwidth (one
-// 16-byte load per lane per 8 FMA); measured per 128 x 128 block: 38.5 us with
-// the pivot row through shared memory and stage 2 on two schedulers, 36.1 us
-// with shuffles and three (bit-identical results).
-// (X <- inv(L_s) X and Y <- Y inv(U_s) for the block-column / block-row factors
-// L = L_0 L_1 L_2 L_3, U = U_3 U_2 U_1 U_0.)  Every stage-1/2 product is a
-// 32 x 32 x 32 block product split into two warp tasks (16-row or 16-column
-// halves, 4 x 4 outputs per lane, float4 operand loads); the row stride kLD
-// keeps rows 16-byte aligned.
-constexpr int kSB = 32;          // sub-block
-constexpr int kNS = kNB / kSB;   // sub-blocks per side (4)
-constexpr int kLD = kNB + 4;     // shared-memory row stride (floats)
-constexpr size_t kDiagSmem = 3 * (size_t)kNB * kLD * sizeof(float);
-constexpr int kPub = 4;                   // columns of L published per flag update
-constexpr int kLinvWarp = 4;              // the inverse-of-L warp: scheduler 0, beside the LU warp
-constexpr long long kDiagSpin = 1LL << 22;  // bounded wait of warp 1 on warp 0
-
-__device__ __forceinline__ float *sblk(float *M, int i, int j) { return M + i * kSB * kLD + j * kSB; }
-__device__ __forceinline__ const float *sblk(const float *M, int i, int j) { return M + i * kSB * kLD + j * kSB; }
-
 __device__ __forceinline__ float rcp_approx(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 
-__device__ __forceinline__ int ld_volatile_s32(const int *p) { return *(const volatile int *)p; }
-
-// Warp 0: row-per-lane LU of P (pivot row by shuffles from lane j) and, in the same sweep,
-// Y = inv(U) by rows (Y U = I solved left to right with the pivot rows already broadcast);
-// publishes column j of L (multipliers, zero on and above the diagonal) to Lc[j][0..32) for the
-// inverse warp, kPub columns at a time.
-__device__ __forceinline__ void lu32_fused(float *P, float *Yb, float *Lc, int *flag, int flag0, int lane, int row0,
-                                           int nb, int64_t k0, int *info) {
-    float a[kSB], y[kSB];
-#pragma unroll
-    for (int c4 = 0; c4 < kSB; c4 += 4) {
-        const float4 v = *reinterpret_cast<const float4 *>(P + lane * kLD + c4);
-        a[c4] = v.x, a[c4 + 1] = v.y, a[c4 + 2] = v.z, a[c4 + 3] = v.w;
-        y[c4] = y[c4 + 1] = y[c4 + 2] = y[c4 + 3] = 0.0f;
-    }
-    unsigned bad = 0;
-#pragma unroll
-    for (int j = 0; j < kSB; j++) {
-        const float piv = __shfl_sync(0xffffffffu, a[j], j);
-        const bool ok = piv != 0.0f && isfinite(piv);
-        bad |= (ok || row0 + j >= nb) ? 0u : (1u << j);
-        const float rp = ok ? rcp_approx(piv) : 0.0f;
-        // Y row `lane`: y[j] = (delta - sum_{k<j} Y_k U_kj) / U_jj, then the later sums
-        const float yj = (((lane == j) ? 1.0f : 0.0f) - y[j]) * rp;
-        y[j] = yj;
-        const float l = lane > j ? a[j] * rp : 0.0f;
-        if (lane > j) a[j] = l;
-        Lc[j * kSB + lane] = l;
-#pragma unroll
-        for (int c = j + 1; c < kSB; c++) {
-            const float u = __shfl_sync(0xffffffffu, a[c], j);  // pivot row j, column c
-            a[c] = fmaf(-l, u, a[c]);
-            y[c] = fmaf(yj, u, y[c]);
-        }
-        if (j % kPub == kPub - 1) {
-            __syncwarp();
-            if (lane == 0) {
-                __threadfence_block();
-                *(volatile int *)flag = flag0 + j + 1;
-            }
-        }
-    }
-    if (bad && lane == 0) atomicCAS(info, 0, (int)(k0 + row0 + __ffs(bad)));
-#pragma unroll
-    for (int c4 = 0; c4 < kSB; c4 += 4) {
-        *reinterpret_cast<float4 *>(P + lane * kLD + c4) = make_float4(a[c4], a[c4 + 1], a[c4 + 2], a[c4 + 3]);
-        *reinterpret_cast<float4 *>(Yb + lane * kLD + c4) = make_float4(y[c4], y[c4 + 1], y[c4 + 2], y[c4 + 3]);
-    }
+// One CTA factors the nb x nb diagonal block (nb <= 128, padded with the identity) in registers:
+// 16 x 16 threads, thread (ty, tx) holding the elements (ty + 16 i, tx + 16 j), so that the
+// shrinking remainder stays spread over all of them.  Two columns make a step with one barrier: the
+// owners of columns and rows j, j + 1 have put their values into shared memory, every thread reads
+// its eight of each and the 2 x 2 pivot block, eliminates the pair by itself and updates its
+// remainder -- the next pair's columns and rows first, which go to the other buffer before the
+// rest.  (One column a step: 29 us a block, the barrier and two shared-memory round trips each.)  The
+// block's inverses, which only the solves read, are left to block_inverse_kernel.  One CTA per
+// system of a batch: system z = blockIdx.x at A + z sA, flags at info + 2 z.
+constexpr int kLuT = 16, kLuR = kNB / kLuT;  // threads per side, elements per thread and side
+struct Lu128Smem {  // [buffer][column or row of the pair][thread of the other side]
+    float4 c[2][2][kLuT][kLuR / 4], u[2][2][kLuT][kLuR / 4];
+};
+template <int JB>
+__device__ __forceinline__ void put8(float4 *o, const float (&v)[kLuR]) {
+    if (JB < 4) o[0] = make_float4(v[0], v[1], v[2], v[3]);
+    o[1] = make_float4(v[4], v[5], v[6], v[7]);
 }
-
-// Warp 4: X = inv(L) column `lane`, right-looking forward substitution over the published columns
-// of L (waits, bounded, for each group of kPub; on a timeout raises info[1] and stops).
-__device__ __forceinline__ void linv32_follow(const float *Lc, float *Xb, const int *flag, int flag0, int lane,
-                                              int *info) {
-    float x[kSB];
-#pragma unroll
-    for (int i = 0; i < kSB; i++) x[i] = (i == lane) ? 1.0f : 0.0f;
-    bool alive = true;
-#pragma unroll
-    for (int k = 0; k < kSB; k++) {
-        if (k % kPub == 0) {
-            long long it = 0;
-            while (alive && ld_volatile_s32(flag) < flag0 + k + kPub) {
-                if (++it > kDiagSpin) {
-                    if (lane == 0) atomicExch(info + 1, 1);
-                    alive = false;
-                }
-            }
-            __syncwarp();
-            __threadfence_block();
-        }
-#pragma unroll
-        for (int i4 = (k + 1) & ~3; i4 < kSB; i4 += 4) {
-            const float4 v = *reinterpret_cast<const float4 *>(Lc + k * kSB + i4);
-            if (i4 > k) x[i4] = fmaf(-v.x, x[k], x[i4]);
-            if (i4 + 1 > k) x[i4 + 1] = fmaf(-v.y, x[k], x[i4 + 1]);
-            if (i4 + 2 > k) x[i4 + 2] = fmaf(-v.z, x[k], x[i4 + 2]);
-            if (i4 + 3 > k) x[i4 + 3] = fmaf(-v.w, x[k], x[i4 + 3]);
-        }
+template <int JB>
+__device__ __forceinline__ void get8(const float4 *o, float (&v)[kLuR]) {
+    if (JB < 4) {
+        const float4 a = o[0];
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
     }
-#pragma unroll
-    for (int i = 0; i < kSB; i++) Xb[i * kLD + lane] = x[i];
+    const float4 b = o[1];
+    v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
 }
-
-// One warp: C (=|-=) A B over k = 32, C of (128 / CG) rows x (4 CG) columns, 4 x 4
-// per lane.  Lane group g = lane / CG owns rows g + G i (G = 32 / CG groups), so the
-// 16-byte A loads of one instruction fall in distinct bank groups (row stride kLD).
-// C may alias A when CG = 8 (row halves read only their own rows of A) or B when
-// CG = 4 (column halves read only their own columns of B): all operands are read
-// before the first store.
-template <int CG, bool SUB>
-__device__ __forceinline__ void warp_mm(const float *A, const float *B, float *C, int lane) {
-    constexpr int G = 32 / CG;
-    const int g = lane / CG, c0 = (lane % CG) * 4;
-    float acc[4][4];
+template <int JB>
+__device__ __forceinline__ void lu128_stage(float (&a)[kLuR][kLuR], Lu128Smem &S, int ty, int tx, int nb, int64_t k0,
+                                            int *info) {
+    // (the first pair of the stage; the later ones are published inside the loop)
+    auto publish = [&](int jp, int b) {
+        if (tx >> 1 == jp) {
+            float v[kLuR];
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        if (SUB) {
-            const float4 v = *reinterpret_cast<const float4 *>(C + (g + G * i) * kLD + c0);
-            acc[i][0] = v.x, acc[i][1] = v.y, acc[i][2] = v.z, acc[i][3] = v.w;
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
+            for (int i = 0; i < kLuR; i++) v[i] = a[i][JB];
+            put8<JB>(S.c[b][tx & 1][ty], v);
         }
-    }
-#pragma unroll 2
-    for (int k = 0; k < kSB; k += 4) {
-        float a[4][4], b[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const float4 v = *reinterpret_cast<const float4 *>(A + (g + G * i) * kLD + k);
-            a[i][0] = SUB ? -v.x : v.x, a[i][1] = SUB ? -v.y : v.y, a[i][2] = SUB ? -v.z : v.z,
-            a[i][3] = SUB ? -v.w : v.w;
-            const float4 w = *reinterpret_cast<const float4 *>(B + (k + i) * kLD + c0);
-            b[i][0] = w.x, b[i][1] = w.y, b[i][2] = w.z, b[i][3] = w.w;
-        }
-#pragma unroll
-        for (int kk = 0; kk < 4; kk++)
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i][kk], b[kk][j], acc[i][j]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-        *reinterpret_cast<float4 *>(C + (g + G * i) * kLD + c0) =
-            make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-    __syncwarp();
-}
-
-// store the finished parts of step s: rows [32s, 32s + 32) of the factored block and of inv(L),
-// columns [32s, 32s + 32) of inv(U) (and the same rows of its transpose); threads t0 .. t0 + nt
-__device__ __forceinline__ void diag_store_step(int s, const float *D, const float *X, const float *Y, float *A,
-                                                int64_t ld, int64_t k0, int nb, bool v4, float *Linv, float *Uinv,
-                                                float *UinvT, int t, int nt) {
-    const int r0 = s * kSB;
-    for (int e = t; e < kSB * kNB / 4; e += nt) {  // 32 rows x 32 float4
-        const int r = r0 + (e >> 5), c4 = (e & 31) * 4;
-        const float4 d = *reinterpret_cast<const float4 *>(D + r * kLD + c4);
-        if (v4) {
-            *reinterpret_cast<float4 *>(A + (k0 + r) * ld + k0 + c4) = d;
-        } else if (r < nb) {
-            const float w[4] = {d.x, d.y, d.z, d.w};
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (c4 + q < nb) A[(k0 + r) * ld + k0 + c4 + q] = w[q];
-        }
-        *reinterpret_cast<float4 *>(Linv + r * kNB + c4) = *reinterpret_cast<const float4 *>(X + r * kLD + c4);
-    }
-    for (int e = t; e < kNB * kSB / 4; e += nt) {  // 128 rows x 8 float4 of column block s
-        const int r = e >> 3, c4 = r0 + (e & 7) * 4;
-        *reinterpret_cast<float4 *>(Uinv + r * kNB + c4) = *reinterpret_cast<const float4 *>(Y + r * kLD + c4);
-    }
-    if (UinvT)
-        for (int e = t; e < kSB * kNB; e += nt) {  // rows r0 .. r0 + 32 of the transpose
-            const int c = r0 + (e >> 7), r = e & (kNB - 1);
-            UinvT[c * kNB + r] = Y[r * kLD + c];
-        }
-}
-
-// One CTA per system of a batch: system z = blockIdx.x at A + z sA, Linv / Uinv + z sD,
-// UinvT + z sT, its flags at info + 2 z.
-__global__ void __launch_bounds__(512) diag_lowp_kernel(float *A, int64_t ld, int64_t k0, int nb, float *Linv,
-                                                        float *Uinv, float *UinvT, int *info, int64_t sA, int64_t sD,
-                                                        int64_t sT) {
-    extern __shared__ __align__(16) float sm[];
-    {
-        const int64_t z = blockIdx.x;
-        A += z * sA, Linv += z * sD, Uinv += z * sD, info += 2 * z;
-        if (UinvT) UinvT += z * sT;
-    }
-    float *D = sm, *X = sm + kNB * kLD, *Y = sm + 2 * kNB * kLD;
-    __shared__ __align__(16) float Lc[kSB * kSB];
-    __shared__ int flag;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nthr = blockDim.x, nwarp = nthr >> 5;
-    if (tid == 0) flag = 0;
-    const bool v4 = nb == kNB && (((uintptr_t)(A + k0 * ld + k0)) & 15) == 0;
-    {
-        const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 buf[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int e = tid + u * 512, r = e >> 5, c4 = (e & 31) * 4;
-            if (v4) {
-                buf[u] = __ldg(reinterpret_cast<const float4 *>(A + (k0 + r) * ld + k0 + c4));
-            } else {
-                float w[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int c = c4 + q;
-                    w[q] = (r < nb && c < nb) ? A[(k0 + r) * ld + k0 + c] : (r == c ? 1.0f : 0.0f);
-                }
-                buf[u] = make_float4(w[0], w[1], w[2], w[3]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int e = tid + u * 512, r = e >> 5, c4 = (e & 31) * 4;
-            *reinterpret_cast<float4 *>(D + r * kLD + c4) = buf[u];
-            *reinterpret_cast<float4 *>(X + r * kLD + c4) = z4;
-            *reinterpret_cast<float4 *>(Y + r * kLD + c4) = z4;
-        }
-    }
+        if (ty >> 1 == jp) put8<JB>(S.u[b][ty & 1][tx], a[JB]);
+    };
+    publish(0, 0);
     __syncthreads();
-    for (int s = 0; s < kNS; s++) {
-        const int m = kNS - 1 - s;
-        // factor D[s][s] (warp 0) and invert L_ss (warp kLinvWarp); the other warps finish stage 2 of s - 1
-        if (warp == 0) lu32_fused(sblk(D, s, s), sblk(Y, s, s), Lc, &flag, s * kSB, lane, s * kSB, nb, k0, info);
-        else if (warp == kLinvWarp) linv32_follow(Lc, sblk(X, s, s), &flag, s * kSB, lane, info);
-        __syncthreads();
-        for (int t = warp; t < 2 * (2 * m + 2 * s); t += nwarp) {
-            const int b = t >> 1, h = (t & 1) * 16;
-            if (b < m) {
-                float *C = sblk(D, s, s + 1 + b) + h;
-                warp_mm<4, false>(sblk(X, s, s), C, C, lane);
-            } else if (b < 2 * m) {
-                float *C = sblk(D, s + 1 + (b - m), s) + h * kLD;
-                warp_mm<8, false>(C, sblk(Y, s, s), C, lane);
-            } else if (b < 2 * m + s) {
-                float *C = sblk(X, s, b - 2 * m) + h;
-                warp_mm<4, false>(sblk(X, s, s), C, C, lane);
-            } else {
-                float *C = sblk(Y, b - 2 * m - s, s) + h * kLD;
-                warp_mm<8, false>(C, sblk(Y, s, s), C, lane);
-            }
+#pragma unroll 1
+    for (int jp = 0; jp < kLuT / 2; jp++) {
+        const int buf = jp & 1, jj = 2 * jp;
+        auto pivot = [&](int col, int row) { return reinterpret_cast<const float *>(S.c[buf][col][row])[JB]; };
+        const float p00 = pivot(0, jj), p10 = pivot(0, jj + 1), p01 = pivot(1, jj), p11 = pivot(1, jj + 1);
+        float l0[kLuR], l1[kLuR], u0[kLuR], u1[kLuR];
+        get8<JB>(S.c[buf][0][ty], l0);
+        get8<JB>(S.c[buf][1][ty], l1);
+        get8<JB>(S.u[buf][0][tx], u0);
+        get8<JB>(S.u[buf][1][tx], u1);
+        const bool ok0 = p00 != 0.0f && isfinite(p00);
+        const float r0 = ok0 ? rcp_approx(p00) : 0.0f, lp = p10 * r0, q11 = fmaf(-lp, p01, p11);
+        const bool ok1 = q11 != 0.0f && isfinite(q11);
+        const float r1 = ok1 ? rcp_approx(q11) : 0.0f;
+        if (!(ok0 && ok1) && threadIdx.x == 0) {
+            const int bad = JB * kLuT + jj + (ok0 ? 1 : 0);
+            if (bad < nb) atomicCAS(info, 0, (int)(k0 + bad + 1));
         }
-        __syncthreads();
-        if (m == 0) break;
-        if (warp == 0 || warp == kLinvWarp) {
-            // look-ahead: the block the next factorization needs, D[s+1][s+1] -= D[s+1][s] D[s][s+1]
-            // (a 16-row half each), then on to step s + 1 while the other warps finish stage 2
-            const int h = warp == 0 ? 0 : 16;
-            warp_mm<8, true>(sblk(D, s + 1, s) + h * kLD, sblk(D, s, s + 1), sblk(D, s + 1, s + 1) + h * kLD, lane);
-            asm volatile("bar.sync 1, 64;" ::: "memory");
-        } else if ((warp & 3) != 0) {
-            // the rest of stage 2 (m^2 - 1 blocks of D, m (s + 1) of X and of Y), then the stores of
-            // step s, on the 12 warps of the three schedulers that warps 0 and kLinvWarp do not use
-            const int w12 = (warp >> 2) * 3 + (warp & 3) - 1;
-            const int nD = m * m - 1, nX = m * (s + 1);
-            for (int t = w12; t < 2 * (nD + 2 * nX); t += 12) {
-                const int b = t >> 1, h = (t & 1) * 16;
-                if (b < nD) {
-                    const int i = (b + 1) / m, j = (b + 1) - ((b + 1) / m) * m;
-                    warp_mm<8, true>(sblk(D, s + 1 + i, s) + h * kLD, sblk(D, s, s + 1 + j),
-                                     sblk(D, s + 1 + i, s + 1 + j) + h * kLD, lane);
-                } else if (b < nD + nX) {
-                    const int i = (b - nD) / (s + 1), q = (b - nD) % (s + 1);
-                    warp_mm<8, true>(sblk(D, s + 1 + i, s) + h * kLD, sblk(X, s, q), sblk(X, s + 1 + i, q) + h * kLD,
-                                     lane);
-                } else {
-                    const int q = (b - nD - nX) / m, j = (b - nD - nX) % m;
-                    warp_mm<8, true>(sblk(Y, q, s) + h * kLD, sblk(D, s, s + 1 + j), sblk(Y, q, s + 1 + j) + h * kLD,
-                                     lane);
-                }
-            }
-            diag_store_step(s, D, X, Y, A, ld, k0, nb, v4, Linv, Uinv, UinvT, w12 * 32 + lane, 12 * 32);
+        // l0, l1: the multipliers of this thread's rows; u1: row j + 1 after row j's elimination.  Rows and
+        // columns up to a pivot take no update from it.
+#pragma unroll
+        for (int i = JB; i < kLuR; i++) {
+            l0[i] *= r0;
+            l1[i] = fmaf(-l0[i], p01, l1[i]) * r1;
+            u1[i] = fmaf(-lp, u0[i], u1[i]);
         }
+        const float m0 = l0[JB], m1 = l1[JB];
+        l0[JB] = ty > jj ? m0 : 0.0f, l1[JB] = ty > jj + 1 ? m1 : 0.0f;
+        u0[JB] = tx > jj ? u0[JB] : 0.0f, u1[JB] = tx > jj + 1 ? u1[JB] : 0.0f;
+#pragma unroll
+        for (int i = JB; i < kLuR; i++) a[i][JB] = fmaf(-l1[i], u1[JB], fmaf(-l0[i], u0[JB], a[i][JB]));
+#pragma unroll
+        for (int j = JB + 1; j < kLuR; j++) a[JB][j] = fmaf(-l1[JB], u1[j], fmaf(-l0[JB], u0[j], a[JB][j]));
+        if (tx >> 1 == jp) {  // the pair's own columns keep the multipliers
+            const bool second = tx & 1;
+#pragma unroll
+            for (int i = JB; i < kLuR; i++)
+                if (i > JB || ty > tx) a[i][JB] = second ? l1[i] : l0[i];
+        }
+        if (jp + 1 < kLuT / 2) publish(jp + 1, buf ^ 1);
+#pragma unroll
+        for (int i = JB + 1; i < kLuR; i++)
+#pragma unroll
+            for (int j = JB + 1; j < kLuR; j++) a[i][j] = fmaf(-l1[i], u1[j], fmaf(-l0[i], u0[j], a[i][j]));
+        __syncthreads();
     }
-    diag_store_step(kNS - 1, D, X, Y, A, ld, k0, nb, v4, Linv, Uinv, UinvT, tid, nthr);
+    if constexpr (JB + 1 < kLuR) lu128_stage<JB + 1>(a, S, ty, tx, nb, k0, info);
+}
+__global__ void __launch_bounds__(kLuT *kLuT) diag_lowp_kernel(float *A, int64_t ld, int64_t k0, int nb, int *info,
+                                                               int64_t sA) {
+    __shared__ Lu128Smem S;
+    A += blockIdx.x * sA;
+    info += 2 * blockIdx.x;
+    const int tx = threadIdx.x % kLuT, ty = threadIdx.x / kLuT;
+    float a[kLuR][kLuR];
+#pragma unroll
+    for (int i = 0; i < kLuR; i++)
+#pragma unroll
+        for (int j = 0; j < kLuR; j++) {
+            const int r = ty + kLuT * i, c = tx + kLuT * j;
+            a[i][j] = r < nb && c < nb ? A[(k0 + r) * ld + k0 + c] : (r == c ? 1.0f : 0.0f);
+        }
+    lu128_stage<0>(a, S, ty, tx, nb, k0, info);
+#pragma unroll
+    for (int i = 0; i < kLuR; i++)
+#pragma unroll
+        for (int j = 0; j < kLuR; j++) {
+            const int r = ty + kLuT * i, c = tx + kLuT * j;
+            if (r < nb && c < nb) A[(k0 + r) * ld + k0 + c] = a[i][j];
+        }
 }
 
-// Panels of one LU step, in place, in one launch (CTA x < ntu: U tiles, else L tiles):
-//   U12[:, 32-col tile] = Linv (128 x 128) * A12[:, tile]  (all 128 rows per CTA; also
-//                         written transposed into Ut (nr rows of 128, row stride ldu, K-major)
-//                         for the tensor cores)
-//   L21[32-row tile, :] = A21[tile, :] * Uinv (128 x 128)  (all 128 columns per CTA)
-// Each CTA reads its whole input tile before writing it back, so in place is safe.
-__global__ void __launch_bounds__(256) lowp_panel_kernel(float *A, int64_t ld, int64_t k0, int64_t nr,
-                                                         const float *Linv, const float *Uinv, float *Ut, int64_t ldu,
-                                                         int ntu) {
-    __shared__ float tile[kNB][33];  // U: [row][col]; L: stored as [col][row]
-    const int64_t c0 = k0 + kNB;
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    if ((int)blockIdx.x < ntu) {
-        const int64_t j0 = (int64_t)blockIdx.x * 32;
-        const int cols = (int)min((int64_t)32, nr - j0);
-        for (int e = t; e < kNB * 32; e += 256) {
-            const int r = e >> 5, c = e & 31;
-            tile[r][c] = c < cols ? A[(k0 + r) * ld + c0 + j0 + c] : 0.0f;
+// The panels of one LU step, U12 = L11^-1 A12 and L21 = A21 U11^-1, both in one launch: a CTA takes 32
+// columns (or rows) and substitutes in 32-row blocks.  Block b's right-hand side loses its products
+// with the blocks before it (warp w four of the 32 rows, lane = column: 16 FMAs per 8 shared loads),
+// and the 32 x 32 diagonal block's inverse, which four warps work out while the CTA loads its
+// columns, is one more such product: no chain longer than 32.  As products with 128 x 128 inverses
+// the panels took a transpose and two tensor-core launches, and the inverses as long as the diagonal
+// block itself.
+// A CTA that has several groups of columns keeps the block and the inverses; with NC = 2 a lane takes
+// two columns (32 FMAs per 12 loads), which pays once the groups of 32 outnumber the CTAs that fit
+// (two per SM).  Whole factorisation with NC = 2 from 1, 2 or 4 groups a CTA on, or never: n = 9,000
+// (tf32) 4.86, 4.98, 4.99, 5.00 ms; n = 24,576 (bf16) 25.6, 25.8, 26.1, 26.5 ms.
+constexpr int kSb = 32, kPanelThreads = 256;
+template <int NC>
+struct LowpPanelSmem {
+    static constexpr int LD = 32 * NC + 1;  // row stride of the CTA's columns
+    float T[kNB][kNB];              // the diagonal block's factors
+    float inv[kNB / kSb][kSb][kSb];  // inverses of L's (U panel) or U's (L panel) 32 x 32 diagonal blocks
+    float H[kNB][LD];               // right-hand sides, then results: element k of column (row) i
+    float R[kSb][LD];
+};
+struct LowpPanelArgs {
+    float *A;
+    int64_t ld, k0, nr, sA;   // trailing rows and columns k0 + 128 ... (per system)
+    float *Ut;                // K-major copy of U12: column c at Ut + c ldu (null: none)
+    int64_t ldu, sU;
+    __nv_bfloat16 *Lb, *Ub;   // BF16 copies of L21 (row r at Lb + r ldb) and of Ut (null: none)
+    int64_t ldb, sB;
+    int ntu;                  // CTAs of the U panel
+};
+// rows [k0, k0 + nb) of the factored block, padded with the identity
+__device__ __forceinline__ void load_factors(const float *A, int64_t ld, int64_t k0, int nb, float (*T)[kNB]) {
+    if (nb == kNB) {
+        float4 v[kNB * kNB / 4 / kPanelThreads];
+#pragma unroll
+        for (int q = 0; q < kNB * kNB / 4 / kPanelThreads; q++) {
+            const int e = threadIdx.x + q * kPanelThreads, r = e / (kNB / 4), c = e % (kNB / 4) * 4;
+            v[q] = *reinterpret_cast<const float4 *>(A + (k0 + r) * ld + k0 + c);
         }
-        __syncthreads();
-        float acc[16];
 #pragma unroll
-        for (int k = 0; k < 16; k++) acc[k] = 0.0f;
-        for (int q = 0; q < kNB; q++) {
-            const float b = tile[q][lane];
-#pragma unroll
-            for (int k = 0; k < 16; k++) acc[k] = fmaf(Linv[(w + 8 * k) * kNB + q], b, acc[k]);
-        }
-        if (lane < cols) {
-#pragma unroll
-            for (int k = 0; k < 16; k++) {
-                const int r = w + 8 * k;
-                A[(k0 + r) * ld + c0 + j0 + lane] = acc[k];
-                Ut[(j0 + lane) * ldu + r] = acc[k];
-            }
+        for (int q = 0; q < kNB * kNB / 4 / kPanelThreads; q++) {
+            const int e = threadIdx.x + q * kPanelThreads;
+            *reinterpret_cast<float4 *>(&T[e / (kNB / 4)][e % (kNB / 4) * 4]) = v[q];
         }
     } else {
-        const int64_t i0 = (int64_t)(blockIdx.x - ntu) * 32;
-        const int rows = (int)min((int64_t)32, nr - i0);
-        for (int e = t; e < 32 * kNB; e += 256) {
-            const int r = e >> 7, c = e & (kNB - 1);
-            tile[c][r] = r < rows ? A[(c0 + i0 + r) * ld + k0 + c] : 0.0f;
+        for (int e = threadIdx.x; e < kNB * kNB; e += kPanelThreads) {
+            const int r = e / kNB, c = e % kNB;
+            T[r][c] = r < nb && c < nb ? A[(k0 + r) * ld + k0 + c] : (r == c ? 1.0f : 0.0f);
+        }
+    }
+}
+// inverse of the unit-lower (or the upper) 32 x 32 block at T[b0][b0], one warp, lane = column; each
+// unknown is a dot product with the ones before it, in four partial sums
+template <bool LOWER>
+__device__ __forceinline__ void inverse32(const float (*T)[kNB], int b0, float (*out)[kSb], int lane) {
+    float x[kSb];
+#pragma unroll
+    for (int s = 0; s < kSb; s++) {
+        const int r = LOWER ? s : kSb - 1 - s;
+        float acc[4] = {r == lane ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f};
+        const float4 *t = reinterpret_cast<const float4 *>(&T[b0 + r][b0]);
+#pragma unroll
+        for (int q = 0; q < kSb / 4; q++) {
+            if (LOWER ? 4 * q >= r : 4 * q + 3 <= r) continue;
+            const float4 v = t[q];
+            const float w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                if (LOWER ? 4 * q + e < r : 4 * q + e > r) acc[e] = fmaf(-w[e], x[4 * q + e], acc[e]);
+        }
+        x[r] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+        if (!LOWER) x[r] *= 1.0f / T[b0 + r][b0 + r];
+    }
+#pragma unroll
+    for (int r = 0; r < kSb; r++) out[r][lane] = x[r];
+}
+// acc[row][column of this lane] -= (or +=) M (4 rows from r0) . V (K rows), four of K at a time; M row-major
+// from m0, or for the L panel its transpose's rows
+template <bool UPANEL, int NC, int K_UNROLL, int MLD, int VLD>
+__device__ __forceinline__ void panel_product(float (&acc)[4][NC], const float *M, const float *V, int K, float sign,
+                                              int lane) {
+#pragma unroll K_UNROLL
+    for (int k = 0; k < K; k += 4) {
+        float h[4][NC];
+        float4 t[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+#pragma unroll
+            for (int c = 0; c < NC; c++) h[e][c] = sign * V[(k + e) * VLD + lane + 32 * c];
+            t[e] = *reinterpret_cast<const float4 *>(UPANEL ? M + e * MLD + k : M + (k + e) * MLD);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+#pragma unroll
+            for (int c = 0; c < NC; c++) {
+                if (UPANEL) {
+                    acc[e][c] = fmaf(t[e].x, h[0][c], acc[e][c]), acc[e][c] = fmaf(t[e].y, h[1][c], acc[e][c]);
+                    acc[e][c] = fmaf(t[e].z, h[2][c], acc[e][c]), acc[e][c] = fmaf(t[e].w, h[3][c], acc[e][c]);
+                } else {
+                    acc[0][c] = fmaf(t[e].x, h[e][c], acc[0][c]), acc[1][c] = fmaf(t[e].y, h[e][c], acc[1][c]);
+                    acc[2][c] = fmaf(t[e].z, h[e][c], acc[2][c]), acc[3][c] = fmaf(t[e].w, h[e][c], acc[3][c]);
+                }
+            }
+    }
+}
+// the substitution of the CTA's columns in S.H
+template <bool UPANEL, int NC>
+__device__ __forceinline__ void panel_solve(LowpPanelSmem<NC> &S, int warp, int lane) {
+    constexpr int LD = LowpPanelSmem<NC>::LD;
+    for (int b = 0; b < kNB / kSb; b++) {
+        const int r0 = b * kSb + 4 * warp;
+        float acc[4][NC];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int c = 0; c < NC; c++) acc[i][c] = S.H[r0 + i][lane + 32 * c];
+        panel_product<UPANEL, NC, 2, kNB, LD>(acc, UPANEL ? &S.T[r0][0] : &S.T[0][r0], &S.H[0][0], b * kSb, -1.0f, lane);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int c = 0; c < NC; c++) S.R[4 * warp + i][lane + 32 * c] = acc[i][c], acc[i][c] = 0.0f;
+        __syncthreads();
+        panel_product<UPANEL, NC, 8, kSb, LD>(acc, UPANEL ? &S.inv[b][4 * warp][0] : &S.inv[b][0][4 * warp], &S.R[0][0],
+                                              kSb, 1.0f, lane);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int c = 0; c < NC; c++) S.H[r0 + i][lane + 32 * c] = acc[i][c];
+        __syncthreads();
+    }
+}
+// row i of the CTA's results (element k of column / row i), 128 contiguous values, one warp
+template <int NC>
+__device__ __forceinline__ float4 result4(const LowpPanelSmem<NC> &S, int i, int lane) {
+    return make_float4(S.H[4 * lane][i], S.H[4 * lane + 1][i], S.H[4 * lane + 2][i], S.H[4 * lane + 3][i]);
+}
+__device__ __forceinline__ void store_bf16x4(__nv_bfloat16 *o, float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2 *>(o) = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+}
+template <int NC>
+__global__ void __launch_bounds__(kPanelThreads, 3 - NC) lowp_panel_kernel(LowpPanelArgs a) {
+    extern __shared__ __align__(16) uint8_t raw[];
+    LowpPanelSmem<NC> &S = *reinterpret_cast<LowpPanelSmem<NC> *>(raw);
+    constexpr int CW = 32 * NC;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, z = blockIdx.y;
+    float *A = a.A + z * a.sA;
+    const bool up = (int)blockIdx.x < a.ntu;
+    load_factors(A, a.ld, a.k0, kNB, S.T);
+    __syncthreads();
+    if (warp < kNB / kSb) {
+        if (up) inverse32<true>(S.T, warp * kSb, S.inv[warp], lane);
+        else inverse32<false>(S.T, warp * kSb, S.inv[warp], lane);
+    }
+    for (int64_t w0 = (int64_t)(up ? blockIdx.x : blockIdx.x - a.ntu) * CW; w0 < a.nr; w0 += (int64_t)a.ntu * CW) {
+        const int cnt = (int)min((int64_t)CW, a.nr - w0);
+        float *A12 = A + a.k0 * a.ld + a.k0 + kNB + w0, *A21 = A + (a.k0 + kNB + w0) * a.ld + a.k0;
+        if (up) {
+            float v[kNB / 8][NC];
+#pragma unroll
+            for (int q = 0; q < kNB / 8; q++)
+#pragma unroll
+                for (int c = 0; c < NC; c++)
+                    v[q][c] = lane + 32 * c < cnt ? A12[(warp + 8 * q) * a.ld + lane + 32 * c] : 0.0f;
+#pragma unroll
+            for (int q = 0; q < kNB / 8; q++)
+#pragma unroll
+                for (int c = 0; c < NC; c++) S.H[warp + 8 * q][lane + 32 * c] = v[q][c];
+        } else {
+            float4 v[4 * NC];
+#pragma unroll
+            for (int q = 0; q < 4 * NC; q++)
+                v[q] = warp + 8 * q < cnt ? *reinterpret_cast<const float4 *>(A21 + (warp + 8 * q) * a.ld + 4 * lane)
+                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < 4 * NC; q++) {
+                const int i = warp + 8 * q;
+                S.H[4 * lane][i] = v[q].x, S.H[4 * lane + 1][i] = v[q].y;
+                S.H[4 * lane + 2][i] = v[q].z, S.H[4 * lane + 3][i] = v[q].w;
+            }
         }
         __syncthreads();
-        // thread: column c = t % 128, rows r = t / 128 + 2 k
-        const int c = t & (kNB - 1), rb = t >> 7;
-        float acc[16];
+        if (up) panel_solve<true, NC>(S, warp, lane);
+        else panel_solve<false, NC>(S, warp, lane);
+        if (up) {
 #pragma unroll
-        for (int k = 0; k < 16; k++) acc[k] = 0.0f;
-        for (int q = 0; q < kNB; q++) {
-            const float u = Uinv[q * kNB + c];
+            for (int q = 0; q < kNB / 8; q++)
 #pragma unroll
-            for (int k = 0; k < 16; k++) acc[k] = fmaf(tile[q][rb + 2 * k], u, acc[k]);
+                for (int c = 0; c < NC; c++)
+                    if (lane + 32 * c < cnt) A12[(warp + 8 * q) * a.ld + lane + 32 * c] = S.H[warp + 8 * q][lane + 32 * c];
         }
-#pragma unroll
-        for (int k = 0; k < 16; k++) {
-            const int r = rb + 2 * k;
-            if (r < rows) A[(c0 + i0 + r) * ld + k0 + c] = acc[k];
+        for (int i = warp; i < cnt; i += 8) {
+            const float4 v = result4<NC>(S, i, lane);
+            const int64_t r = w0 + i;
+            if (!up) *reinterpret_cast<float4 *>(A21 + i * a.ld + 4 * lane) = v;
+            else if (a.Ut) *reinterpret_cast<float4 *>(a.Ut + z * a.sU + r * a.ldu + 4 * lane) = v;
+            if (a.Lb) store_bf16x4((up ? a.Ub : a.Lb) + z * a.sB + r * a.ldb + 4 * lane, v);
         }
+        __syncthreads();  // every result is out before the next group's columns come in
+    }
+}
+static int lowp_panels(LowpPanelArgs &a, int nbat, cudaStream_t st) {
+    // groups of 32 columns or rows in each panel against two CTAs per SM
+    const int64_t groups = ceil_div(a.nr, 32) * nbat, slots = 2LL * sm_count();
+    static bool attr_set = false;
+    if (!attr_set) {
+        FLG_CUDA(cudaFuncSetAttribute(lowp_panel_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(LowpPanelSmem<1>)));
+        FLG_CUDA(cudaFuncSetAttribute(lowp_panel_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(LowpPanelSmem<2>)));
+        attr_set = true;
+    }
+    if (2 * groups <= slots) {
+        a.ntu = (int)std::min<int64_t>(ceil_div(a.nr, 32), std::max<int64_t>(1, slots / 2 / nbat));
+        lowp_panel_kernel<1><<<dim3(2 * a.ntu, nbat), kPanelThreads, sizeof(LowpPanelSmem<1>), st>>>(a);
+    } else {
+        a.ntu = (int)std::min<int64_t>(ceil_div(a.nr, 64), std::max<int64_t>(1, slots / 4 / nbat));
+        lowp_panel_kernel<2><<<dim3(2 * a.ntu, nbat), kPanelThreads, sizeof(LowpPanelSmem<2>), st>>>(a);
+    }
+    FLG_LAUNCH_CHECK();
+    return FLG_OK;
+}
+
+// The inverses of the diagonal blocks' unit-lower and upper factors (the solves use them), all blocks
+// of all systems in one launch after the factorization: the panels' substitution applied to the
+// identity.  blockIdx = (block and its 32 columns or rows, inverse of L or of U, system)
+__global__ void __launch_bounds__(kPanelThreads, 2) block_inverse_kernel(const float *A, int64_t ld, int64_t n, int64_t sA,
+                                                                         float *Linv, float *Uinv, int64_t sD) {
+    extern __shared__ __align__(16) uint8_t raw[];
+    LowpPanelSmem<1> &S = *reinterpret_cast<LowpPanelSmem<1> *>(raw);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, w0 = (int)(blockIdx.x % 4) * 32;
+    const int64_t k0 = (int64_t)(blockIdx.x / 4) * kNB;
+    const bool up = blockIdx.y == 0;
+    A += blockIdx.z * sA;
+    float *o = (up ? Linv : Uinv) + blockIdx.z * sD + k0 * kNB;
+    load_factors(A, ld, k0, (int)min((int64_t)kNB, n - k0), S.T);
+    for (int k = warp; k < kNB; k += 8) S.H[k][lane] = k == w0 + lane ? 1.0f : 0.0f;
+    __syncthreads();
+    if (warp < kNB / kSb) {
+        if (up) inverse32<true>(S.T, warp * kSb, S.inv[warp], lane);
+        else inverse32<false>(S.T, warp * kSb, S.inv[warp], lane);
+    }
+    __syncthreads();
+    if (up) {
+        panel_solve<true, 1>(S, warp, lane);
+        for (int k = warp; k < kNB; k += 8) o[k * kNB + w0 + lane] = S.H[k][lane];
+    } else {
+        panel_solve<false, 1>(S, warp, lane);
+        for (int i = warp; i < 32; i += 8) reinterpret_cast<float4 *>(o + (w0 + i) * kNB)[lane] = result4<1>(S, i, lane);
     }
 }
 
@@ -970,29 +972,6 @@ __global__ void __launch_bounds__(256) sgemm_kernel(int64_t M, int64_t N, int64_
     }
 }
 
-__global__ void copy2d_f32_kernel(const float *src, int64_t lds, float *dst, int64_t ldd, int64_t rows, int64_t cols) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (int64_t r = blockIdx.y; r < rows; r += gridDim.y)
-        if (c < cols) dst[r * ldd + c] = src[r * lds + c];
-}
-
-// dst (cols x rows, ldd) = src^T (rows x cols, lds); system blockIdx.z at src + z ss, dst + z sd
-__global__ void transpose_f32_kernel(const float *src, int64_t lds, float *dst, int64_t ldd, int64_t rows,
-                                     int64_t cols, int64_t ss, int64_t sd) {
-    __shared__ float t[32][33];
-    src += blockIdx.z * ss, dst += blockIdx.z * sd;
-    const int64_t r0 = (int64_t)blockIdx.y * 32, c0 = (int64_t)blockIdx.x * 32;
-    for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-        const int64_t r = r0 + i, c = c0 + threadIdx.x;
-        t[i][threadIdx.x] = (r < rows && c < cols) ? src[r * lds + c] : 0.0f;
-    }
-    __syncthreads();
-    for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-        const int64_t c = c0 + i, r = r0 + threadIdx.x;
-        if (c < cols && r < rows) dst[c * ldd + r] = t[threadIdx.x][i];
-    }
-}
-
 // tensor-core update (tc_gemm.cu): C (m x nc, ldc) -= Lp (m x K, ldl) * Ut^T (nc x K, ldu), K % 128 == 0,
 // for one system or a batch of them (TcBatch)
 size_t tc_update_bytes(int64_t m, int64_t nc, int64_t K, int mode, int nb = 1);
@@ -1004,39 +983,11 @@ int tc_update_bf16(float *C, int64_t ldc, const void *La, int64_t ldl, const voi
                    int64_t nc, int64_t K, void *work, size_t work_bytes, cudaStream_t st, int *err_dev, int tile,
                    int max_ctas, const TcBatch &bt);
 
-// BF16 copies of one step's finished panels for the BF16 trailing updates: blockIdx.y = 0
-// rounds the L panel (nr rows x 128, row stride lda) into Lb, 1 the K-major U panel (nr rows
-// x 128, row stride ldu) into Ub (row stride ldb); system blockIdx.z at + z (sA, sU, sB).
-__global__ void __launch_bounds__(256) panel_bf16_kernel(const float *L21, int64_t lda, const float *Ut, int64_t ldu,
-                                                         __nv_bfloat16 *Lb, __nv_bfloat16 *Ub, int64_t ldb,
-                                                         int64_t nr, int64_t sA, int64_t sU, int64_t sB) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, r = i >> 5;
-    if (r >= nr) return;
-    const int c4 = (int)(i & 31) * 4;
-    const int64_t z = blockIdx.z;
-    const float *src = blockIdx.y == 0 ? L21 + z * sA + r * lda : Ut + z * sU + r * ldu;
-    __nv_bfloat16 *dst = (blockIdx.y == 0 ? Lb : Ub) + z * sB + r * ldb;
-    const float4 v = *reinterpret_cast<const float4 *>(src + c4);
-    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-    uint2 w;
-    w.x = *reinterpret_cast<uint32_t *>(&lo);
-    w.y = *reinterpret_cast<uint32_t *>(&hi);
-    *reinterpret_cast<uint2 *>(dst + c4) = w;
-}
-
 static int sgemm(cudaStream_t st, int64_t M, int64_t N, int64_t K, float alpha, const float *A, int64_t lda,
                  const float *B, int64_t ldb, float beta, float *C, int64_t ldc) {
     if (M == 0 || N == 0) return FLG_OK;
     dim3 grid((unsigned)ceil_div(N, SG_BN), (unsigned)ceil_div(M, SG_BM));
     sgemm_kernel<<<grid, 256, 0, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
-    FLG_LAUNCH_CHECK();
-    return FLG_OK;
-}
-
-static int copy2d(cudaStream_t st, const float *src, int64_t lds, float *dst, int64_t ldd, int64_t rows, int64_t cols) {
-    if (rows == 0 || cols == 0) return FLG_OK;
-    dim3 grid((unsigned)ceil_div(cols, 256), (unsigned)std::min<int64_t>(rows, 65535));
-    copy2d_f32_kernel<<<grid, 256, 0, st>>>(src, lds, dst, ldd, rows, cols);
     FLG_LAUNCH_CHECK();
     return FLG_OK;
 }
@@ -1632,7 +1583,7 @@ extern "C" int flg_lu_solve_f64(int64_t n, int64_t nrhs, const double *LU, int64
 struct SideStream {
     int dev = -1;
     cudaStream_t s = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr, tail = nullptr, lfork = nullptr, ljoin = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
 };
 constexpr int kSideStreamDevices = 64;
 static int side_stream(SideStream **out) {
@@ -1647,9 +1598,6 @@ static int side_stream(SideStream **out) {
         FLG_CUDA(cudaStreamCreateWithPriority(&ss.s, cudaStreamNonBlocking, hi));
         FLG_CUDA(cudaEventCreateWithFlags(&ss.fork, cudaEventDisableTiming));
         FLG_CUDA(cudaEventCreateWithFlags(&ss.join, cudaEventDisableTiming));
-        FLG_CUDA(cudaEventCreateWithFlags(&ss.tail, cudaEventDisableTiming));
-        FLG_CUDA(cudaEventCreateWithFlags(&ss.lfork, cudaEventDisableTiming));
-        FLG_CUDA(cudaEventCreateWithFlags(&ss.ljoin, cudaEventDisableTiming));
         ss.dev = dev;
     }
     *out = &ss;
@@ -1671,16 +1619,14 @@ extern "C" int64_t flg_lu_lowp_dinv_elems(int64_t n) { return 2 * ceil_div(std::
 // faster from n = 12,288 up and 2% slower at n = 4,608, so 512 below n = 8,192.
 static int64_t outer_width(int64_t n) { return (n >= 8192 ? 8 : 4) * (int64_t)kNB; }
 
-// scratch of nbat systems, system z's at + z * (kNB n, n kNB, n W) floats; BF16 mode: the
-// BF16 copies of the outer panel's L columns and of UtB (n W each per system) in PB
+// scratch of nbat systems, system z's at + z n W floats; BF16 mode: the BF16 copies of the outer
+// panel's L columns and of UtB (n W each per system) in PB
 template <class Ar>
-static void lowp_carve(Ar &ar, int64_t n, int nbat, int mode, float **U12, float **L21, float **UtB, char **tcw,
-                       size_t *tcb, __nv_bfloat16 **PB) {
-    *U12 = ar.template take<float>((size_t)nbat * kNB * n);
-    *L21 = ar.template take<float>((size_t)nbat * n * kNB);
+static void lowp_carve(Ar &ar, int64_t n, int nbat, int mode, float **UtB, char **tcw, size_t *tcb,
+                       __nv_bfloat16 **PB) {
     const int64_t W = outer_width(n);
     *UtB = ar.template take<float>((size_t)nbat * n * W);
-    // the panel products run in TF32 (no operand workspace); the BF16 updates read PB
+    // the updates take their operands as they are (TF32, or PB's BF16 copies): no operand workspace
     *tcb = (mode == FLG_LU_FP32) ? 0 : tc_update_bytes(n, n, W, FLG_LU_TF32, nbat);
     *tcw = ar.template take<char>(*tcb);
     *PB = mode == FLG_LU_BF16 ? ar.template take<__nv_bfloat16>((size_t)2 * nbat * n * W) : nullptr;
@@ -1692,22 +1638,22 @@ static int lu_prec(int mode) { return mode & ~(FLG_LU_TILE_N128 | FLG_LU_TILE_N2
 extern "C" size_t flg_lu_factor_lowp_workspace(int64_t n, int mode) {
     mode = lu_prec(mode);
     CountingArena c;
-    float *a, *b, *d;
+    float *d;
     char *w;
     size_t t;
     __nv_bfloat16 *pb;
-    lowp_carve(c, n, 1, mode, &a, &b, &d, &w, &t, &pb);
+    lowp_carve(c, n, 1, mode, &d, &w, &t, &pb);
     return c.bytes() + 256;  // + the flags of flg_lu_factor_lowp, at the end
 }
 
 extern "C" size_t flg_lu_factor_lowp_batched_workspace(int64_t n, int nbat, int mode) {
     mode = lu_prec(mode);
     CountingArena c;
-    float *a, *b, *d;
+    float *d;
     char *w;
     size_t t;
     __nv_bfloat16 *pb;
-    lowp_carve(c, n, std::max(nbat, 1), mode, &a, &b, &d, &w, &t, &pb);
+    lowp_carve(c, n, std::max(nbat, 1), mode, &d, &w, &t, &pb);
     return c.bytes();
 }
 
@@ -1731,20 +1677,18 @@ static int lowp_factor(int64_t n, int nbat, float *A, int64_t ld, int64_t sA, in
     if (n == 0) return FLG_OK;
     FLG_REQUIRE(A && dinv, "null pointer");
     Arena ar(work, work_bytes);
-    float *U12, *L21, *UtB;
+    float *UtB;
     char *tcw;
     size_t tcb;
     __nv_bfloat16 *PB;
-    lowp_carve(ar, n, nbat, mode, &U12, &L21, &UtB, &tcw, &tcb, &PB);
-    FLG_REQUIRE(U12 && L21 && UtB && (tcb == 0 || tcw) && (mode != FLG_LU_BF16 || PB),
-                "workspace too small for LU (%zu bytes)", work_bytes);
-    // the tensor-core panels use the partial-block scratch: U12 for A12^T, L21 for Uinv^T
-    float *T12 = U12, *UinvT = L21;
+    lowp_carve(ar, n, nbat, mode, &UtB, &tcw, &tcb, &PB);
+    FLG_REQUIRE(UtB && (tcb == 0 || tcw) && (mode != FLG_LU_BF16 || PB), "workspace too small for LU (%zu bytes)",
+                work_bytes);
     int *dinfo = flags;  // [0] first bad pivot, [1] tensor-core wait timed out
     const int64_t W = outer_width(n);  // outer panel width
-    // per-system strides: the matrix, the block inverses, A12^T / Uinv^T scratch, U's K-major copy
-    const int64_t sD = flg_lu_lowp_dinv_elems(n), sT = (int64_t)kNB * n, sUt = n * W;
-    const TcBatch bA{nbat, sA, sA, sUt}, bU{nbat, sUt, sT, sD}, bL{nbat, sA, sA, sT};
+    // per-system strides: the matrix, the block inverses, U's K-major copy
+    const int64_t sD = flg_lu_lowp_dinv_elems(n), sUt = n * W;
+    const TcBatch bA{nbat, sA, sA, sUt};
     // BF16 mode: each step's finished L and U panels are rounded once into LB (row r, column
     // c - K0 of the outer panel at LB + r W + c - K0) and UB (laid out as UtB), and every
     // trailing update of the outer panel reads them
@@ -1760,64 +1704,40 @@ static int lowp_factor(int64_t n, int nbat, float *A, int64_t ld, int64_t sA, in
         }
         return tc_update(C, ld, Lp, ld, Up, W, m, nc, K, mode, tcw, tcb, st, dinfo + 1, false, tile, ctas, bA);
     };
-    const size_t dsmem = kDiagSmem;
     static bool attr_set = false;  // set once, so a later call can be captured in a graph
     if (!attr_set) {
-        FLG_CUDA(cudaFuncSetAttribute(diag_lowp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem));
+        FLG_CUDA(cudaFuncSetAttribute(block_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(LowpPanelSmem<1>)));
         attr_set = true;
     }
     const bool tc = mode != FLG_LU_FP32;
     const int64_t nblk = ceil_div(n, kNB);
-    float *Linv = dinv, *Uinv = dinv + nblk * kNB * kNB;
     SideStream *side = nullptr;
     if (tc) FLG_TRY(side_stream(&side));
     // the persistent updates that run beside the look-ahead diagonal blocks leave them an SM each
     const int cap = std::max(1, sm_count() - nbat);
     auto diag = [&](int64_t d0, cudaStream_t s) {
-        const int64_t kd = d0 / kNB;
-        const int nbd = (int)std::min<int64_t>(kNB, n - d0);
-        const bool tcp = tc && nbd == kNB && n - (d0 + nbd) > 0;  // tensor-core panels follow
         prof_begin(FLG_SLOT_LU_DIAG, s);
-        diag_lowp_kernel<<<nbat, 512, dsmem, s>>>(A, ld, d0, nbd, Linv + kd * kNB * kNB, Uinv + kd * kNB * kNB,
-                                                  tcp ? UinvT : nullptr, dinfo, sA, sD, sT);
+        diag_lowp_kernel<<<nbat, kLuT * kLuT, 0, s>>>(A, ld, d0, (int)std::min<int64_t>(kNB, n - d0), dinfo, sA);
         prof_end(FLG_SLOT_LU_DIAG, s);
     };
     // Look-ahead: once the 128 x 128 block at d0 has its last update (launched on st), the
     // diagonal kernel of that block runs on the side stream while st goes on with the rest of
-    // the trailing update; the next panels wait for it.  Only for a full block with a
-    // trailing part (the block's own panels then run on the tensor cores).
-    bool pending = false, side_busy = false;
-    const dim3 tb(32, 8);
-    // Ut of an inner step back into the row block A12 (U12 row-major, read only by the solves):
-    // off the critical path, after the join on the side stream.  The next panels write other
-    // K slots of UtB and another row block; the next outer panel rewrites UtB only after a
-    // later diagonal kernel on the side stream, so every deferred transpose has run by then.
-    struct Deferred {
-        const float *Ut = nullptr;
-        float *A12 = nullptr;
-        int64_t nr = 0;
-    };
-    auto look_ahead = [&](int64_t d0, Deferred t) -> int {
+    // the trailing update; the next panels wait for it.
+    bool pending = false;
+    auto look_ahead = [&](int64_t d0) -> int {
         FLG_CUDA(cudaEventRecord(side->fork, st));
         FLG_CUDA(cudaStreamWaitEvent(side->s, side->fork, 0));
         diag(d0, side->s);
         FLG_LAUNCH_CHECK();
         FLG_CUDA(cudaEventRecord(side->join, side->s));
-        if (t.Ut) {
-            transpose_f32_kernel<<<dim3(kNB / 32, (unsigned)ceil_div(t.nr, 32), nbat), tb, 0, side->s>>>(
-                t.Ut, W, t.A12, ld, t.nr, kNB, sUt, sA);
-            FLG_LAUNCH_CHECK();
-            side_busy = true;
-        }
         pending = true;
         return FLG_OK;
     };
     for (K0 = 0; K0 < n; K0 += W) {
         const int64_t E = std::min<int64_t>(n, K0 + W);
         for (int64_t k0 = K0; k0 < E; k0 += kNB) {
-            const int64_t k = k0 / kNB;
             const int nb = (int)std::min<int64_t>(kNB, n - k0);
-            const bool tcp = tc && nb == kNB && n - (k0 + nb) > 0;  // tensor-core panels
             if (pending) {  // this block's diagonal kernel ran ahead on the side stream
                 FLG_CUDA(cudaStreamWaitEvent(st, side->join, 0));
                 pending = false;
@@ -1831,58 +1751,19 @@ static int lowp_factor(int64_t n, int nbat, float *A, int64_t ld, int64_t sA, in
             // (nb < kNB only for the last block, which has no trailing part)
             float *A12 = A + k0 * ld + c0, *A21 = A + c0 * ld + k0, *A22 = A + c0 * ld + c0;
             float *Ut = UtB + (c0 - K0) * W + (k0 - K0);  // row: column - K0; K offset: k0 - K0
-            // an inner step whose next diagonal block runs ahead defers its transpose-back
-            const bool defer_t = tcp && E > c0 && n - c0 > kNB;
-            if (tcp) {
-                // panels on the tensor cores (TF32 in both tensor-core modes):
-                //   Ut = A12^T Linv^T (the K-major copy the updates read), then A12 = Ut^T;
-                //   L21 = A21 Uinv, in place (each tile's rows are read in full before they are stored),
-                //   on the side stream beside the U panel (TF32 store mode touches no shared
-                //   workspace); the updates below join it, and the next diagonal kernel, which
-                //   rewrites Uinv^T, follows it on the side stream
-                FLG_CUDA(cudaEventRecord(side->lfork, st));
-                FLG_CUDA(cudaStreamWaitEvent(side->s, side->lfork, 0));
-                FLG_TRY(tc_update(A21, ld, A21, ld, UinvT, kNB, nr, kNB, kNB, FLG_LU_TF32, tcw, tcb, side->s,
-                                  dinfo + 1, true, 0, 0, bL));
-                FLG_CUDA(cudaEventRecord(side->ljoin, side->s));
-                transpose_f32_kernel<<<dim3((unsigned)ceil_div(nr, 32), kNB / 32, nbat), tb, 0, st>>>(
-                    A12, ld, T12, kNB, kNB, nr, sA, sT);
-                FLG_LAUNCH_CHECK();
-                FLG_TRY(tc_update(Ut, W, T12, kNB, Linv + k * kNB * kNB, kNB, nr, kNB, kNB, FLG_LU_TF32, tcw,
-                                  tcb, st, dinfo + 1, true, 0, 0, bU));
-                if (!defer_t) {
-                    transpose_f32_kernel<<<dim3(kNB / 32, (unsigned)ceil_div(nr, 32), nbat), tb, 0, st>>>(
-                        Ut, W, A12, ld, nr, kNB, sUt, sA);
-                    FLG_LAUNCH_CHECK();
-                }
-                FLG_CUDA(cudaStreamWaitEvent(st, side->ljoin, 0));
-                if (mode == FLG_LU_BF16) {  // both panels of this step, rounded once for every update
-                    panel_bf16_kernel<<<dim3((unsigned)ceil_div(nr * 32, 256), 2, nbat), 256, 0, st>>>(
-                        A21, ld, Ut, W, LB + c0 * W + (k0 - K0), UB + (Ut - UtB), W, nr, sA, sUt, n * W);
-                    FLG_LAUNCH_CHECK();
-                }
-            } else if (nb == kNB) {
-                // U12 = Linv A12 (+ its K-major copy), L21 = A21 Uinv: one launch, in place
-                const int ntu = (int)ceil_div(nr, 32), ntl = (int)ceil_div(nr, 32);
-                lowp_panel_kernel<<<ntu + ntl, 256, 0, st>>>(A, ld, k0, nr, Linv + k * kNB * kNB, Uinv + k * kNB * kNB,
-                                                             Ut, W, ntu);
-                FLG_LAUNCH_CHECK();
-            } else {
-                FLG_TRY(sgemm(st, nb, nr, nb, 1.0f, Linv + k * kNB * kNB, kNB, A12, ld, 0.0f, U12, nr));
-                FLG_TRY(copy2d(st, U12, nr, A12, ld, nb, nr));
-                FLG_TRY(sgemm(st, nr, nb, nb, 1.0f, A21, ld, Uinv + k * kNB * kNB, kNB, 0.0f, L21, kNB));
-                FLG_TRY(copy2d(st, L21, kNB, A21, ld, nr, nb));
-            }
+            LowpPanelArgs pa{A, ld, k0, nr, sA, tc ? Ut : nullptr, W, sUt, nullptr, nullptr, W, n * W, 0};
+            if (mode == FLG_LU_BF16) pa.Ut = nullptr, pa.Lb = LB + c0 * W + (k0 - K0), pa.Ub = UB + (Ut - UtB);
+            FLG_TRY(lowp_panels(pa, nbat, st));
             prof_end(FLG_SLOT_LU_PANEL, st);
             prof_begin(FLG_SLOT_LU_UPDATE, st);
-            if (!tc || nb < kNB) {
+            if (!tc) {
                 FLG_TRY(sgemm(st, nr, nr, nb, -1.0f, A21, ld, A12, ld, 1.0f, A22, ld));
             } else if (E > c0) {
                 if (n - c0 > kNB) {
                     // the next diagonal block first, then it factors beside the rest:
                     // rows > c0 + 128 x its columns, rows > k0 x columns (c0 + 128, E)
                     FLG_TRY(upd(A22, A21, Ut, kNB, kNB, kNB, 0));
-                    FLG_TRY(look_ahead(c0, Deferred{Ut, A12, nr}));
+                    FLG_TRY(look_ahead(c0));
                     FLG_TRY(upd(A22 + kNB * ld, A21 + kNB * ld, Ut, nr - kNB, kNB, kNB, cap));
                     if (E > c0 + kNB) FLG_TRY(upd(A22 + kNB, A21, Ut + kNB * W, nr, E - c0 - kNB, kNB, cap));
                 } else {
@@ -1900,7 +1781,7 @@ static int lowp_factor(int64_t n, int nbat, float *A, int64_t ld, int64_t sA, in
             if (n - E > kNB) {
                 // the next outer panel's first diagonal block first, then it factors beside the rest
                 FLG_TRY(upd(C, Lp, Up, kNB, kNB, E - K0, 0));
-                FLG_TRY(look_ahead(E, Deferred{}));
+                FLG_TRY(look_ahead(E));
                 FLG_TRY(upd(C + kNB * ld, Lp + kNB * ld, Up, n - E - kNB, kNB, E - K0, cap));
                 FLG_TRY(upd(C + kNB, Lp, Up + kNB * W, n - E, n - E - kNB, E - K0, cap));
             } else {
@@ -1910,10 +1791,9 @@ static int lowp_factor(int64_t n, int nbat, float *A, int64_t ld, int64_t sA, in
         }
     }
     if (pending) FLG_CUDA(cudaStreamWaitEvent(st, side->join, 0));  // (every look-ahead is joined above)
-    if (side_busy) {  // the deferred transposes
-        FLG_CUDA(cudaEventRecord(side->tail, side->s));
-        FLG_CUDA(cudaStreamWaitEvent(st, side->tail, 0));
-    }
+    block_inverse_kernel<<<dim3((unsigned)(4 * nblk), 2, nbat), kPanelThreads, sizeof(LowpPanelSmem<1>), st>>>(
+        A, ld, n, sA, dinv, dinv + nblk * kNB * kNB, sD);
+    FLG_LAUNCH_CHECK();
     return FLG_OK;
 }
 
