@@ -155,9 +155,8 @@ FLG_HD q60 qmul36(q60 a, int b) {
     const Qf f = qf(a);
     return (((q60)f.h * b) >> 6) + (((q60)f.l * b) >> 36);
 }
-// e^-z = m 2^-n, m in (1/2, 1], for z = zm 2^kz with zm in [1/2, 1), 0 <= kz <= 6
-FLG_HD q60 q_expneg(q60 zm, int kz, int *n) {
-    const q60 v = qmul(qf(zm), qf(1663314137230540311ll));  // zm log2(e), in (0.7, 1.45)
+// 2^-(v 2^kz) = m 2^-n, m in (1/2, 1], for v in [0, 1.45), 0 <= kz <= 7
+FLG_HD q60 q_exp2neg(q60 v, int kz, int *n) {
     const q60 frac = (q60)((uint64_t)v << kz) & (kQ1 - 1);
     *n = (int)(v >> (60 - kz));
     const int i = (int)(frac >> 54);
@@ -169,7 +168,19 @@ FLG_HD q60 q_expneg(q60 zm, int kz, int *n) {
     const q60 p = kQ1 - x + qmul(qf(qmul(xf, xf)), qf(u));
     return qmul(qf(q_exp_table(i)), qf(p));
 }
+// e^-z for z = zm 2^kz with zm in [1/2, 1): zm log2(e) is in (0.7, 1.45)
+FLG_HD q60 q_expneg(q60 zm, int kz, int *n) { return q_exp2neg(qmul(qf(zm), qf(1663314137230540311ll)), kz, n); }
 
+// bits that |x| < 2 can move up so that the larger ones of or-ed x are in [1/2, 1); q_abs1 is |x| or |x| - 1
+FLG_HD uint64_t q_abs1(q60 x) { return (uint64_t)(x ^ (x >> 63)); }
+FLG_HD int q_room(uint64_t m) {
+#if defined(__CUDA_ARCH__)
+    const int lz = __clz((int)(m >> 32));
+#else
+    const int lz = (m >> 32) ? __builtin_clz((unsigned)(m >> 32)) : 32;
+#endif
+    return lz > 4 ? lz - 4 : 0;
+}
 FLG_HD q60 q_shift(q60 x, int s) {  // x 2^-s
     return s >= 0 ? x >> (s < 63 ? s : 63) : x << -s;
 }
@@ -212,7 +223,10 @@ FLG_HD FxRadial fx_brinkman(const FxDir &g, const FxAlpha &al) {
     const Qf kf = qf(k << sk), f2 = qf(F2h << sf);
     r.A = qmul(qf(((F1 << sf) >> 1) + qmul(f2, qf(g.w2))), kf);
     r.B = qmul(f2, kf);
-    r.x = 1 + al.iae - 3 * E - sk - sf;
+    // A and B up to [1/2, 1): a sum keeps its terms to 2^-58 of the largest exponent it has met
+    const int s = q_room(q_abs1(r.A) | q_abs1(r.B));
+    r.A <<= s, r.B <<= s;
+    r.x = 1 + al.iae - 3 * E - sk - sf - s;
     return r;
 }
 
@@ -224,6 +238,203 @@ FLG_HD void fx_radial_apply(const FxDir &g, const FxRadial &r, const q60 *F, q60
     u[0] = qmul(A, f0) + qmul(b, n0);
     u[1] = qmul(A, f1) + qmul(b, n1);
     u[2] = qmul(A, f2) + qmul(b, n2);
+}
+
+// ---- complex alpha --------------------------------------------------------------------------------
+// The same functions of the complex z = |alpha| sqrt(Q) u, u = alpha / |alpha| (Re u >= 1/2, so that
+// e^-z has vanished beside one from |z| = 128 on).  Imaginary parts carry an exponent of their own,
+// xi, so that they keep their precision where z is small.
+struct FxAlphaC {
+    q60 am;        // |alpha| = am 2^ae, am in [1/2, 1)
+    int ae, iae;   // 1 / alpha^2 = i 2^iae, |i| in [1/2, 1)
+    q60 ur, ui;    // u
+    q60 u2r, u2i;  // u^2
+    q60 ir, ii;
+    q60 cx, cy;    // Re(u) log2(e), Im(u) 2 / pi
+};
+// which alpha the fixed-point path takes: a finite one that decays, with an imaginary part that an
+// absolute error of 2^-59 |alpha| still leaves its FP64 precision
+inline bool fx_alpha_c_ok(double re, double im) {
+    return std::fabs(re) < 1e150 && std::fabs(im) < 1e150 && re > 1e-150 && std::fabs(im) <= 1.7 * re &&
+           std::fabs(im) >= re / 4;
+}
+inline FxAlphaC fx_alpha_c(double re, double im) {
+    FxAlphaC a;
+    const long double r = re, i = im, m2 = r * r + i * i, m = sqrtl(m2), ur = r / m, ui = i / m;
+    auto q = [](long double x) { return (q60)llroundl(ldexpl(x, 60)); };
+    int e;
+    a.am = q(frexpl(m, &e));
+    if (a.am >= kQ1) a.am = kQ1 - 1;
+    a.ae = e;
+    a.ur = q(ur), a.ui = q(ui);
+    const long double u2r = ur * ur - ui * ui, u2i = 2 * ur * ui;
+    a.u2r = q(u2r), a.u2i = q(u2i);
+    const long double im2 = frexpl(1.0L / m2, &e);
+    a.iae = e;
+    a.ir = q(u2r * im2), a.ii = q(-u2i * im2);
+    a.cx = q(ur * 1.442695040888963407359924681001892137L);
+    a.cy = q(ui * 0.636619772367581343075535053490057448L);
+    return a;
+}
+
+// cos and sin of 2 pi i / 64
+struct alignas(16) QTrig {
+    q60 c, s;
+};
+#define FLG_TRIG_TABLE \
+    {1152921504606846976ll, 0ll}, {1147369872436662991ll, 113006068906017470ll}, \
+    {1130768441178740757ll, 224923827593068887ll}, {1103277091691359535ll, 334675446864527722ll}, \
+    {1065160580698383124ll, 441203958630471860ll}, {1016785991037278313ll, 543483435088187080ll}, \
+    {958619196450722178ll, 640528868967736374ll}, {891220374967787610ll, 731405659690429196ll}, \
+    {815238614083298888ll, 815238614083298888ll}, {731405659690429196ll, 891220374967787610ll}, \
+    {640528868967736374ll, 958619196450722178ll}, {543483435088187080ll, 1016785991037278313ll}, \
+    {441203958630471860ll, 1065160580698383124ll}, {334675446864527722ll, 1103277091691359535ll}, \
+    {224923827593068887ll, 1130768441178740757ll}, {113006068906017470ll, 1147369872436662991ll}, \
+    {0ll, 1152921504606846976ll}, {-113006068906017470ll, 1147369872436662991ll}, \
+    {-224923827593068887ll, 1130768441178740757ll}, {-334675446864527722ll, 1103277091691359535ll}, \
+    {-441203958630471860ll, 1065160580698383124ll}, {-543483435088187080ll, 1016785991037278313ll}, \
+    {-640528868967736374ll, 958619196450722178ll}, {-731405659690429196ll, 891220374967787610ll}, \
+    {-815238614083298888ll, 815238614083298888ll}, {-891220374967787610ll, 731405659690429196ll}, \
+    {-958619196450722178ll, 640528868967736374ll}, {-1016785991037278313ll, 543483435088187080ll}, \
+    {-1065160580698383124ll, 441203958630471860ll}, {-1103277091691359535ll, 334675446864527722ll}, \
+    {-1130768441178740757ll, 224923827593068887ll}, {-1147369872436662991ll, 113006068906017470ll}, \
+    {-1152921504606846976ll, 0ll}, {-1147369872436662991ll, -113006068906017470ll}, \
+    {-1130768441178740757ll, -224923827593068887ll}, {-1103277091691359535ll, -334675446864527722ll}, \
+    {-1065160580698383124ll, -441203958630471860ll}, {-1016785991037278313ll, -543483435088187080ll}, \
+    {-958619196450722178ll, -640528868967736374ll}, {-891220374967787610ll, -731405659690429196ll}, \
+    {-815238614083298888ll, -815238614083298888ll}, {-731405659690429196ll, -891220374967787610ll}, \
+    {-640528868967736374ll, -958619196450722178ll}, {-543483435088187080ll, -1016785991037278313ll}, \
+    {-441203958630471860ll, -1065160580698383124ll}, {-334675446864527722ll, -1103277091691359535ll}, \
+    {-224923827593068887ll, -1130768441178740757ll}, {-113006068906017470ll, -1147369872436662991ll}, \
+    {0ll, -1152921504606846976ll}, {113006068906017470ll, -1147369872436662991ll}, \
+    {224923827593068887ll, -1130768441178740757ll}, {334675446864527722ll, -1103277091691359535ll}, \
+    {441203958630471860ll, -1065160580698383124ll}, {543483435088187080ll, -1016785991037278313ll}, \
+    {640528868967736374ll, -958619196450722178ll}, {731405659690429196ll, -891220374967787610ll}, \
+    {815238614083298888ll, -815238614083298888ll}, {891220374967787610ll, -731405659690429196ll}, \
+    {958619196450722178ll, -640528868967736374ll}, {1016785991037278313ll, -543483435088187080ll}, \
+    {1065160580698383124ll, -441203958630471860ll}, {1103277091691359535ll, -334675446864527722ll}, \
+    {1130768441178740757ll, -224923827593068887ll}, {1147369872436662991ll, -113006068906017470ll}
+#if defined(__CUDACC__)
+static __device__ const QTrig c_q_trig[64] = {FLG_TRIG_TABLE};
+#endif
+static const QTrig h_q_trig[64] = {FLG_TRIG_TABLE};
+FLG_HD QTrig q_trig_table(int i) {
+#if defined(__CUDA_ARCH__)
+    const longlong2 v = *reinterpret_cast<const longlong2 *>(&c_q_trig[i]);
+    return {v.x, v.y};
+#else
+    return h_q_trig[i];
+#endif
+}
+// cos and sin of v quarter turns (v in Q60, any multiple of a whole turn may be missing): the
+// nearest of 64 angles and Taylor polynomials of the rest, at most pi / 64
+FLG_HD QTrig q_cos_sin(q60 v) {
+    const q60 k = (q60)((uint64_t)v + (1ull << 55)) >> 56;  // sixteenths of a quarter turn
+    const q60 rem = (q60)((uint64_t)v - ((uint64_t)k << 56));
+    const Qf x = qf(qmul(qf(rem << 4), qf(113187804032455044ll)));
+    const q60 x2 = qmul(x, x);
+    const int s2 = (int)(x2 >> 24);
+    const q60 s4 = (kQ1 / 120) - qmul36((kQ1 / 5040) - qmul36(kQ1 / 362880, s2), s2);
+    const q60 c4 = (kQ1 / 24) - qmul36((kQ1 / 720) - qmul36(kQ1 / 40320, s2), s2);
+    const Qf xf2 = qf(x2);
+    // sin x = x - x^3 (1/6 - x^2 s4), cos x = 1 - x^2 (1/2 - x^2 c4)
+    const q60 sn = qmul(x, qf(kQ1 - qmul(xf2, qf((kQ1 / 6) - qmul(xf2, qf(s4))))));
+    const q60 cs1 = qmul(xf2, qf((kQ1 / 2) - qmul(xf2, qf(c4))));  // 1 - cos x
+    const QTrig t = q_trig_table((int)k & 63);
+    const Qf tc = qf(t.c), ts = qf(t.s), sf = qf(sn), cf = qf(cs1);
+    return {t.c - qmul(tc, cf) - qmul(ts, sf), t.s - qmul(ts, cf) + qmul(tc, sf)};
+}
+
+// u = (A f + B (f.n) n) 2^x, A = (Ar + i Ai 2^xi), B alike; all below 1.5
+struct FxRadialC {
+    q60 Ar, Br, Ai, Bi;
+    int x, xi;
+};
+FLG_HD FxRadialC fx_brinkman_c(const FxDir &g, const FxAlphaC &al) {
+    const Qf y = qf(g.r.y), w2 = qf(g.w2);
+    const int E = g.r.e - 1023;
+    q60 zm = qmul(qf(al.am), qf(qmul(qf(g.r.qh), y)));  // in [1/4, 1)
+    const int low = zm < kQ1 / 2;
+    zm <<= low;
+    const int kz = al.ae + E + 1 - low;  // |z| = zm 2^kz, zm in [1/2, 1)
+    const Qf zf = qf(zm), ui = qf(al.ui);
+    FxRadialC r;
+    if (kz < 0) {
+        // a polynomial with real coefficients at a complex point: b_k = a_k + 2 Re(z) b_{k+1} - |z|^2 b_{k+2}
+        const q60 zq = q_shift(zm, -kz), zr = qmul(qf(zq), qf(al.ur));
+        const Qf p = qf(2 * zr), m = qf(qmul(qf(zq), qf(zq)));
+        q60 b1 = q_br1(15), c1 = 0, b2 = q_br2(15), c2 = 0;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+        for (int n = 14; n >= 1; n--) {
+            const Qf h1 = qf(b1), h2 = qf(b2);
+            q60 t = q_br1(n) + qmul(h1, p);
+            if (n < 14) t -= qmul(qf(c1), m);
+            c1 = b1, b1 = t;
+            t = q_br2(n) + qmul(h2, p);
+            if (n < 14) t -= qmul(qf(c2), m);
+            c2 = b2, b2 = t;
+        }
+        const Qf z0 = qf(zr), h1 = qf(b1), h2 = qf(b2);
+        const q60 f1 = q_br1(0) + qmul(h1, z0) - qmul(qf(c1), m), f2 = q_br2(0) + qmul(h2, z0) - qmul(qf(c2), m);
+        const Qf zi = qf(qmul(qf(qmul(zf, ui)), y));  // Im(z) y 2^-kz
+        r.Ar = qmul(qf(f1 + qmul(qf(f2), w2)), y);
+        r.Br = qmul(qf(f2), y);
+        r.Ai = qmul(qf(b1 + qmul(h2, w2)), zi);
+        r.Bi = qmul(h2, zi);
+        r.x = -E;
+        r.xi = kz;
+        return r;
+    }
+    // F1 and F2 over 2^sc: below 1 at |z| < 1, up to 4 and 7 above
+    const int sc = kz == 0 ? 0 : 3;
+    q60 F1r = -(kQ1 >> sc), F1i = 0, F2r = 3 * (kQ1 >> sc), F2i = 0;
+    if (kz < 8) {
+        const q60 v = qmul(zf, qf(al.cx));  // Re(z) log2(e) 2^-kz
+        int n;
+        const Qf em = qf(q_exp2neg(v, kz, &n));
+        const QTrig t = q_cos_sin((q60)((uint64_t)qmul(zf, qf(al.cy)) << kz));
+        const Qf er = qf(qmul(em, qf(t.c))), ei = qf(-qmul(em, qf(t.s)));
+        // 1 + z + z^2 and 3 + 3 z + z^2 over 4^kz 2^h
+        const Qf zz = qf(qmul(zf, zf));
+        const q60 z2r = qmul(zz, qf(al.u2r)), z2i = qmul(zz, qf(al.u2i));
+        const q60 z1r = qmul(zf, qf(al.ur)) >> kz, z1i = qmul(zf, ui) >> kz, z0 = kQ1 >> (2 * kz);
+        const int h1 = kz == 0, h2 = kz < 2 ? 2 - kz : 0;
+        const Qf pr = qf((z2r + z1r + z0) >> h1), pi = qf((z2i + z1i) >> h1);
+        const Qf qr = qf((z2r + 3 * (z1r + z0)) >> h2), qi = qf((z2i + 3 * z1i) >> h2);
+        const int s1 = n - 2 * kz - h1 + sc, s2 = n - 2 * kz - h2 + sc;
+        F1r += q_shift(qmul(er, pr) - qmul(ei, pi), s1);
+        F1i += q_shift(qmul(er, pi) + qmul(ei, pr), s1);
+        F2r -= q_shift(qmul(er, qr) - qmul(ei, qi), s2);
+        F2i -= q_shift(qmul(er, qi) + qmul(ei, qr), s2);
+    }
+    const q60 y3 = qmul(qf(qmul(y, y)), y);
+    const int s3 = y3 < kQ1 / 4 ? 2 : 0;
+    const Qf y3f = qf(y3 << s3);
+    const Qf kr = qf(qmul(y3f, qf(al.ir))), ki = qf(qmul(y3f, qf(al.ii))), f2r = qf(F2r), f2i = qf(F2i);
+    const Qf ar = qf(F1r + qmul(f2r, w2)), ai = qf(F1i + qmul(f2i, w2));
+    r.Ar = qmul(ar, kr) - qmul(ai, ki);
+    r.Ai = qmul(ar, ki) + qmul(ai, kr);
+    r.Br = qmul(f2r, kr) - qmul(f2i, ki);
+    r.Bi = qmul(f2r, ki) + qmul(f2i, kr);
+    const int s = q_room(q_abs1(r.Ar) | q_abs1(r.Ai) | q_abs1(r.Br) | q_abs1(r.Bi));  // as in fx_brinkman
+    r.Ar <<= s, r.Ai <<= s, r.Br <<= s, r.Bi <<= s;
+    r.x = sc + al.iae - 3 * E - s3 - s;
+    r.xi = 0;
+    return r;
+}
+// the two parts of one real strength vector: ur = (Ar F + Br t n), ui = (Ai F + Bi t n), t = F.n
+FLG_HD void fx_radial_apply_c(const FxDir &g, const FxRadialC &r, const q60 *F, q60 *ur, q60 *ui) {
+    const Qf n0 = qf(g.n[0]), n1 = qf(g.n[1]), n2 = qf(g.n[2]), f0 = qf(F[0]), f1 = qf(F[1]), f2 = qf(F[2]);
+    const Qf t = qf(qmul(f0, n0) + qmul(f1, n1) + qmul(f2, n2));
+    const Qf br = qf(qmul(t, qf(r.Br))), bi = qf(qmul(t, qf(r.Bi))), Ar = qf(r.Ar), Ai = qf(r.Ai);
+    ur[0] = qmul(Ar, f0) + qmul(br, n0);
+    ur[1] = qmul(Ar, f1) + qmul(br, n1);
+    ur[2] = qmul(Ar, f2) + qmul(br, n2);
+    ui[0] = qmul(Ai, f0) + qmul(bi, n0);
+    ui[1] = qmul(Ai, f1) + qmul(bi, n1);
+    ui[2] = qmul(Ai, f2) + qmul(bi, n2);
 }
 
 // wall: everything that does not depend on the strengths

@@ -3,8 +3,10 @@
 // Replaces fluidlets.evaluate (core/matvec.py:24-49) and its Numba loop
 // _apply (core/matvec.py:10-21).  Two precisions:
 //
-//  FLG_PREC_FP64  sum_f64_kernel: one target per thread, sources staged in
-//                 shared memory in tiles of 128, FP64 arithmetic throughout.
+//  FLG_PREC_FP64  sum_fx_kernel: one target per thread, sources staged in
+//                 shared memory in tiles of 64, displacements in FP64 and the
+//                 pairs in 60-bit fixed point; sum_f64_kernel, FP64 throughout,
+//                 for the complex alpha that the fixed-point pairs do not take.
 //  FLG_PREC_MIXED far_f32_kernel: TPT targets per thread, 256-source tiles of
 //                 packed FP32 sources (float4 x,y,z,eps^2 | f0,f1,f2,thr) in
 //                 cell order, register-prefetched; pairs with r < 4 eps_j are
@@ -22,6 +24,7 @@
 // combined in a fixed order (bitwise deterministic results).
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "flg_common.cuh"
 #include "pair_fixed.cuh"
@@ -30,9 +33,6 @@
 
 namespace flg {
 
-#ifndef FLG_FX_MINB
-#define FLG_FX_MINB 4
-#endif
 constexpr int kF64Threads = 128;
 constexpr int kF64Tile = 128;
 constexpr int kF32Threads = 256;
@@ -159,38 +159,109 @@ __global__ void __launch_bounds__(kF64Threads) sum_f64_kernel(SumArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// The same sum for real kernels with the pairs in 60-bit fixed point (pair_fixed.cuh): the FP64
-// pipe (19 clocks per warp instruction and SM) keeps the displacements and squared distances, six
-// operations of a Stokeslet pair's 27 and eight of a wall pair's 56; the rest runs on the integer
-// pipe beside it.  Sums of 16 terms stay in 64-bit integers relative to their largest exponent.
-// A pair outside the fixed-point ranges takes the FP64 function.  The wall kernel's factor t is
-// applied once at the end, its factor h in the staged strengths.
+// The same sum with the pairs in 60-bit fixed point (pair_fixed.cuh): the FP64 pipe (19 clocks per
+// warp instruction and SM) keeps the displacements and squared distances, six operations of a
+// Stokeslet pair's 27, eight of a wall pair's 56 and six of a complex Brinkman pair's 350; the rest
+// runs on the integer pipe beside it.  Sums of 16 terms stay in 64-bit integers relative to their
+// largest exponent, real and imaginary parts each to their own.  A pair outside the fixed-point
+// ranges takes the FP64 function; a complex alpha that fx_alpha_c_ok refuses takes sum_f64_kernel.
+// The wall kernel's factor t is applied once at the end, its factor h in the staged strengths.
+// Bound by the integer pipe.  FP64 pairs -> fixed point: 32,768 x 1,003 wall 3.6 -> 1.2 ms, 16,384 x
+// 16,384 Brinkman 33 -> 12 ms, 4,099 x 2,500 complex Brinkman 6.0 -> 1.7 ms (four CTAs per SM; the
+// complex pair's registers allow three: 1.81 ms a call with two or three, 1.84 with four).
 // ---------------------------------------------------------------------------
 constexpr int kFxThreads = 128, kFxTile = 64;
+template <bool CK>
+using FxAlphaOf = typename std::conditional<CK, FxAlphaC, FxAlpha>::type;
+template <int NF>
 struct FxSource {
     double x, y, z, e2, e;
-    int ef;  // exponent of the strengths, or kFxBad
+    int ef[NF];  // exponents of the strengths, or kFxBad
 };
+// strengths (for the wall times h) as mantissas and exponents
 template <int KIND, int NF>
-__device__ __noinline__ void pair_f64_slow(double tx, double ty, double tz, const FxSource &s, const double *f,
-                                           int64_t j, double alpha, double *u) {
+__device__ __forceinline__ void fx_strengths(double *f, double h, q60 *F, int *ef) {
+    if (KIND == FLG_WALL)
+#pragma unroll
+        for (int c = 0; c < 3 * NF; c++) f[c] *= h;
+#pragma unroll
+    for (int c = 0; c < NF; c++) ef[c] = fx_strength(f + 3 * c, 3, F + 3 * c);
+}
+// pairs between two readings of the accumulators: 16 terms
+template <int NF, bool CK>
+constexpr int kFxPairs = CK ? kFxSeg / NF : kFxSeg;
+// adds one pair; false: outside the fixed-point ranges
+template <int KIND, int NF, bool CK>
+__device__ __forceinline__ bool pair_fx(double tx, double ty, double tz, double sx, double sy, double sz, double e,
+                                        double e2, const q60 *F, const int *ef, const FxAlphaOf<CK> &al,
+                                        FxAcc<3> *acc) {
+    const double d0 = tx - sx, d1 = ty - sy, d2 = tz - sz;
+    if (ef[0] == kFxBad || (NF == 2 && ef[NF - 1] == kFxBad)) return false;
+    q60 t[3];
+    if constexpr (KIND == FLG_WALL) {
+        const double dp = tz + sz;
+        const double rq = fma(d1, d1, fma(d0, d0, e2)), QF = fma(d2, d2, rq), QI = fma(dp, dp, rq);
+        if (!q_in_range(QF) || !q_in_range(QI) || (d_neg(tz) ^ d_neg(sz))) return false;
+        const FxWall w = fx_wall(d0, d1, d2, dp, QF, QI, e);
+#pragma unroll
+        for (int c = 0; c < NF; c++) {
+            const int x = fx_wall_apply(w, F + 3 * c, t) + ef[c];
+            acc[c].scale(x);
+            acc[c].add(0, t, x);
+        }
+    } else {
+        const double Q = fma(d2, d2, fma(d1, d1, fma(d0, d0, e2)));
+        if (!q_in_range(Q)) return false;
+        const FxDir g = fx_dir(d0, d1, d2, Q, e);
+        if constexpr (CK) {
+            const FxRadialC r = fx_brinkman_c(g, al);
+#pragma unroll
+            for (int c = 0; c < NF; c++) {  // i f: real part -A_im f, imaginary part A_re f
+                q60 im[3];
+                fx_radial_apply_c(g, r, F + 3 * c, t, im);
+                if (c == 1)
+#pragma unroll
+                    for (int k = 0; k < 3; k++) im[k] = -im[k];
+                const int x = r.x + ef[c];
+                acc[c].scale(x);
+                acc[c].add(0, t, x);
+                acc[1 - c].scale(x + r.xi);
+                acc[1 - c].add(0, im, x + r.xi);
+            }
+        } else {
+            const FxRadial r = KIND == FLG_STOKESLET ? fx_stokeslet(g) : fx_brinkman(g, al);
+#pragma unroll
+            for (int c = 0; c < NF; c++) {
+                acc[c].scale(r.x + ef[c]);
+                fx_radial_apply(g, r, F + 3 * c, t);
+                acc[c].add(0, t, r.x + ef[c]);
+            }
+        }
+    }
+    return true;
+}
+template <int KIND, int NF, bool CK>
+__device__ __noinline__ void pair_f64_slow(double tx, double ty, double tz, const FxSource<NF> &s, const double *f,
+                                           int64_t j, double are, double aim, double *u) {
     double fj[3 * NF];
     load_strength<NF>(f, j, fj);
-    pair_f64<KIND, NF, false>(tx, ty, tz, 2.0, s.x, s.y, s.z, s.e2, fj, alpha, 0.0, u);
+    pair_f64<KIND, NF, CK>(tx, ty, tz, 2.0, s.x, s.y, s.z, s.e2, fj, are, aim, u);
 }
-template <int KIND, int NF>
-__global__ void __launch_bounds__(kFxThreads, FLG_FX_MINB) sum_fx_kernel(SumArgs a, FxAlpha al) {
-    constexpr int NC = 3 * NF;
-    __shared__ FxSource s_src[kFxTile];
-    __shared__ q60 s_f[kFxTile][NC];
+template <int KIND, int NF, bool CK>
+__global__ void __launch_bounds__(kFxThreads, CK ? 3 : 4)
+sum_fx_kernel(SumArgs a, FxAlphaOf<CK> al) {
+    constexpr int OUTW = (NF == 2 || CK) ? 6 : 3, SEG = kFxPairs<NF, CK>;
+    __shared__ FxSource<NF> s_src[kFxTile];
+    __shared__ q60 s_f[kFxTile][3 * NF];
     const int64_t i = (int64_t)blockIdx.x * kFxThreads + threadIdx.x;
     const int64_t ii = i < a.M ? i : a.M - 1;
     const double tx = a.tg[3 * ii], ty = a.tg[3 * ii + 1], tz = a.tg[3 * ii + 2];
-    double u[NC], us[NC];
-    FxAcc<NC> acc;
-    acc.init();
+    double u[OUTW], us[OUTW];
+    FxAcc<3> acc[OUTW / 3];
 #pragma unroll
-    for (int c = 0; c < NC; c++) u[c] = us[c] = 0.0;
+    for (int c = 0; c < OUTW / 3; c++) acc[c].init();
+#pragma unroll
+    for (int c = 0; c < OUTW; c++) u[c] = us[c] = 0.0;
     const int64_t j0 = (int64_t)blockIdx.y * a.split_len;
     const int64_t j1 = min(a.N, j0 + a.split_len);
     for (int64_t jt = j0; jt < j1; jt += kFxTile) {
@@ -198,65 +269,34 @@ __global__ void __launch_bounds__(kFxThreads, FLG_FX_MINB) sum_fx_kernel(SumArgs
         __syncthreads();
         for (int k = threadIdx.x; k < cnt; k += kFxThreads) {
             const int64_t j = jt + k;
-            FxSource s;
+            FxSource<NF> s;
             s.x = a.src[3 * j], s.y = a.src[3 * j + 1], s.z = a.src[3 * j + 2];
             s.e = fabs(a.eps[j]);
             s.e2 = s.e * s.e;
-            double f[NC];
+            double f[3 * NF];
             load_strength<NF>(a.f, j, f);
-            if (KIND == FLG_WALL)
-#pragma unroll
-                for (int c = 0; c < NC; c++) f[c] *= s.z;
-            s.ef = fx_strength(f, NC, s_f[k]);
+            fx_strengths<KIND, NF>(f, s.z, s_f[k], s.ef);
             s_src[k] = s;
         }
         __syncthreads();
-        for (int k0 = 0; k0 < cnt; k0 += kFxSeg) {
-            acc.clear();
-            const int k1 = min(cnt, k0 + kFxSeg);
+        for (int k0 = 0; k0 < cnt; k0 += SEG) {
+#pragma unroll
+            for (int c = 0; c < OUTW / 3; c++) acc[c].clear();
+            const int k1 = min(cnt, k0 + SEG);
 #pragma unroll 1
             for (int k = k0; k < k1; k++) {
-                const FxSource &s = s_src[k];
-                const double d0 = tx - s.x, d1 = ty - s.y, d2 = tz - s.z;
-                if constexpr (KIND == FLG_WALL) {
-                    const double dp = tz + s.z;
-                    const double rq = fma(d1, d1, fma(d0, d0, s.e2)), QF = fma(d2, d2, rq), QI = fma(dp, dp, rq);
-                    if (q_in_range(QF) && q_in_range(QI) && s.ef < kFxBad && !(d_neg(tz) ^ d_neg(s.z))) {
-                        const FxWall w = fx_wall(d0, d1, d2, dp, QF, QI, s.e);
-#pragma unroll
-                        for (int c = 0; c < NC; c += 3) {
-                            q60 t[3];
-                            const int x = fx_wall_apply(w, s_f[k] + c, t) + s.ef;
-                            acc.scale(x);
-                            acc.add(c, t, x);
-                        }
-                        continue;
-                    }
-                } else {
-                    const double Q = fma(d2, d2, fma(d1, d1, fma(d0, d0, s.e2)));
-                    if (q_in_range(Q) && s.ef < kFxBad) {
-                        const FxDir g = fx_dir(d0, d1, d2, Q, s.e);
-                        const FxRadial r = KIND == FLG_STOKESLET ? fx_stokeslet(g) : fx_brinkman(g, al);
-                        acc.scale(r.x + s.ef);
-#pragma unroll
-                        for (int c = 0; c < NC; c += 3) {
-                            q60 t[3];
-                            fx_radial_apply(g, r, s_f[k] + c, t);
-                            acc.add(c, t, r.x + s.ef);
-                        }
-                        continue;
-                    }
-                }
-                pair_f64_slow<KIND, NF>(tx, ty, tz, s, a.f, jt + k, a.alpha_re, us);
+                const FxSource<NF> &s = s_src[k];
+                if (!pair_fx<KIND, NF, CK>(tx, ty, tz, s.x, s.y, s.z, s.e, s.e2, s_f[k], s.ef, al, acc))
+                    pair_f64_slow<KIND, NF, CK>(tx, ty, tz, s, a.f, jt + k, a.alpha_re, a.alpha_im, us);
             }
 #pragma unroll
-            for (int c = 0; c < NC; c++) u[c] += acc.value(c);
+            for (int c = 0; c < OUTW; c++) u[c] += acc[c / 3].value(c % 3);
         }
     }
     if (i < a.M) {
-        double *p = a.partial + ((int64_t)blockIdx.y * a.M + i) * NC;
+        double *p = a.partial + ((int64_t)blockIdx.y * a.M + i) * OUTW;
 #pragma unroll
-        for (int c = 0; c < NC; c++) p[c] = KIND == FLG_WALL ? tz * (u[c] + us[c]) : u[c] + us[c];
+        for (int c = 0; c < OUTW; c++) p[c] = KIND == FLG_WALL ? tz * (u[c] + us[c]) : u[c] + us[c];
     }
 }
 
@@ -985,7 +1025,7 @@ struct NearArgs {
 // (pair_fixed.cuh).  Measured against a thread per target with FP64 pairs: see sum_plan_geometry.
 constexpr int kNearThreads = 128, kNearLanes = 8, kNearTargets = kNearThreads / kNearLanes, kNearList = 64;
 template <int KIND, int NF, bool CK>
-__global__ void __launch_bounds__(kNearThreads) near_f64_kernel(NearArgs a, FxAlpha al) {
+__global__ void __launch_bounds__(kNearThreads) near_f64_kernel(NearArgs a, FxAlphaOf<CK> al) {
     constexpr int OUTW = (NF == 2 || CK) ? 6 : 3;
     __shared__ int list[kNearTargets][kNearList];
     const int lane = threadIdx.x & 31, l = lane & (kNearLanes - 1), gs = lane & ~(kNearLanes - 1), grp = threadIdx.x / kNearLanes;
@@ -1031,55 +1071,28 @@ __global__ void __launch_bounds__(kNearThreads) near_f64_kernel(NearArgs a, FxAl
         total += __shfl_sync(0xffffffffu, rn[q / kNearLanes], gs + q % kNearLanes);
     }
     const int rounds = (int)(__reduce_max_sync(0xffffffffu, (unsigned)total) + kNearLanes - 1) / kNearLanes;
-    FxAcc<3 * NF> acc;
-    if constexpr (!CK) acc.init();
+    FxAcc<3> acc[OUTW / 3];
+#pragma unroll
+    for (int c = 0; c < OUTW / 3; c++) acc[c].init();
     int terms = 0, cnt = 0;
     auto evaluate = [&]() {
         for (int q = l; q < cnt; q += kNearLanes) {
             const int64_t j = a.sorted[list[grp][q]];
             const double sx = a.src[3 * j], sy = a.src[3 * j + 1], sz = a.src[3 * j + 2], e = fabs(a.eps[j]);
-            double fj[3 * NF];
+            double fj[3 * NF], fh[3 * NF];
             load_strength<NF>(a.f, j, fj);
-            if constexpr (!CK) {
-                const double d0 = tx - sx, d1 = ty - sy, d2 = tz - sz, e2 = e * e;
-                double fh[3 * NF];
+            if (!CK || al.am != 0) {
+                q60 F[3 * NF];
+                int ef[NF];
 #pragma unroll
-                for (int c = 0; c < 3 * NF; c++) fh[c] = KIND == FLG_WALL ? fj[c] * sz : fj[c];
-                q60 F[3 * NF], t[3];
-                const int ef = fx_strength(fh, 3 * NF, F);
-                bool done = false;
-                if constexpr (KIND == FLG_WALL) {
-                    const double dp = tz + sz;
-                    const double rq = fma(d1, d1, fma(d0, d0, e2)), QF = fma(d2, d2, rq), QI = fma(dp, dp, rq);
-                    if (q_in_range(QF) && q_in_range(QI) && ef < kFxBad && !(d_neg(tz) ^ d_neg(sz))) {
-                        const FxWall w = fx_wall(d0, d1, d2, dp, QF, QI, e);
+                for (int c = 0; c < 3 * NF; c++) fh[c] = fj[c];
+                fx_strengths<KIND, NF>(fh, sz, F, ef);
+                if (pair_fx<KIND, NF, CK>(tx, ty, tz, sx, sy, sz, e, e * e, F, ef, al, acc)) {
+                    if (++terms == kFxPairs<NF, CK>) {
 #pragma unroll
-                        for (int c = 0; c < 3 * NF; c += 3) {
-                            const int x = fx_wall_apply(w, F + c, t) + ef;
-                            acc.scale(x);
-                            acc.add(c, t, x);
-                        }
-                        done = true;
-                    }
-                } else {
-                    const double Q = fma(d2, d2, fma(d1, d1, fma(d0, d0, e2)));
-                    if (q_in_range(Q) && ef < kFxBad) {
-                        const FxDir g = fx_dir(d0, d1, d2, Q, e);
-                        const FxRadial r = KIND == FLG_STOKESLET ? fx_stokeslet(g) : fx_brinkman(g, al);
-                        acc.scale(r.x + ef);
+                        for (int c = 0; c < OUTW; c++) uf[c] += acc[c / 3].value(c % 3);
 #pragma unroll
-                        for (int c = 0; c < 3 * NF; c += 3) {
-                            fx_radial_apply(g, r, F + c, t);
-                            acc.add(c, t, r.x + ef);
-                        }
-                        done = true;
-                    }
-                }
-                if (done) {
-                    if (++terms == kFxSeg) {
-#pragma unroll
-                        for (int c = 0; c < 3 * NF; c++) uf[c] += acc.value(c);
-                        acc.clear();
+                        for (int c = 0; c < OUTW / 3; c++) acc[c].clear();
                         terms = 0;
                     }
                     continue;
@@ -1113,12 +1126,10 @@ __global__ void __launch_bounds__(kNearThreads) near_f64_kernel(NearArgs a, FxAl
     __syncwarp();
     evaluate();
     __syncwarp();
-    if constexpr (!CK) {
 #pragma unroll
-        for (int c = 0; c < 3 * NF; c++) {
-            uf[c] += acc.value(c);
-            u[c] += KIND == FLG_WALL ? tz * uf[c] : uf[c];
-        }
+    for (int c = 0; c < OUTW; c++) {
+        uf[c] += acc[c / 3].value(c % 3);
+        u[c] += KIND == FLG_WALL ? tz * uf[c] : uf[c];
     }
 #pragma unroll
     for (int o = 1; o < kNearLanes; o <<= 1)
@@ -1315,6 +1326,12 @@ static int sort_targets(const double *tg, int64_t M, const SumPlan *p, cudaStrea
     return FLG_OK;
 }
 
+template <int KIND, bool CK>
+static FxAlphaOf<CK> alpha_of(const SumRun &r) {
+    if constexpr (CK) return fx_alpha_c_ok(r.alpha_re, r.alpha_im) ? fx_alpha_c(r.alpha_re, r.alpha_im) : FxAlphaC{};
+    else return KIND == FLG_BRINKMANLET ? fx_alpha(r.alpha_re) : FxAlpha{};
+}
+
 template <int KIND, int NF, bool CK>
 static int launch_sum(const SumRun &r, const SumLayout &L, int precision, const SumPlan *p, cudaStream_t st) {
     FinalArgs fin{};
@@ -1332,14 +1349,15 @@ static int launch_sum(const SumRun &r, const SumLayout &L, int precision, const 
             SumArgs a{r.tg, r.M, r.src, r.eps, r.f, r.N, L.split_len, r.alpha_re, r.alpha_im, p->partial};
             dim3 grid((unsigned)ceil_div(r.M, kF64Threads), (unsigned)L.S);
             prof_begin(FLG_SLOT_SUM_F64, st);
-            if constexpr (!CK) {
-                static_assert(kFxThreads == kF64Threads, "one grid for both");
-                FxAlpha al{};
-                if (KIND == FLG_BRINKMANLET) al = fx_alpha(r.alpha_re);
-                sum_fx_kernel<KIND, NF><<<grid, kFxThreads, 0, st>>>(a, al);
-            } else {
-                sum_f64_kernel<KIND, NF, CK><<<grid, kF64Threads, 0, st>>>(a);
+            static_assert(kFxThreads == kF64Threads, "one grid for both");
+            bool done = false;
+            if constexpr (CK) {
+                if (!fx_alpha_c_ok(r.alpha_re, r.alpha_im)) {
+                    sum_f64_kernel<KIND, NF, CK><<<grid, kF64Threads, 0, st>>>(a);
+                    done = true;
+                }
             }
+            if (!done) sum_fx_kernel<KIND, NF, CK><<<grid, kFxThreads, 0, st>>>(a, alpha_of<KIND, CK>(r));
             FLG_LAUNCH_CHECK();
             prof_end(FLG_SLOT_SUM_F64, st);
         } else {
@@ -1375,9 +1393,8 @@ static int launch_sum(const SumRun &r, const SumLayout &L, int precision, const 
     NearArgs na{r.tg, r.M, tperm, r.src, r.eps, r.f, r.N, p->packed, L.NQ, p->grid, p->offsets, p->sorted,
                 r.alpha_re, r.alpha_im, fin};
     prof_begin(FLG_SLOT_NEAR_F64, st);
-    FxAlpha al{};
-    if (KIND == FLG_BRINKMANLET && !CK) al = fx_alpha(r.alpha_re);
-    near_f64_kernel<KIND, NF, CK><<<(unsigned)ceil_div(r.M, kNearTargets), kNearThreads, 0, st>>>(na, al);
+    near_f64_kernel<KIND, NF, CK><<<(unsigned)ceil_div(r.M, kNearTargets), kNearThreads, 0, st>>>(
+        na, alpha_of<KIND, CK>(r));
     FLG_LAUNCH_CHECK();
     prof_end(FLG_SLOT_NEAR_F64, st);
     return FLG_OK;

@@ -112,6 +112,59 @@ def test_zero_blob_on_a_source_is_not_finite():
     assert not np.isfinite(u[0]).any() and np.isfinite(u[1]).all()
 
 
+COMPLEX = [complex(0.7, 0.7), 3.0 - 1.0j, 1.0 + 1.6j, 60.0 * (1 + 1j), 1e-4 * (1 + 1j), 0.05 + 0.9j, 2.0 + 0.01j]
+
+
+@pytest.mark.parametrize("m,n", [(1, 1), (3, 8), (129, 17), (40, 1025)])
+@pytest.mark.parametrize("alpha", COMPLEX)
+@pytest.mark.parametrize("strengths", ["real", "complex"])
+def test_complex_alpha(alpha, strengths, m, n):
+    """All of |z| from the series to vanished exponentials; the last two alphas take the FP64 pairs."""
+    rng = np.random.default_rng(m * 1000 + n)
+    X, Y = points(rng, m, n)
+    X[0] = Y[0]
+    F = rng.normal(size=(n, 3))
+    F = F + 1j * rng.normal(size=(n, 3)) if strengths == "complex" else F
+    e = 0.05 * rng.uniform(0.5, 2.0, n)
+    u, ref = check(fl.Brinkmanlet3D(alpha), "brinkman", alpha, X, Y, F, e, 1e-13)
+    if strengths == "real":  # both parts to their own precision (a loss of |Re| / |Im| <= 100 in the last)
+        for a, b in ((u.real, ref.real), (u.imag, ref.imag)):
+            assert np.linalg.norm(a - b) <= 1e-11 * np.linalg.norm(b)
+
+
+def test_complex_alpha_scales_and_tiny_imaginary_strengths():
+    rng = np.random.default_rng(8)
+    X, Y = points(rng, 50, 70)
+    F = rng.normal(size=(70, 3)) + 1e-9j * rng.normal(size=(70, 3))
+    for s in (1e-40, 1.0, 1e40):  # alpha L fixed: homogeneous of degree -1
+        u = fl.evaluate(fl.Brinkmanlet3D((0.8 + 0.6j) / s), X * s, Y * s, F, 0.03 * s) * s
+        ref = O.evaluate("brinkman", X, Y, F, 0.03, alpha=0.8 + 0.6j)
+        assert np.linalg.norm(u - ref) <= 1e-13 * np.linalg.norm(ref)
+    for kernel, name in ((fl.Stokeslet3D(), "stokeslet"), (fl.WallStokeslet3D(), "wall")):
+        u, ref = fl.evaluate(kernel, X, Y, F, 0.03), O.evaluate(name, X, Y, F, 0.03)
+        assert np.linalg.norm(u.imag - ref.imag) <= 1e-12 * np.linalg.norm(ref.imag)
+
+
+def test_complex_alpha_non_finite_strengths():
+    rng = np.random.default_rng(9)
+    X, Y = points(rng, 20, 40)
+    F = rng.normal(size=(40, 3)) + 1j * rng.normal(size=(40, 3))
+    F[7, 1] = complex(0.0, np.nan)
+    assert np.all(np.isnan(fl.evaluate(fl.Brinkmanlet3D(1 + 1j), X, Y, F, 0.05)).any(axis=1))
+
+
+@pytest.mark.parametrize("strengths", ["real", "complex"])
+def test_complex_alpha_near_field(strengths):
+    rng = np.random.default_rng(10)
+    X, Y = points(rng, 600, 900)
+    F = rng.normal(size=(900, 3))
+    F = F + 1j * rng.normal(size=(900, 3)) if strengths == "complex" else F
+    for alpha in (2.0 + 2.0j, 0.3 + 2.0j):
+        ref = O.evaluate("brinkman", X, Y, F, 0.05, alpha=alpha)
+        u = fl.evaluate(fl.Brinkmanlet3D(alpha), X, Y, F, 0.05, precision="mixed")
+        assert np.linalg.norm(u - ref) <= 5e-6 * np.linalg.norm(ref)
+
+
 # ---- matrices ---------------------------------------------------------------------------------
 def oracle_matrix(name, alpha, *args):
     return O.assemble(name, *args, alpha=alpha) if name == "brinkman" else O.assemble(name, *args)
