@@ -185,29 +185,37 @@ FLG_HD q60 q_shift(q60 x, int s) {  // x 2^-s
     return s >= 0 ? x >> (s < 63 ? s : 63) : x << -s;
 }
 
-FLG_HD FxRadial fx_brinkman(const FxDir &g, const FxAlpha &al) {
-    const Qf y = qf(g.r.y);
-    const int E = g.r.e - 1023;
-    q60 zm = qmul(qf(al.am), qf(qmul(qf(g.r.qh), y)));  // in [1/4, 1)
+// |alpha| sqrt(Q) = m 2^k, m in [1/2, 1)
+struct FxZ {
+    q60 m;
+    int k;
+};
+FLG_HD FxZ fx_z(const FxDir &g, q60 am, int ae) {
+    const q60 zm = qmul(qf(am), qf(qmul(qf(g.r.qh), qf(g.r.y))));  // in [1/4, 1)
     const int low = zm < kQ1 / 2;
-    zm <<= low;
-    const int kz = al.ae + E + 1 - low;  // z = zm 2^kz, zm in [1/2, 1)
-    FxRadial r;
-    if (kz < 0) {
-        const Qf z = qf(q_shift(zm, -kz));
-        q60 f1 = q_br1(15), f2 = q_br2(15);
+    return {zm << low, ae + (g.r.e - 1023) + 1 - low};
+}
+FLG_HD FxRadial fx_series(const FxDir &g, const FxZ &zz, const FxAlpha &) {  // k < 0
+    const Qf y = qf(g.r.y), z = qf(q_shift(zz.m, -zz.k));
+    q60 f1 = q_br1(15), f2 = q_br2(15);
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
-        for (int n = 14; n >= 0; n--) {
-            f1 = qmul(qf(f1), z) + q_br1(n);
-            f2 = qmul(qf(f2), z) + q_br2(n);
-        }
-        r.A = qmul(qf(f1 + qmul(qf(f2), qf(g.w2))), y);
-        r.B = qmul(qf(f2), y);
-        r.x = -E;
-        return r;
+    for (int n = 14; n >= 0; n--) {
+        f1 = qmul(qf(f1), z) + q_br1(n);
+        f2 = qmul(qf(f2), z) + q_br2(n);
     }
+    FxRadial r;
+    r.A = qmul(qf(f1 + qmul(qf(f2), qf(g.w2))), y);
+    r.B = qmul(qf(f2), y);
+    r.x = 1023 - g.r.e;
+    return r;
+}
+FLG_HD FxRadial fx_closed(const FxDir &g, const FxZ &zz, const FxAlpha &al) {  // k >= 0
+    const Qf y = qf(g.r.y);
+    const int E = g.r.e - 1023, kz = zz.k;
+    const q60 zm = zz.m;
+    FxRadial r;
     q60 F1 = -kQ1, F2h = kQ1 + kQ1 / 2;  // F1, F2 / 2 where E has vanished
     if (kz < 6 || (kz == 6 && zm < kQ1 / 64 * 52)) {
         int n;
@@ -228,6 +236,10 @@ FLG_HD FxRadial fx_brinkman(const FxDir &g, const FxAlpha &al) {
     r.A <<= s, r.B <<= s;
     r.x = 1 + al.iae - 3 * E - sk - sf - s;
     return r;
+}
+FLG_HD FxRadial fx_brinkman(const FxDir &g, const FxAlpha &al) {
+    const FxZ z = fx_z(g, al.am, al.ae);
+    return z.k < 0 ? fx_series(g, z, al) : fx_closed(g, z, al);
 }
 
 // u / 2^x for strengths F; |u| < 2
@@ -350,43 +362,39 @@ struct FxRadialC {
     q60 Ar, Br, Ai, Bi;
     int x, xi;
 };
-FLG_HD FxRadialC fx_brinkman_c(const FxDir &g, const FxAlphaC &al) {
-    const Qf y = qf(g.r.y), w2 = qf(g.w2);
-    const int E = g.r.e - 1023;
-    q60 zm = qmul(qf(al.am), qf(qmul(qf(g.r.qh), y)));  // in [1/4, 1)
-    const int low = zm < kQ1 / 2;
-    zm <<= low;
-    const int kz = al.ae + E + 1 - low;  // |z| = zm 2^kz, zm in [1/2, 1)
-    const Qf zf = qf(zm), ui = qf(al.ui);
+FLG_HD FxRadialC fx_series(const FxDir &g, const FxZ &zz, const FxAlphaC &al) {
+    const Qf y = qf(g.r.y), w2 = qf(g.w2), zf = qf(zz.m), ui = qf(al.ui);
+    const q60 zm = zz.m;
+    const int kz = zz.k;
     FxRadialC r;
-    if (kz < 0) {
-        // a polynomial with real coefficients at a complex point: b_k = a_k + 2 Re(z) b_{k+1} - |z|^2 b_{k+2}
-        const q60 zq = q_shift(zm, -kz), zr = qmul(qf(zq), qf(al.ur));
-        const Qf p = qf(2 * zr), m = qf(qmul(qf(zq), qf(zq)));
-        q60 b1 = q_br1(15), c1 = 0, b2 = q_br2(15), c2 = 0;
+    // a polynomial with real coefficients at a complex point: b_k = a_k + 2 Re(z) b_{k+1} - |z|^2 b_{k+2}
+    const q60 zq = q_shift(zm, -kz), zr = qmul(qf(zq), qf(al.ur));
+    const Qf p = qf(2 * zr), m = qf(qmul(qf(zq), qf(zq)));
+    q60 b1 = q_br1(15), c1 = 0, b2 = q_br2(15), c2 = 0;
 #if defined(__CUDA_ARCH__)
-#pragma unroll
+#pragma unroll 1  // unrolled, the pair outgrows the instruction cache: 4,099 x 2,500 1.81 ms, not 1.56
 #endif
-        for (int n = 14; n >= 1; n--) {
-            const Qf h1 = qf(b1), h2 = qf(b2);
-            q60 t = q_br1(n) + qmul(h1, p);
-            if (n < 14) t -= qmul(qf(c1), m);
-            c1 = b1, b1 = t;
-            t = q_br2(n) + qmul(h2, p);
-            if (n < 14) t -= qmul(qf(c2), m);
-            c2 = b2, b2 = t;
-        }
-        const Qf z0 = qf(zr), h1 = qf(b1), h2 = qf(b2);
-        const q60 f1 = q_br1(0) + qmul(h1, z0) - qmul(qf(c1), m), f2 = q_br2(0) + qmul(h2, z0) - qmul(qf(c2), m);
-        const Qf zi = qf(qmul(qf(qmul(zf, ui)), y));  // Im(z) y 2^-kz
-        r.Ar = qmul(qf(f1 + qmul(qf(f2), w2)), y);
-        r.Br = qmul(qf(f2), y);
-        r.Ai = qmul(qf(b1 + qmul(h2, w2)), zi);
-        r.Bi = qmul(h2, zi);
-        r.x = -E;
-        r.xi = kz;
-        return r;
+    for (int n = 14; n >= 1; n--) {
+        const Qf h1 = qf(b1), h2 = qf(b2);
+        const q60 t1 = q_br1(n) + qmul(h1, p) - qmul(qf(c1), m), t2 = q_br2(n) + qmul(h2, p) - qmul(qf(c2), m);
+        c1 = b1, b1 = t1;
+        c2 = b2, b2 = t2;
     }
+    const Qf z0 = qf(zr), h1 = qf(b1), h2 = qf(b2);
+    const q60 f1 = q_br1(0) + qmul(h1, z0) - qmul(qf(c1), m), f2 = q_br2(0) + qmul(h2, z0) - qmul(qf(c2), m);
+    const Qf zi = qf(qmul(qf(qmul(zf, ui)), y));  // Im(z) y 2^-kz
+    r.Ar = qmul(qf(f1 + qmul(qf(f2), w2)), y);
+    r.Br = qmul(qf(f2), y);
+    r.Ai = qmul(qf(b1 + qmul(h2, w2)), zi);
+    r.Bi = qmul(h2, zi);
+    r.x = 1023 - g.r.e;
+    r.xi = kz;
+    return r;
+}
+FLG_HD FxRadialC fx_closed(const FxDir &g, const FxZ &zz, const FxAlphaC &al) {
+    const Qf y = qf(g.r.y), w2 = qf(g.w2), zf = qf(zz.m), ui = qf(al.ui);
+    const int E = g.r.e - 1023, kz = zz.k;
+    FxRadialC r;
     // F1 and F2 over 2^sc: below 1 at |z| < 1, up to 4 and 7 above
     const int sc = kz == 0 ? 0 : 3;
     q60 F1r = -(kQ1 >> sc), F1i = 0, F2r = 3 * (kQ1 >> sc), F2i = 0;
@@ -424,6 +432,11 @@ FLG_HD FxRadialC fx_brinkman_c(const FxDir &g, const FxAlphaC &al) {
     r.xi = 0;
     return r;
 }
+FLG_HD FxRadialC fx_brinkman(const FxDir &g, const FxAlphaC &al) {
+    const FxZ z = fx_z(g, al.am, al.ae);
+    return z.k < 0 ? fx_series(g, z, al) : fx_closed(g, z, al);
+}
+
 // the two parts of one real strength vector: ur = (Ar F + Br t n), ui = (Ai F + Bi t n), t = F.n
 FLG_HD void fx_radial_apply_c(const FxDir &g, const FxRadialC &r, const q60 *F, q60 *ur, q60 *ui) {
     const Qf n0 = qf(g.n[0]), n1 = qf(g.n[1]), n2 = qf(g.n[2]), f0 = qf(F[0]), f1 = qf(F[1]), f2 = qf(F[2]);

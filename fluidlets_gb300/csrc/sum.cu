@@ -167,10 +167,17 @@ __global__ void __launch_bounds__(kF64Threads) sum_f64_kernel(SumArgs a) {
 // ranges takes the FP64 function; a complex alpha that fx_alpha_c_ok refuses takes sum_f64_kernel.
 // The wall kernel's factor t is applied once at the end, its factor h in the staged strengths.
 // Bound by the integer pipe.  FP64 pairs -> fixed point: 32,768 x 1,003 wall 3.6 -> 1.2 ms, 16,384 x
-// 16,384 Brinkman 33 -> 12 ms, 4,099 x 2,500 complex Brinkman 6.0 -> 1.7 ms (four CTAs per SM; the
-// complex pair's registers allow three: 1.81 ms a call with two or three, 1.84 with four).
+// 16,384 Brinkman 33 -> 12 ms, 4,099 x 2,500 complex Brinkman 6.0 -> 1.2 ms (four CTAs per SM; three
+// for the complex pair: 1.33 ms a call, 1.34 with two).
 // ---------------------------------------------------------------------------
 constexpr int kFxThreads = 128, kFxTile = 64;
+static_assert(kFxTile <= 64, "one bit per source of a tile");
+// Brinkman pairs of small z take a series, the others an exponential.  Where fewer than this many lanes
+// of a warp are in the series' range, they put it off to the end of the tile, where each lane
+// works through its own list: with one pair in sixteen in the range a warp runs the series for 9 of
+// 64 sources and not for 55.  16,384 x 16,384 (two sums within a solve): 58.6 ms of the solve with
+// the series at once, 55.7 with 12, 56.0 with 20; 4,099 x 2,500 complex: 1.56, 1.33, 1.32 ms.
+constexpr int kFxLowNow = 12;
 template <bool CK>
 using FxAlphaOf = typename std::conditional<CK, FxAlphaC, FxAlpha>::type;
 template <int NF>
@@ -190,14 +197,36 @@ __device__ __forceinline__ void fx_strengths(double *f, double h, q60 *F, int *e
 // pairs between two readings of the accumulators: 16 terms
 template <int NF, bool CK>
 constexpr int kFxPairs = CK ? kFxSeg / NF : kFxSeg;
+// adds the velocity of the strengths F 2^ef
+template <int NF, class R>
+__device__ __forceinline__ void fx_add_radial(const FxDir &g, const R &r, const q60 *F, const int *ef, FxAcc<3> *acc) {
+#pragma unroll
+    for (int c = 0; c < NF; c++) {
+        q60 t[3], im[3];
+        const int x = r.x + ef[c];
+        acc[c].scale(x);
+        if constexpr (std::is_same<R, FxRadialC>::value) {
+            fx_radial_apply_c(g, r, F + 3 * c, t, im);
+            if (c == 1)  // i f: real part -A_im f, imaginary part A_re f
+#pragma unroll
+                for (int k = 0; k < 3; k++) im[k] = -im[k];
+            acc[1 - c].scale(x + r.xi);
+            acc[1 - c].add(0, im, x + r.xi);
+        } else {
+            fx_radial_apply(g, r, F + 3 * c, t);
+        }
+        acc[c].add(0, t, x);
+    }
+}
+template <int NF>
+__device__ __forceinline__ bool fx_ok(const int *ef) { return ef[0] != kFxBad && (NF == 1 || ef[NF - 1] != kFxBad); }
 // adds one pair; false: outside the fixed-point ranges
 template <int KIND, int NF, bool CK>
 __device__ __forceinline__ bool pair_fx(double tx, double ty, double tz, double sx, double sy, double sz, double e,
                                         double e2, const q60 *F, const int *ef, const FxAlphaOf<CK> &al,
                                         FxAcc<3> *acc) {
     const double d0 = tx - sx, d1 = ty - sy, d2 = tz - sz;
-    if (ef[0] == kFxBad || (NF == 2 && ef[NF - 1] == kFxBad)) return false;
-    q60 t[3];
+    if (!fx_ok<NF>(ef)) return false;
     if constexpr (KIND == FLG_WALL) {
         const double dp = tz + sz;
         const double rq = fma(d1, d1, fma(d0, d0, e2)), QF = fma(d2, d2, rq), QI = fma(dp, dp, rq);
@@ -205,6 +234,7 @@ __device__ __forceinline__ bool pair_fx(double tx, double ty, double tz, double 
         const FxWall w = fx_wall(d0, d1, d2, dp, QF, QI, e);
 #pragma unroll
         for (int c = 0; c < NF; c++) {
+            q60 t[3];
             const int x = fx_wall_apply(w, F + 3 * c, t) + ef[c];
             acc[c].scale(x);
             acc[c].add(0, t, x);
@@ -213,30 +243,8 @@ __device__ __forceinline__ bool pair_fx(double tx, double ty, double tz, double 
         const double Q = fma(d2, d2, fma(d1, d1, fma(d0, d0, e2)));
         if (!q_in_range(Q)) return false;
         const FxDir g = fx_dir(d0, d1, d2, Q, e);
-        if constexpr (CK) {
-            const FxRadialC r = fx_brinkman_c(g, al);
-#pragma unroll
-            for (int c = 0; c < NF; c++) {  // i f: real part -A_im f, imaginary part A_re f
-                q60 im[3];
-                fx_radial_apply_c(g, r, F + 3 * c, t, im);
-                if (c == 1)
-#pragma unroll
-                    for (int k = 0; k < 3; k++) im[k] = -im[k];
-                const int x = r.x + ef[c];
-                acc[c].scale(x);
-                acc[c].add(0, t, x);
-                acc[1 - c].scale(x + r.xi);
-                acc[1 - c].add(0, im, x + r.xi);
-            }
-        } else {
-            const FxRadial r = KIND == FLG_STOKESLET ? fx_stokeslet(g) : fx_brinkman(g, al);
-#pragma unroll
-            for (int c = 0; c < NF; c++) {
-                acc[c].scale(r.x + ef[c]);
-                fx_radial_apply(g, r, F + 3 * c, t);
-                acc[c].add(0, t, r.x + ef[c]);
-            }
-        }
+        if constexpr (KIND == FLG_STOKESLET) fx_add_radial<NF>(g, fx_stokeslet(g), F, ef, acc);
+        else fx_add_radial<NF>(g, fx_brinkman(g, al), F, ef, acc);
     }
     return true;
 }
@@ -279,6 +287,7 @@ sum_fx_kernel(SumArgs a, FxAlphaOf<CK> al) {
             s_src[k] = s;
         }
         __syncthreads();
+        unsigned long long later = 0;  // sources of this target whose series is put off
         for (int k0 = 0; k0 < cnt; k0 += SEG) {
 #pragma unroll
             for (int c = 0; c < OUTW / 3; c++) acc[c].clear();
@@ -286,11 +295,53 @@ sum_fx_kernel(SumArgs a, FxAlphaOf<CK> al) {
 #pragma unroll 1
             for (int k = k0; k < k1; k++) {
                 const FxSource<NF> &s = s_src[k];
-                if (!pair_fx<KIND, NF, CK>(tx, ty, tz, s.x, s.y, s.z, s.e, s.e2, s_f[k], s.ef, al, acc))
+                if constexpr (KIND == FLG_BRINKMANLET) {
+                    const double d0 = tx - s.x, d1 = ty - s.y, d2 = tz - s.z;
+                    const double Q = fma(d2, d2, fma(d1, d1, fma(d0, d0, s.e2)));
+                    const bool ok = fx_ok<NF>(s.ef) && q_in_range(Q);
+                    FxDir g;
+                    FxZ z{0, 0};
+                    if (ok) {
+                        g = fx_dir(d0, d1, d2, Q, s.e);
+                        z = fx_z(g, al.am, al.ae);
+                    }
+                    const bool low = z.k < 0, now = __popc(__ballot_sync(0xffffffffu, low)) >= kFxLowNow;
+                    if (low && !now)
+                        later |= 1ull << k;
+                    else if (ok)
+                        fx_add_radial<NF>(g, low ? fx_series(g, z, al) : fx_closed(g, z, al), s_f[k], s.ef, acc);
+                    else
+                        pair_f64_slow<KIND, NF, CK>(tx, ty, tz, s, a.f, jt + k, a.alpha_re, a.alpha_im, us);
+                } else if (!pair_fx<KIND, NF, CK>(tx, ty, tz, s.x, s.y, s.z, s.e, s.e2, s_f[k], s.ef, al, acc)) {
                     pair_f64_slow<KIND, NF, CK>(tx, ty, tz, s, a.f, jt + k, a.alpha_re, a.alpha_im, us);
+                }
             }
 #pragma unroll
             for (int c = 0; c < OUTW; c++) u[c] += acc[c / 3].value(c % 3);
+        }
+        if constexpr (KIND == FLG_BRINKMANLET) {
+            if (__any_sync(0xffffffffu, later != 0)) {
+                int terms = SEG;
+#pragma unroll
+                for (int c = 0; c < OUTW / 3; c++) acc[c].clear();
+                while (later) {
+                    const int k = __ffsll((long long)later) - 1;
+                    later &= later - 1;
+                    const FxSource<NF> &s = s_src[k];
+                    const double d0 = tx - s.x, d1 = ty - s.y, d2 = tz - s.z;
+                    const FxDir g = fx_dir(d0, d1, d2, fma(d2, d2, fma(d1, d1, fma(d0, d0, s.e2))), s.e);
+                    fx_add_radial<NF>(g, fx_series(g, fx_z(g, al.am, al.ae), al), s_f[k], s.ef, acc);
+                    if (--terms == 0) {
+                        terms = SEG;
+#pragma unroll
+                        for (int c = 0; c < OUTW; c++) u[c] += acc[c / 3].value(c % 3);
+#pragma unroll
+                        for (int c = 0; c < OUTW / 3; c++) acc[c].clear();
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < OUTW; c++) u[c] += acc[c / 3].value(c % 3);
+            }
         }
     }
     if (i < a.M) {
