@@ -677,26 +677,37 @@ __global__ void __launch_bounds__(kLuT *kLuT) diag_lowp_kernel(float *A, int64_t
         }
 }
 
-// The panels of one LU step, U12 = L11^-1 A12 and L21 = A21 U11^-1, both in one launch: a CTA takes 32
-// columns (or rows) and substitutes in 32-row blocks.  Block b's right-hand side loses its products
-// with the blocks before it (warp w four of the 32 rows, lane = column: 16 FMAs per 8 shared loads),
-// and the 32 x 32 diagonal block's inverse, which four warps work out while the CTA loads its
-// columns, is one more such product: no chain longer than 32.  As products with 128 x 128 inverses
-// the panels took a transpose and two tensor-core launches, and the inverses as long as the diagonal
-// block itself.
-// A CTA that has several groups of columns keeps the block and the inverses; with NC = 2 a lane takes
-// two columns (32 FMAs per 12 loads), which pays once the groups of 32 outnumber the CTAs that fit
-// (two per SM).  Whole factorisation with NC = 2 from 1, 2 or 4 groups a CTA on, or never: n = 9,000
-// (tf32) 4.86, 4.98, 4.99, 5.00 ms; n = 24,576 (bf16) 25.6, 25.8, 26.1, 26.5 ms.
-constexpr int kSb = 32, kPanelThreads = 256;
+// The panels of one LU step, U12 = L11^-1 A12 and L21 = A21 U11^-1, both in one launch: a team of warps
+// takes 32 NC columns (or rows) and substitutes in 32-row blocks.  Block b's right-hand side loses its
+// products with the blocks before it (a warp RW of the 32 rows, lane = column), and the 32 x 32
+// diagonal block's inverse, which four warps work out while the teams load their columns, is one
+// more such product: no chain longer than 32.  As products with 128 x 128 inverses the panels took a
+// transpose and two tensor-core launches, and the inverses as long as the diagonal block itself.
+// Bound by the latency of few warps (2 per scheduler, 48 % of issue slots).  Small panels: 32 columns a
+// CTA of eight warps, 4 rows each, two CTAs per SM.  Once the groups of 32 outnumber those, CTAs
+// that go through several groups with the block and its inverses kept: two teams of four warps,
+// 8 rows x 2 columns a lane (64 FMAs per 16 loads).  Whole factorisation at n = 9,000 (tf32) and 24,576
+// (bf16), ms: 32 columns throughout 5.00, 26.5; one team of eight warps, 4 rows x 2 columns 4.92, 23.7;
+// two 4.86, 23.8; two of four warps, 8 x 2 4.82, 23.7; 8 x 4 5.20, 24.2; three teams 5.03, 23.9.
+constexpr int kSb = 32;
 template <int NC>
-struct LowpPanelSmem {
-    static constexpr int LD = 32 * NC + 1;  // row stride of the CTA's columns
-    float T[kNB][kNB];              // the diagonal block's factors
-    float inv[kNB / kSb][kSb][kSb];  // inverses of L's (U panel) or U's (L panel) 32 x 32 diagonal blocks
-    float H[kNB][LD];               // right-hand sides, then results: element k of column (row) i
-    float R[kSb][LD];
+struct LowpTeam {
+    static constexpr int LD = 32 * NC + 1;  // row stride of the team's columns
+    float H[kNB][LD];                // right-hand sides, then results: element k of column (row) i
 };
+template <int NC, int NT>
+struct LowpPanelSmem {
+    float T[kNB][kNB];               // the diagonal block's factors
+    float inv[kNB / kSb][kSb][kSb];  // inverses of L's (U panel) or U's (L panel) 32 x 32 diagonal blocks
+    LowpTeam<NC> team[NT];
+};
+// a team: 32 / RW warps of RW rows of each 32-row block
+template <int RW>
+constexpr int kTeamThreads = 32 * (kSb / RW);
+template <int RW>
+__device__ __forceinline__ void team_sync(int team) {
+    asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kTeamThreads<RW>) : "memory");
+}
 struct LowpPanelArgs {
     float *A;
     int64_t ld, k0, nr, sA;   // trailing rows and columns k0 + 128 ... (per system)
@@ -707,21 +718,23 @@ struct LowpPanelArgs {
     int ntu;                  // CTAs of the U panel
 };
 // rows [k0, k0 + nb) of the factored block, padded with the identity
+template <int THREADS>
 __device__ __forceinline__ void load_factors(const float *A, int64_t ld, int64_t k0, int nb, float (*T)[kNB]) {
     if (nb == kNB) {
-        float4 v[kNB * kNB / 4 / kPanelThreads];
+        constexpr int Q = (kNB * kNB / 4 + THREADS - 1) / THREADS;
+        float4 v[Q];
 #pragma unroll
-        for (int q = 0; q < kNB * kNB / 4 / kPanelThreads; q++) {
-            const int e = threadIdx.x + q * kPanelThreads, r = e / (kNB / 4), c = e % (kNB / 4) * 4;
-            v[q] = *reinterpret_cast<const float4 *>(A + (k0 + r) * ld + k0 + c);
+        for (int q = 0; q < Q; q++) {
+            const int e = threadIdx.x + q * THREADS, r = e / (kNB / 4), c = e % (kNB / 4) * 4;
+            if (e < kNB * kNB / 4) v[q] = *reinterpret_cast<const float4 *>(A + (k0 + r) * ld + k0 + c);
         }
 #pragma unroll
-        for (int q = 0; q < kNB * kNB / 4 / kPanelThreads; q++) {
-            const int e = threadIdx.x + q * kPanelThreads;
-            *reinterpret_cast<float4 *>(&T[e / (kNB / 4)][e % (kNB / 4) * 4]) = v[q];
+        for (int q = 0; q < Q; q++) {
+            const int e = threadIdx.x + q * THREADS;
+            if (e < kNB * kNB / 4) *reinterpret_cast<float4 *>(&T[e / (kNB / 4)][e % (kNB / 4) * 4]) = v[q];
         }
     } else {
-        for (int e = threadIdx.x; e < kNB * kNB; e += kPanelThreads) {
+        for (int e = threadIdx.x; e < kNB * kNB; e += THREADS) {
             const int r = e / kNB, c = e % kNB;
             T[r][c] = r < nb && c < nb ? A[(k0 + r) * ld + k0 + c] : (r == c ? 1.0f : 0.0f);
         }
@@ -752,167 +765,196 @@ __device__ __forceinline__ void inverse32(const float (*T)[kNB], int b0, float (
 #pragma unroll
     for (int r = 0; r < kSb; r++) out[r][lane] = x[r];
 }
-// acc[row][column of this lane] -= (or +=) M (4 rows from r0) . V (K rows), four of K at a time; M row-major
+// acc[row][column of this lane] -= (or +=) M (RW rows from r0) . V (K rows), four of K at a time; M row-major
 // from m0, or for the L panel its transpose's rows
-template <bool UPANEL, int NC, int K_UNROLL, int MLD, int VLD>
-__device__ __forceinline__ void panel_product(float (&acc)[4][NC], const float *M, const float *V, int K, float sign,
+template <bool UPANEL, int RW, int NC, int K_UNROLL, int MLD, int VLD>
+__device__ __forceinline__ void panel_product(float (&acc)[RW][NC], const float *M, const float *V, int K, float sign,
                                               int lane) {
 #pragma unroll K_UNROLL
     for (int k = 0; k < K; k += 4) {
         float h[4][NC];
-        float4 t[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-#pragma unroll
-            for (int c = 0; c < NC; c++) h[e][c] = sign * V[(k + e) * VLD + lane + 32 * c];
-            t[e] = *reinterpret_cast<const float4 *>(UPANEL ? M + e * MLD + k : M + (k + e) * MLD);
-        }
 #pragma unroll
         for (int e = 0; e < 4; e++)
 #pragma unroll
-            for (int c = 0; c < NC; c++) {
-                if (UPANEL) {
-                    acc[e][c] = fmaf(t[e].x, h[0][c], acc[e][c]), acc[e][c] = fmaf(t[e].y, h[1][c], acc[e][c]);
-                    acc[e][c] = fmaf(t[e].z, h[2][c], acc[e][c]), acc[e][c] = fmaf(t[e].w, h[3][c], acc[e][c]);
-                } else {
-                    acc[0][c] = fmaf(t[e].x, h[e][c], acc[0][c]), acc[1][c] = fmaf(t[e].y, h[e][c], acc[1][c]);
-                    acc[2][c] = fmaf(t[e].z, h[e][c], acc[2][c]), acc[3][c] = fmaf(t[e].w, h[e][c], acc[3][c]);
+            for (int c = 0; c < NC; c++) h[e][c] = sign * V[(k + e) * VLD + lane + 32 * c];
+        if (UPANEL) {
+#pragma unroll
+            for (int i = 0; i < RW; i++) {
+                const float4 t = *reinterpret_cast<const float4 *>(M + i * MLD + k);
+#pragma unroll
+                for (int c = 0; c < NC; c++) {
+                    acc[i][c] = fmaf(t.x, h[0][c], acc[i][c]), acc[i][c] = fmaf(t.y, h[1][c], acc[i][c]);
+                    acc[i][c] = fmaf(t.z, h[2][c], acc[i][c]), acc[i][c] = fmaf(t.w, h[3][c], acc[i][c]);
                 }
             }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+#pragma unroll
+                for (int i = 0; i < RW; i += 4) {
+                    const float4 t = *reinterpret_cast<const float4 *>(M + (k + e) * MLD + i);
+#pragma unroll
+                    for (int c = 0; c < NC; c++) {
+                        acc[i][c] = fmaf(t.x, h[e][c], acc[i][c]), acc[i + 1][c] = fmaf(t.y, h[e][c], acc[i + 1][c]);
+                        acc[i + 2][c] = fmaf(t.z, h[e][c], acc[i + 2][c]);
+                        acc[i + 3][c] = fmaf(t.w, h[e][c], acc[i + 3][c]);
+                    }
+                }
+        }
     }
 }
-// the substitution of the CTA's columns in S.H
-template <bool UPANEL, int NC>
-__device__ __forceinline__ void panel_solve(LowpPanelSmem<NC> &S, int warp, int lane) {
-    constexpr int LD = LowpPanelSmem<NC>::LD;
+// the substitution of the team's columns in its H, RW rows of each block per warp
+template <bool UPANEL, int RW, int NC, int NT>
+__device__ __forceinline__ void panel_solve(LowpPanelSmem<NC, NT> &S, int team, int warp, int lane) {
+    constexpr int LD = LowpTeam<NC>::LD;
+    LowpTeam<NC> &m = S.team[team];
     for (int b = 0; b < kNB / kSb; b++) {
-        const int r0 = b * kSb + 4 * warp;
-        float acc[4][NC];
+        const int r0 = b * kSb + RW * warp;
+        float acc[RW][NC];
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < RW; i++)
 #pragma unroll
-            for (int c = 0; c < NC; c++) acc[i][c] = S.H[r0 + i][lane + 32 * c];
-        panel_product<UPANEL, NC, 2, kNB, LD>(acc, UPANEL ? &S.T[r0][0] : &S.T[0][r0], &S.H[0][0], b * kSb, -1.0f, lane);
+            for (int c = 0; c < NC; c++) acc[i][c] = m.H[r0 + i][lane + 32 * c];
+        panel_product<UPANEL, RW, NC, 2, kNB, LD>(acc, UPANEL ? &S.T[r0][0] : &S.T[0][r0], &m.H[0][0], b * kSb, -1.0f,
+                                                  lane);
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < RW; i++)
 #pragma unroll
-            for (int c = 0; c < NC; c++) S.R[4 * warp + i][lane + 32 * c] = acc[i][c], acc[i][c] = 0.0f;
-        __syncthreads();
-        panel_product<UPANEL, NC, 8, kSb, LD>(acc, UPANEL ? &S.inv[b][4 * warp][0] : &S.inv[b][0][4 * warp], &S.R[0][0],
-                                              kSb, 1.0f, lane);
+            for (int c = 0; c < NC; c++) m.H[r0 + i][lane + 32 * c] = acc[i][c], acc[i][c] = 0.0f;
+        team_sync<RW>(team);
+        panel_product<UPANEL, RW, NC, RW == 4 ? 8 : 2, kSb, LD>(
+            acc, UPANEL ? &S.inv[b][RW * warp][0] : &S.inv[b][0][RW * warp], &m.H[b * kSb][0], kSb, 1.0f, lane);
+        team_sync<RW>(team);  // the block's right-hand sides have been read
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < RW; i++)
 #pragma unroll
-            for (int c = 0; c < NC; c++) S.H[r0 + i][lane + 32 * c] = acc[i][c];
-        __syncthreads();
+            for (int c = 0; c < NC; c++) m.H[r0 + i][lane + 32 * c] = acc[i][c];
+        team_sync<RW>(team);
     }
 }
-// row i of the CTA's results (element k of column / row i), 128 contiguous values, one warp
+// row i of the team's results (element k of column / row i), 128 contiguous values, one warp
 template <int NC>
-__device__ __forceinline__ float4 result4(const LowpPanelSmem<NC> &S, int i, int lane) {
-    return make_float4(S.H[4 * lane][i], S.H[4 * lane + 1][i], S.H[4 * lane + 2][i], S.H[4 * lane + 3][i]);
+__device__ __forceinline__ float4 result4(const LowpTeam<NC> &m, int i, int lane) {
+    return make_float4(m.H[4 * lane][i], m.H[4 * lane + 1][i], m.H[4 * lane + 2][i], m.H[4 * lane + 3][i]);
 }
 __device__ __forceinline__ void store_bf16x4(__nv_bfloat16 *o, float4 v) {
     const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
     *reinterpret_cast<uint2 *>(o) = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
 }
-template <int NC>
-__global__ void __launch_bounds__(kPanelThreads, 3 - NC) lowp_panel_kernel(LowpPanelArgs a) {
+template <int NC, int NT, int RW>
+__global__ void __launch_bounds__(kTeamThreads<RW> *NT, NT == 1 ? 2 : 1) lowp_panel_kernel(LowpPanelArgs a) {
     extern __shared__ __align__(16) uint8_t raw[];
-    LowpPanelSmem<NC> &S = *reinterpret_cast<LowpPanelSmem<NC> *>(raw);
-    constexpr int CW = 32 * NC;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, z = blockIdx.y;
+    LowpPanelSmem<NC, NT> &S = *reinterpret_cast<LowpPanelSmem<NC, NT> *>(raw);
+    constexpr int CW = 32 * NC, TW = kSb / RW;  // columns and warps of a team
+    constexpr int LU = 16 / NC, LL = 8;         // rows (columns of A21^T) of a warp in flight while loading
+    const int team = threadIdx.x / kTeamThreads<RW>, warp = (threadIdx.x % kTeamThreads<RW>) >> 5,
+              lane = threadIdx.x & 31;
+    const int z = blockIdx.y;
+    LowpTeam<NC> &m = S.team[team];
     float *A = a.A + z * a.sA;
     const bool up = (int)blockIdx.x < a.ntu;
-    load_factors(A, a.ld, a.k0, kNB, S.T);
+    load_factors<kTeamThreads<RW> * NT>(A, a.ld, a.k0, kNB, S.T);
     __syncthreads();
-    if (warp < kNB / kSb) {
-        if (up) inverse32<true>(S.T, warp * kSb, S.inv[warp], lane);
-        else inverse32<false>(S.T, warp * kSb, S.inv[warp], lane);
+    if (threadIdx.x < 32 * (kNB / kSb)) {
+        const int b = threadIdx.x >> 5;
+        if (up) inverse32<true>(S.T, b * kSb, S.inv[b], lane);
+        else inverse32<false>(S.T, b * kSb, S.inv[b], lane);
     }
-    for (int64_t w0 = (int64_t)(up ? blockIdx.x : blockIdx.x - a.ntu) * CW; w0 < a.nr; w0 += (int64_t)a.ntu * CW) {
-        const int cnt = (int)min((int64_t)CW, a.nr - w0);
+    bool first = true;
+    const int64_t cta = up ? blockIdx.x : blockIdx.x - a.ntu;
+    for (int64_t w0 = (cta * NT + team) * CW; first || w0 < a.nr; w0 += (int64_t)a.ntu * NT * CW) {
+        const int cnt = (int)max((int64_t)0, min((int64_t)CW, a.nr - w0));
         float *A12 = A + a.k0 * a.ld + a.k0 + kNB + w0, *A21 = A + (a.k0 + kNB + w0) * a.ld + a.k0;
         if (up) {
-            float v[kNB / 8][NC];
+#pragma unroll 1
+            for (int q0 = warp; q0 < kNB; q0 += TW * LU) {
+                float v[LU][NC];
 #pragma unroll
-            for (int q = 0; q < kNB / 8; q++)
+                for (int q = 0; q < LU; q++)
 #pragma unroll
-                for (int c = 0; c < NC; c++)
-                    v[q][c] = lane + 32 * c < cnt ? A12[(warp + 8 * q) * a.ld + lane + 32 * c] : 0.0f;
+                    for (int c = 0; c < NC; c++)
+                        v[q][c] = lane + 32 * c < cnt ? A12[(q0 + TW * q) * a.ld + lane + 32 * c] : 0.0f;
 #pragma unroll
-            for (int q = 0; q < kNB / 8; q++)
+                for (int q = 0; q < LU; q++)
 #pragma unroll
-                for (int c = 0; c < NC; c++) S.H[warp + 8 * q][lane + 32 * c] = v[q][c];
+                    for (int c = 0; c < NC; c++) m.H[q0 + TW * q][lane + 32 * c] = v[q][c];
+            }
         } else {
-            float4 v[4 * NC];
+            constexpr int LB = LL < CW / TW ? LL : CW / TW;
+#pragma unroll 1
+            for (int q0 = warp; q0 < CW; q0 += TW * LB) {
+                float4 v[LB];
 #pragma unroll
-            for (int q = 0; q < 4 * NC; q++)
-                v[q] = warp + 8 * q < cnt ? *reinterpret_cast<const float4 *>(A21 + (warp + 8 * q) * a.ld + 4 * lane)
-                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int q = 0; q < LB; q++)
+                    v[q] = q0 + TW * q < cnt ? *reinterpret_cast<const float4 *>(A21 + (q0 + TW * q) * a.ld + 4 * lane)
+                                             : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int q = 0; q < 4 * NC; q++) {
-                const int i = warp + 8 * q;
-                S.H[4 * lane][i] = v[q].x, S.H[4 * lane + 1][i] = v[q].y;
-                S.H[4 * lane + 2][i] = v[q].z, S.H[4 * lane + 3][i] = v[q].w;
+                for (int q = 0; q < LB; q++) {
+                    const int i = q0 + TW * q;
+                    m.H[4 * lane][i] = v[q].x, m.H[4 * lane + 1][i] = v[q].y;
+                    m.H[4 * lane + 2][i] = v[q].z, m.H[4 * lane + 3][i] = v[q].w;
+                }
             }
         }
-        __syncthreads();
-        if (up) panel_solve<true, NC>(S, warp, lane);
-        else panel_solve<false, NC>(S, warp, lane);
+        if (first) __syncthreads();  // the inverses are there, too
+        else team_sync<RW>(team);
+        first = false;
+        if (up) panel_solve<true, RW>(S, team, warp, lane);
+        else panel_solve<false, RW>(S, team, warp, lane);
         if (up) {
-#pragma unroll
-            for (int q = 0; q < kNB / 8; q++)
+#pragma unroll 4
+            for (int q = warp; q < kNB; q += TW)
 #pragma unroll
                 for (int c = 0; c < NC; c++)
-                    if (lane + 32 * c < cnt) A12[(warp + 8 * q) * a.ld + lane + 32 * c] = S.H[warp + 8 * q][lane + 32 * c];
+                    if (lane + 32 * c < cnt) A12[q * a.ld + lane + 32 * c] = m.H[q][lane + 32 * c];
         }
-        for (int i = warp; i < cnt; i += 8) {
-            const float4 v = result4<NC>(S, i, lane);
+#pragma unroll 2
+        for (int i = warp; i < cnt; i += TW) {
+            const float4 v = result4<NC>(m, i, lane);
             const int64_t r = w0 + i;
             if (!up) *reinterpret_cast<float4 *>(A21 + i * a.ld + 4 * lane) = v;
             else if (a.Ut) *reinterpret_cast<float4 *>(a.Ut + z * a.sU + r * a.ldu + 4 * lane) = v;
             if (a.Lb) store_bf16x4((up ? a.Ub : a.Lb) + z * a.sB + r * a.ldb + 4 * lane, v);
         }
-        __syncthreads();  // every result is out before the next group's columns come in
+        team_sync<RW>(team);  // every result is out before the next group's columns come in
     }
+}
+template <int NC, int NT, int RW>
+static int launch_panels(LowpPanelArgs &a, int nbat, int64_t ctas, cudaStream_t st) {
+    constexpr size_t smem = sizeof(LowpPanelSmem<NC, NT>);
+    static bool attr_set = false;
+    if (!attr_set) {
+        FLG_CUDA(cudaFuncSetAttribute(lowp_panel_kernel<NC, NT, RW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
+        attr_set = true;
+    }
+    a.ntu = (int)std::min<int64_t>(ceil_div(a.nr, 32 * NC * NT), std::max<int64_t>(1, ctas / 2 / nbat));
+    lowp_panel_kernel<NC, NT, RW><<<dim3(2 * a.ntu, nbat), kTeamThreads<RW> * NT, smem, st>>>(a);
+    FLG_LAUNCH_CHECK();
+    return FLG_OK;
 }
 static int lowp_panels(LowpPanelArgs &a, int nbat, cudaStream_t st) {
     // groups of 32 columns or rows in each panel against two CTAs per SM
     const int64_t groups = ceil_div(a.nr, 32) * nbat, slots = 2LL * sm_count();
-    static bool attr_set = false;
-    if (!attr_set) {
-        FLG_CUDA(cudaFuncSetAttribute(lowp_panel_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sizeof(LowpPanelSmem<1>)));
-        FLG_CUDA(cudaFuncSetAttribute(lowp_panel_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sizeof(LowpPanelSmem<2>)));
-        attr_set = true;
-    }
-    if (2 * groups <= slots) {
-        a.ntu = (int)std::min<int64_t>(ceil_div(a.nr, 32), std::max<int64_t>(1, slots / 2 / nbat));
-        lowp_panel_kernel<1><<<dim3(2 * a.ntu, nbat), kPanelThreads, sizeof(LowpPanelSmem<1>), st>>>(a);
-    } else {
-        a.ntu = (int)std::min<int64_t>(ceil_div(a.nr, 64), std::max<int64_t>(1, slots / 4 / nbat));
-        lowp_panel_kernel<2><<<dim3(2 * a.ntu, nbat), kPanelThreads, sizeof(LowpPanelSmem<2>), st>>>(a);
-    }
-    FLG_LAUNCH_CHECK();
-    return FLG_OK;
+    return 2 * groups <= slots ? launch_panels<1, 1, 4>(a, nbat, slots, st)
+                               : launch_panels<2, 2, 8>(a, nbat, slots / 2, st);
 }
 
 // The inverses of the diagonal blocks' unit-lower and upper factors (the solves use them), all blocks
 // of all systems in one launch after the factorization: the panels' substitution applied to the
 // identity.  blockIdx = (block and its 32 columns or rows, inverse of L or of U, system)
-__global__ void __launch_bounds__(kPanelThreads, 2) block_inverse_kernel(const float *A, int64_t ld, int64_t n, int64_t sA,
+__global__ void __launch_bounds__(kTeamThreads<4>, 2) block_inverse_kernel(const float *A, int64_t ld, int64_t n, int64_t sA,
                                                                          float *Linv, float *Uinv, int64_t sD) {
     extern __shared__ __align__(16) uint8_t raw[];
-    LowpPanelSmem<1> &S = *reinterpret_cast<LowpPanelSmem<1> *>(raw);
+    LowpPanelSmem<1, 1> &S = *reinterpret_cast<LowpPanelSmem<1, 1> *>(raw);
+    LowpTeam<1> &m = S.team[0];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, w0 = (int)(blockIdx.x % 4) * 32;
     const int64_t k0 = (int64_t)(blockIdx.x / 4) * kNB;
     const bool up = blockIdx.y == 0;
     A += blockIdx.z * sA;
     float *o = (up ? Linv : Uinv) + blockIdx.z * sD + k0 * kNB;
-    load_factors(A, ld, k0, (int)min((int64_t)kNB, n - k0), S.T);
-    for (int k = warp; k < kNB; k += 8) S.H[k][lane] = k == w0 + lane ? 1.0f : 0.0f;
+    load_factors<kTeamThreads<4>>(A, ld, k0, (int)min((int64_t)kNB, n - k0), S.T);
+    for (int k = warp; k < kNB; k += 8) m.H[k][lane] = k == w0 + lane ? 1.0f : 0.0f;
     __syncthreads();
     if (warp < kNB / kSb) {
         if (up) inverse32<true>(S.T, warp * kSb, S.inv[warp], lane);
@@ -920,11 +962,11 @@ __global__ void __launch_bounds__(kPanelThreads, 2) block_inverse_kernel(const f
     }
     __syncthreads();
     if (up) {
-        panel_solve<true, 1>(S, warp, lane);
-        for (int k = warp; k < kNB; k += 8) o[k * kNB + w0 + lane] = S.H[k][lane];
+        panel_solve<true, 4>(S, 0, warp, lane);
+        for (int k = warp; k < kNB; k += 8) o[k * kNB + w0 + lane] = m.H[k][lane];
     } else {
-        panel_solve<false, 1>(S, warp, lane);
-        for (int i = warp; i < 32; i += 8) reinterpret_cast<float4 *>(o + (w0 + i) * kNB)[lane] = result4<1>(S, i, lane);
+        panel_solve<false, 4>(S, 0, warp, lane);
+        for (int i = warp; i < 32; i += 8) reinterpret_cast<float4 *>(o + (w0 + i) * kNB)[lane] = result4<1>(m, i, lane);
     }
 }
 
@@ -1606,25 +1648,31 @@ static int side_stream(SideStream **out) {
 
 extern "C" int64_t flg_lu_lowp_dinv_elems(int64_t n) { return 2 * ceil_div(std::max<int64_t>(n, 1), kNB) * kNB * kNB; }
 
-// Tensor-core modes defer most of the trailing update: blocks are grouped into
-// outer panels of W columns [K0, E), W = outer_width(n).  Inner step k0 (diagonal block,
-// panels) updates only the L-shaped part of the Schur complement that the next
-// inner steps read -- rows > k0 x columns (k0, E), and rows (k0, E) x columns
-// >= E -- with rank-128 updates; the rest, rows and columns >= E, receives one
-// rank-(E - K0) update per outer panel, which moves the trailing matrix through
-// HBM W / 128 times less often.  The K-major copy of U (UtB: one row of W
-// per column >= K0) feeds both.  A wider W halves the trailing traffic again but
-// lengthens the chain of inner steps that nothing overlaps; measured on the
-// tensor-core modes (TF32 / BF16, factor + refinement): 1,024 columns is 6-9%
-// faster from n = 12,288 up and 2% slower at n = 4,608, so 512 below n = 8,192.
-static int64_t outer_width(int64_t n) { return (n >= 8192 ? 8 : 4) * (int64_t)kNB; }
+// Tensor-core modes defer most of the trailing update, on two levels: blocks are grouped into middle
+// panels of W1 columns [K1, E) and those into outer panels of W columns [K0, E2).  Inner step k0
+// (diagonal block, panels) updates only the L-shaped part of the Schur complement that the next
+// inner steps read -- rows > k0 x columns (k0, E), and rows (k0, E) x columns >= E -- with
+// rank-128 updates; after a middle panel the rest of the outer panel's columns and rows get one
+// rank-W1 update, and rows and columns >= E2 one rank-W update per outer panel.  A tile of C
+// costs the update kernel 1.9 GB of traffic per 472 million elements whatever the depth (rank 1,024 at
+// 15,360: 268 us of products alone, 358 us of C alone, 464 us together), so a deeper rank moves the trailing
+// matrix less often.  The K-major copy of U (UtB: one row of W per column >= K0) feeds all three.
+// Measured, factor with copies: W1 = W = 512 / W1 = W = 1,024 / 512 and 1,024 / 512 and 2,048:
+// n = 9,000 tf32 4.96 / 4.87 / 4.87 / 4.93 ms, bf16 4.58 / 4.44 / 4.40 / 4.43; n = 24,576 tf32
+// 34.2 / 32.0 / 31.2 / 31.7, bf16 30.4 / 25.5 / 24.4 / 23.5 (bf16 products take half as long, so that
+// C's traffic weighs more).  Below 8,192 unknowns one level of 512 is the fastest (4,608: 1.99, two
+// levels 2.05).
+static int64_t inner_width() { return 4 * (int64_t)kNB; }
+static int64_t outer_width(int64_t n, int mode) {
+    return inner_width() * (n < 8192 ? 1 : mode == FLG_LU_BF16 ? 4 : 2);
+}
 
 // scratch of nbat systems, system z's at + z n W floats; BF16 mode: the BF16 copies of the outer
 // panel's L columns and of UtB (n W each per system) in PB
 template <class Ar>
 static void lowp_carve(Ar &ar, int64_t n, int nbat, int mode, float **UtB, char **tcw, size_t *tcb,
                        __nv_bfloat16 **PB) {
-    const int64_t W = outer_width(n);
+    const int64_t W = outer_width(n, mode);
     *UtB = ar.template take<float>((size_t)nbat * n * W);
     // the updates take their operands as they are (TF32, or PB's BF16 copies): no operand workspace
     *tcb = (mode == FLG_LU_FP32) ? 0 : tc_update_bytes(n, n, W, FLG_LU_TF32, nbat);
@@ -1685,7 +1733,7 @@ static int lowp_factor(int64_t n, int nbat, float *A, int64_t ld, int64_t sA, in
     FLG_REQUIRE(UtB && (tcb == 0 || tcw) && (mode != FLG_LU_BF16 || PB), "workspace too small for LU (%zu bytes)",
                 work_bytes);
     int *dinfo = flags;  // [0] first bad pivot, [1] tensor-core wait timed out
-    const int64_t W = outer_width(n);  // outer panel width
+    const int64_t W = outer_width(n, mode), W1 = inner_width();  // outer and middle panel width
     // per-system strides: the matrix, the block inverses, U's K-major copy
     const int64_t sD = flg_lu_lowp_dinv_elems(n), sUt = n * W;
     const TcBatch bA{nbat, sA, sA, sUt};
@@ -1707,7 +1755,7 @@ static int lowp_factor(int64_t n, int nbat, float *A, int64_t ld, int64_t sA, in
     static bool attr_set = false;  // set once, so a later call can be captured in a graph
     if (!attr_set) {
         FLG_CUDA(cudaFuncSetAttribute(block_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sizeof(LowpPanelSmem<1>)));
+                                      (int)sizeof(LowpPanelSmem<1, 1>)));
         attr_set = true;
     }
     const bool tc = mode != FLG_LU_FP32;
@@ -1734,64 +1782,65 @@ static int lowp_factor(int64_t n, int nbat, float *A, int64_t ld, int64_t sA, in
         pending = true;
         return FLG_OK;
     };
+    // C[r0:, c0:] -= L U^T over columns [ka, kb) for rows [r0, r1) and columns [c0, c1): the first
+    // diagonal block of it, at (r0, c0), first when `ahead`, so that it factors beside the rest
+    auto block = [&](int64_t r0, int64_t r1, int64_t c0, int64_t c1, int64_t ka, int64_t kb, bool ahead) -> int {
+        float *C = A + r0 * ld + c0, *Lp = A + r0 * ld + ka, *Up = UtB + (c0 - K0) * W + (ka - K0);
+        const int64_t m = r1 - r0, nc = c1 - c0, K = kb - ka;
+        if (!ahead || m <= kNB) return upd(C, Lp, Up, m, nc, K, pending ? cap : 0);
+        FLG_TRY(upd(C, Lp, Up, std::min<int64_t>(kNB, m), std::min<int64_t>(kNB, nc), K, 0));
+        FLG_TRY(look_ahead(r0));
+        FLG_TRY(upd(C + kNB * ld, Lp + kNB * ld, Up, m - kNB, std::min<int64_t>(kNB, nc), K, cap));
+        if (nc > kNB) FLG_TRY(upd(C + kNB, Lp, Up + kNB * W, m, nc - kNB, K, cap));
+        return FLG_OK;
+    };
     for (K0 = 0; K0 < n; K0 += W) {
-        const int64_t E = std::min<int64_t>(n, K0 + W);
-        for (int64_t k0 = K0; k0 < E; k0 += kNB) {
-            const int nb = (int)std::min<int64_t>(kNB, n - k0);
-            if (pending) {  // this block's diagonal kernel ran ahead on the side stream
-                FLG_CUDA(cudaStreamWaitEvent(st, side->join, 0));
-                pending = false;
-            } else {
-                diag(k0, st);
-                FLG_LAUNCH_CHECK();
-            }
-            const int64_t c0 = k0 + nb, nr = n - c0;
-            if (nr <= 0) continue;
-            prof_begin(FLG_SLOT_LU_PANEL, st);
-            // (nb < kNB only for the last block, which has no trailing part)
-            float *A12 = A + k0 * ld + c0, *A21 = A + c0 * ld + k0, *A22 = A + c0 * ld + c0;
-            float *Ut = UtB + (c0 - K0) * W + (k0 - K0);  // row: column - K0; K offset: k0 - K0
-            LowpPanelArgs pa{A, ld, k0, nr, sA, tc ? Ut : nullptr, W, sUt, nullptr, nullptr, W, n * W, 0};
-            if (mode == FLG_LU_BF16) pa.Ut = nullptr, pa.Lb = LB + c0 * W + (k0 - K0), pa.Ub = UB + (Ut - UtB);
-            FLG_TRY(lowp_panels(pa, nbat, st));
-            prof_end(FLG_SLOT_LU_PANEL, st);
-            prof_begin(FLG_SLOT_LU_UPDATE, st);
-            if (!tc) {
-                FLG_TRY(sgemm(st, nr, nr, nb, -1.0f, A21, ld, A12, ld, 1.0f, A22, ld));
-            } else if (E > c0) {
-                if (n - c0 > kNB) {
-                    // the next diagonal block first, then it factors beside the rest:
-                    // rows > c0 + 128 x its columns, rows > k0 x columns (c0 + 128, E)
-                    FLG_TRY(upd(A22, A21, Ut, kNB, kNB, kNB, 0));
-                    FLG_TRY(look_ahead(c0));
-                    FLG_TRY(upd(A22 + kNB * ld, A21 + kNB * ld, Ut, nr - kNB, kNB, kNB, cap));
-                    if (E > c0 + kNB) FLG_TRY(upd(A22 + kNB, A21, Ut + kNB * W, nr, E - c0 - kNB, kNB, cap));
+        const int64_t E2 = std::min<int64_t>(n, K0 + W);
+        for (int64_t K1 = K0; K1 < E2; K1 += W1) {
+            const int64_t E = std::min<int64_t>(n, K1 + W1);
+            for (int64_t k0 = K1; k0 < E; k0 += kNB) {
+                const int nb = (int)std::min<int64_t>(kNB, n - k0);
+                if (pending) {  // this block's diagonal kernel ran ahead on the side stream
+                    FLG_CUDA(cudaStreamWaitEvent(st, side->join, 0));
+                    pending = false;
                 } else {
-                    // rows > k0 x columns (k0, E)
-                    FLG_TRY(upd(A22, A21, Ut, nr, E - c0, kNB, 0));
+                    diag(k0, st);
+                    FLG_LAUNCH_CHECK();
                 }
-                // rows (k0, E) x columns >= E
-                if (n > E) FLG_TRY(upd(A + c0 * ld + E, A21, Ut + (E - c0) * W, E - c0, n - E, kNB, pending ? cap : 0));
+                const int64_t c0 = k0 + nb, nr = n - c0;
+                if (nr <= 0) continue;
+                prof_begin(FLG_SLOT_LU_PANEL, st);
+                // (nb < kNB only for the last block, which has no trailing part)
+                float *A12 = A + k0 * ld + c0, *A21 = A + c0 * ld + k0;
+                float *Ut = UtB + (c0 - K0) * W + (k0 - K0);  // row: column - K0; K offset: k0 - K0
+                LowpPanelArgs pa{A, ld, k0, nr, sA, tc ? Ut : nullptr, W, sUt, nullptr, nullptr, W, n * W, 0};
+                if (mode == FLG_LU_BF16) pa.Ut = nullptr, pa.Lb = LB + c0 * W + (k0 - K0), pa.Ub = UB + (Ut - UtB);
+                FLG_TRY(lowp_panels(pa, nbat, st));
+                prof_end(FLG_SLOT_LU_PANEL, st);
+                prof_begin(FLG_SLOT_LU_UPDATE, st);
+                if (!tc) {
+                    FLG_TRY(sgemm(st, nr, nr, nb, -1.0f, A21, ld, A12, ld, 1.0f, A + c0 * ld + c0, ld));
+                } else if (E > c0) {
+                    FLG_TRY(block(c0, n, c0, E, k0, c0, true));         // rows > k0 x columns (k0, E)
+                    if (n > E) FLG_TRY(block(c0, E, E, n, k0, c0, false));  // rows (k0, E) x columns >= E
+                }
+                prof_end(FLG_SLOT_LU_UPDATE, st);
             }
-            prof_end(FLG_SLOT_LU_UPDATE, st);
+            if (tc && E2 > E) {  // the middle panel's rank-W1 update of the rest of the outer panel
+                prof_begin(FLG_SLOT_LU_UPDATE, st);
+                FLG_TRY(block(E, n, E, E2, K1, E, true));
+                if (n > E2) FLG_TRY(block(E, E2, E2, n, K1, E, false));
+                prof_end(FLG_SLOT_LU_UPDATE, st);
+            }
         }
-        if (tc && n > E) {  // the deferred rank-(E - K0) update of rows and columns >= E (E - K0 = W here)
+        if (tc && n > E2) {  // the deferred rank-W update of rows and columns >= E2
             prof_begin(FLG_SLOT_LU_UPDATE, st);
-            float *C = A + E * ld + E, *Lp = A + E * ld + K0, *Up = UtB + (E - K0) * W;
-            if (n - E > kNB) {
-                // the next outer panel's first diagonal block first, then it factors beside the rest
-                FLG_TRY(upd(C, Lp, Up, kNB, kNB, E - K0, 0));
-                FLG_TRY(look_ahead(E));
-                FLG_TRY(upd(C + kNB * ld, Lp + kNB * ld, Up, n - E - kNB, kNB, E - K0, cap));
-                FLG_TRY(upd(C + kNB, Lp, Up + kNB * W, n - E, n - E - kNB, E - K0, cap));
-            } else {
-                FLG_TRY(upd(C, Lp, Up, n - E, n - E, E - K0, 0));
-            }
+            FLG_TRY(block(E2, n, E2, n, K0, E2, true));
             prof_end(FLG_SLOT_LU_UPDATE, st);
         }
     }
     if (pending) FLG_CUDA(cudaStreamWaitEvent(st, side->join, 0));  // (every look-ahead is joined above)
-    block_inverse_kernel<<<dim3((unsigned)(4 * nblk), 2, nbat), kPanelThreads, sizeof(LowpPanelSmem<1>), st>>>(
+    block_inverse_kernel<<<dim3((unsigned)(4 * nblk), 2, nbat), kTeamThreads<4>, sizeof(LowpPanelSmem<1, 1>), st>>>(
         A, ld, n, sA, dinv, dinv + nblk * kNB * kNB, sD);
     FLG_LAUNCH_CHECK();
     return FLG_OK;
