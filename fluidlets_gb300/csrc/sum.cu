@@ -394,32 +394,45 @@ __device__ __forceinline__ void final_store(const FinalArgs &a, int64_t i, const
     }
 }
 
-// u += the splits' partial sums of target i in split order, eight splits' loads in flight (one at a time
-// they cost an L2 round trip each: 17 of a 226 x 226 call's 27 us)
-template <int OUTW>
-__device__ __forceinline__ void sum_partials(const double *partial, int S, int64_t M, int64_t i, double *u) {
-    for (int s0 = 0; s0 < S; s0 += 8) {
+// u += the splits' partial sums of target i in split order, every LANES-th from s0 on, eight splits' loads in
+// flight (one at a time they cost an L2 round trip each: 17 of a 226 x 226 call's 27 us)
+template <int OUTW, int LANES>
+__device__ __forceinline__ void sum_partials(const double *partial, int S, int64_t M, int64_t i, int s0, double *u) {
+    for (; s0 < S; s0 += 8 * LANES) {
         double v[8][OUTW];
 #pragma unroll
         for (int s = 0; s < 8; s++)
 #pragma unroll
             for (int c = 0; c < OUTW; c++)
-                v[s][c] = s0 + s < S ? partial[((int64_t)(s0 + s) * M + i) * OUTW + c] : 0.0;
+                v[s][c] = s0 + s * LANES < S ? partial[((int64_t)(s0 + s * LANES) * M + i) * OUTW + c] : 0.0;
 #pragma unroll
         for (int s = 0; s < 8; s++)
-            if (s0 + s < S)
+            if (s0 + s * LANES < S)
 #pragma unroll
                 for (int c = 0; c < OUTW; c++) u[c] += v[s][c];
     }
 }
 
-__global__ void finalize_kernel(FinalArgs a) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.M) return;
+// LANES lanes per target, each a share of the splits: one lane's additions are a chain of 64 clocks each
+template <int OUTW, int LANES>
+__global__ void __launch_bounds__(64) finalize_kernel(FinalArgs a) {
+    const int64_t t = (int64_t)blockIdx.x * 64 + threadIdx.x, i = t / LANES;
+    const int l = (int)(t % LANES);
     double u[6] = {0, 0, 0, 0, 0, 0};
-    if (a.outw == 3) sum_partials<3>(a.partial, a.S, a.M, i, u);
-    else sum_partials<6>(a.partial, a.S, a.M, i, u);
-    final_store(a, i, u);
+    if (i < a.M) sum_partials<OUTW, LANES>(a.partial, a.S, a.M, i, l, u);
+#pragma unroll
+    for (int o = 1; o < LANES; o <<= 1)
+#pragma unroll
+        for (int c = 0; c < OUTW; c++) u[c] += __shfl_xor_sync(0xffffffffu, u[c], o);
+    if (i < a.M && l == 0) final_store(a, i, u);
+}
+// Eight lanes per target where there are many splits of few targets (4,099 targets, 30 splits: a call of
+// 1.29 ms with one lane, 1.26 with eight); more targets fill the chip by themselves, and 32 of them
+// per warp read whole sectors (32,768 targets, 19 splits: 1.24 ms with one lane, 1.26 with eight).
+template <int OUTW>
+static void launch_finalize(const FinalArgs &a, cudaStream_t st) {
+    if (a.S < 16 || a.M > 8192) finalize_kernel<OUTW, 1><<<(unsigned)ceil_div(a.M, 64), 64, 0, st>>>(a);
+    else finalize_kernel<OUTW, 8><<<(unsigned)ceil_div(a.M, 8), 64, 0, st>>>(a);
 }
 
 // ---------------------------------------------------------------------------
@@ -1414,7 +1427,8 @@ static int launch_sum(const SumRun &r, const SumLayout &L, int precision, const 
         } else {
             fin.S = 0;
         }
-        finalize_kernel<<<(unsigned)ceil_div(r.M, 64), 64, 0, st>>>(fin);
+        if (L.outw == 3) launch_finalize<3>(fin, st);
+        else launch_finalize<6>(fin, st);
         FLG_LAUNCH_CHECK();
         return FLG_OK;
     }
