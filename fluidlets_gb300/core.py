@@ -49,6 +49,8 @@ def _blob_widths(eps, n) -> torch.Tensor:
         e = eps.to(dtype=torch.float64)
         return dv.to_dev(torch.broadcast_to(e, (n,)), torch.float64)
     e = np.asarray(eps, dtype=np.float64)
+    if e.ndim < 2 and e.size == 1:  # filled on the device: an upload would wait for the stream
+        return torch.full((n,), float(e.reshape(-1)[0]), dtype=torch.float64, device=dv.require_cuda())
     return dv.to_dev(np.broadcast_to(e, (n,)), torch.float64)
 
 
