@@ -442,6 +442,7 @@ __global__ void __launch_bounds__(kTrsmThreads) swap_trsm_kernel(double *A, int6
                 *reinterpret_cast<const uint4 *>(stg + row * kTrsmStgLd + ch);
     }
 }
+constexpr int kTrsmWide = 2 * 8;
 static int swap_trsm(double *A, int64_t ld, const int32_t *ipiv, int64_t k0, int64_t c0, int64_t c1, uint16_t *SB,
                      int64_t cap, int *eb, cudaStream_t st) {
     const int64_t nc = c1 - c0;
@@ -454,7 +455,7 @@ static int swap_trsm(double *A, int64_t ld, const int32_t *ipiv, int64_t k0, int
         attr_set = true;
     }
     // G = 4 once its warps (8 columns each) fill half of the schedulers; below, G = 16's shorter chain
-    const bool wide = nc >= (int64_t)sm_count() * 2 * 8;
+    const bool wide = nc >= kTrsmWide * (int64_t)sm_count();
     const int cols = wide ? 8 : 2;
     const int w = (int)std::min<int64_t>(kTrsmWarps, ceil_div(nc, (int64_t)cols * sm_count()));
     const unsigned grid = (unsigned)ceil_div(nc, (int64_t)w * cols);
@@ -1526,10 +1527,14 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
         ahead = false;
         if (c0 >= n) break;
         const int64_t nc = n - c0;
-        FLG_TRY(swap_trsm(A, ld, ipiv, k0, c0, n, sb.B, n, sb.eb, st));
+        const int64_t nn = std::min<int64_t>(kPanel, nc);  // the next panel's columns first
+        // where the substitution of all columns is a long launch (37 us from 2,432 columns on, 12 for the next
+        // panel's), the rest of them follows beside the panel: n = 4,608 15.26 -> 14.94 ms; at fewer columns
+        // the launch costs what it saves (2,304: 5.71, 5.82 ms)
+        const bool split = nc >= kTrsmWide * (int64_t)sm_count() && nc <= kClusterPanelRows;
+        FLG_TRY(swap_trsm(A, ld, ipiv, k0, c0, split ? c0 + nn : n, sb.B, n, sb.eb, st));
         prof_begin(FLG_SLOT_LU_UPDATE, st);
         const int b = (int)(k0 / kPanel) & 1;
-        const int64_t nn = std::min<int64_t>(kPanel, nc);  // the next panel's columns first
         FLG_TRY(slice_update(A + c0 * ld + c0, ld, nc, nn, sb.A[b], n, 0, sb.ea[b], sb.B, n, 0, sb.eb, &bar->err, maxblk,
                              st));
         if (nc > nn) {
@@ -1542,6 +1547,7 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
             FLG_CUDA(cudaEventRecord(fs->panel_done, fs->panel));
             ahead = true;
             if (cluster) FLG_CUDA(cudaStreamWaitEvent(st, fs->panel_on, 0));
+            if (split) FLG_TRY(swap_trsm(A, ld, ipiv, k0, c0 + nn, n, sb.B + nn * kSliceK, n, sb.eb + nn, st));
             FLG_TRY(slice_update(A + c0 * ld + c0 + nn, ld, nc, nc - nn, sb.A[b], n, 0, sb.ea[b], sb.B, n, nn, sb.eb,
                                  &bar->err, cluster ? maxblk - kPanelCtas : maxblk, st));
         }
