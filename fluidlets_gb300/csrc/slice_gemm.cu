@@ -18,13 +18,17 @@
 // in row order, so that A's eight slices (128 KB) stay in shared memory over a row of tiles:
 //   * warp 0 (one lane): TMA, A's block when the row changes, B's block (8 x 4 KB) into a
 //     two-stage ring;
-//   * warp 1 (one lane): 36 x 4 tcgen05.mma (M = 128, N = 32, K = 16) per tile into one of two
-//     sets of eight 32-column accumulators (all 512 TMEM columns);
+//   * warp 1 (one lane): 8 x 4 tcgen05.mma per tile (M = 128, K = 16) into one of two sets of eight
+//     32-column accumulators (all 512 TMEM columns).  Slice q of A meets slices 0 .. 7 - q of B in one
+//     instruction of N = 32 (8 - q): those slices follow one another in shared memory as the
+//     orders' accumulators q .. 7 do in TMEM;
 //   * warps 2-9: the epilogue of the other set, 16 columns per warp, the tile's C through a small
 //     shared-memory transpose so that global accesses cover 64-byte row segments.
-// What bounds it: the epilogue's four FP64 operations per element on the two-lane pipe (128 x 32
-// x 4 / 2 = 8,192 clocks per tile) against about 6,000 clocks of MMAs; N = 32 with two accumulator
-// sets hides the MMAs behind the epilogue, where N = 64 would have used all of TMEM for one.
+// What bounds it: the epilogue's latency (two warps per scheduler).  As 36 x 4 instructions of N = 32
+// each read a slice of A for 32 columns, and with three FP64 operations per element to join the
+// orders (the pipe has two lanes), a factorization took, n = 4,608 / 7,000, ms: 14.94 / 33.8; with the
+// wide instructions 14.36 / 32.2; with the integer join as well 14.12 / 30.3.  Sixteen epilogue warps
+// (15.0 / 33.8) or loads of C one chunk ahead (14.7 / 31.5) are slower.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -55,9 +59,25 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
 }
-// the integer h (|h| < 2^51) as a double: its bits added to those of 2^52 + 2^51
-__device__ __forceinline__ double int_to_double(long long h) {
-    return __longlong_as_double(0x4338000000000000ll + h) - 6755399441055744.0;
+// H + L 2^-32 for 64-bit integers below 2^62, rounded to a double by integer instructions: sign and magnitude,
+// the top 64 of its 96 bits normalized, rounded to 53 (a tie away from zero).  As two conversions
+// and an FMA it took three FP64 operations, 48 of the 64 clocks per 32 elements that the pipe needed.
+__device__ __forceinline__ double join_orders(long long H, long long L) {
+    const long long hi = H + (L >> 32);
+    uint32_t w0 = (uint32_t)L, w1 = (uint32_t)hi, w2 = (uint32_t)((unsigned long long)hi >> 32);
+    const uint32_t sign = w2 & 0x80000000u;
+    if (sign)  // -(w2 w1 w0)
+        asm("sub.cc.u32 %0, 0, %0;\n\tsubc.cc.u32 %1, 0, %1;\n\tsubc.u32 %2, 0, %2;" : "+r"(w0), "+r"(w1), "+r"(w2));
+    int e = 1085;  // the exponent field, less one, for a leading bit at the top of w2
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+        if (w2 == 0) w2 = w1, w1 = w0, w0 = 0, e -= 32;
+    const int lz = __clz((int)w2);
+    const uint32_t m1 = __funnelshift_l(w1, w2, lz), m0 = __funnelshift_l(w0, w1, lz);
+    const unsigned long long m = (unsigned long long)m1 << 32 | m0;
+    const unsigned long long r = (m >> 11) + ((m0 >> 10) & 1) + ((unsigned long long)(uint32_t)(e - lz) << 52);
+    const unsigned long long x = (w2 == 0 ? 0ull : r) | (unsigned long long)sign << 32;
+    return __longlong_as_double((long long)x);
 }
 // t 2^e; the exponent field is added directly where neither side can leave the normal range
 __device__ __forceinline__ double scale_pow2(double t, int e) {
@@ -79,8 +99,8 @@ __global__ void __launch_bounds__(SG_THREADS, 1) slice_update_kernel(const __gri
     const int ntx = (nc + SG_BN - 1) / SG_BN, nty = (m + TC_BM - 1) / TC_BM;
     const int64_t ntiles = (int64_t)ntx * nty;
     const int64_t t0 = ntiles * blockIdx.x / gridDim.x, t1 = ntiles * (blockIdx.x + 1) / gridDim.x;
-    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(SG_BN >> 3) << 17) |
-                               ((uint32_t)(TC_BM >> 4) << 24);  // FP32 accumulators, BF16, K-major, 128 x 32
+    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) |
+                               ((uint32_t)(TC_BM >> 4) << 24);  // FP32 accumulators, BF16, K-major, 128 x (N at bit 17)
 
     if (threadIdx.x == 0) {
         mbar_init(&afull, 1);
@@ -150,19 +170,20 @@ __global__ void __launch_bounds__(SG_THREADS, 1) slice_update_kernel(const __gri
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d0 = tmem + s * (kSlices * SG_BN);
                 const uint8_t *b0 = sB + s * SG_B_BYTES;
-#pragma unroll 1
-                for (int p = 0; p < kSlices; p++)
-#pragma unroll 1
-                    for (int q = 0; q <= p; q++) {
-                        const uint64_t ad = sw128_desc(sA + q * SG_A_SLICE), bd = sw128_desc(b0 + (p - q) * SG_B_SLICE);
+                // A's slice q meets B's slices 0 .. 7 - q at once: they lie one after the other like the orders'
+                // accumulators q .. 7, so that N = 32 (8 - q) columns share one pass over A's slice
 #pragma unroll
-                        for (int kk = 0; kk < 4; kk++)  // 16 of the 64 K elements: 32 bytes of each row
-                            asm volatile(
-                                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                                " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d0 + p * SG_BN),
-                                "l"(ad + kk * 2), "l"(bd + kk * 2), "r"(IDESC), "r"((q | kk) ? 1u : 0u)
-                                : "memory");
-                    }
+                for (int q = 0; q < kSlices; q++) {
+                    const uint64_t ad = sw128_desc(sA + q * SG_A_SLICE), bd = sw128_desc(b0);
+                    const uint32_t idesc = IDESC | ((uint32_t)((kSlices - q) * SG_BN >> 3) << 17);
+#pragma unroll
+                    for (int kk = 0; kk < 4; kk++)  // 16 of the 64 K elements: 32 bytes of each row
+                        asm volatile(
+                            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d0 + q * SG_BN),
+                            "l"(ad + kk * 2), "l"(bd + kk * 2), "r"(idesc), "r"((q | kk) ? 1u : 0u)
+                            : "memory");
+                }
                 mma_commit(&bempty[s]);
                 mma_commit(&accf[s]);
                 if (t + 1 == t1 || (t + 1) / ntx != rb) mma_commit(&aempty);
@@ -210,7 +231,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) slice_update_kernel(const __gri
                     // orders 0..3 in units of 2^-24 of the top order's, 4..7 in units of 2^-56
                     const long long H = (long long)(d[0] * 256 + d[1]) * 65536 + (d[2] * 256 + d[3]);
                     const long long L = (long long)(d[4] * 256 + d[5]) * 65536 + (d[6] * 256 + d[7]);
-                    const double x = fma(int_to_double(L), 0x1p-32, int_to_double(H));
+                    const double x = join_orders(H, L);
                     const int ec = cc + c < nc ? eb[cc + c] : 0;
                     st[lane * SG_STG_LD + c] = scale_pow2(x, er + ec - 36);
                 }
