@@ -78,3 +78,23 @@ def test_lowp_lu_edges(n, nbat, mode):
             err = (D[:, h, k] @ I - torch.eye(128, device="cuda", dtype=torch.float64)).abs().max()
             assert float(err) <= 8 * 256 * 2.0 ** -24, (k, h, float(err))
     assert not np.isnan(dinv.cpu().numpy()).any()
+
+
+@pytest.mark.parametrize("nr,nc,lds,ldd,off", [(1, 1, 1, 1, 0), (3, 7, 9, 8, 0), (5, 4096, 4096, 4096, 0), (2, 4099, 4100, 4128, 0),
+                                               (7, 33, 34, 36, 1), (70000, 5, 6, 8, 0)])
+def test_fp32_copies_are_rounded_as_the_conversion(nr, nc, lds, ldd, off):
+    """Whole bits: ties, denormals, overflow, infinities and NaN, aligned rows and others."""
+    L = _lib.load()
+    rng = np.random.default_rng(nc)
+    x = rng.normal(size=nr * lds + off) * 10.0 ** rng.integers(-50, 50, nr * lds + off)
+    x[::5] = np.ldexp(2.0 * rng.integers(2 ** 23, 2 ** 24, x[::5].size) + 1.0, rng.integers(-160, 110, x[::5].size))  # ties
+    x[::11] = np.resize([0.0, -0.0, np.inf, -np.inf, np.nan, 3.4028235677973366e38, 1.1754943e-38, 1e-45, 7e-46, 5e-324],
+                        x[::11].size)
+    src = torch.from_numpy(x).cuda()[off:].reshape(nr, lds)
+    a, b = (torch.full((nr, ldd), 7.0, dtype=torch.float32, device="cuda") for _ in range(2))
+    _lib.check(L.flg_convert_f64_f32x2(nr, nc, dv.ptr(src), lds, dv.ptr(a), dv.ptr(b), ldd, dv.stream()))
+    ref = src[:, :nc].cpu().float()
+    for d in (a, b):
+        assert torch.equal(torch.isnan(d[:, :nc].cpu()), torch.isnan(ref)) and torch.all(d[:, nc:] == 7.0)
+        assert torch.equal(torch.nan_to_num(d[:, :nc].cpu(), nan=1.0).view(torch.int32),
+                           torch.nan_to_num(ref, nan=1.0).view(torch.int32))
