@@ -3,7 +3,9 @@
 // FP64 (the drop-in for scipy.linalg.solve, core/solve.py:64-67, and
 // np.linalg.solve, swimming.py:101): right-looking blocked LU with partial
 // pivoting, row-major storage, block width kPanel = 64.
-//   panel_f64_kernel  cooperative launch over up to one CTA per SM; each CTA
+//   cluster_panel     (panel.cu) panels of up to 8,192 rows, in two halves of 32
+//                     columns on one 16-CTA cluster.
+//   panel_f64_kernel  taller panels: cooperative launch over up to one CTA per SM; each CTA
 //                     keeps a slab of panel rows in shared memory; one round of
 //                     published candidates per column (pivot search is a
 //                     grid-wide argmax, first index on ties as LAPACK's idamax),
@@ -11,19 +13,18 @@
 //   swap_rows_kernel  the panel's row swaps on the columns left of it.
 //   swap_trsm_kernel  the swaps and U12 = L11^-1 A12 right of it, and U12's BF16 slices.
 //   slice_update      A22 -= L21 U12 in FP64 accuracy on the tensor cores (slice_gemm.cu).
+//   trsv_cluster      (trsv.cu) the triangular solves of few right-hand sides.
 //
 // Low precision (preconditioner of FP64 GMRES-IR): blocked LU WITHOUT
-// pivoting in FP32 storage, block FLG_LU_LOWP_BLOCK = 128; the diagonal block
-// is factored by one CTA, which also writes the inverses of its L and U
-// factors (kept in `dinv` for the solves); the panels are GEMMs with those
-// inverses; the trailing update runs on the tensor cores (tc_gemm.cu, deferred
-// to one rank-512 update per outer panel of four blocks) or on CUDA cores
-// (FLG_LU_FP32).  With the tensor cores the next diagonal block runs ahead on
-// a side stream while the rest of each update finishes.
+// pivoting in FP32 storage, block FLG_LU_LOWP_BLOCK = 128: the diagonal block in
+// the registers of one CTA, both panels by substitution in one launch, the
+// trailing update on the tensor cores (tc_gemm.cu, deferred on two levels) or on
+// CUDA cores (FLG_LU_FP32).  With the tensor cores the next diagonal block runs
+// ahead on a side stream while the rest of each update finishes.  The inverses
+// of the diagonal blocks' factors, kept in `dinv` for the solves, are one launch at the end.
 //
-// Every spin-wait (the grid barrier, the solves' dataflow, waits.cuh; the
-// diagonal block's warp handshake, an iteration count) is bounded and reports
-// failure through a device flag instead of hanging.
+// Every spin-wait (the grid barrier, the cluster exchanges, the solves' dataflow, waits.cuh)
+// is bounded and reports failure through a device flag instead of hanging.
 #include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -1883,7 +1884,7 @@ extern "C" int flg_lu_factor_lowp(int64_t n, float *A, int64_t ld, int mode, flo
     FLG_CUDA(cudaMemcpyAsync(hflags, flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
     FLG_CUDA(cudaStreamSynchronize(st));
     if (hflags[1]) {
-        set_error("a bounded device wait timed out (tensor-core update or diagonal block)");
+        set_error("a bounded device wait timed out (tensor-core update)");
         return FLG_ERR_TIMEOUT;
     }
     *info = hflags[0];

@@ -235,9 +235,11 @@ int flg_lu_solve_f64(int64_t n, int64_t nrhs, const double *LU, int64_t ld, cons
 /* Low-precision LU without pivoting for the mixed-precision path: A is FP32
  * (n x n, ld; ld a multiple of 4 so every row starts on a 16-byte boundary),
  * factored in place (unit L, U) in blocks of FLG_LU_LOWP_BLOCK.  With mode
- * FLG_LU_TF32 or FLG_LU_BF16 the panels (TF32) and the trailing updates (the
- * mode's type; rank 128 inside 512-column outer panels, rank 512 for the rest)
- * run on the tcgen05 tensor cores; FLG_LU_FP32 uses CUDA cores throughout.
+ * FLG_LU_TF32 or FLG_LU_BF16 the trailing updates (rank 128 inside 512-column
+ * panels, rank 512 inside outer panels of 1,024 (TF32) or 2,048 (BF16) columns
+ * from n = 8,192 on, rank of the outer panel for the rest) run on the tcgen05
+ * tensor cores in the mode's type; the panels are FP32 substitutions.
+ * FLG_LU_FP32 uses CUDA cores throughout.
  * A tensor-core mode may carry FLG_LU_TILE_N128 or FLG_LU_TILE_N256 (the tile
  * width of the trailing updates; the workspace does not depend on it).
  * dinv (FP32, size flg_lu_lowp_dinv_elems(n)) receives the inverses of the
@@ -252,8 +254,7 @@ int flg_lu_factor_lowp(int64_t n, float *A, int64_t ld, int mode, float *dinv, i
 /* The same factorization without any host synchronization (so it can be
  * captured in a CUDA graph): the pivot / timeout flags are written to the
  * device array flags[2] (flags[0] = 1 + first bad pivot row, flags[1] = 1 if
- * a bounded device wait -- tensor-core pipeline or diagonal-block warps --
- * timed out) for the caller to check after the stream. */
+ * a bounded device wait of the tensor-core pipeline timed out) for the caller to check after the stream. */
 int flg_lu_factor_lowp_async(int64_t n, float *A, int64_t ld, int mode, float *dinv, int *flags,
                              void *work, size_t work_bytes, void *stream);
 /* The same for nbat (1 .. 64) independent systems of order n in one sequence
@@ -261,9 +262,9 @@ int flg_lu_factor_lowp_async(int64_t n, float *A, int64_t ld, int mode, float *d
  * its block inverses at dinv + z flg_lu_lowp_dinv_elems(n), its flags at
  * flags[2 z], flags[2 z + 1] (2 nbat ints; flags[1] also reports a timed-out
  * tensor-core wait of any system).  Every kernel of a step covers all systems:
- * the diagonal blocks as one CTA per system, the panels and trailing updates
- * as one tensor-core launch over the tiles of all systems (3-D tensor maps,
- * the system index outermost).  Tensor-core modes only (TF32 / BF16, with or
+ * the diagonal blocks as one CTA per system, both panels as one launch, the
+ * trailing updates as one tensor-core launch over the tiles of all systems
+ * (3-D tensor maps, the system index outermost).  Tensor-core modes only (TF32 / BF16, with or
  * without a tile-width bit).  Each system's factors are bit-identical to its
  * own flg_lu_factor_lowp_async call.  No counterpart in the reference. */
 size_t flg_lu_factor_lowp_batched_workspace(int64_t n, int nbat, int mode);
