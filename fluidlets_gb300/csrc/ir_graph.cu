@@ -10,7 +10,7 @@
 //
 //   x = 0, r = b, ||b||                              (prologue)
 //   WHILE the residual is above rtol ||b||:          (refinement steps)
-//     v0 = M^-1 r, beta = ||v0||, ptol = 1e-6 beta   (inner GMRES on M^-1 A d = M^-1 r)
+//     v0 = M^-1 r, beta = ||v0||, ptol = ir_inner_tolerance beta   (inner GMRES on M^-1 A d = M^-1 r)
 //     WHILE the inner residual estimate is above ptol and columns remain:
 //       w = M^-1 (A32 v_k); two classical Gram-Schmidt passes; Givens update
 //     x += V y (upper-triangular least squares)
@@ -40,11 +40,6 @@ int lu_solve_lowp_prepare();
 constexpr int kIrMaxM = 64;             // inner columns at most
 constexpr int kIrThreads = 256;
 constexpr int64_t kIrChunk = 8192;      // elements per CTA of a dot product
-// Inner (preconditioned) tolerance.  An inner step gains about three digits (TF32 factors), so an
-// inner solve ends some way below the tolerance: at 1e-4 many ended just below it after one step,
-// and a third FP64 residual was needed (wall, 8,192 blobs, tf32: 3 refinement steps of 45.4 ms in
-// all); 1e-6 has two steps of two iterations each reach 1e-12 (42.1 ms; bf16 factors: 35.8 both).
-constexpr double kIrInner = 1e-6;
 constexpr double kEps = 2.220446049250313e-16;
 
 // the device state of one refinement (one graph)
@@ -164,7 +159,7 @@ __global__ void ir_ctrl_init(IrState *S, double rtol, int m, int max_outer, cuda
 // start of an inner solve: beta = ||M^-1 r||, its tolerance, g = beta e1
 __global__ void ir_ctrl_inner_init(IrState *S, cudaGraphConditionalHandle h_inner) {
     S->beta = sqrt(fmax(S->dot, 0.0));
-    S->ptol = S->beta * kIrInner;
+    S->ptol = S->beta * ir_inner_tolerance(S->tol, S->rn);
     for (int q = 0; q <= S->m; q++) S->g[q] = 0.0;
     S->g[0] = S->beta;
     S->k = 0;

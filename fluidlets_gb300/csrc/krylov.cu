@@ -651,7 +651,7 @@ extern "C" int flg_gmres_ir_dense(int64_t n, const double *A, int64_t ld, const 
     char *lw = ar.take<char>(lsb);
     float *xs = ar.take<float>(2 * n);
     FLG_REQUIRE(d && lw && xs, "workspace too small for GMRES-IR");
-    // outer residuals with the FP64 matrix; inner (preconditioned, tolerance 1e-6) matvecs
+    // outer residuals with the FP64 matrix; inner (preconditioned, ir_inner_tolerance) matvecs
     // with the FP32 copy when the caller provides one
     g.A = [&](const double *v, double *out) { return flg_gemv_f64(n, n, A, ld, v, out, st); };
     if (A32)
@@ -665,7 +665,6 @@ extern "C" int flg_gmres_ir_dense(int64_t n, const double *A, int64_t ld, const 
         FLG_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * n, st));
         return FLG_OK;
     }
-    const double inner = 1e-6;  // as ir_graph.cu, which has the figures
     double rn = 0.0, prev = INFINITY;
     int stall = 0;
     for (int o = 0; o <= 60; o++) {
@@ -681,7 +680,7 @@ extern "C" int flg_gmres_ir_dense(int64_t n, const double *A, int64_t ld, const 
         prev = rn;
         FLG_CUDA(cudaMemsetAsync(d, 0, sizeof(double) * n, st));
         double rin;
-        int s2 = gi.solve(g.r, d, inner, maxiter, *iters, rin, rn, true);
+        int s2 = gi.solve(g.r, d, ir_inner_tolerance(rtol * bn, rn), maxiter, *iters, rin, rn, true);
         if (s2 != FLG_OK && s2 != FLG_ERR_NOT_CONVERGED) return s2;
         add_kernel<double><<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(x, d, n);
         FLG_LAUNCH_CHECK();
