@@ -208,13 +208,14 @@ __global__ void __launch_bounds__(kTvThreads, 1) trsv_cluster_kernel(const doubl
                 send(&y[b * kTb + lane], &pb[b], warp + d * kTvWarps, o);
             if (up && warp == 0 && row < n) B[(int64_t)row * ldb] = o;
         }
-        // the backward pass reads this CTA's own forward results from y and every CTA must have them: the
-        // last block's arrival implies all others
-        if (pass == 0)
-            for (int k = 0; k < own_max; k++)
-                if (k * kTvCtas + c < nb) cluster_wait(&pb[k * kTvCtas + c], 0, &S.err);
+        // Every value sent to this CTA has arrived before any CTA goes on: nothing orders two st.async to one
+        // address, so a forward value still under way could land on the backward one that replaces it
+        // (a CTA waits for a block by itself only where it needs the block), and a CTA that has
+        // ended must not be a store's target.
+        for (int e = t; e < nb; e += kTvThreads) cluster_wait(&pb[e], 0, &S.err);
+        __syncthreads();
+        cluster_sync();
     }
-    cluster_sync();  // no CTA leaves while a block is on its way to it
 }
 
 static size_t trsv_smem(int64_t n) {
