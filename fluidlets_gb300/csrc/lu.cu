@@ -357,23 +357,24 @@ __global__ void __launch_bounds__(kSwapThreads) swap_rows_kernel(double *A, int6
 
 // The interchanges and U12 = L11^-1 A12 (unit lower L11 = A[k0:k0+64, k0:k0+64]) on the columns
 // [c0, c1) right of a full panel, and the slices of U12's columns for the trailing update
-// (slices.cuh): SB [8][cap][64] BF16 with column c at row c - c0, exponents eb[c - c0].  G lanes per
+// (slices.cuh): SB [8][cap][64] BF16 with column c at row c - c0, exponents and masks eb, mb[c - c0].  G lanes per
 // column, lane group g holding rows G i + g: the substitution runs column by column of L11
 // (every row's FMAs in the same order as row by row, but independent of one another).  An FP64
 // warp instruction takes 64 clocks of its scheduler, so a warp's 544 (G = 4) or 160 (G = 16) of them
 // are the kernel's time: 16 lanes per column spread the few hundred columns of a small system over all
 // schedulers, 4 waste fewer FMAs on rows already solved where there are columns for every
 // scheduler anyway.  `warps` of a CTA's eight have columns; all load L11 and work out the
-// interchanges.
+// interchanges.  Two CTAs per SM (128 registers): the wide launch beside a cluster panel has more
+// CTAs than SMs left (one per SM: 14.8 ms for 4,608 unknowns, two: 14.7).
 constexpr int kTrsmThreads = 256, kTrsmWarps = kTrsmThreads / 32;
 constexpr int kTrsmStgLd = kPanel + 8;              // 16-bit words per staged slice row (no bank conflicts)
 constexpr size_t trsm_smem(int G, int warps) {
     return sizeof(double) * kPanel * kPanel + sizeof(uint16_t) * kSlices * (32 / G) * kTrsmStgLd * warps;
 }
 template <int G>
-__global__ void __launch_bounds__(kTrsmThreads) swap_trsm_kernel(double *A, int64_t ld, const int32_t *ipiv, int64_t k0,
+__global__ void __launch_bounds__(kTrsmThreads, 2) swap_trsm_kernel(double *A, int64_t ld, const int32_t *ipiv, int64_t k0,
                                                                  int64_t c0, int64_t c1, int warps, uint16_t *SB,
-                                                                 int64_t cap, int *eb) {
+                                                                 int64_t cap, int *eb, SliceMask *mb, int near_range) {
     extern __shared__ __align__(16) double Lt[];  // [64][64]: Lt[q][r] = L11[r][q]; then the warps' staged slices
     __shared__ int piv[kPanel], dst[2 * kPanel], src[2 * kPanel];
     constexpr int COLS = 32 / G, R = kPanel / G;  // columns per warp, rows per lane
@@ -425,6 +426,24 @@ __global__ void __launch_bounds__(kTrsmThreads) swap_trsm_kernel(double *A, int6
 #pragma unroll
     for (int o = COLS; o < 32; o <<= 1) exmax = max(exmax, __shfl_xor_sync(0xffffffffu, exmax, o));
     if (live && g == 0) eb[c - c0] = slice_scale(exmax);
+    {  // this lane's rows have the parity of g, so their bits lie in one word of each mask
+        unsigned near = 0, set = 0;
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            const unsigned bit = 1u << ((G * i + g) >> 1);
+            near |= slice_near(x[i], exmax, near_range) ? bit : 0u;
+            set |= x[i] != 0.0 ? bit : 0u;
+        }
+#pragma unroll
+        for (int o = 2 * COLS; o < 32; o <<= 1) {
+            near |= __shfl_xor_sync(0xffffffffu, near, o);
+            set |= __shfl_xor_sync(0xffffffffu, set, o);
+        }
+        if (live && g < 2) {
+            unsigned *w = reinterpret_cast<unsigned *>(mb + (c - c0)) + g;
+            w[0] = near, w[2] = set;
+        }
+    }
     uint16_t *stg = (uint16_t *)(Lt + kPanel * kPanel) + warp * (kSlices * COLS * kTrsmStgLd);
 #pragma unroll
     for (int i = 0; i < R; i++) {
@@ -445,7 +464,7 @@ __global__ void __launch_bounds__(kTrsmThreads) swap_trsm_kernel(double *A, int6
 }
 constexpr int kTrsmWide = 2 * 8;
 static int swap_trsm(double *A, int64_t ld, const int32_t *ipiv, int64_t k0, int64_t c0, int64_t c1, uint16_t *SB,
-                     int64_t cap, int *eb, cudaStream_t st) {
+                     int64_t cap, int *eb, SliceMask *mb, int near, cudaStream_t st) {
     const int64_t nc = c1 - c0;
     static bool attr_set = false;
     if (!attr_set) {
@@ -460,16 +479,18 @@ static int swap_trsm(double *A, int64_t ld, const int32_t *ipiv, int64_t k0, int
     const int cols = wide ? 8 : 2;
     const int w = (int)std::min<int64_t>(kTrsmWarps, ceil_div(nc, (int64_t)cols * sm_count()));
     const unsigned grid = (unsigned)ceil_div(nc, (int64_t)w * cols);
-    if (wide) swap_trsm_kernel<4><<<grid, kTrsmThreads, trsm_smem(4, w), st>>>(A, ld, ipiv, k0, c0, c1, w, SB, cap, eb);
-    else swap_trsm_kernel<16><<<grid, kTrsmThreads, trsm_smem(16, w), st>>>(A, ld, ipiv, k0, c0, c1, w, SB, cap, eb);
+    if (wide) swap_trsm_kernel<4><<<grid, kTrsmThreads, trsm_smem(4, w), st>>>(A, ld, ipiv, k0, c0, c1, w, SB, cap, eb, mb, near);
+    else swap_trsm_kernel<16><<<grid, kTrsmThreads, trsm_smem(16, w), st>>>(A, ld, ipiv, k0, c0, c1, w, SB, cap, eb, mb, near);
     FLG_LAUNCH_CHECK();
     return FLG_OK;
 }
 
 // the trailing update on the tensor cores (slice_gemm.cu)
-int slice_rows(const double *A, int64_t lda, int64_t rows, int64_t cap, void *S, int *e, cudaStream_t st);
-int slice_update(double *C, int64_t ldc, int64_t m, int64_t nc, const void *SA, int64_t capA, int64_t a0, const int *ea,
-                 const void *SB, int64_t capB, int64_t b0, const int *eb, int *err, int max_ctas, cudaStream_t st);
+int slice_rows(const double *A, int64_t lda, int64_t rows, int64_t cap, void *S, int *e, SliceMask *mask, int near,
+               cudaStream_t st);
+int slice_update(double *C, int64_t ldc, int64_t m, int64_t nc, const double *A, const double *B, const void *SA,
+                 int64_t capA, const int *ea, const SliceMask *ma, const void *SB, int64_t capB, int64_t b0, const int *eb,
+                 const SliceMask *mb, int near, int *err, int max_ctas, cudaStream_t st);
 
 // ---- FP64 triangular solves (getrs) ------------------------------------------------
 // Row interchanges in LAPACK order (swap rows r and ipiv[r] for r = 0, 1, ...).
@@ -1383,19 +1404,22 @@ static int panel_geometry(int64_t m, int &nblk, int &rpc) {
 }
 
 // operand slices of the trailing update: L21's rows (two buffers: the next panel's slices are
-// written while this panel's update still reads its own) and U12's columns, with their exponents
+// written while this panel's update still reads its own) and U12's columns, with their exponents and masks
 struct SliceBufs {
     uint16_t *A[2] = {}, *B = nullptr;
     int *ea[2] = {}, *eb = nullptr;
+    SliceMask *ma[2] = {}, *mb = nullptr;
     template <class Ar>
     void carve(Ar &ar, int64_t n) {
         const size_t rows = n > kPanel ? (size_t)n : 0;
         for (int k = 0; k < 2; k++) {
             A[k] = ar.template take<uint16_t>(kSlices * rows * kSliceK);
             ea[k] = ar.template take<int>(rows);
+            ma[k] = ar.template take<SliceMask>(rows);
         }
         B = ar.template take<uint16_t>(kSlices * rows * kSliceK);
         eb = ar.template take<int>(rows);
+        mb = ar.template take<SliceMask>(rows);
     }
 };
 
@@ -1451,14 +1475,14 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
                 sm_count() * 384);
     cudaStream_t st = as_stream(stream);
     Arena ar(work, work_bytes);
-    const int maxblk = sm_count();
+    const int maxblk = sm_count(), near = slice_near_range(n);
     GridBar *bar = ar.take<GridBar>(1);
     unsigned long long *word = ar.take<unsigned long long>(2 * maxblk);
     double *rowbuf = ar.take<double>((size_t)2 * maxblk * kRowBufLd);
     double *diagbuf = ar.take<double>(2 * kPanel);
     SliceBufs sb;
     sb.carve(ar, n);
-    FLG_REQUIRE(diagbuf != nullptr && (n <= kPanel || sb.eb != nullptr), "workspace too small for LU (%zu bytes)",
+    FLG_REQUIRE(diagbuf != nullptr && (n <= kPanel || sb.mb != nullptr), "workspace too small for LU (%zu bytes)",
                 work_bytes);
     F64Streams *fs = nullptr;
     FLG_TRY(f64_streams(&fs));
@@ -1489,7 +1513,7 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
                                       nullptr, s));
             }
             prof_end(FLG_SLOT_LU_PANEL, s);
-            return slice_rows(A + (k0 + kb) * ld + k0, ld, m - kb, n, sb.A[b], sb.ea[b], s);
+            return slice_rows(A + (k0 + kb) * ld + k0, ld, m - kb, n, sb.A[b], sb.ea[b], sb.ma[b], near, s);
         }
         int nblk, rpc;
         panel_geometry(m, nblk, rpc);
@@ -1505,7 +1529,7 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
         FLG_CUDA(cudaLaunchCooperativeKernel((void *)panel_f64_kernel, dim3(nblk), dim3(256), args, smem, s));
         count_launch();
         prof_end(FLG_SLOT_LU_PANEL, s);
-        return slice_rows(A + (k0 + kb) * ld + k0, ld, m - kb, n, sb.A[b], sb.ea[b], s);
+        return slice_rows(A + (k0 + kb) * ld + k0, ld, m - kb, n, sb.A[b], sb.ea[b], sb.ma[b], near, s);
     };
     // Look-ahead: after each panel's trailing update has reached the next panel's 64 columns,
     // the next panel factors on the panel stream while the main stream updates the rest.
@@ -1533,11 +1557,12 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
         // panel's), the rest of them follows beside the panel: n = 4,608 15.26 -> 14.94 ms; at fewer columns
         // the launch costs what it saves (2,304: 5.71, 5.82 ms)
         const bool split = nc >= kTrsmWide * (int64_t)sm_count() && nc <= kClusterPanelRows;
-        FLG_TRY(swap_trsm(A, ld, ipiv, k0, c0, split ? c0 + nn : n, sb.B, n, sb.eb, st));
+        FLG_TRY(swap_trsm(A, ld, ipiv, k0, c0, split ? c0 + nn : n, sb.B, n, sb.eb, sb.mb, near, st));
         prof_begin(FLG_SLOT_LU_UPDATE, st);
         const int b = (int)(k0 / kPanel) & 1;
-        FLG_TRY(slice_update(A + c0 * ld + c0, ld, nc, nn, sb.A[b], n, 0, sb.ea[b], sb.B, n, 0, sb.eb, &bar->err, maxblk,
-                             st));
+        const double *L21 = A + c0 * ld + k0, *U12 = A + k0 * ld + c0;
+        FLG_TRY(slice_update(A + c0 * ld + c0, ld, nc, nn, L21, U12, sb.A[b], n, sb.ea[b], sb.ma[b], sb.B, n, 0, sb.eb,
+                             sb.mb, near, &bar->err, maxblk, st));
         if (nc > nn) {
             FLG_CUDA(cudaEventRecord(fs->next_ready, st));
             FLG_CUDA(cudaStreamWaitEvent(fs->panel, fs->next_ready, 0));
@@ -1548,9 +1573,9 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
             FLG_CUDA(cudaEventRecord(fs->panel_done, fs->panel));
             ahead = true;
             if (cluster) FLG_CUDA(cudaStreamWaitEvent(st, fs->panel_on, 0));
-            if (split) FLG_TRY(swap_trsm(A, ld, ipiv, k0, c0 + nn, n, sb.B + nn * kSliceK, n, sb.eb + nn, st));
-            FLG_TRY(slice_update(A + c0 * ld + c0 + nn, ld, nc, nc - nn, sb.A[b], n, 0, sb.ea[b], sb.B, n, nn, sb.eb,
-                                 &bar->err, cluster ? maxblk - kPanelCtas : maxblk, st));
+            if (split) FLG_TRY(swap_trsm(A, ld, ipiv, k0, c0 + nn, n, sb.B + nn * kSliceK, n, sb.eb + nn, sb.mb + nn, near, st));
+            FLG_TRY(slice_update(A + c0 * ld + c0 + nn, ld, nc, nc - nn, L21, U12 + nn, sb.A[b], n, sb.ea[b], sb.ma[b],
+                                 sb.B, n, nn, sb.eb, sb.mb, near, &bar->err, cluster ? maxblk - kPanelCtas : maxblk, st));
         }
         prof_end(FLG_SLOT_LU_UPDATE, st);
         if (!ahead) FLG_TRY(panel(c0, st, nullptr));  // the last panel: nothing to overlap it with

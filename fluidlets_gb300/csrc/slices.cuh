@@ -7,6 +7,13 @@
 // factor 2^9 of 2^e, rounded to 2^(e - 63) below.  A digit is exact in BF16 (8 significant
 // bits), a product of two digits is an integer of at most 2^14, and 64 x 8 such products sum to
 // at most 2^23, which FP32 accumulates exactly.
+//
+// What that costs a dot product of a row and a column depends on where their large values meet: its
+// error is about 2^-59 of 2^(ea + eb), which is small beside the FP64 rounding errors of a term that
+// is large in both and not small at all where every product lies far below the two maxima (rows
+// of different units among the 64 pivots).  The masks of a row or column say which of its 64 values
+// reach 2^(e - 1 - near), and which are not zero; slice_gemm.cu recomputes in FP64 what the masks of a row
+// and a column leave open.
 #pragma once
 #include <stdint.h>
 
@@ -15,6 +22,7 @@ namespace flg {
 constexpr int kSlices = 8;            // digits per value
 constexpr int kSliceK = 64;           // depth of one operand block: 64 BF16 = 128 bytes
 constexpr int kSliceNonFinite = 1 << 20;  // exponent of a row or column that holds an Inf or NaN
+typedef uint4 SliceMask;              // near (x, y), non-zero (z, w); value k: bit k / 2 of the first word, odd k of the second
 
 // biased exponent of x, 1 for zero and denormals (they scale like the smallest normals)
 __device__ __forceinline__ int slice_exponent(double x) {
@@ -23,6 +31,18 @@ __device__ __forceinline__ int slice_exponent(double x) {
 }
 // the common exponent e (|x| < 2^e) from the largest biased exponent of the row
 __device__ __forceinline__ int slice_scale(int exmax) { return exmax == 0x7ff ? kSliceNonFinite : exmax - 1022; }
+
+// whether x counts as near the maximum of its row or column
+__device__ __forceinline__ bool slice_near(double x, int exmax, int near) {
+    return exmax == 0x7ff || slice_exponent(x) >= exmax - near;
+}
+// the masks' range for n unknowns: products of near values reach 2^(ea + eb - (2 near + 2)), and 2 near + 2 is at
+// most log2 n + 4 (slice_gemm.cu)
+inline int slice_near_range(int64_t n) {
+    int lg = 0;
+    while (n >> (lg + 1)) lg++;
+    return (lg + 2) / 2;
+}
 
 // the eight digits of x relative to the row's largest biased exponent, biased by 128: digit k is
 // byte 7 - k of the result minus 128 (zero digits for a row with non-finite entries)
