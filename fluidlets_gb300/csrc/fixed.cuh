@@ -141,17 +141,22 @@ FLG_HD q60 q_rcp1p(q60 x) {
     return ((q60)r0 << 30) + qmul30(qf(c), r0);
 }
 
-// x 2^p (x in Q60) as a double, rounded once
+// x 2^p (x in Q60) as a double, rounded once (on the device by integer instructions, a tie away from zero: the FP64
+// pipe, which converts, is what bounds the matrix kernels)
 FLG_HD double q_to_double(q60 x, int p) {
+    const int ex = p - 60;
 #if defined(__CUDA_ARCH__)
-    const double d = __ll2double_rn(x);
+    if (ex > 900 || ex < -900) return scalbn(__ll2double_rn(x), ex);
+    const uint64_t s = (uint64_t)(x >> 63), m = ((uint64_t)x ^ s) - s;
+    const int lz = __clzll((long long)m);
+    const uint64_t n = m << (lz & 63);
+    const uint64_t r = (n >> 11) + (n >> 10 & 1) + ((uint64_t)(uint32_t)(1085 - lz + ex) << 52);
+    return bitsd(m == 0 ? 0 : r | (s & 0x8000000000000000ull));
 #else
     const double d = (double)x;
-#endif
-    const int ex = p - 60;
     if (ex > 900 || ex < -900) return scalbn(d, ex);
-    const uint64_t u = dbits(d);
-    return x == 0 ? 0.0 : bitsd(u + ((uint64_t)(int64_t)ex << 52));
+    return x == 0 ? 0.0 : bitsd(dbits(d) + ((uint64_t)(int64_t)ex << 52));
+#endif
 }
 
 }  // namespace flg

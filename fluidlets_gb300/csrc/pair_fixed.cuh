@@ -453,6 +453,8 @@ FLG_HD void fx_radial_apply_c(const FxDir &g, const FxRadialC &r, const q60 *F, 
 // wall: everything that does not depend on the strengths
 struct FxWall {
     q60 nx, ny, nm, nI, rho, rho2, Z3h, cq, czq, g, yF;
+    q60 r3;  // rho^3 = r3 2^r3x, r3 in [1/8, 1): with its relative precision where rho is small
+    int r3x;
     int eF;  // sF = yF 2^-eF
     int x;  // bracket / 8 . g . 2^x, without the factor t h
 };
@@ -467,6 +469,10 @@ FLG_HD FxWall fx_wall(double d0, double d1, double dm, double dp, double QF, dou
     const q60 half = qmul(yI, qf(qmul(qf(f.r.qh), qf(f.r.y))));
     w.rho = q_shift(half << 1, i.e - f.r.e);
     if (w.rho > kQ1) w.rho = kQ1;
+    const int low = half < kQ1 / 2;  // (1/4 < half < 1)
+    const Qf rm = qf(half << low);
+    w.r3 = qmul(rm, qf(qmul(rm, rm)));
+    w.r3x = 3 * (1 - low - (i.e - f.r.e));
     const Qf rho = qf(w.rho);
     w.rho2 = qmul(rho, rho);
     const q60 Z1h = q_rcp1p(w.rho);  // Z1 / 2
@@ -524,7 +530,10 @@ FLG_HD void fx_radial_block(const FxDir &g, const FxRadial &r, const FxConst &c,
     *B = q_to_double(qmul(qf(qmul(qf(r.B), qf(qmul(y, y)))), cm), r.x + c.x - 2 * (g.r.e - 1023));
 }
 // the wall block from d0, d1 and: G_jk = a d_j d_k + c delta_jk, G_jz = d_j b1, G_zj = d_j b2, G_zz = z
-// (j, k = x, y); th: t h times the constant
+// (j, k = x, y); t, h: the two heights, one of them times the constant.  With P = Z3 k, R = 3 rho^3 k of
+// the common factor k, a = P + R, b1 = P dm - R dp, b2 = P dm + R dp in FP64: beside the distance dm and dp may be small,
+// and b1 and b2 keep their precision to 2^-53 of their own terms.  (As fixed-point n_z and n_I to 2^-60 of the
+// distance, at heights of 1e-6 of it b1 and b2 were exact to 5e-13.)
 struct FxWallBlock {
     double a, b1, b2, c, z;
 };
@@ -541,17 +550,17 @@ FLG_HD FxWallBlock fx_wall_block(double d0, double d1, double dm, double dp, dou
 #endif
     const int s = lz < 12 ? lz - 4 : 0;  // |k| < 1: lz >= 4 (0: t = 0)
     k <<= s;
-    const Qf kf = qf(k), yf = qf(w.yF), nm = qf(w.nm), nI = qf(w.nI), rho = qf(w.rho);
-    const q60 r2n = qmul(qf(w.rho2), nI), zn = qmul(qf(w.Z3h), nm), r3 = qmul(qf(w.rho2), rho);
-    const q60 i2n = r2n + qhalf(r2n);  // 3/2 rho^2 nI
-    const q60 a4 = qhalf(w.Z3h + r3 + qhalf(r3)), b14 = qhalf(zn - i2n), b24 = qhalf(zn + i2n);
-    const q60 rn2 = qmul(rho, qf(qmul(nI, nI)));
-    const q60 z4 = w.czq + qhalf(qmul(nm, qf(zn)) - rn2 - qhalf(rn2));
+    const Qf kf = qf(k), yf = qf(w.yF), nm = qf(w.nm), nI = qf(w.nI);
+    const q60 rn2 = qmul(qf(w.rho), qf(qmul(nI, nI)));
+    const q60 z4 = w.czq + qhalf(qmul(nm, qf(qmul(qf(w.Z3h), nm))) - rn2 - qhalf(rn2));
     const int x = w.x - 1 - s + t.x + h.x;  // (the bracket over 4 here, over 8 in w.x)
+    const Qf y2k = qf(qmul(qf(qmul(yf, yf)), kf));
+    const double P = q_to_double(qmul(qf(w.Z3h), y2k), x - 1 - 2 * w.eF);
+    const double R = q_to_double(qmul(qf(w.r3 + qhalf(w.r3)), y2k), x - 1 - 2 * w.eF + w.r3x), Rd = R * dp;
     FxWallBlock b;
-    b.a = q_to_double(qmul(qf(qmul(qf(a4), qf(qmul(yf, yf)))), kf), x - 2 * w.eF);
-    b.b1 = q_to_double(qmul(qf(qmul(qf(b14), yf)), kf), x - w.eF);
-    b.b2 = q_to_double(qmul(qf(qmul(qf(b24), yf)), kf), x - w.eF);
+    b.a = P + R;
+    b.b1 = fma(P, dm, -Rd);
+    b.b2 = fma(P, dm, Rd);
     b.c = q_to_double(qmul(qf(w.cq), kf), x);
     b.z = q_to_double(qmul(qf(z4), kf), x);
     return b;
