@@ -173,7 +173,7 @@ __device__ __forceinline__ void bucket_system(AsmArgs &a, const int64_t *&n_real
 // ---- real FP64 matrices in fixed point ---------------------------------------------------------
 // The block's coefficients (A, B of a radial kernel; five for the wall) come from pair_fixed.cuh with
 // the kernel's scale and 1 / mu in them; the entries are FP64 products of them with the displacement,
-// so each keeps its precision beside its own terms.  A wall block takes 21 operations of the FP64 pipe
+// so each keeps its precision beside its own terms.  A wall block takes 20 operations of the FP64 pipe
 // instead of 108 (1,501 x 2,003: 0.53 -> 0.154 ms).  Pairs outside the fixed-point ranges take block_f64.
 struct FxAsm {
     FxAlpha al;
@@ -212,7 +212,7 @@ __device__ __forceinline__ void block_fx(double tx, double ty, double tz, const 
         const double dp = tz + s.z;
         const double rq = fma(d1, d1, fma(d0, d0, s.e2)), QF = fma(d2, d2, rq), QI = fma(dp, dp, rq);
         if (cok && s.ok && q_in_range(QF) && q_in_range(QI) && fx_const_ok(tz) && !(d_neg(tz) ^ d_neg(s.z))) {
-            const FxWallBlock w = fx_wall_block(d0, d1, d2, dp, QF, QI, s.e, fx_const(tz), s.h);
+            const FxWallBlock w = fx_wall_block(d2, dp, QF, QI, s.e, fx_const(tz), s.h);
             const double a0 = w.a * d0, a1 = w.a * d1;
             G[0] = fma(a0, d0, w.c), G[1] = a0 * d1, G[2] = d0 * w.b1;
             G[3] = G[1], G[4] = fma(a1, d1, w.c), G[5] = d1 * w.b1;
@@ -222,7 +222,7 @@ __device__ __forceinline__ void block_fx(double tx, double ty, double tz, const 
     } else {
         const double Q = fma(d2, d2, fma(d1, d1, fma(d0, d0, s.e2)));
         if (cok && q_in_range(Q)) {
-            const FxDir g = fx_dir(d0, d1, d2, Q, s.e);
+            const FxDir g = fx_dir(Q, s.e);
             double A, B;
             fx_radial_block(g, KIND == FLG_STOKESLET ? fx_stokeslet(g) : fx_brinkman(g, f.al), f.c, &A, &B);
             const double b0 = B * d0, b1 = B * d1, b2 = B * d2;

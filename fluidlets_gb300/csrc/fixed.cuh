@@ -41,9 +41,8 @@ FLG_HD q60 qmul(Qf a, Qf b) {
 }
 // a b for a 30-bit b (Q30)
 FLG_HD q60 qmul30(Qf a, int b) { return (q60)a.h * b + (((q60)a.l * b + (1ll << 29)) >> 30); }
-// x / 2 and x 2^-s (s >= 1), rounded
+// x / 2, rounded
 FLG_HD q60 qhalf(q60 x) { return (x + 1) >> 1; }
-FLG_HD q60 qshr(q60 x, int s) { return ((x >> (s - 1)) + 1) >> 1; }
 
 FLG_HD uint64_t dbits(double x) {
 #if defined(__CUDA_ARCH__)

@@ -1,63 +1,53 @@
-// pair_fixed.cuh -- the FP64 pair kernels in 60-bit fixed point (fixed.cuh).
+// pair_fixed.cuh -- the FP64 pair kernels' coefficients in 60-bit fixed point (fixed.cuh).
 //
-// The same formulas as pair_math.cuh's, written in bounded quantities.  With Q = |d|^2 + e^2 =
-// q 2^(2E), y = q^-1/2, the unit vector n = d / sqrt(Q) and w = e / sqrt(Q):
-//   Stokeslet     8 pi u = s [(1 + w^2) f + (f.n) n],                       s = y 2^-E
-//   Brinkmanlet   4 pi u = s [(f1 + w^2 f2) f + f2 (f.n) n]                 below z = 1/2 (series), and
-//                        = s^3 / alpha^2 [(F1 + w^2 F2) f + F2 (f.n) n],    F = z^2 f, above:
+// The same formulas as pair_math.cuh's, the coefficients written in bounded quantities.  With Q = |d|^2 + e^2 =
+// q 2^(2E), y = q^-1/2, s = Q^-1/2 = y 2^-E and w = e s:
+//   Stokeslet     8 pi u = A f + B (f.d) d,  A = s (1 + w^2), B = s^3
+//   Brinkmanlet   4 pi u = A f + B (f.d) d,  A = s (f1 + w^2 f2), B = s^3 f2         below z = 1/2 (series), and
+//                        A = s^3 / alpha^2 (F1 + w^2 F2), B = s^5 / alpha^2 F2, F = z^2 f, above:
 //     F1 = E (1 + z + z^2) - 1, F2 = 3 - E (3 + 3 z + z^2), E = e^-z from 2^-n 2^(-i/64) e^-x with a table
 //     (P. T. P. Tang, "Table-driven implementation of the exponential function in IEEE
 //     floating-point arithmetic", ACM TOMS 15, 1989)
-//   wall          8 pi u = 2 t h sF s^2 [...] with rho = s / sF <= 1, nI = dp s and the bracket
-//     c f_j + n_j (Z3 (f.n) - 3 rho^2 B)           (j = x, y),  c = Z1 + w^2 Z3 - rho + 3 w^2 rho^3
-//     c' f_z + n_z Z3 (f.n) - 3 rho nI B,                       c' = Z1 + w^2 Z3 - rho - 3 w^2 rho^3
-//     Z1 = 2 / (1 + rho), Z3 = Z1 (1 + rho + rho^2) = 2 + ... , B = nI f_z - rho (n_x f_x + n_y f_y)
+//   wall          8 pi u_j = 2 t h sF s^2 [c f_j + d_j sF^2 (Z3 (f.d) + 3 rho^3 (D - dp f_z))]      (j = x, y)
+//                 8 pi u_z = 2 t h sF s^2 [z f_z + D sF^2 (Z3 dm + 3 rho^3 dp)]
+//     with rho = s / sF <= 1 (s of the image), D = d_x f_x + d_y f_y, dm = t - h, dp = t + h,
+//     Z1 = 2 / (1 + rho), Z3 = Z1 (1 + rho + rho^2) = 2 + ... , c = Z1 + w^2 Z3 - rho + 3 w^2 rho^3,
+//     z = Z1 + w^2 Z3 - rho - 3 w^2 rho^3 + Z3 n^2 - 3 rho nI^2, n = dm sF, nI = dp s
 //   (the bracket is the image form of pair_math.cuh divided by sF^3 rho^2, which keeps its
 //   precision where the wall is far: rho -> 0).
-// Displacements and Q stay in FP64 (their rounding is the FP64 kernel's own); everything after them
-// is an integer of 2^-59 absolute error in quantities of order one, where an FP64 chain of the
-// same length has several 2^-54 relative ones.  Pairs outside the ranges where this holds (Q
-// not a normal number far from the limits, strengths that are not finite, targets and sources on
+// A coefficient is a double of 2^-54 relative accuracy or better (of its terms, where they cancel).  Displacements,
+// Q, and the products with displacement and strength stay in FP64, so that every component of a
+// velocity keeps the precision of an FP64 sum of its own terms: a component may be small beside the
+// others, as may the displacement along it, and fixed point against a common exponent would round
+// it to 2^-58 of the largest.  (The Stokeslet's sums are integers with an exponent for each component.)
+// Pairs outside the ranges (Q not a normal number far from the limits, targets and sources on
 // opposite sides of the wall) go to the FP64 functions, pair by pair.
 #pragma once
 #include "fixed.cuh"
 
 namespace flg {
 
-// exponents of Q that the fixed-point path takes: every exponent sum stays far inside the range
-constexpr int kQExpMin = 1023 - 1000, kQExpMax = 1023 + 1000;
-FLG_HD bool q_in_range(double Q) {
+// exponents of Q that the fixed-point path takes: every exponent sum stays far inside the range, and so do the
+// coefficients (s^3 of a radial kernel's sum, with one height s^4 of the wall's)
+constexpr int kQExpMax = 1000, kQExpRadial = 640, kQExpWall = 360;
+FLG_HD bool q_in_range(double Q, int limit = kQExpMax) {
     const int ex = (int)(dbits(Q) >> 52);  // (a sign bit makes it too large)
-    return ex >= kQExpMin && ex <= kQExpMax;
+    return ex >= 1023 - limit && ex <= 1023 + limit;
 }
 
-// strengths of one source, f = F 2^e with the largest |F_k| in [1/4, 1/2); e = kFxBad: not finite
-constexpr int kFxBad = 1 << 28, kFxZero = -(1 << 20);
-FLG_HD int fx_strength(const double *f, int n, q60 *F) {
-    int em = 0;
-    for (int k = 0; k < n; k++) em = dexp(f[k]) > em ? dexp(f[k]) : em;
-    if (em == 0x7ff) return kFxBad;
-    for (int k = 0; k < n; k++) F[k] = q_of(f[k], em) >> 2;  // |f| 2^-em < 2: a quarter of it below 1/2
-    return em < 64 ? (em == 0 ? kFxZero : kFxBad) : em - 1023 + 2;
-}
-
-// what the pair kernels give: the coefficients of u = (A f + B (f.n) n) 2^x for a radial kernel
+// what the pair kernels give: u = (A f + B (f.n) n) 2^x of a radial kernel, n = d / sqrt(Q)
 struct FxRadial {
     q60 A, B;  // A in [-1.8, 1.8], B in [0, 1.6]
     int x;
 };
-struct FxDir {  // unit vector and w^2, with the root
-    q60 n[3], w2;
+struct FxDir {  // the root and w^2
+    q60 w2;
     QRsqrt r;
 };
-FLG_HD FxDir fx_dir(double d0, double d1, double d2, double Q, double e) {
+FLG_HD FxDir fx_dir(double Q, double e) {
     FxDir g;
     g.r = q_rsqrt(Q);
-    const Qf y = qf(g.r.y);
-    g.n[0] = q_sign(qmul(qf(q_mag(d0, g.r.e)), y), d_neg(d0));
-    g.n[1] = q_sign(qmul(qf(q_mag(d1, g.r.e)), y), d_neg(d1));
-    g.n[2] = q_sign(qmul(qf(q_mag(d2, g.r.e)), y), d_neg(d2));
-    const Qf w = qf(qmul(qf(q_mag(e, g.r.e)), y));
+    const Qf w = qf(qmul(qf(q_mag(e, g.r.e)), qf(g.r.y)));
     g.w2 = qmul(w, w);
     return g;
 }
@@ -242,14 +232,84 @@ FLG_HD FxRadial fx_brinkman(const FxDir &g, const FxAlpha &al) {
     return z.k < 0 ? fx_series(g, z, al) : fx_closed(g, z, al);
 }
 
-// u / 2^x for strengths F; |u| < 2
-FLG_HD void fx_radial_apply(const FxDir &g, const FxRadial &r, const q60 *F, q60 *u) {
-    const Qf n0 = qf(g.n[0]), n1 = qf(g.n[1]), n2 = qf(g.n[2]), f0 = qf(F[0]), f1 = qf(F[1]), f2 = qf(F[2]);
-    const q60 t = qmul(f0, n0) + qmul(f1, n1) + qmul(f2, n2);
-    const Qf b = qf(qmul(qf(t), qf(r.B))), A = qf(r.A);
-    u[0] = qmul(A, f0) + qmul(b, n0);
-    u[1] = qmul(A, f1) + qmul(b, n1);
-    u[2] = qmul(A, f2) + qmul(b, n2);
+// A and B of u = A f + B (f.d) d
+struct FxCoef {
+    double A, B;
+};
+FLG_HD FxCoef fx_coef(const FxDir &g, const FxRadial &r) {
+    const Qf y = qf(g.r.y);
+    return {q_to_double(r.A, r.x), q_to_double(qmul(qf(r.B), qf(qmul(y, y))), r.x - 2 * (g.r.e - 1023))};
+}
+
+// ---- Stokeslet sums in integers ---------------------------------------------------------------------
+// A Stokeslet pair has so few operations that the ten FP64 products with displacement and strength would be what
+// bounds its sum, so they are integers too, every component with an exponent of its own: strengths,
+// displacement, and the sums, so that a component's rounding stays 2^-56 of its own largest term.
+struct FxNum {
+    q60 m;  // [1/2, 1), with the sign; 0 for zero
+    int e;  // x = m 2^e
+};
+constexpr int kFxTiny = -(1 << 20);  // exponent of a zero
+FLG_HD FxNum fx_num(double x) {      // (denormals count as zero)
+    const uint64_t u = dbits(x);
+    const int ex = (int)(u >> 52) & 0x7ff;
+    if (ex == 0) return {0, kFxTiny};
+    return {q_sign((q60)((u & 0x000fffffffffffffull) << 7 | 0x0800000000000000ull), d_neg(x)), ex - 1022};
+}
+FLG_HD bool fx_num_ok(double x) { return (dexp(x) != 0 || x == 0.0) && dexp(x) != 0x7ff; }
+// Sums of three components over up to 32 terms m 2^x, |m| < 1: 64-bit integers of 57 fractional bits relative
+// to the component's largest exponent so far, which outlives the 32 terms
+struct FxAcc {
+    q60 a[3];
+    int x[3];
+    FLG_HD void init() {
+        clear();
+        x[0] = x[1] = x[2] = -(1 << 24);
+    }
+    FLG_HD void clear() { a[0] = a[1] = a[2] = 0; }
+    FLG_HD void add(int c, q60 m, int xt) {
+        if (xt > x[c]) {  // makes room (rare once the first few terms have passed)
+            const int s = xt - x[c] < 63 ? xt - x[c] : 63;
+            a[c] >>= s;
+            x[c] = xt;
+        }
+        const int s = x[c] - xt + 3 < 63 ? x[c] - xt + 3 : 63;
+        a[c] += ((m >> (s - 1)) + 1) >> 1;
+    }
+    FLG_HD double value(int c) const { return q_to_double(a[c], x[c] + 3); }
+};
+// adds one pair's velocities of NF strengths f[3 NF] into acc[NF]
+template <int NF>
+FLG_HD void fx_add_stokeslet(double d0, double d1, double d2, double Q, double e, const FxNum *f, FxAcc *acc) {
+    const FxDir g = fx_dir(Q, e);
+    const int E = g.r.e - 1023;
+    const Qf y = qf(g.r.y), A = qf(qmul(qf((kQ1 + g.w2) >> 1), y));  // (1 + w^2) s / 2
+    const q60 y3 = qmul(qf(qmul(y, y)), y);
+    const int n3 = q_room((uint64_t)y3);  // s^3 with its leading bit at 2^59
+    const Qf B = qf(y3 << n3);
+    const FxNum d[3] = {fx_num(d0), fx_num(d1), fx_num(d2)};
+    const Qf D[3] = {qf(d[0].m), qf(d[1].m), qf(d[2].m)};
+    for (int c = 0; c < NF; c++) {
+        const FxNum *F = f + 3 * c;
+        Qf Fm[3];
+        q60 p[3];
+        int xp[3];
+        for (int k = 0; k < 3; k++) {
+            Fm[k] = qf(F[k].m);
+            p[k] = qmul(Fm[k], D[k]);
+            xp[k] = F[k].e + d[k].e;
+        }
+        int xt = xp[0] > xp[1] ? xp[0] : xp[1];
+        xt = (xt > xp[2] ? xt : xp[2]) + 2;  // f.d / 4 below 3/4
+        q60 t = 0;
+        for (int k = 0; k < 3; k++) t += p[k] >> (xt - xp[k] < 63 ? xt - xp[k] : 63);
+        const Qf b = qf(qmul(qf(t), B));
+        const int xb = xt - 3 * E - n3;
+        for (int k = 0; k < 3; k++) {
+            acc[c].add(k, qmul(A, Fm[k]), 1 - E + F[k].e);
+            acc[c].add(k, qmul(b, D[k]), xb + d[k].e);
+        }
+    }
 }
 
 // ---- complex alpha --------------------------------------------------------------------------------
@@ -437,80 +497,16 @@ FLG_HD FxRadialC fx_brinkman(const FxDir &g, const FxAlphaC &al) {
     return z.k < 0 ? fx_series(g, z, al) : fx_closed(g, z, al);
 }
 
-// the two parts of one real strength vector: ur = (Ar F + Br t n), ui = (Ai F + Bi t n), t = F.n
-FLG_HD void fx_radial_apply_c(const FxDir &g, const FxRadialC &r, const q60 *F, q60 *ur, q60 *ui) {
-    const Qf n0 = qf(g.n[0]), n1 = qf(g.n[1]), n2 = qf(g.n[2]), f0 = qf(F[0]), f1 = qf(F[1]), f2 = qf(F[2]);
-    const Qf t = qf(qmul(f0, n0) + qmul(f1, n1) + qmul(f2, n2));
-    const Qf br = qf(qmul(t, qf(r.Br))), bi = qf(qmul(t, qf(r.Bi))), Ar = qf(r.Ar), Ai = qf(r.Ai);
-    ur[0] = qmul(Ar, f0) + qmul(br, n0);
-    ur[1] = qmul(Ar, f1) + qmul(br, n1);
-    ur[2] = qmul(Ar, f2) + qmul(br, n2);
-    ui[0] = qmul(Ai, f0) + qmul(bi, n0);
-    ui[1] = qmul(Ai, f1) + qmul(bi, n1);
-    ui[2] = qmul(Ai, f2) + qmul(bi, n2);
-}
-
-// wall: everything that does not depend on the strengths
-struct FxWall {
-    q60 nx, ny, nm, nI, rho, rho2, Z3h, cq, czq, g, yF;
-    q60 r3;  // rho^3 = r3 2^r3x, r3 in [1/8, 1): with its relative precision where rho is small
-    int r3x;
-    int eF;  // sF = yF 2^-eF
-    int x;  // bracket / 8 . g . 2^x, without the factor t h
+struct FxCoefC {
+    double Ar, Ai, Br, Bi;
 };
-FLG_HD FxWall fx_wall(double d0, double d1, double dm, double dp, double QF, double QI, double e) {
-    const FxDir f = fx_dir(d0, d1, dm, QF, e);
-    const QRsqrt i = q_rsqrt(QI);
-    const Qf yI = qf(i.y);
-    FxWall w;
-    w.nx = f.n[0], w.ny = f.n[1], w.nm = f.n[2];
-    w.nI = q_sign(qmul(qf(q_mag(dp, i.e)), yI), d_neg(dp));
-    // rho = (yI / yF) 2^(EF - EI), 1 / yF = q yF
-    const q60 half = qmul(yI, qf(qmul(qf(f.r.qh), qf(f.r.y))));
-    w.rho = q_shift(half << 1, i.e - f.r.e);
-    if (w.rho > kQ1) w.rho = kQ1;
-    const int low = half < kQ1 / 2;  // (1/4 < half < 1)
-    const Qf rm = qf(half << low);
-    w.r3 = qmul(rm, qf(qmul(rm, rm)));
-    w.r3x = 3 * (1 - low - (i.e - f.r.e));
-    const Qf rho = qf(w.rho);
-    w.rho2 = qmul(rho, rho);
-    const q60 Z1h = q_rcp1p(w.rho);  // Z1 / 2
-    w.Z3h = kQ1 + qmul(qf(w.rho2), qf(Z1h));  // Z3 / 2 = 1 + rho^2 / (1 + rho)
-    const q60 w2r3 = qmul(qf(f.w2), qf(qmul(qf(w.rho2), rho)));
-    const q60 base = Z1h + qmul(qf(f.w2), qf(w.Z3h)) - qhalf(w.rho), i3 = w2r3 + qhalf(w2r3);
-    w.cq = qhalf(base + i3), w.czq = qhalf(base - i3);  // c / 4, c' / 4
-    w.g = qmul(qf(f.r.y), qf(qmul(yI, yI)));
-    w.yF = f.r.y, w.eF = f.r.e - 1023;
-    w.x = 4 - w.eF - 2 * (i.e - 1023);  // 8 from the bracket, 2 of 2 t h
-    return w;
-}
-// the exponent of u 2^x is returned: the bracket cancels near the wall and for far images, so it is
-// scaled up to [1/2, 1) before its last product
-FLG_HD int fx_wall_apply(const FxWall &w, const q60 *F, q60 *u) {
-    const Qf nx = qf(w.nx), ny = qf(w.ny), nm = qf(w.nm), nI = qf(w.nI), f0 = qf(F[0]), f1 = qf(F[1]), f2 = qf(F[2]);
-    const q60 D = qmul(f0, nx) + qmul(f1, ny);
-    const Qf B = qf(qmul(nI, f2) - qmul(qf(w.rho), qf(D)));
-    const q60 t1 = qmul(qf(w.Z3h), qf(D + qmul(f2, nm)));  // Z3 (f.n) / 2
-    const q60 r2B = qmul(qf(w.rho2), B), zB = qmul(qf(w.rho), qf(qmul(nI, B)));
-    const Qf b = qf(qhalf(t1 - r2B - qhalf(r2B))), cq = qf(w.cq), g = qf(w.g);
-    const q60 ux = qmul(cq, f0) + qmul(b, nx), uy = qmul(cq, f1) + qmul(b, ny);
-    const q60 uz = qmul(qf(w.czq), f2) + qhalf(qmul(nm, qf(t1)) - zB - qhalf(zB));
-    const uint64_t m = (uint64_t)((ux ^ (ux >> 63)) | (uy ^ (uy >> 63)) | (uz ^ (uz >> 63)));
-#if defined(__CUDA_ARCH__)
-    const int lz = __clz((int)(m >> 32));
-#else
-    const int lz = (m >> 32) ? __builtin_clz((unsigned)(m >> 32)) : 32;
-#endif
-    // |bracket| / 4 < 2.4: lz >= 2; one shift left of lz - 3 after the shift right that makes room
-    const int s = lz < 5 ? 0 : lz - 5;
-    u[0] = qmul(qf(qhalf(ux << s)), g);
-    u[1] = qmul(qf(qhalf(uy << s)), g);
-    u[2] = qmul(qf(qhalf(uz << s)), g);
-    return w.x - s;
+FLG_HD FxCoefC fx_coef(const FxDir &g, const FxRadialC &r) {
+    const Qf y = qf(g.r.y), y2 = qf(qmul(y, y));
+    const int x = r.x - 2 * (g.r.e - 1023);
+    return {q_to_double(r.Ar, r.x), q_to_double(r.Ai, r.x + r.xi), q_to_double(qmul(qf(r.Br), y2), x),
+            q_to_double(qmul(qf(r.Bi), y2), x + r.xi)};
 }
 
-// ---- matrix blocks ------------------------------------------------------------------------------
 // a real factor c = m 2^x with |m| in [1/2, 1) (0 for c = 0)
 struct FxConst {
     q60 m;
@@ -523,6 +519,56 @@ FLG_HD FxConst fx_const(double c) {  // (not for denormals, infinities or NaN)
 }
 FLG_HD bool fx_const_ok(double c) { return c == 0.0 || (dexp(c) > 64 && dexp(c) < 1982); }
 
+// wall, times a factor k 2^kx (|k| in [1/4, 1) or 0): P = Z3, R = 3 rho^3 and their sum a (with the factor
+// sF^2), c and z of the header.
+// Where dm and dp are small beside the distance, P dm and R dp in FP64 keep their precision.  (As fixed-point n
+// and nI, to 2^-60 of the distance, the xz entries were exact to 5e-13 at heights of 1e-6 of it.)
+struct FxWall {
+    double P, R, a, c, z;
+};
+FLG_HD FxWall fx_wall(double dm, double dp, double QF, double QI, double e, q60 k, int kx) {
+    const FxDir f = fx_dir(QF, e);
+    const QRsqrt i = q_rsqrt(QI);
+    const Qf yI = qf(i.y), yF = qf(f.r.y), nm = qf(qmul(qf(q_mag(dm, f.r.e)), yF)), nI = qf(qmul(qf(q_mag(dp, i.e)), yI));
+    // rho = (yI / yF) 2^(EF - EI), 1 / yF = q yF
+    const q60 half = qmul(yI, qf(qmul(qf(f.r.qh), yF)));
+    q60 r = q_shift(half << 1, i.e - f.r.e);
+    if (r > kQ1) r = kQ1;
+    // rho^3 with its relative precision where rho is small: r3 2^r3x, r3 in [1/8, 1)
+    const int low = half < kQ1 / 2;  // (1/4 < half < 1)
+    const Qf rho = qf(r), rm = qf(half << low);
+    const q60 r3 = qmul(rm, qf(qmul(rm, rm)));
+    const int r3x = 3 * (1 - low - (i.e - f.r.e));
+    const q60 rho2 = qmul(rho, rho);
+    const q60 Z1h = q_rcp1p(r);  // Z1 / 2
+    const q60 Z3h = kQ1 + qmul(qf(rho2), qf(Z1h));  // Z3 / 2 = 1 + rho^2 / (1 + rho)
+    const q60 rho3 = qmul(qf(rho2), rho), w2r3 = qmul(qf(f.w2), qf(rho3));
+    const q60 base = Z1h + qmul(qf(f.w2), qf(Z3h)) - qhalf(r), i3 = w2r3 + qhalf(w2r3);
+    const q60 c4 = qhalf(base + i3);  // c / 4
+    const q60 rn2 = qmul(rho, qf(qmul(nI, nI)));
+    const q60 z4 = qhalf(base - i3) + qhalf(qmul(nm, qf(qmul(qf(Z3h), nm))) - rn2 - qhalf(rn2));
+    // the common factor k sF s^2, scaled up to [1/2, 1)
+    q60 g = qmul(qf(qmul(yF, qf(qmul(yI, yI)))), qf(k));
+    const uint32_t hi = (uint32_t)((uint64_t)(g ^ (g >> 63)) >> 32);
+#if defined(__CUDA_ARCH__)
+    const int lz = __clz((int)hi);
+#else
+    const int lz = hi ? __builtin_clz(hi) : 32;
+#endif
+    const int s = lz < 12 ? lz - 4 : 0;  // |g| < 1: lz >= 4 (32: k = 0)
+    g <<= s;
+    const int eF = f.r.e - 1023, x = 3 - eF - 2 * (i.e - 1023) - s + kx;  // (4 from the bracket, 2 of 2 t h)
+    const Qf gf = qf(g), y2g = qf(qmul(qf(qmul(yF, yF)), gf));
+    FxWall w;
+    w.P = q_to_double(qmul(qf(Z3h), y2g), x - 1 - 2 * eF);
+    w.R = q_to_double(qmul(qf(r3 + qhalf(r3)), y2g), x - 1 - 2 * eF + r3x);
+    w.a = q_to_double(qmul(qf(qhalf(Z3h + rho3 + qhalf(rho3))), y2g), x - 2 * eF);
+    w.c = q_to_double(qmul(qf(c4), gf), x);
+    w.z = q_to_double(qmul(qf(z4), gf), x);
+    return w;
+}
+
+// ---- matrix blocks ------------------------------------------------------------------------------
 // G = A I + B d d^T, both times c
 FLG_HD void fx_radial_block(const FxDir &g, const FxRadial &r, const FxConst &c, double *A, double *B) {
     const Qf cm = qf(c.m), y = qf(g.r.y);
@@ -530,71 +576,14 @@ FLG_HD void fx_radial_block(const FxDir &g, const FxRadial &r, const FxConst &c,
     *B = q_to_double(qmul(qf(qmul(qf(r.B), qf(qmul(y, y)))), cm), r.x + c.x - 2 * (g.r.e - 1023));
 }
 // the wall block from d0, d1 and: G_jk = a d_j d_k + c delta_jk, G_jz = d_j b1, G_zj = d_j b2, G_zz = z
-// (j, k = x, y); t, h: the two heights, one of them times the constant.  With P = Z3 k, R = 3 rho^3 k of
-// the common factor k, a = P + R, b1 = P dm - R dp, b2 = P dm + R dp in FP64: beside the distance dm and dp may be small,
-// and b1 and b2 keep their precision to 2^-53 of their own terms.  (As fixed-point n_z and n_I to 2^-60 of the
-// distance, at heights of 1e-6 of it b1 and b2 were exact to 5e-13.)
+// (j, k = x, y); t, h: the two heights, one of them times the constant
 struct FxWallBlock {
     double a, b1, b2, c, z;
 };
-FLG_HD FxWallBlock fx_wall_block(double d0, double d1, double dm, double dp, double QF, double QI, double e,
-                                 const FxConst &t, const FxConst &h) {
-    const FxWall w = fx_wall(d0, d1, dm, dp, QF, QI, e);
-    // g t h, scaled up to [1/2, 1)
-    q60 k = qmul(qf(w.g), qf(qmul(qf(t.m), qf(h.m))));
-    const uint32_t hi = (uint32_t)((uint64_t)(k ^ (k >> 63)) >> 32);
-#if defined(__CUDA_ARCH__)
-    const int lz = __clz((int)hi);
-#else
-    const int lz = hi ? __builtin_clz(hi) : 32;
-#endif
-    const int s = lz < 12 ? lz - 4 : 0;  // |k| < 1: lz >= 4 (0: t = 0)
-    k <<= s;
-    const Qf kf = qf(k), yf = qf(w.yF), nm = qf(w.nm), nI = qf(w.nI);
-    const q60 rn2 = qmul(qf(w.rho), qf(qmul(nI, nI)));
-    const q60 z4 = w.czq + qhalf(qmul(nm, qf(qmul(qf(w.Z3h), nm))) - rn2 - qhalf(rn2));
-    const int x = w.x - 1 - s + t.x + h.x;  // (the bracket over 4 here, over 8 in w.x)
-    const Qf y2k = qf(qmul(qf(qmul(yf, yf)), kf));
-    const double P = q_to_double(qmul(qf(w.Z3h), y2k), x - 1 - 2 * w.eF);
-    const double R = q_to_double(qmul(qf(w.r3 + qhalf(w.r3)), y2k), x - 1 - 2 * w.eF + w.r3x), Rd = R * dp;
-    FxWallBlock b;
-    b.a = P + R;
-    b.b1 = fma(P, dm, -Rd);
-    b.b2 = fma(P, dm, Rd);
-    b.c = q_to_double(qmul(qf(w.cq), kf), x);
-    b.z = q_to_double(qmul(qf(z4), kf), x);
-    return b;
+FLG_HD FxWallBlock fx_wall_block(double dm, double dp, double QF, double QI, double e, const FxConst &t, const FxConst &h) {
+    const FxWall w = fx_wall(dm, dp, QF, QI, e, qmul(qf(t.m), qf(h.m)), t.x + h.x);
+    const double Rd = w.R * dp;
+    return {w.a, fma(w.P, dm, -Rd), fma(w.P, dm, Rd), w.c, w.z};
 }
-
-// Sums of up to 16 terms u 2^x with |u| < 2: 64-bit integers of 57 fractional bits (a term is
-// rounded to 2^-58 of its unit, the sum stays below 2^62) relative to the largest exponent so far,
-// which outlives the 16 terms.
-constexpr int kFxSeg = 16;
-template <int NC>
-struct FxAcc {
-    q60 a[NC];
-    int x;
-    FLG_HD void init() {
-        clear();
-        x = -(1 << 24);
-    }
-    FLG_HD void clear() {
-        for (int k = 0; k < NC; k++) a[k] = 0;
-    }
-    // makes room for a term of exponent xt (rare once the first few pairs have passed)
-    FLG_HD void scale(int xt) {
-        if (xt > x) {
-            const int s = xt - x < 63 ? xt - x : 63;
-            for (int k = 0; k < NC; k++) a[k] = qshr(a[k], s);
-            x = xt;
-        }
-    }
-    // term u[0..3) of exponent xt at component c0 of the sum
-    FLG_HD void add(int c0, const q60 *u, int xt) {
-        const int s = x - xt + 3 < 63 ? x - xt + 3 : 63;
-        for (int k = 0; k < 3; k++) a[c0 + k] += qshr(u[k], s);
-    }
-    FLG_HD double value(int k) const { return q_to_double(a[k], x + 3); }
-};
 
 }  // namespace flg

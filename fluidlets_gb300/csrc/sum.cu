@@ -157,115 +157,130 @@ __global__ void __launch_bounds__(kF64Threads) sum_f64_kernel(SumArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// The same sum with the pairs in 60-bit fixed point (pair_fixed.cuh): the FP64 pipe (19 clocks per
-// warp instruction and SM) keeps the displacements and squared distances, six operations of a
-// Stokeslet pair's 27, eight of a wall pair's 56 and six of a complex Brinkman pair's 350; the rest
-// runs on the integer pipe beside it.  Sums of 16 terms stay in 64-bit integers relative to their
-// largest exponent, real and imaginary parts each to their own.  A pair outside the fixed-point
-// ranges takes the FP64 function; a complex alpha that fx_alpha_c_ok refuses takes sum_f64_kernel.
-// The wall kernel's factor t is applied once at the end, its factor h in the staged strengths.
-// Bound by the integer pipe.  FP64 pairs -> fixed point: 32,768 x 1,003 wall 3.6 -> 1.2 ms, 16,384 x
-// 16,384 Brinkman 33 -> 12 ms, 4,099 x 2,500 complex Brinkman 6.0 -> 1.2 ms (four CTAs per SM; three
-// for the complex pair: 1.33 ms a call, 1.34 with two).
+// The same sum with the pairs' coefficients in 60-bit fixed point (pair_fixed.cuh): the FP64 pipe (19 clocks
+// per warp instruction and SM) keeps displacements, squared distances and the products with displacement and
+// strength, 21 operations of a wall pair's 56, 16 of a Brinkman pair's 60 or so and 23 of a complex one's 350; the
+// rest runs on the integer pipe beside it.  The Stokeslet's products and sums are integers too (6 operations of
+// 27).  A pair outside the fixed-point ranges takes the FP64 function; a complex alpha that fx_alpha_c_ok
+// refuses takes sum_f64_kernel.  The wall kernel's factor t is applied once at the end, its factor h in the coefficients.
+// Every component of a velocity keeps the precision of an FP64 sum of its own terms.  Bound by the integer
+// pipe, the wall kernel by the FP64 pipe (86 % busy).  FP64 pairs -> these: 32,768 x 1,003 wall 3.6 -> 1.34 ms,
+// 16,384 x 16,384 Stokeslet 11.4 -> 5.8 ms (with its products in FP64 7.8), Brinkman 47 -> 10.4 ms, 4,099 x 2,500
+// complex Brinkman and strengths 7.4 -> 0.93 ms (four CTAs per SM; three for the complex pair, with four 0.95).  With
+// one exponent for the three components of strengths and sums the wall took 1.24 and the Stokeslet 5.1 ms,
+// and the z components of a sheet bent by 1e-6 of its size were exact to 2e-11.
 // ---------------------------------------------------------------------------
 constexpr int kFxThreads = 128, kFxTile = 64;
 static_assert(kFxTile <= 64, "one bit per source of a tile");
 // Brinkman pairs of small z take a series, the others an exponential.  Where fewer than this many lanes
 // of a warp are in the series' range, they put it off to the end of the tile, where each lane
 // works through its own list: with one pair in sixteen in the range a warp runs the series for 9 of
-// 64 sources and not for 55.  16,384 x 16,384 (two sums within a solve): 58.6 ms of the solve with
-// the series at once, 55.7 with 12, 56.0 with 20; 4,099 x 2,500 complex: 1.56, 1.33, 1.32 ms.
+// 64 sources and not for 55.  16,384 x 16,384 (two sums within a solve): 58.7 ms of the solve with
+// the series at once, 56.1 with 8, 55.9 with 12, 55.7 with 20; 4,099 x 2,500 complex: 1.17, 0.93, 0.93, 0.93 ms.
 constexpr int kFxLowNow = 12;
 template <bool CK>
 using FxAlphaOf = typename std::conditional<CK, FxAlphaC, FxAlpha>::type;
-template <int NF>
 struct FxSource {
     double x, y, z, e2, e;
-    int ef[NF];  // exponents of the strengths, or kFxBad
+    FxConst h;  // wall: the height
+    bool ok;
 };
-// strengths (for the wall times h) as mantissas and exponents
-template <int KIND, int NF>
-__device__ __forceinline__ void fx_strengths(double *f, double h, q60 *F, int *ef) {
-    if (KIND == FLG_WALL)
-#pragma unroll
-        for (int c = 0; c < 3 * NF; c++) f[c] *= h;
-#pragma unroll
-    for (int c = 0; c < NF; c++) ef[c] = fx_strength(f + 3 * c, 3, F + 3 * c);
-}
-// pairs between two readings of the accumulators: 16 terms
-template <int NF, bool CK>
-constexpr int kFxPairs = CK ? kFxSeg / NF : kFxSeg;
-// adds the velocity of the strengths F 2^ef
-template <int NF, class R>
-__device__ __forceinline__ void fx_add_radial(const FxDir &g, const R &r, const q60 *F, const int *ef, FxAcc<3> *acc) {
-#pragma unroll
-    for (int c = 0; c < NF; c++) {
-        q60 t[3], im[3];
-        const int x = r.x + ef[c];
-        acc[c].scale(x);
-        if constexpr (std::is_same<R, FxRadialC>::value) {
-            fx_radial_apply_c(g, r, F + 3 * c, t, im);
-            if (c == 1)  // i f: real part -A_im f, imaginary part A_re f
-#pragma unroll
-                for (int k = 0; k < 3; k++) im[k] = -im[k];
-            acc[1 - c].scale(x + r.xi);
-            acc[1 - c].add(0, im, x + r.xi);
-        } else {
-            fx_radial_apply(g, r, F + 3 * c, t);
-        }
-        acc[c].add(0, t, x);
+template <int KIND>
+__device__ __forceinline__ FxSource fx_source(const double *src, const double *eps, int64_t j) {
+    FxSource s{src[3 * j], src[3 * j + 1], src[3 * j + 2], 0.0, fabs(eps[j]), {0, 0}, true};
+    s.e2 = s.e * s.e;
+    if (KIND == FLG_WALL) {
+        s.ok = fx_const_ok(s.z);
+        if (s.ok) s.h = fx_const(s.z);
     }
+    return s;
+}
+// u += the velocity of the strengths f for a radial kernel's coefficients
+template <int NF>
+__device__ __forceinline__ void fx_add_radial(const FxCoef &c, double d0, double d1, double d2, const double *f, double *u) {
+    radial_apply(c.A, c.B, d0, d1, d2, f[0], f[1], f[2], u);
+    if constexpr (NF == 2) radial_apply(c.A, c.B, d0, d1, d2, f[3], f[4], f[5], u + 3);
 }
 template <int NF>
-__device__ __forceinline__ bool fx_ok(const int *ef) { return ef[0] != kFxBad && (NF == 1 || ef[NF - 1] != kFxBad); }
-// adds one pair; false: outside the fixed-point ranges
+__device__ __forceinline__ void fx_add_radial(const FxCoefC &c, double d0, double d1, double d2, const double *f, double *u) {
+    if constexpr (NF == 1) {
+        radial_apply(c.Ar, c.Br, d0, d1, d2, f[0], f[1], f[2], u);
+        radial_apply(c.Ai, c.Bi, d0, d1, d2, f[0], f[1], f[2], u + 3);
+    } else {
+        const double d[3] = {d0, d1, d2};
+        const double tr = fma(d2, f[2], fma(d1, f[1], d0 * f[0])), ti = fma(d2, f[5], fma(d1, f[4], d0 * f[3]));
+        const double br = fma(c.Br, tr, -c.Bi * ti), bi = fma(c.Br, ti, c.Bi * tr);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            u[k] = fma(c.Ar, f[k], fma(-c.Ai, f[3 + k], fma(br, d[k], u[k])));
+            u[3 + k] = fma(c.Ar, f[3 + k], fma(c.Ai, f[k], fma(bi, d[k], u[3 + k])));
+        }
+    }
+}
+// u += one pair (the wall's without its factor t); false: outside the fixed-point ranges
 template <int KIND, int NF, bool CK>
-__device__ __forceinline__ bool pair_fx(double tx, double ty, double tz, double sx, double sy, double sz, double e,
-                                        double e2, const q60 *F, const int *ef, const FxAlphaOf<CK> &al,
-                                        FxAcc<3> *acc) {
-    const double d0 = tx - sx, d1 = ty - sy, d2 = tz - sz;
-    if (!fx_ok<NF>(ef)) return false;
+__device__ __forceinline__ bool pair_fx(double tx, double ty, double tz, const FxSource &s, const double *f,
+                                        const FxAlphaOf<CK> &al, double *u) {
+    const double d0 = tx - s.x, d1 = ty - s.y, d2 = tz - s.z;
     if constexpr (KIND == FLG_WALL) {
-        const double dp = tz + sz;
-        const double rq = fma(d1, d1, fma(d0, d0, e2)), QF = fma(d2, d2, rq), QI = fma(dp, dp, rq);
-        if (!q_in_range(QF) || !q_in_range(QI) || (d_neg(tz) ^ d_neg(sz))) return false;
-        const FxWall w = fx_wall(d0, d1, d2, dp, QF, QI, e);
+        const double dp = tz + s.z;
+        const double rq = fma(d1, d1, fma(d0, d0, s.e2)), QF = fma(d2, d2, rq), QI = fma(dp, dp, rq);
+        if (!s.ok || !q_in_range(QF, kQExpWall) || !q_in_range(QI) || (d_neg(tz) ^ d_neg(s.z))) return false;
+        const FxWall w = fx_wall(d2, dp, QF, QI, s.e, s.h.m, s.h.x);
+        const double Rd = w.R * dp, b1 = fma(w.P, d2, -Rd), b2 = fma(w.P, d2, Rd);
 #pragma unroll
         for (int c = 0; c < NF; c++) {
-            q60 t[3];
-            const int x = fx_wall_apply(w, F + 3 * c, t) + ef[c];
-            acc[c].scale(x);
-            acc[c].add(0, t, x);
+            const double fx = f[3 * c], fy = f[3 * c + 1], fz = f[3 * c + 2], D = fma(d1, fy, d0 * fx);
+            const double m = fma(w.a, D, b1 * fz);
+            u[3 * c] = fma(w.c, fx, fma(d0, m, u[3 * c]));
+            u[3 * c + 1] = fma(w.c, fy, fma(d1, m, u[3 * c + 1]));
+            u[3 * c + 2] = fma(w.z, fz, fma(b2, D, u[3 * c + 2]));
         }
     } else {
-        const double Q = fma(d2, d2, fma(d1, d1, fma(d0, d0, e2)));
-        if (!q_in_range(Q)) return false;
-        const FxDir g = fx_dir(d0, d1, d2, Q, e);
-        if constexpr (KIND == FLG_STOKESLET) fx_add_radial<NF>(g, fx_stokeslet(g), F, ef, acc);
-        else fx_add_radial<NF>(g, fx_brinkman(g, al), F, ef, acc);
+        const double Q = fma(d2, d2, fma(d1, d1, fma(d0, d0, s.e2)));
+        if (!q_in_range(Q, kQExpRadial)) return false;
+        const FxDir g = fx_dir(Q, s.e);
+        if constexpr (KIND == FLG_STOKESLET) fx_add_radial<NF>(fx_coef(g, fx_stokeslet(g)), d0, d1, d2, f, u);
+        else fx_add_radial<NF>(fx_coef(g, fx_brinkman(g, al)), d0, d1, d2, f, u);
     }
     return true;
 }
+// a pair outside those ranges: the FP64 function (the wall's without its factor t).  Where powers of s would leave the
+// range, at coordinates scaled by a power of two c: u(x) = c u(c x) at alpha / c.
 template <int KIND, int NF, bool CK>
-__device__ __noinline__ void pair_f64_slow(double tx, double ty, double tz, const FxSource<NF> &s, const double *f,
-                                           int64_t j, double are, double aim, double *u) {
-    double fj[3 * NF];
-    load_strength<NF>(f, j, fj);
-    pair_f64<KIND, NF, CK>(tx, ty, tz, 2.0, s.x, s.y, s.z, s.e2, fj, are, aim, u);
+__device__ __noinline__ void pair_f64_slow(double tx, double ty, double tz, const FxSource &s, const double *f, double are,
+                                           double aim, double *u) {
+    const double d0 = tx - s.x, d1 = ty - s.y, d2 = tz - s.z;
+    const int ex = dexp(fma(d2, d2, fma(d1, d1, fma(d0, d0, s.e2)))) - 1023, k = -(ex >> 1);
+    if ((k >= -100 && k <= 100) || ex == -1023 || ex == 1024) {
+        pair_f64<KIND, NF, CK>(tx, ty, tz, 2.0, s.x, s.y, s.z, s.e2, f, are, aim, u);
+        return;
+    }
+    constexpr int OUTW = (NF == 2 || CK) ? 6 : 3;
+    const double c = scalbn(1.0, k), ic = scalbn(1.0, -k), e = c * s.e;
+    double w[OUTW];
+#pragma unroll
+    for (int i = 0; i < OUTW; i++) w[i] = 0.0;
+    pair_f64<KIND, NF, CK>(c * tx, c * ty, c * tz, 2.0, c * s.x, c * s.y, c * s.z, e * e, f, ic * are, ic * aim, w);
+#pragma unroll
+    for (int i = 0; i < OUTW; i++) u[i] += KIND == FLG_WALL ? c * (c * w[i]) : c * w[i];
 }
 template <int KIND, int NF, bool CK>
 __global__ void __launch_bounds__(kFxThreads, CK ? 3 : 4)
 sum_fx_kernel(SumArgs a, FxAlphaOf<CK> al) {
-    constexpr int OUTW = (NF == 2 || CK) ? 6 : 3, SEG = kFxPairs<NF, CK>;
-    __shared__ FxSource<NF> s_src[kFxTile];
-    __shared__ q60 s_f[kFxTile][3 * NF];
+    constexpr int OUTW = (NF == 2 || CK) ? 6 : 3;
+    __shared__ FxSource s_src[kFxTile];
+    constexpr bool INT = KIND == FLG_STOKESLET;  // products and sums in integers, too
+    constexpr int SEG = 16;                      // pairs between two readings of their accumulators
+    __shared__ double s_f[kFxTile][3 * NF];
+    __shared__ FxNum s_n[INT ? kFxTile : 1][3 * NF];
     const int64_t i = (int64_t)blockIdx.x * kFxThreads + threadIdx.x;
     const int64_t ii = i < a.M ? i : a.M - 1;
     const double tx = a.tg[3 * ii], ty = a.tg[3 * ii + 1], tz = a.tg[3 * ii + 2];
     double u[OUTW], us[OUTW];
-    FxAcc<3> acc[OUTW / 3];
+    FxAcc acc[NF];
 #pragma unroll
-    for (int c = 0; c < OUTW / 3; c++) acc[c].init();
+    for (int c = 0; c < NF; c++) acc[c].init();
 #pragma unroll
     for (int c = 0; c < OUTW; c++) u[c] = us[c] = 0.0;
     const int64_t j0 = (int64_t)blockIdx.y * a.split_len;
@@ -274,71 +289,67 @@ sum_fx_kernel(SumArgs a, FxAlphaOf<CK> al) {
         const int cnt = (int)(j1 - jt < kFxTile ? j1 - jt : kFxTile);
         __syncthreads();
         for (int k = threadIdx.x; k < cnt; k += kFxThreads) {
-            const int64_t j = jt + k;
-            FxSource<NF> s;
-            s.x = a.src[3 * j], s.y = a.src[3 * j + 1], s.z = a.src[3 * j + 2];
-            s.e = fabs(a.eps[j]);
-            s.e2 = s.e * s.e;
-            double f[3 * NF];
-            load_strength<NF>(a.f, j, f);
-            fx_strengths<KIND, NF>(f, s.z, s_f[k], s.ef);
-            s_src[k] = s;
+            s_src[k] = fx_source<KIND>(a.src, a.eps, jt + k);
+            load_strength<NF>(a.f, jt + k, s_f[k]);
+            if constexpr (INT)
+#pragma unroll
+                for (int c = 0; c < 3 * NF; c++) {
+                    s_n[k][c] = fx_num(s_f[k][c]);
+                    s_src[k].ok = s_src[k].ok && fx_num_ok(s_f[k][c]);
+                }
         }
         __syncthreads();
-        unsigned long long later = 0;  // sources of this target whose series is put off
-        for (int k0 = 0; k0 < cnt; k0 += SEG) {
+        if constexpr (INT) {
+            for (int k0 = 0; k0 < cnt; k0 += SEG) {
 #pragma unroll
-            for (int c = 0; c < OUTW / 3; c++) acc[c].clear();
-            const int k1 = min(cnt, k0 + SEG);
+                for (int c = 0; c < NF; c++) acc[c].clear();
+                const int k1 = min(cnt, k0 + SEG);
 #pragma unroll 1
-            for (int k = k0; k < k1; k++) {
-                const FxSource<NF> &s = s_src[k];
-                if constexpr (KIND == FLG_BRINKMANLET) {
+                for (int k = k0; k < k1; k++) {
+                    const FxSource &s = s_src[k];
                     const double d0 = tx - s.x, d1 = ty - s.y, d2 = tz - s.z;
                     const double Q = fma(d2, d2, fma(d1, d1, fma(d0, d0, s.e2)));
-                    const bool ok = fx_ok<NF>(s.ef) && q_in_range(Q);
-                    FxDir g;
-                    FxZ z{0, 0};
-                    if (ok) {
-                        g = fx_dir(d0, d1, d2, Q, s.e);
-                        z = fx_z(g, al.am, al.ae);
-                    }
-                    const bool low = z.k < 0, now = __popc(__ballot_sync(0xffffffffu, low)) >= kFxLowNow;
-                    if (low && !now)
-                        later |= 1ull << k;
-                    else if (ok)
-                        fx_add_radial<NF>(g, low ? fx_series(g, z, al) : fx_closed(g, z, al), s_f[k], s.ef, acc);
-                    else
-                        pair_f64_slow<KIND, NF, CK>(tx, ty, tz, s, a.f, jt + k, a.alpha_re, a.alpha_im, us);
-                } else if (!pair_fx<KIND, NF, CK>(tx, ty, tz, s.x, s.y, s.z, s.e, s.e2, s_f[k], s.ef, al, acc)) {
-                    pair_f64_slow<KIND, NF, CK>(tx, ty, tz, s, a.f, jt + k, a.alpha_re, a.alpha_im, us);
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < OUTW; c++) u[c] += acc[c / 3].value(c % 3);
-        }
-        if constexpr (KIND == FLG_BRINKMANLET) {
-            if (__any_sync(0xffffffffu, later != 0)) {
-                int terms = SEG;
-#pragma unroll
-                for (int c = 0; c < OUTW / 3; c++) acc[c].clear();
-                while (later) {
-                    const int k = __ffsll((long long)later) - 1;
-                    later &= later - 1;
-                    const FxSource<NF> &s = s_src[k];
-                    const double d0 = tx - s.x, d1 = ty - s.y, d2 = tz - s.z;
-                    const FxDir g = fx_dir(d0, d1, d2, fma(d2, d2, fma(d1, d1, fma(d0, d0, s.e2))), s.e);
-                    fx_add_radial<NF>(g, fx_series(g, fx_z(g, al.am, al.ae), al), s_f[k], s.ef, acc);
-                    if (--terms == 0) {
-                        terms = SEG;
-#pragma unroll
-                        for (int c = 0; c < OUTW; c++) u[c] += acc[c / 3].value(c % 3);
-#pragma unroll
-                        for (int c = 0; c < OUTW / 3; c++) acc[c].clear();
-                    }
+                    if (s.ok && q_in_range(Q, kQExpRadial)) fx_add_stokeslet<NF>(d0, d1, d2, Q, s.e, s_n[k], acc);
+                    else pair_f64_slow<KIND, NF, CK>(tx, ty, tz, s, s_f[k], a.alpha_re, a.alpha_im, us);
                 }
 #pragma unroll
                 for (int c = 0; c < OUTW; c++) u[c] += acc[c / 3].value(c % 3);
+            }
+            continue;
+        }
+        unsigned long long later = 0;  // sources of this target whose series is put off
+#pragma unroll 1
+        for (int k = 0; k < cnt; k++) {
+            const FxSource &s = s_src[k];
+            if constexpr (KIND == FLG_BRINKMANLET) {
+                const double d0 = tx - s.x, d1 = ty - s.y, d2 = tz - s.z;
+                const double Q = fma(d2, d2, fma(d1, d1, fma(d0, d0, s.e2)));
+                const bool ok = q_in_range(Q, kQExpRadial);
+                FxDir g;
+                FxZ z{0, 0};
+                if (ok) {
+                    g = fx_dir(Q, s.e);
+                    z = fx_z(g, al.am, al.ae);
+                }
+                const bool low = z.k < 0, now = __popc(__ballot_sync(0xffffffffu, low)) >= kFxLowNow;
+                if (low && !now)
+                    later |= 1ull << k;
+                else if (ok)
+                    fx_add_radial<NF>(fx_coef(g, low ? fx_series(g, z, al) : fx_closed(g, z, al)), d0, d1, d2, s_f[k], u);
+                else
+                    pair_f64_slow<KIND, NF, CK>(tx, ty, tz, s, s_f[k], a.alpha_re, a.alpha_im, us);
+            } else if (!pair_fx<KIND, NF, CK>(tx, ty, tz, s, s_f[k], al, u)) {
+                pair_f64_slow<KIND, NF, CK>(tx, ty, tz, s, s_f[k], a.alpha_re, a.alpha_im, us);
+            }
+        }
+        if constexpr (KIND == FLG_BRINKMANLET) {
+            while (later) {
+                const int k = __ffsll((long long)later) - 1;
+                later &= later - 1;
+                const FxSource &s = s_src[k];
+                const double d0 = tx - s.x, d1 = ty - s.y, d2 = tz - s.z;
+                const FxDir g = fx_dir(fma(d2, d2, fma(d1, d1, fma(d0, d0, s.e2))), s.e);
+                fx_add_radial<NF>(fx_coef(g, fx_series(g, fx_z(g, al.am, al.ae), al)), d0, d1, d2, s_f[k], u);
             }
         }
     }
@@ -1097,9 +1108,9 @@ __global__ void __launch_bounds__(kNearThreads) near_f64_kernel(NearArgs a, FxAl
     const CellGrid G = *a.grid;
     const double tx = a.tg[3 * i], ty = a.tg[3 * i + 1], tz = a.tg[3 * i + 2];
     const float fx = __double2float_rn(tx), fy = __double2float_rn(ty), fz = __double2float_rn(tz);
-    double u[OUTW], uf[OUTW];  // uf: fixed-point pairs (the wall's without their factor t)
+    double u[OUTW], uf[OUTW], us[OUTW];  // far field; near pairs (the wall's without their factor t), in fixed point and not
 #pragma unroll
-    for (int c = 0; c < OUTW; c++) u[c] = uf[c] = 0.0;
+    for (int c = 0; c < OUTW; c++) u[c] = uf[c] = us[c] = 0.0;
     // the nine runs of candidates: run q is cell row (y, z) = (cy + q % 3 - 1, cz + q / 3 - 1)
     const int cx = cell_coord(tx, G.ox, G.inv_h, G.nx);
     const int cy = cell_coord(ty, G.oy, G.inv_h, G.ny);
@@ -1133,34 +1144,20 @@ __global__ void __launch_bounds__(kNearThreads) near_f64_kernel(NearArgs a, FxAl
         total += __shfl_sync(0xffffffffu, rn[q / kNearLanes], gs + q % kNearLanes);
     }
     const int rounds = (int)(__reduce_max_sync(0xffffffffu, (unsigned)total) + kNearLanes - 1) / kNearLanes;
-    FxAcc<3> acc[OUTW / 3];
-#pragma unroll
-    for (int c = 0; c < OUTW / 3; c++) acc[c].init();
-    int terms = 0, cnt = 0;
+    int cnt = 0;
     auto evaluate = [&]() {
         for (int q = l; q < cnt; q += kNearLanes) {
             const int64_t j = a.sorted[list[grp][q]];
-            const double sx = a.src[3 * j], sy = a.src[3 * j + 1], sz = a.src[3 * j + 2], e = fabs(a.eps[j]);
-            double fj[3 * NF], fh[3 * NF];
+            const FxSource s = fx_source<KIND>(a.src, a.eps, j);
+            double fj[3 * NF];
             load_strength<NF>(a.f, j, fj);
-            if (!CK || al.am != 0) {
-                q60 F[3 * NF];
-                int ef[NF];
-#pragma unroll
-                for (int c = 0; c < 3 * NF; c++) fh[c] = fj[c];
-                fx_strengths<KIND, NF>(fh, sz, F, ef);
-                if (pair_fx<KIND, NF, CK>(tx, ty, tz, sx, sy, sz, e, e * e, F, ef, al, acc)) {
-                    if (++terms == kFxPairs<NF, CK>) {
-#pragma unroll
-                        for (int c = 0; c < OUTW; c++) uf[c] += acc[c / 3].value(c % 3);
-#pragma unroll
-                        for (int c = 0; c < OUTW / 3; c++) acc[c].clear();
-                        terms = 0;
-                    }
+            if constexpr (CK)
+                if (al.am == 0) {  // an alpha that the fixed-point pairs do not take
+                    pair_f64<KIND, NF, CK>(tx, ty, tz, 2.0, s.x, s.y, s.z, s.e2, fj, a.alpha_re, a.alpha_im, uf);
                     continue;
                 }
-            }
-            pair_f64<KIND, NF, CK>(tx, ty, tz, 2.0 * tz, sx, sy, sz, e * e, fj, a.alpha_re, a.alpha_im, u);
+            if (!pair_fx<KIND, NF, CK>(tx, ty, tz, s, fj, al, uf))
+                pair_f64_slow<KIND, NF, CK>(tx, ty, tz, s, fj, a.alpha_re, a.alpha_im, us);
         }
     };
     for (int r = 0; r < rounds; r++) {
@@ -1190,7 +1187,7 @@ __global__ void __launch_bounds__(kNearThreads) near_f64_kernel(NearArgs a, FxAl
     __syncwarp();
 #pragma unroll
     for (int c = 0; c < OUTW; c++) {
-        uf[c] += acc[c / 3].value(c % 3);
+        uf[c] += us[c];
         u[c] += KIND == FLG_WALL ? tz * uf[c] : uf[c];
     }
 #pragma unroll
