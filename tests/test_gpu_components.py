@@ -173,3 +173,25 @@ def test_scales_outside_the_fixed_point_ranges(scale):
     G, S = wall_blocks(X, Y, 0.05)
     ref, size = np.einsum("ijab,jb->ia", G, F.astype(LD)), np.einsum("ijab,jb->ia", S, abs(F).astype(LD))
     assert np.all(abs(u - ref) <= 100 * U * size)
+
+
+@pytest.mark.parametrize("strengths", ["real", "complex"])
+@pytest.mark.parametrize("order", ["mixed", "sorted", "all below"])
+def test_heights_of_both_signs(order, strengths):
+    """Targets and sources above and below the wall, alternating within a warp and a tile or in runs."""
+    rng = np.random.default_rng(8)
+    X, Y = rng.uniform(-1, 1, (300, 3)), rng.uniform(-1, 1, (150, 3))
+    if order == "sorted":
+        X, Y = X[X[:, 2].argsort()], Y[Y[:, 2].argsort()]
+    elif order == "all below":
+        X[:, 2], Y[:, 2] = -abs(X[:, 2]), abs(Y[:, 2])
+    X[7, 2] = Y[9, 2] = 0.0
+    F = rng.normal(size=(150, 3))
+    if strengths == "complex":
+        F = F + 1j * rng.normal(size=(150, 3))
+    u = fl.evaluate(fl.WallStokeslet3D(), X, Y, F, 0.3)
+    G, S = wall_blocks(X, Y, 0.3)
+    ref = np.einsum("ijab,jb->ia", G, F.astype(np.clongdouble if strengths == "complex" else LD))
+    # (the terms of opposite heights do not cancel to the factor 2 t h: each counts by itself)
+    size = np.einsum("ijab,jb->ia", abs(S), abs(F.real).astype(LD) + abs(F.imag))
+    assert np.all(abs(u - ref) <= (30 + 150) * U * size)
