@@ -1141,20 +1141,21 @@ int gemv_f32_presplit(int64_t n_rows, int64_t n_cols, const float *A, int64_t ld
 }  // namespace flg
 
 // nearest force point of every quadrature point (the reference's k-d tree query,
-// core/assemble.py:61-65): exhaustive, FP64 squared distances, the first index on ties.  A warp per
-// query, each lane every 32nd force point, distances compared as integers (non-negative doubles order
-// like their bits; a NaN is above infinity and never taken): a thread per query walked all points
-// alone, seven FP64 instructions of 64 clocks each (896 x 226: 112 us, this form 7 us).
+// core/assemble.py:61-65): exhaustive, FP64 squared distances, the first index on ties.  LANES lanes per
+// query, each every LANES-th force point, distances compared as integers (non-negative doubles order
+// like their bits; a NaN is above infinity and never taken): with a thread per query few queries walk all
+// points alone, seven FP64 instructions of 64 clocks each (896 x 226: 112 us, a warp per query 7 us).
+template <int LANES>
 __global__ void __launch_bounds__(256) nearest_kernel(const double *quad, int64_t Q, const double *force, int64_t N,
                                                       int64_t *out) {
-    const int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (q >= Q) return;
-    const double px = quad[3 * q], py = quad[3 * q + 1], pz = quad[3 * q + 2];
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, q = t / LANES;
+    const bool live = q < Q;
+    const int64_t qq = live ? q : Q - 1;
+    const double px = quad[3 * qq], py = quad[3 * qq + 1], pz = quad[3 * qq + 2];
     unsigned long long best = 0x7ff0000000000000ull;  // infinity
     long long bi = INT64_MAX;
 #pragma unroll 4
-    for (int64_t k = lane; k < N; k += 32) {
+    for (int64_t k = t % LANES; k < N; k += LANES) {
         const double dx = px - force[3 * k], dy = py - force[3 * k + 1], dz = pz - force[3 * k + 2];
         const double d2 = dx * dx + dy * dy + dz * dz;
         const unsigned long long b = (unsigned long long)__double_as_longlong(d2);
@@ -1164,7 +1165,7 @@ __global__ void __launch_bounds__(256) nearest_kernel(const double *quad, int64_
         }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = LANES / 2; o > 0; o >>= 1) {
         const unsigned long long ob = __shfl_xor_sync(0xffffffffu, best, o);
         const long long oi = __shfl_xor_sync(0xffffffffu, bi, o);
         if (ob < best || (ob == best && oi < bi)) {
@@ -1172,7 +1173,11 @@ __global__ void __launch_bounds__(256) nearest_kernel(const double *quad, int64_
             bi = oi;
         }
     }
-    if (lane == 0) out[q] = bi == INT64_MAX ? 0 : bi;
+    if (live && t % LANES == 0) out[q] = bi == INT64_MAX ? 0 : bi;
+}
+template <int LANES>
+static void launch_nearest(const double *quad, int64_t Q, const double *force, int64_t N, int64_t *out, cudaStream_t st) {
+    nearest_kernel<LANES><<<(unsigned)ceil_div(Q * LANES, 256), 256, 0, st>>>(quad, Q, force, N, out);
 }
 
 extern "C" int flg_nearest_neighbors(const double *quad, int64_t Q, const double *force, int64_t N, int64_t *out,
@@ -1182,7 +1187,10 @@ extern "C" int flg_nearest_neighbors(const double *quad, int64_t Q, const double
     if (Q == 0) return FLG_OK;
     FLG_REQUIRE(N > 0, "no force points to search");
     FLG_REQUIRE(quad && force && out, "null pointer");
-    nearest_kernel<<<(unsigned)ceil_div(Q, 8), 256, 0, as_stream(stream)>>>(quad, Q, force, N, out);
+    // Eight lanes per query, whose reduction is shorter, once they leave two warps per scheduler.  us with 32 / 8 / 1
+    // lanes: 896 x 1,000: 28 / 70 / 461; 4,000 x 100: 24 / 19 / 57; 9,000 x 1,000: 130 / 119 / 462; 400,000 x 100: 985 / 467 / 474
+    if (Q * 8 >= 2 * 32 * 4LL * sm_count()) launch_nearest<8>(quad, Q, force, N, out, as_stream(stream));
+    else launch_nearest<32>(quad, Q, force, N, out, as_stream(stream));
     FLG_LAUNCH_CHECK();
     return FLG_OK;
 }
