@@ -7,6 +7,7 @@
 #include <string.h>
 
 #include "../../include/fluidlets_gb300.h"
+#include "ir_tolerance.cuh"
 
 namespace flg {
 
@@ -113,16 +114,5 @@ struct TcBatch {
     int count = 1;
     int64_t sC = 0, sL = 0, sU = 0;
 };
-
-// Inner (preconditioned) tolerance of a step of the dense refinement at residual norm rn, aimed at tol.  At 1e-4 many
-// inner solves ended just below it after one iteration, and a third FP64 residual was needed (wall, 8,192
-// blobs, tf32: 3 steps, 45.4 ms); at 1e-6 two steps reach 1e-12 (42.1 ms).  The last step aims at a twentieth
-// of tol, so that forces do not end with the whole tolerance as their error; a step gains eight digits at most
-// (its operator is the FP32 copy of the matrix).
-__host__ __device__ inline double ir_inner_tolerance(double tol, double rn) {
-    const double need = tol / rn;
-    if (!(need >= 1e-8)) return 1e-6;
-    return fmin(1e-6, fmax(0.05 * need, 2e-8));
-}
 
 }  // namespace flg

@@ -57,7 +57,7 @@ struct IrState {
     int m;                              // inner columns allowed
     int k;                              // inner columns done in this step
     int breakdown;
-    int outer, max_outer, iters, stall;
+    int outer, max_outer, iters, stall, beyond;
     int status;                         // 0 running, 1 converged, 2 stopped (stall / step limit)
 };
 
@@ -152,6 +152,7 @@ __global__ void ir_ctrl_init(IrState *S, double rtol, int m, int max_outer, cuda
     S->max_outer = max_outer;
     S->iters = 0;
     S->stall = 0;
+    S->beyond = 0;
     S->status = S->rn <= S->tol ? 1 : 0;  // b = 0: x = 0 is the answer
     cudaGraphSetConditional(h_outer, S->status == 0 ? 1u : 0u);
 }
@@ -242,11 +243,12 @@ __global__ void ir_ctrl_outer(IrState *S, cudaGraphConditionalHandle h_outer) {
     S->rn = sqrt(fmax(S->dot, 0.0));
     S->outer++;
     int go = 1;
-    if (S->rn <= S->tol) {
+    S->stall = S->rn > 0.5 * S->prev_rn ? S->stall + 1 : 0;
+    if (ir_done(S->tol, S->rn, S->beyond || S->stall > 0 || S->outer >= S->max_outer)) {
         S->status = 1;
         go = 0;
     } else {
-        S->stall = S->rn > 0.5 * S->prev_rn ? S->stall + 1 : 0;
+        S->beyond = S->beyond || S->rn <= S->tol;
         S->prev_rn = S->rn;
         if (S->stall >= 3 || S->outer >= S->max_outer) {
             S->status = 2;

@@ -1,0 +1,32 @@
+// ir_tolerance.cuh -- how far the steps of the dense refinement go (krylov.cu, ir_graph.cu).
+#pragma once
+#include <math.h>
+
+#if defined(__CUDACC__)
+#define FLG_IR_HD __host__ __device__
+#else
+#define FLG_IR_HD
+#endif
+
+namespace flg {
+
+// Inner (preconditioned) tolerance of a step at residual norm rn, aimed at tol.  At 1e-4 many
+// inner solves ended just below it after one iteration, and a third FP64 residual was needed (wall, 8,192
+// blobs, tf32: 3 steps, 45.4 ms); at 1e-6 two steps reach 1e-12 (42.1 ms).  A step gains eight digits at most (its
+// operator is the FP32 copy of the matrix); one that needs no more than that aims at a fiftieth of tol, as far as
+// those eight digits go.
+FLG_IR_HD inline double ir_inner_tolerance(double tol, double rn) {
+    const double need = tol / rn;
+    if (need >= 1.0) return 1e-4;  // (a step beyond the tolerance, see below)
+    if (!(need >= 1e-8)) return 1e-6;
+    return fmin(1e-6, fmax(0.02 * need, 2e-8));
+}
+
+// Whether the refinement is done at residual norm rn.  The error of the solution is the residual times the condition
+// number, and two steps end anywhere below tol where ones of 1e-4 had overshot it (swimmer of 1,470 unknowns: residual
+// 2.5e-13, forces exact to 5e-11 instead of 9e-14): above a fiftieth of tol one more step follows.  Largest errors over
+// 60 bodies and 14 swimmers, steps of 1e-4 / these: 1.0e-12, 5.1e-13 / 2.0e-13, 5.1e-13; above a twentieth 3.6e-13,
+// 2.3e-12; above a hundredth 5e-15, 6e-14, but nearly every solve takes a third step (24,576 unknowns 32.9 -> 37.6 ms).
+FLG_IR_HD inline bool ir_done(double tol, double rn, bool beyond) { return rn <= tol && (beyond || rn <= 0.02 * tol); }
+
+}  // namespace flg

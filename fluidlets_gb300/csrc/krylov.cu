@@ -665,22 +665,26 @@ extern "C" int flg_gmres_ir_dense(int64_t n, const double *A, int64_t ld, const 
         FLG_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * n, st));
         return FLG_OK;
     }
+    const double tol = rtol * bn;
     double rn = 0.0, prev = INFINITY;
     int stall = 0;
+    bool beyond = false;  // the step beyond the tolerance has been taken
     for (int o = 0; o <= 60; o++) {
         bool is_b = false;
         FLG_TRY(o == 0 ? g.residual_from(b, x, &is_b) : g.residual(b, x));
         if (is_b) rn = bn;
         else FLG_TRY(g.norm(g.r, &rn));
         *resid = rn / bn;
-        if (rn <= rtol * bn) return FLG_OK;
-        if (*iters >= restart * maxiter) break;
+        const bool last = *iters >= restart * maxiter;
         stall = (rn > 0.5 * prev) ? stall + 1 : 0;
+        if (ir_done(tol, rn, beyond || stall > 0 || last || o == 60)) return FLG_OK;
+        if (last) break;
+        beyond = beyond || rn <= tol;
         if (stall >= 3) break;
         prev = rn;
         FLG_CUDA(cudaMemsetAsync(d, 0, sizeof(double) * n, st));
         double rin;
-        int s2 = gi.solve(g.r, d, ir_inner_tolerance(rtol * bn, rn), maxiter, *iters, rin, rn, true);
+        int s2 = gi.solve(g.r, d, ir_inner_tolerance(tol, rn), maxiter, *iters, rin, rn, true);
         if (s2 != FLG_OK && s2 != FLG_ERR_NOT_CONVERGED) return s2;
         add_kernel<double><<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(x, d, n);
         FLG_LAUNCH_CHECK();
