@@ -7,6 +7,7 @@
 #include <string.h>
 
 #include "../../include/fluidlets_gb300.h"
+#include "device_once.cuh"
 #include "ir_tolerance.cuh"
 
 namespace flg {

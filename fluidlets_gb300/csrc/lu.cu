@@ -466,14 +466,11 @@ constexpr int kTrsmWide = 2 * 8;
 static int swap_trsm(double *A, int64_t ld, const int32_t *ipiv, int64_t k0, int64_t c0, int64_t c1, uint16_t *SB,
                      int64_t cap, int *eb, SliceMask *mb, int near, cudaStream_t st) {
     const int64_t nc = c1 - c0;
-    static bool attr_set = false;
-    if (!attr_set) {
-        FLG_CUDA(cudaFuncSetAttribute(swap_trsm_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)trsm_smem(4, kTrsmWarps)));
-        FLG_CUDA(cudaFuncSetAttribute(swap_trsm_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)trsm_smem(16, kTrsmWarps)));
-        attr_set = true;
-    }
+    FLG_ONCE_PER_DEVICE(
+        FLG_CUDA(cudaFuncSetAttribute(swap_trsm_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem(4,
+                                      kTrsmWarps)));
+        FLG_CUDA(cudaFuncSetAttribute(swap_trsm_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem(16,
+                                      kTrsmWarps))));
     // G = 4 once its warps (8 columns each) fill half of the schedulers; below, G = 16's shorter chain
     const bool wide = nc >= kTrsmWide * (int64_t)sm_count();
     const int cols = wide ? 8 : 2;
@@ -945,12 +942,9 @@ __global__ void __launch_bounds__(kTeamThreads<RW> *NT, NT == 1 ? 2 : 1) lowp_pa
 template <int NC, int NT, int RW>
 static int launch_panels(LowpPanelArgs &a, int nbat, int64_t ctas, cudaStream_t st) {
     constexpr size_t smem = sizeof(LowpPanelSmem<NC, NT>);
-    static bool attr_set = false;
-    if (!attr_set) {
+    FLG_ONCE_PER_DEVICE(
         FLG_CUDA(cudaFuncSetAttribute(lowp_panel_kernel<NC, NT, RW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-        attr_set = true;
-    }
+                                      (int)smem)));
     a.ntu = (int)std::min<int64_t>(ceil_div(a.nr, 32 * NC * NT), std::max<int64_t>(1, ctas / 2 / nbat));
     lowp_panel_kernel<NC, NT, RW><<<dim3(2 * a.ntu, nbat), kTeamThreads<RW> * NT, smem, st>>>(a);
     FLG_LAUNCH_CHECK();
@@ -1347,11 +1341,9 @@ size_t lu_solve_lowp_bytes(int64_t n) {
 
 // the kernel attributes of the solve, set once (before any graph capture that includes it)
 int lu_solve_lowp_prepare() {
-    static bool attr_set = false;
-    if (!attr_set) {
-        FLG_CUDA(cudaFuncSetAttribute(lowp_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kApplySmem));
-        attr_set = true;
-    }
+    FLG_ONCE_PER_DEVICE(
+        FLG_CUDA(cudaFuncSetAttribute(lowp_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kApplySmem)));
     return FLG_OK;
 }
 
@@ -1486,12 +1478,9 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
                 work_bytes);
     F64Streams *fs = nullptr;
     FLG_TRY(f64_streams(&fs));
-    static bool attr_set = false;
-    if (!attr_set) {
+    FLG_ONCE_PER_DEVICE(
         FLG_CUDA(cudaFuncSetAttribute(panel_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      384 * kPanel * (int)sizeof(double)));
-        attr_set = true;
-    }
+                                      384 * kPanel * (int)sizeof(double))));
     FLG_CUDA(cudaMemsetAsync(bar, 0, sizeof(GridBar), st));
     // the panel of columns [k0, k0 + kb), rows k0.. on stream s, and the slices of its L21;
     // started (optional) completes once the panel's first kernel is resident
@@ -1612,12 +1601,9 @@ extern "C" int flg_lu_solve_f64(int64_t n, int64_t nrhs, const double *LU, int64
     FLG_REQUIRE(nrhs <= 65535, "at most 65,535 right-hand sides per call");
     if (solve_on_cluster(n, nrhs)) return trsv_cluster(n, nrhs, LU, ld, ipiv, B, ldb, st);
     if (n <= kPivSmemMax) {
-        static bool attr_set = false;
-        if (!attr_set) {
+        FLG_ONCE_PER_DEVICE(
             FLG_CUDA(cudaFuncSetAttribute(apply_pivots_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          kPivSmemMax * (int)sizeof(double)));
-            attr_set = true;
-        }
+                                          kPivSmemMax * (int)sizeof(double))));
         apply_pivots_smem_kernel<<<(unsigned)nrhs, 256, n * sizeof(double), st>>>(B, ldb, ipiv, n);
     } else {
         apply_pivots_kernel<<<(unsigned)ceil_div(nrhs, 32), 32, 0, st>>>(B, ldb, nrhs, ipiv, n);
@@ -1784,12 +1770,9 @@ static int lowp_factor(int64_t n, int nbat, float *A, int64_t ld, int64_t sA, in
         }
         return tc_update(C, ld, Lp, ld, Up, W, m, nc, K, mode, tcw, tcb, st, dinfo + 1, false, tile, ctas, bA);
     };
-    static bool attr_set = false;  // set once, so a later call can be captured in a graph
-    if (!attr_set) {
-        FLG_CUDA(cudaFuncSetAttribute(block_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sizeof(LowpPanelSmem<1, 1>)));
-        attr_set = true;
-    }
+    FLG_ONCE_PER_DEVICE(
+        FLG_CUDA(cudaFuncSetAttribute(block_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LowpPanelSmem<1,
+                                      1>))));
     const bool tc = mode != FLG_LU_FP32;
     const int64_t nblk = ceil_div(n, kNB);
     SideStream *side = nullptr;

@@ -326,13 +326,10 @@ int cluster_panel(const ClusterPanelArgs &in, cudaEvent_t started, cudaStream_t 
     ClusterPanelArgs a = in;
     const int64_t m = a.n - a.k0;
     FLG_REQUIRE(a.kb >= 1 && a.kb <= kHalf && m <= kClusterPanelRows, "bad cluster panel");
-    static bool attr_set = false;
-    if (!attr_set) {
+    FLG_ONCE_PER_DEVICE(
         FLG_CUDA(cudaFuncSetAttribute(panel_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         FLG_CUDA(cudaFuncSetAttribute(panel_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)panel_smem(32 * kMaxRowWarps)));
-        attr_set = true;
-    }
+                                      (int)panel_smem(32 * kMaxRowWarps))));
     int ncta = 1;
     while (ncta < kPanelCtas && (int64_t)ncta * 32 < m) ncta *= 2;
     a.rpc = (int)ceil_div(m, ncta);

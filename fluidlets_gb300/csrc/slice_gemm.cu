@@ -439,11 +439,9 @@ int slice_update(double *C, int64_t ldc, int64_t m, int64_t nc, const double *A,
     const __nv_bfloat16 *b = (const __nv_bfloat16 *)SB + b0 * kSliceK;
     FLG_TRY(make_operand_map(&tma, SA, m, kSliceK, kSliceK, FLG_LU_BF16, TC_BM, kSlices, capA * kSliceK, kSlices));
     FLG_TRY(make_operand_map(&tmb, b, nc, kSliceK, kSliceK, FLG_LU_BF16, SG_BN, kSlices, capB * kSliceK, kSlices));
-    static bool attr_set = false;
-    if (!attr_set) {
-        FLG_CUDA(cudaFuncSetAttribute(slice_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SG_SMEM));
-        attr_set = true;
-    }
+    FLG_ONCE_PER_DEVICE(
+        FLG_CUDA(cudaFuncSetAttribute(slice_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)SG_SMEM)));
     const int64_t ntiles = ceil_div(m, TC_BM) * ceil_div(nc, SG_BN);
     const unsigned grid = (unsigned)std::min<int64_t>(ntiles, std::max(1, max_ctas));
     slice_update_kernel<<<grid, SG_THREADS, SG_SMEM, st>>>(tma, tmb, C, ldc, (int)m, (int)nc, A, B, ea, eb + b0,

@@ -1345,11 +1345,8 @@ int sum_plan_geometry(int kind, const double *src, const double *eps, int64_t N,
     if (N <= kClusterPlanMax) {
         PlanArgs a{src, eps, f, N, L.NQ, kind == FLG_WALL ? 1 : 0, p->bounds, p->grid, p->cell_of, p->counts, p->offsets,
                    p->block_sums, p->slots, p->sorted, p->packed, p->tile_box};
-        static bool attr_set = false;
-        if (!attr_set) {
-            FLG_CUDA(cudaFuncSetAttribute(plan_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            attr_set = true;
-        }
+        FLG_ONCE_PER_DEVICE(
+            FLG_CUDA(cudaFuncSetAttribute(plan_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)));
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(kPlanCtas);
         cfg.blockDim = dim3(kPlanThreads);

@@ -355,12 +355,9 @@ int tc_pick_tile(int64_t m, int64_t nc, int sms, int nb = 1) {
 template <int MODE, int BN>
 static int tc_launch(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, int64_t m, int64_t nc,
                      int nkb, int nb, bool store, int *err, int sms, cudaStream_t st) {
-    static bool attr_set = false;  // set once, so a later call can be captured in a graph
-    if (!attr_set) {
+    FLG_ONCE_PER_DEVICE(
         FLG_CUDA(cudaFuncSetAttribute(tc_update_kernel<MODE, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)TcTile<BN>::SMEM));
-        attr_set = true;
-    }
+                                      (int)TcTile<BN>::SMEM)));
     const int64_t ntiles = nb * ceil_div(m, TC_BM) * ceil_div(nc, BN);
     FLG_REQUIRE(ntiles < (1LL << 31), "too many tiles");
     const unsigned grid = (unsigned)std::min<int64_t>(ntiles, sms);

@@ -226,12 +226,9 @@ bool trsv_fits(int64_t n) { return trsv_smem(n) <= 232448; }
 
 int trsv_cluster(int64_t n, int64_t nrhs, const double *LU, int64_t ld, const int32_t *ipiv, double *B, int64_t ldb,
                  cudaStream_t st) {
-    static bool attr_set = false;
-    if (!attr_set) {
+    FLG_ONCE_PER_DEVICE(
         FLG_CUDA(cudaFuncSetAttribute(trsv_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        FLG_CUDA(cudaFuncSetAttribute(trsv_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
-        attr_set = true;
-    }
+        FLG_CUDA(cudaFuncSetAttribute(trsv_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448)));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(kTvCtas * nrhs));
     cfg.blockDim = dim3(kTvThreads);
