@@ -58,6 +58,7 @@ SIGNATURES = {
     "flg_lu_factor_f64_workspace": (c_size_t, [c_int64]),
     "flg_lu_factor_f64": (c_int, [c_int64, _P, c_int64, _P, POINTER(c_int), _P, c_size_t, _P]),
     "flg_lu_solve_f64": (c_int, [c_int64, c_int64, _P, c_int64, _P, _P, c_int64, _P]),
+    "flg_lu_solve_f64_flag": (c_int, [c_int64, c_int64, _P, c_int64, _P, _P, c_int64, _P, _P]),
     "flg_lu_lowp_dinv_elems": (c_int64, [c_int64]),
     "flg_lu_factor_lowp_workspace": (c_size_t, [c_int64, c_int]),
     "flg_lu_factor_lowp": (c_int, [c_int64, _P, c_int64, c_int, _P, POINTER(c_int), _P, c_size_t, _P]),

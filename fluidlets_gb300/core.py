@@ -261,9 +261,23 @@ class SolveInfo:
     ir_steps: int = 0        # FP64 refinement steps of the mixed-precision path
 
 
-def _lu_solve_dev(K: torch.Tensor, U: torch.Tensor) -> torch.Tensor:
+class _SolveFlag:
+    """Outcome of the bounded waits of an FP64 triangular solve: a wait that ran out leaves NaN in the
+    solution and raises the flag.  Callers that read a result back look at the flag only when it is
+    NaN, so that the usual solve costs no round trip."""
+
+    def __init__(self, device):
+        self.word = torch.empty(1, dtype=torch.int32, device=device)
+
+    def check(self):
+        if int(self.word):
+            raise RuntimeError("LU solve: a bounded device wait timed out")
+
+
+def _lu_solve_dev(K: torch.Tensor, U: torch.Tensor, flag: _SolveFlag | None = None) -> torch.Tensor:
     """Dense FP64 LU with partial pivoting (getrf + getrs) on the device; K is overwritten.
-    U holds one right-hand side (n values, returned flat) or several as the columns of (n, k)."""
+    U holds one right-hand side (n values, returned flat) or several as the columns of (n, k).
+    With a flag the caller checks it after a NaN; without, the solve is waited for and checked."""
     n = K.shape[0]
     L = load()
     if K.is_complex():
@@ -275,7 +289,7 @@ def _lu_solve_dev(K: torch.Tensor, U: torch.Tensor) -> torch.Tensor:
         R[n:, n:] = K.real
         b = torch.cat([U.real, U.imag]).to(torch.float64).contiguous() if U.is_complex() else \
             torch.cat([U, torch.zeros_like(U)]).contiguous()
-        x = _lu_solve_dev(R, b)
+        x = _lu_solve_dev(R, b, flag)
         return torch.complex(x[:n], x[n:])
     piv = torch.empty(n, dtype=torch.int32, device=K.device)
     nbytes = L.flg_lu_factor_f64_workspace(n)
@@ -284,13 +298,19 @@ def _lu_solve_dev(K: torch.Tensor, U: torch.Tensor) -> torch.Tensor:
     check(L.flg_lu_factor_f64(n, dv.ptr(K), n, dv.ptr(piv), ctypes.byref(info), dv.ptr(ws), nbytes, dv.stream()),
           "LU factorization")
     # the solve overwrites its right-hand side: always work on a copy of U
-    B = U.reshape(n, -1).to(torch.float64).clone() if not U.is_complex() else None
-    if B is None:  # real matrix, complex right-hand side: two real columns
+    if U.is_complex():  # real matrix, complex right-hand side: two real columns
         B = torch.stack([U.real, U.imag], 1).contiguous()
-        check(L.flg_lu_solve_f64(n, 2, dv.ptr(K), n, dv.ptr(piv), dv.ptr(B), 2, dv.stream()), "LU solve")
-        return torch.complex(B[:, 0], B[:, 1])
+    else:
+        B = U.reshape(n, -1).to(torch.float64).clone()
     nrhs = B.shape[1]
-    check(L.flg_lu_solve_f64(n, nrhs, dv.ptr(K), n, dv.ptr(piv), dv.ptr(B), nrhs, dv.stream()), "LU solve")
+    own = flag is None
+    flag = _SolveFlag(K.device) if own else flag
+    check(L.flg_lu_solve_f64_flag(n, nrhs, dv.ptr(K), n, dv.ptr(piv), dv.ptr(B), nrhs, dv.ptr(flag.word), dv.stream()),
+          "LU solve")
+    if own:
+        flag.check()
+    if U.is_complex():
+        return torch.complex(B[:, 0], B[:, 1])
     return B.reshape(-1) if nrhs == 1 else B
 
 
@@ -530,6 +550,7 @@ def resistance(kernel, points, velocities, eps, mu=1.0, method="auto", rtol=1e-1
         method = "lu" if U.numel() <= DENSE_MAX else "gmres"
     prec = _prec(precision)
     ir_steps = 0
+    flag = None
     # mixed precision refines to rtol / 100 so that the FORCE error against the FP64 solve,
     # not only the residual, is within rtol (error <= condition number x residual)
     rtol_ir = rtol * 1e-2 if prec == PREC["mixed"] else rtol
@@ -543,7 +564,8 @@ def resistance(kernel, points, velocities, eps, mu=1.0, method="auto", rtol=1e-1
             # the refinement's last residual is ||U - K f|| / ||U|| with the FP64 K: reported as is
             f, iterations, ir_steps, resid = _mixed_lu_solve_dev(K, U, rtol_ir, restart, maxiter, lu, required=rtol)
         else:
-            f = _lu_solve_dev(K, U.to(K.dtype) if K.is_complex() else U)
+            flag = _SolveFlag(K.device)
+            f = _lu_solve_dev(K, U.to(K.dtype) if K.is_complex() else U, flag)
             iterations = 1
         del K
     elif method == "gmres":
@@ -560,4 +582,6 @@ def resistance(kernel, points, velocities, eps, mu=1.0, method="auto", rtol=1e-1
         # return exactly this quantity, ||b - A x|| / ||b|| with the FP64 operator, already)
         Kf = _evaluate_dev(kernel, X, X, F.contiguous(), e, mu, "fp64").reshape(-1)
         resid = float(torch.linalg.vector_norm(Kf - U) / torch.linalg.vector_norm(U))
+        if flag is not None and resid != resid:
+            flag.check()
     return _out(F, as_torch), SolveInfo(method, int(iterations), resid, precision, int(ir_steps))

@@ -27,28 +27,4 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ bool cluster_try_wait(uint64_t *bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// bounded; after a timeout (the error word) every later wait gives up at once and the kernel runs to
-// its end on garbage, which the host reports
-__device__ __forceinline__ void cluster_wait(uint64_t *bar, uint32_t parity, int *err) {
-    if (cluster_try_wait(bar, parity)) return;
-    const unsigned long long t0 = global_ns();
-    while (!cluster_try_wait(bar, parity)) {
-        if (*(volatile int *)err) return;
-        if (global_ns() - t0 > kWaitLimitNs) {
-            atomicExch(err, 1);
-            return;
-        }
-    }
-}
-
 }  // namespace flg

@@ -23,8 +23,8 @@
 // ahead on a side stream while the rest of each update finishes.  The inverses
 // of the diagonal blocks' factors, kept in `dinv` for the solves, are one launch at the end.
 //
-// Every spin-wait (the grid barrier, the cluster exchanges, the solves' dataflow, waits.cuh)
-// is bounded and reports failure through a device flag instead of hanging.
+// Every spin-wait (the panels' exchanges, the solves' dataflow, waits.cuh) is bounded and reports
+// failure through a device flag instead of hanging.
 #include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -81,11 +81,6 @@ struct PanelArgs {
 
 __device__ __forceinline__ void st_release_u64(unsigned long long *p, unsigned long long v) {
     asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long *p) {
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
 }
 
 constexpr int kRowBufLd = kPanel + 8;  // a published row: kb values, then the reciprocal of its pivot
@@ -196,17 +191,8 @@ __global__ void __launch_bounds__(256) panel_f64_kernel(PanelArgs a) {
                 const int q = q0 + t;
                 if (q < nblk) {
                     const unsigned long long *w = a.word + (int64_t)buf * nblk + q;
-                    unsigned long long u = ld_relaxed_u64(w);
-                    if ((u >> 63) != par) {
-                        const unsigned long long t0 = global_ns();
-                        while (((u = ld_relaxed_u64(w)) >> 63) != par) {
-                            if (*(volatile int *)&a.bar->err || global_ns() - t0 > kWaitLimitNs) {
-                                atomicExch(&a.bar->err, 1);
-                                s_abort = 1;
-                                break;
-                            }
-                        }
-                    }
+                    unsigned long long u;
+                    if (!wait_parity(w, par, u, kWaitLimitNs, &a.bar->err)) s_abort = 1;
                     const unsigned long long val = u & 0x7fffffffffffffffull;
                     if (val > bv) {
                         bv = val;
@@ -467,10 +453,10 @@ static int swap_trsm(double *A, int64_t ld, const int32_t *ipiv, int64_t k0, int
                      int64_t cap, int *eb, SliceMask *mb, int near, cudaStream_t st) {
     const int64_t nc = c1 - c0;
     FLG_ONCE_PER_DEVICE(
-        FLG_CUDA(cudaFuncSetAttribute(swap_trsm_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem(4,
-                                      kTrsmWarps)));
-        FLG_CUDA(cudaFuncSetAttribute(swap_trsm_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem(16,
-                                      kTrsmWarps))));
+        FLG_CUDA(cudaFuncSetAttribute(swap_trsm_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)trsm_smem(4, kTrsmWarps)));
+        FLG_CUDA(cudaFuncSetAttribute(swap_trsm_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)trsm_smem(16, kTrsmWarps))));
     // G = 4 once its warps (8 columns each) fill half of the schedulers; below, G = 16's shorter chain
     const bool wide = nc >= kTrsmWide * (int64_t)sm_count();
     const int cols = wide ? 8 : 2;
@@ -1395,6 +1381,12 @@ static int panel_geometry(int64_t m, int &nblk, int &rpc) {
     return rpc <= 384 ? FLG_OK : FLG_ERR_INVALID;
 }
 
+// the identity interchanges: what the interchange kernels queued behind a panel whose wait ran out find for its columns
+__global__ void identity_pivots_kernel(int32_t *ipiv, int64_t n) {
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) ipiv[k] = (int32_t)k;
+}
+
 // operand slices of the trailing update: L21's rows (two buffers: the next panel's slices are
 // written while this panel's update still reads its own) and U12's columns, with their exponents and masks
 struct SliceBufs {
@@ -1482,6 +1474,10 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
         FLG_CUDA(cudaFuncSetAttribute(panel_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       384 * kPanel * (int)sizeof(double))));
     FLG_CUDA(cudaMemsetAsync(bar, 0, sizeof(GridBar), st));
+    if (n > kClusterPanelRows) {
+        identity_pivots_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(ipiv, n);
+        FLG_LAUNCH_CHECK();
+    }
     // the panel of columns [k0, k0 + kb), rows k0.. on stream s, and the slices of its L21;
     // started (optional) completes once the panel's first kernel is resident
     auto panel = [&](int64_t k0, cudaStream_t s, cudaEvent_t started) -> int {
@@ -1592,14 +1588,10 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
 // n = 4,608: 1: 1.25 / 4.67, 32: 6.2 / 9.6, 64: 13.7 / 14.6.
 static bool solve_on_cluster(int64_t n, int64_t nrhs) { return nrhs <= (n >= 2048 ? 32 : 16) && trsv_fits(n); }
 
-extern "C" int flg_lu_solve_f64(int64_t n, int64_t nrhs, const double *LU, int64_t ld, const int32_t *ipiv, double *B,
-                                int64_t ldb, void *stream) {
-    FLG_RANGE("flg_lu_solve_f64");
-    FLG_REQUIRE(n >= 0 && nrhs >= 0 && ld >= n && ldb >= nrhs, "bad LU solve arguments");
-    if (n == 0 || nrhs == 0) return FLG_OK;
-    cudaStream_t st = as_stream(stream);
-    FLG_REQUIRE(nrhs <= 65535, "at most 65,535 right-hand sides per call");
-    if (solve_on_cluster(n, nrhs)) return trsv_cluster(n, nrhs, LU, ld, ipiv, B, ldb, st);
+// err (optional): a device word that a timed-out wait of the solve raises
+static int lu_solve_f64(int64_t n, int64_t nrhs, const double *LU, int64_t ld, const int32_t *ipiv, double *B, int64_t ldb,
+                        int *err, cudaStream_t st) {
+    if (solve_on_cluster(n, nrhs)) return trsv_cluster(n, nrhs, LU, ld, ipiv, B, ldb, err, st);
     if (n <= kPivSmemMax) {
         FLG_ONCE_PER_DEVICE(
             FLG_CUDA(cudaFuncSetAttribute(apply_pivots_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1632,6 +1624,28 @@ extern "C" int flg_lu_solve_f64(int64_t n, int64_t nrhs, const double *LU, int64
         }
     }
     return FLG_OK;
+}
+
+static int check_solve(int64_t n, int64_t nrhs, int64_t ld, int64_t ldb) {
+    FLG_REQUIRE(n >= 0 && nrhs >= 0 && ld >= n && ldb >= nrhs, "bad LU solve arguments");
+    FLG_REQUIRE(nrhs <= 65535 || n == 0, "at most 65,535 right-hand sides per call");
+    return FLG_OK;
+}
+extern "C" int flg_lu_solve_f64(int64_t n, int64_t nrhs, const double *LU, int64_t ld, const int32_t *ipiv, double *B,
+                                int64_t ldb, void *stream) {
+    FLG_RANGE("flg_lu_solve_f64");
+    FLG_TRY(check_solve(n, nrhs, ld, ldb));
+    if (n == 0 || nrhs == 0) return FLG_OK;
+    return lu_solve_f64(n, nrhs, LU, ld, ipiv, B, ldb, nullptr, as_stream(stream));
+}
+extern "C" int flg_lu_solve_f64_flag(int64_t n, int64_t nrhs, const double *LU, int64_t ld, const int32_t *ipiv, double *B,
+                                     int64_t ldb, int *flag, void *stream) {
+    FLG_RANGE("flg_lu_solve_f64_flag");
+    FLG_TRY(check_solve(n, nrhs, ld, ldb));
+    FLG_REQUIRE(flag != nullptr, "null flag");
+    FLG_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), as_stream(stream)));
+    if (n == 0 || nrhs == 0) return FLG_OK;
+    return lu_solve_f64(n, nrhs, LU, ld, ipiv, B, ldb, flag, as_stream(stream));
 }
 
 // ---- low-precision LU entry points ----------------------------------------------------
@@ -1771,8 +1785,8 @@ static int lowp_factor(int64_t n, int nbat, float *A, int64_t ld, int64_t sA, in
         return tc_update(C, ld, Lp, ld, Up, W, m, nc, K, mode, tcw, tcb, st, dinfo + 1, false, tile, ctas, bA);
     };
     FLG_ONCE_PER_DEVICE(
-        FLG_CUDA(cudaFuncSetAttribute(block_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LowpPanelSmem<1,
-                                      1>))));
+        FLG_CUDA(cudaFuncSetAttribute(block_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(LowpPanelSmem<1, 1>))));
     const bool tc = mode != FLG_LU_FP32;
     const int64_t nblk = ceil_div(n, kNB);
     SideStream *side = nullptr;

@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(32 * (kMaxRowWarps + kPubWarps), 1) panel_clus
             }
         }
         if (CG > 1) asm volatile("bar.sync 1, %0;" ::"r"(32 * rw) : "memory");  // the other groups' columns of this row
-        cluster_wait((uint64_t *)&S.bar[buf], parity, a.err);
+        cluster_wait((uint64_t *)&S.bar[buf], parity, a.err, kWaitLimitNs);
         __syncwarp();
         const int win = warp_argmax(lane < ncta ? S.rx_key[buf][lane] : 0ull);
         // no candidate anywhere (a column of NaN): row g stays, as the pivot
@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(32 * (kMaxRowWarps + kPubWarps), 1) panel_clus
         rcp = win >= 0 ? S.rx_rcp[buf][win] : 0.0;
         ok = finite_nonzero(pv[j]);
         prow = win >= 0 ? k0 + win * rpc + (int)S.rx_lrow[buf][win] : g;
+        prow = min(max(prow, g), (int)a.n - 1);  // (in range also after a wait that ran out: it indexes memory)
         if (warp == 0 && lane == 0) {
             S.swin[j & 1] = win;
             S.piv[j] = prow;

@@ -30,7 +30,7 @@ struct TrsvShared {
 };
 
 __global__ void __launch_bounds__(kTvThreads, 1) trsv_cluster_kernel(const double *LU, int64_t ld, const int32_t *ipiv,
-                                                                     double *B, int64_t ldb, int n) {
+                                                                     double *B, int64_t ldb, int n, int *err) {
     extern __shared__ __align__(16) uint8_t raw[];
     TrsvShared &S = *reinterpret_cast<TrsvShared *>(raw);
     const int nb = (n + kTb - 1) / kTb, own_max = (nb + kTvCtas - 1) / kTvCtas;
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(kTvThreads, 1) trsv_cluster_kernel(const doubl
                 for (int s = 0; s < 4; s++)
                     if (p0 + s + 1 < np) {
                         const int j = block(p0 + s);
-                        cluster_wait(&pb[j], 0, &S.err);
+                        cluster_wait(&pb[j], 0, &S.err, kWaitLimitNs);
 #pragma unroll
                         for (int q = 0; q < 4; q++) acc = fma(m[s][q], y[j * kTb + cw + q], acc);
                     }
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kTvThreads, 1) trsv_cluster_kernel(const doubl
             }
             if (np > 0) {
                 if (warp < 4) {
-                    cluster_wait(&pb[jl], 0, &S.err);
+                    cluster_wait(&pb[jl], 0, &S.err, kWaitLimitNs);
                     double a = 0.0;
 #pragma unroll
                     for (int q = 0; q < 8; q++) a = fma(ml[q], y[jl * kTb + warp * 8 + q], a);
@@ -212,10 +212,12 @@ __global__ void __launch_bounds__(kTvThreads, 1) trsv_cluster_kernel(const doubl
         // address, so a forward value still under way could land on the backward one that replaces it
         // (a CTA waits for a block by itself only where it needs the block), and a CTA that has
         // ended must not be a store's target.
-        for (int e = t; e < nb; e += kTvThreads) cluster_wait(&pb[e], 0, &S.err);
+        for (int e = t; e < nb; e += kTvThreads) cluster_wait(&pb[e], 0, &S.err, kWaitLimitNs);
         __syncthreads();
         cluster_sync();
     }
+    // a wait that ran out: the results behind it are NaN
+    if (t == 0 && S.err && err) atomicExch(err, 1);
 }
 
 static size_t trsv_smem(int64_t n) {
@@ -225,7 +227,7 @@ static size_t trsv_smem(int64_t n) {
 bool trsv_fits(int64_t n) { return trsv_smem(n) <= 232448; }
 
 int trsv_cluster(int64_t n, int64_t nrhs, const double *LU, int64_t ld, const int32_t *ipiv, double *B, int64_t ldb,
-                 cudaStream_t st) {
+                 int *err, cudaStream_t st) {
     FLG_ONCE_PER_DEVICE(
         FLG_CUDA(cudaFuncSetAttribute(trsv_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         FLG_CUDA(cudaFuncSetAttribute(trsv_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448)));
@@ -240,7 +242,7 @@ int trsv_cluster(int64_t n, int64_t nrhs, const double *LU, int64_t ld, const in
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    FLG_CUDA(cudaLaunchKernelEx(&cfg, trsv_cluster_kernel, LU, ld, ipiv, B, ldb, (int)n));
+    FLG_CUDA(cudaLaunchKernelEx(&cfg, trsv_cluster_kernel, LU, ld, ipiv, B, ldb, (int)n, err));
     count_launch();
     return FLG_OK;
 }

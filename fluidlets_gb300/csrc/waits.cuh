@@ -1,8 +1,8 @@
 // waits.cuh -- the library's bounded device waits.
 //
-// Every spin-wait in a kernel of this library (the FP64 LU panel's grid
-// barrier, the low-precision solve's dataflow polls, the tensor-core update's
-// mbarrier waits) goes through one of the functions below.  Each takes a
+// Every spin-wait in a kernel of this library (the tall FP64 LU panel's polls of published
+// candidates, the grid barrier, the low-precision solve's dataflow polls, the tensor-core updates'
+// mbarrier waits, the cluster exchanges of the FP64 panel and solve) goes through one of the functions below.  Each takes a
 // wall-clock limit in nanoseconds (the %globaltimer register, so the limit
 // does not depend on the SM clock) and an error word: when the limit runs out
 // the wait raises the word and returns false, and the kernel then skips its
@@ -61,6 +61,27 @@ __device__ __forceinline__ bool wait_published4(const unsigned *p, int count, un
             return false;
         }
     }
+}
+
+// ---- published word with a parity ------------------------------------------------------
+// Waits until the top bit of the 64-bit word at p (relaxed loads; the caller fences) is `parity`; v receives the word.
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ bool wait_parity(const unsigned long long *p, unsigned long long parity, unsigned long long &v,
+                                            unsigned long long limit_ns, int *err) {
+    v = ld_relaxed_u64(p);
+    if ((v >> 63) == parity) return true;
+    const unsigned long long t0 = global_ns();
+    while (((v = ld_relaxed_u64(p)) >> 63) != parity) {
+        if (*(volatile int *)err || global_ns() - t0 > limit_ns) {
+            atomicExch(err, 1);
+            return false;
+        }
+    }
+    return true;
 }
 
 // ---- grid barrier -------------------------------------------------------------------
@@ -125,6 +146,33 @@ __device__ __forceinline__ bool mbar_drain(uint64_t *bar, uint32_t parity, int *
     if (mbar_try_wait(bar, parity)) return true;
     const unsigned long long t0 = global_ns();
     while (!mbar_try_wait(bar, parity)) {
+        if (global_ns() - t0 > limit_ns) {
+            atomicExch(err, 1);
+            return false;
+        }
+    }
+    return true;
+}
+
+// ---- cluster exchange -------------------------------------------------------------------
+// The phase of an mbarrier that other CTAs of the cluster complete (st.async), acquired at cluster scope.  After a
+// wait that ran out every later one gives up at once, and the kernel runs to its end on whatever it has, its
+// indexes kept in range, so that the CTAs still meet at their cluster barriers.
+__device__ __forceinline__ bool cluster_try_wait(uint64_t *bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool cluster_wait(uint64_t *bar, uint32_t parity, int *err, unsigned long long limit_ns) {
+    if (cluster_try_wait(bar, parity)) return true;
+    const unsigned long long t0 = global_ns();
+    while (!cluster_try_wait(bar, parity)) {
+        if (*(volatile int *)err) return false;
         if (global_ns() - t0 > limit_ns) {
             atomicExch(err, 1);
             return false;

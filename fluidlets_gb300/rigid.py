@@ -19,8 +19,8 @@ import numpy as np
 import torch
 
 from . import _device as dv
-from .core import (_assemble_dev, _blob_widths, _gmres_ir_dense_dev, _lowp_factor_dev, _lu_solve_dev, _points, _prec,
-                   _uniform_eps)
+from .core import (_SolveFlag, _assemble_dev, _blob_widths, _gmres_ir_dense_dev, _lowp_factor_dev, _lu_solve_dev,
+                   _points, _prec, _uniform_eps)
 from .kernels import Stokeslet3D
 from .swimming import _system_dev
 
@@ -45,12 +45,16 @@ def rigid_body_mobility(kernel, points, eps, force, torque=(0.0, 0.0, 0.0), mu=1
     rhs = torch.zeros(3 * N + 6, dtype=torch.float64, device=A.device)
     rhs[3 * N:3 * N + 3] = torch.from_numpy(F).to(A.device)
     rhs[3 * N + 3:] = torch.from_numpy(T).to(A.device)
+    flag = None
     if _prec(precision) == 1:
         K32, ld32, dinv, A32 = _lowp_factor_dev(A, lu)
         sol, *_ = _gmres_ir_dense_dev(A, K32, ld32, dinv, rhs, rtol * 1e-2, 60, 200, required=rtol, A32=A32)
     else:
-        sol = _lu_solve_dev(A, rhs)
+        flag = _SolveFlag(A.device)
+        sol = _lu_solve_dev(A, rhs, flag)
     sol = dv.to_host(sol)
+    if flag is not None and np.isnan(sol).any():
+        flag.check()
     return sol[3 * N:3 * N + 3], sol[3 * N + 3:], sol[:3 * N].reshape(N, 3)
 
 

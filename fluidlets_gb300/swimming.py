@@ -23,7 +23,8 @@ import torch
 
 from . import _device as dv
 from ._lib import F64, check, load, lu_mode
-from .core import _assemble_nearest_dev, _gmres_ir_dense_dev, _lowp_factor_dev, _lu_solve_dev, _prec, nearest_neighbors
+from .core import (_SolveFlag, _assemble_nearest_dev, _gmres_ir_dense_dev, _lowp_factor_dev, _lu_solve_dev, _prec,
+                   nearest_neighbors)
 from .kernels import Stokeslet3D, kernel_params
 
 
@@ -81,12 +82,16 @@ def swimming_problem(shape: SwimmerShape, x0, B, eps, mu=1.0, kernel=None, neare
     A = _system_dev(kernel, x, X, nearest, x0, eps, mu)
     rhs = torch.zeros(3 * N + 6, dtype=torch.float64, device=A.device)
     rhs[:3 * N] = torch.from_numpy(v.ravel()).to(A.device)
+    flag = None
     if _prec(precision) == 1:
         K32, ld32, dinv, A32 = _lowp_factor_dev(A, lu)
         sol, *_ = _gmres_ir_dense_dev(A, K32, ld32, dinv, rhs, rtol * 1e-2, 60, 200, required=rtol, A32=A32)
     else:
-        sol = _lu_solve_dev(A, rhs)
+        flag = _SolveFlag(A.device)
+        sol = _lu_solve_dev(A, rhs, flag)
     sol = dv.to_host(sol)
+    if flag is not None and np.isnan(sol).any():
+        flag.check()
     return SwimState(sol[3 * N:3 * N + 3], sol[3 * N + 3:], sol[:3 * N].reshape(N, 3), x, X, nearest)
 
 

@@ -228,9 +228,14 @@ size_t flg_lu_factor_f64_workspace(int64_t n);
 int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv, int *info,
                       void *work, size_t work_bytes, void *stream);
 /* Solves A X = B with the factors of flg_lu_factor_f64; B is (n x nrhs)
- * row-major with leading dimension ldb, overwritten by X. */
+ * row-major with leading dimension ldb, overwritten by X.  Asynchronous: a
+ * bounded wait that ran out leaves NaN in X. */
 int flg_lu_solve_f64(int64_t n, int64_t nrhs, const double *LU, int64_t ld, const int32_t *ipiv,
                      double *B, int64_t ldb, void *stream);
+/* The same, with the outcome of its waits in the device word flag (0, or 1 where
+ * a wait ran out) for the caller to read after the stream. */
+int flg_lu_solve_f64_flag(int64_t n, int64_t nrhs, const double *LU, int64_t ld, const int32_t *ipiv,
+                          double *B, int64_t ldb, int *flag, void *stream);
 
 /* Low-precision LU without pivoting for the mixed-precision path: A is FP32
  * (n x n, ld; ld a multiple of 4 so every row starts on a 16-byte boundary),
@@ -489,10 +494,11 @@ int64_t flg_launch_count(void);
  * No counterpart in the reference (its solvers run on the host; their only
  * failure report is RuntimeError on GMRES non-convergence, core/solve.py:77-78).
  * flg_wait_selftest drives one kind of wait to expiry on a condition nothing
- * satisfies, with a limit of `limit_ms`: which = 0 the grid barrier of the FP64
- * LU panel (one arrival never comes), 1 the low-precision solve's poll of a
- * published value (nothing publishes it), 2 the tensor-core update's mbarrier
- * wait (no arrival completes the phase).  It returns FLG_ERR_TIMEOUT, as the
+ * satisfies, with a limit of `limit_ms`: which = 0 the grid barrier (one arrival
+ * never comes), 1 the polls of published values, the low-precision solve's and
+ * the tall FP64 panel's (nothing publishes them), 2 the mbarrier waits, the
+ * tensor-core updates' and the cluster exchanges' of the FP64 panel and solve
+ * (no arrival completes the phase).  It returns FLG_ERR_TIMEOUT, as the
  * production entry points do for such a wait, after about limit_ms, with the
  * context still usable.  Synchronizes. */
 size_t flg_wait_selftest_workspace(void);

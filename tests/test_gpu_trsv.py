@@ -52,3 +52,31 @@ def test_repeated_solves_give_the_same_bits(n):
     scale = np.abs(np.tril(F, -1) + np.eye(n)) @ (np.abs(np.triu(F)) @ np.abs(x).astype(float))
     # backward error of the factors and the substitutions, 3 n u |L| |U| |x| in all, in the largest row
     assert np.abs(A @ x - b).max() <= 3 * n * 2.0**-53 * scale.max()
+
+
+@pytest.mark.parametrize("n,nrhs", [(1, 1), (513, 2), (100, 40)])
+def test_flagged_solves(n, nrhs):
+    """The same bits, with the outcome of the waits in a word of the caller's."""
+    _, LU, piv = factored(n, n + 7)
+    L = _lib.load()
+    B = torch.randn((n, nrhs), dtype=torch.float64, device="cuda")
+    X, Y = B.clone(), B.clone()
+    flag = torch.full((1,), 77, dtype=torch.int32, device="cuda")
+    args = (n, nrhs, dv.ptr(LU), n, dv.ptr(piv))
+    _lib.check(L.flg_lu_solve_f64(*args, dv.ptr(X), nrhs, dv.stream()))
+    _lib.check(L.flg_lu_solve_f64_flag(*args, dv.ptr(Y), nrhs, dv.ptr(flag), dv.stream()))
+    assert torch.equal(X, Y) and int(flag) == 0
+    assert L.flg_lu_solve_f64_flag(*args, dv.ptr(Y), nrhs, None, dv.stream()) == _lib.FLG_ERR_INVALID
+    assert L.flg_lu_solve_f64_flag(n, nrhs, dv.ptr(LU), n - 1, dv.ptr(piv), dv.ptr(Y), nrhs, dv.ptr(flag),
+                                   dv.stream()) == _lib.FLG_ERR_INVALID
+
+
+def test_a_raised_flag_reaches_python():
+    from fluidlets_gb300.core import _SolveFlag
+
+    flag = _SolveFlag("cuda")
+    flag.word.zero_()
+    flag.check()
+    flag.word.fill_(1)
+    with pytest.raises(RuntimeError, match="timed out"):
+        flag.check()
