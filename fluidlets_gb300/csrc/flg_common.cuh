@@ -70,16 +70,19 @@ inline int sm_count() {
     return n;
 }
 
-// Bump allocator over a caller-provided workspace (256-byte aligned slices).
+// Bump allocator over a caller-provided workspace (256-byte aligned slices).  After a slice that did not fit every
+// later one is null, too, so that the last one taken tells whether all were.
 struct Arena {
     char *base;
     size_t cap, used;
+    bool full = false;
     Arena(void *p, size_t n) : base((char *)p), cap(n), used(0) {}
     template <typename T>
     T *take(size_t count) {
         size_t off = (used + 255) & ~size_t(255);
         size_t bytes = count * sizeof(T);
-        if (off + bytes > cap || (base == nullptr && bytes > 0)) return nullptr;
+        full = full || off + bytes > cap || (base == nullptr && bytes > 0);
+        if (full) return nullptr;
         used = off + bytes;
         return (T *)(base + off);
     }
