@@ -1234,5 +1234,7 @@ extern "C" int flg_convert_f64_f32x2(int64_t n_rows, int64_t n_cols, const doubl
 
 extern "C" int flg_convert_f64_f32(int64_t n_rows, int64_t n_cols, const double *src, int64_t lds, float *dst,
                                    int64_t ldd, void *stream) {
+    FLG_REQUIRE(n_rows >= 0 && n_cols >= 0 && lds >= n_cols && ldd >= n_cols, "bad conversion shape");
+    if (n_rows == 0 || n_cols == 0) return FLG_OK;  // (nothing to write: dst may be null)
     return flg_convert_f64_f32x2(n_rows, n_cols, src, lds, dst, nullptr, ldd, stream);
 }
