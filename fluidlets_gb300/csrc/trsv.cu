@@ -147,6 +147,7 @@ __global__ void __launch_bounds__(kTvThreads, 1) trsv_cluster_kernel(const doubl
             }
             __syncthreads();
             double v = 0.0, tr[kTb], rd = 1.0;
+            bool divide = false;
             if (warp == 0) {
                 v = up ? y[b * kTb + lane] : rhs[own * kTb + lane];
 #pragma unroll
@@ -154,9 +155,18 @@ __global__ void __launch_bounds__(kTvThreads, 1) trsv_cluster_kernel(const doubl
 #pragma unroll
                 for (int q = 0; q < kTb; q++) tr[q] = S.T[lane][q];
                 if (up) {  // T x = T D^-1 (D x): the columns scaled ahead take the multiplication off the chain
+                    const int ex = (__double2hiint(S.T[lane][lane]) >> 20) & 0x7ff;
+                    bool bad = ex < 64 || ex > 1982;
                     rd = __drcp_rn(S.T[lane][lane]);
 #pragma unroll
-                    for (int q = 0; q < kTb; q++) tr[q] *= __shfl_sync(0xffffffffu, rd, q);
+                    for (int q = 0; q < kTb; q++) {
+                        const double t0 = tr[q];
+                        tr[q] *= __shfl_sync(0xffffffffu, rd, q);
+                        const int hi = __double2hiint(tr[q]), e = (hi >> 20) & 0x7ff;
+                        bad = bad || (q > lane && (e == 0x7ff || (e == 0 && t0 != 0.0)));
+                    }
+                    // a reciprocal or a scaled entry outside the normal range loses accuracy, or is infinite: divide there
+                    divide = __any_sync(0xffffffffu, bad);
                 }
             }
             if (np > 0) {
@@ -180,9 +190,7 @@ __global__ void __launch_bounds__(kTvThreads, 1) trsv_cluster_kernel(const doubl
                         v = lane > q ? w : v;
                     }
                 } else {
-                    // 1 / u loses accuracy where it leaves the normal range: divide there
-                    const int ex = (__double2hiint(S.T[lane][lane]) >> 20) & 0x7ff;
-                    if (__any_sync(0xffffffffu, ex < 64 || ex > 1982)) {
+                    if (divide) {
                         for (int q = kTb - 1; q >= 0; q--) {
                             const double x = v / S.T[lane][lane];
                             const double xq = __shfl_sync(0xffffffffu, x, q);

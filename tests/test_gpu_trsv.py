@@ -80,3 +80,25 @@ def test_a_raised_flag_reaches_python():
     flag.word.fill_(1)
     with pytest.raises(RuntimeError, match="timed out"):
         flag.check()
+
+
+@pytest.mark.parametrize("n,col", [(20, 19), (32, 31), (40, 39), (70, 50)])
+@pytest.mark.parametrize("big,small", [(1e160, 1e-160), (1e-200, 1e150)])
+def test_columns_far_from_their_pivots(n, col, big, small):
+    """An upper-triangular matrix with one column that is 1e320 times its diagonal entry (or 1e-350 of it): the
+    quotient of the two is not a number, the solution is."""
+    rng = np.random.default_rng(n)
+    A = np.eye(n)
+    A[:col, col] = big * rng.uniform(1, 2, col)
+    A[col, col] = small
+    b = rng.normal(size=(n, 1))
+    b[col] = 1e-200 * small if big > 1 else 1e130 * small
+    x = b.copy()
+    x[col] = b[col] / small
+    x[:col] -= A[:col, col:col + 1] * x[col]
+    L = _lib.load()
+    Ad, B = torch.tensor(A, device="cuda"), torch.tensor(b, device="cuda")
+    piv = torch.arange(n, dtype=torch.int32, device="cuda")
+    _lib.check(L.flg_lu_solve_f64(n, 1, dv.ptr(Ad), n, dv.ptr(piv), dv.ptr(B), 1, dv.stream()))
+    got = B.cpu().numpy()
+    assert np.all(np.abs(got - x) <= 4 * 2.0**-53 * (np.abs(b) + np.abs(A[:, col:col + 1] * x[col])) + 4 * 2.0**-53 * np.abs(x))
