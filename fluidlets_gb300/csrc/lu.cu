@@ -1022,7 +1022,7 @@ __global__ void __launch_bounds__(256) sgemm_kernel(int64_t M, int64_t N, int64_
 size_t tc_update_bytes(int64_t m, int64_t nc, int64_t K, int mode, int nb = 1);
 int tc_update(float *C, int64_t ldc, const float *Lp, int64_t ldl, const float *Ut, int64_t ldu, int64_t m,
               int64_t nc, int64_t K, int mode, void *work, size_t work_bytes, cudaStream_t st, int *err_dev,
-              bool store = false, int tile = 0, int max_ctas = 0, const TcBatch &bt = TcBatch{});
+              int tile = 0, int max_ctas = 0, const TcBatch &bt = TcBatch{});
 // the BF16 update from operands already rounded to BF16 (La, Ub: K-major __nv_bfloat16)
 int tc_update_bf16(float *C, int64_t ldc, const void *La, int64_t ldl, const void *Ub, int64_t ldu, int64_t m,
                    int64_t nc, int64_t K, void *work, size_t work_bytes, cudaStream_t st, int *err_dev, int tile,
@@ -1782,7 +1782,7 @@ static int lowp_factor(int64_t n, int nbat, float *A, int64_t ld, int64_t sA, in
             return tc_update_bf16(C, ld, LB + r * W + (c - K0), W, UB + (Up - UtB), W, m, nc, K, tcw, tcb, st,
                                   dinfo + 1, tile, ctas, bB);
         }
-        return tc_update(C, ld, Lp, ld, Up, W, m, nc, K, mode, tcw, tcb, st, dinfo + 1, false, tile, ctas, bA);
+        return tc_update(C, ld, Lp, ld, Up, W, m, nc, K, mode, tcw, tcb, st, dinfo + 1, tile, ctas, bA);
     };
     FLG_ONCE_PER_DEVICE(
         FLG_CUDA(cudaFuncSetAttribute(block_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -1,7 +1,6 @@
 // tc_gemm.cu -- tcgen05 tensor-core rank-K update for the low-precision LU.
 //
 //   C (m x nc, FP32, row-major, ldc)  -=  A (m x K) * B^T,  B given as Bt (nc x K)
-//   (or, in store mode, C = A * B^T)
 //
 // Both operands are K-major (K contiguous per row, K a multiple of 128).  A
 // batch of equally shaped updates of independent systems (fixed strides
@@ -55,7 +54,7 @@ template <int MODE, int TC_BN>
 __global__ void __launch_bounds__(TC_THREADS, 1) tc_update_kernel(const __grid_constant__ CUtensorMap tmA,
                                                                   const __grid_constant__ CUtensorMap tmB,
                                                                   const __grid_constant__ CUtensorMap tmC, int m,
-                                                                  int nc, int nkb, int nbat, int store, int *err) {
+                                                                  int nc, int nkb, int nbat, int *err) {
     constexpr int KBLK = MODE == FLG_LU_TF32 ? 32 : 64;  // elements per 128-byte row
     constexpr int KSTEP_BYTES = 32;                       // one MMA consumes 32 bytes of each row
     constexpr uint32_t IDESC = tc_idesc(MODE == FLG_LU_TF32 ? 2u : 1u, TC_BN);
@@ -200,18 +199,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_update_kernel(const __grid_c
                 if (nst >= 2 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                 __syncwarp();
                 // row `lane`, 16-byte chunk c at chunk position c ^ (row % 8) (128-byte swizzle)
-                const float sg = store ? 1.0f : -1.0f;  // C = acc, or C += -acc
 #pragma unroll
                 for (int c = 0; c < 8; c++) {
-                    const float4 w = make_float4(sg * __uint_as_float(v[4 * c]), sg * __uint_as_float(v[4 * c + 1]),
-                                                 sg * __uint_as_float(v[4 * c + 2]), sg * __uint_as_float(v[4 * c + 3]));
+                    const float4 w = make_float4(-__uint_as_float(v[4 * c]), -__uint_as_float(v[4 * c + 1]),
+                                                 -__uint_as_float(v[4 * c + 2]), -__uint_as_float(v[4 * c + 3]));
                     *reinterpret_cast<float4 *>(box + lane * 128 + ((c ^ (lane & 7)) << 4)) = w;
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) {
-                    if (store) tma_store_3d(&tmC, box, n0 + ch * 32, m0 + q * 32, z);
-                    else tma_reduce_add_3d(&tmC, box, n0 + ch * 32, m0 + q * 32, z);
+                    tma_reduce_add_3d(&tmC, box, n0 + ch * 32, m0 + q * 32, z);
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
             }
@@ -354,22 +351,21 @@ int tc_pick_tile(int64_t m, int64_t nc, int sms, int nb = 1) {
 
 template <int MODE, int BN>
 static int tc_launch(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, int64_t m, int64_t nc,
-                     int nkb, int nb, bool store, int *err, int sms, cudaStream_t st) {
+                     int nkb, int nb, int *err, int sms, cudaStream_t st) {
     FLG_ONCE_PER_DEVICE(
         FLG_CUDA(cudaFuncSetAttribute(tc_update_kernel<MODE, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)TcTile<BN>::SMEM)));
     const int64_t ntiles = nb * ceil_div(m, TC_BM) * ceil_div(nc, BN);
     FLG_REQUIRE(ntiles < (1LL << 31), "too many tiles");
     const unsigned grid = (unsigned)std::min<int64_t>(ntiles, sms);
-    tc_update_kernel<MODE, BN><<<grid, TC_THREADS, TcTile<BN>::SMEM, st>>>(ma, mb, mc, (int)m, (int)nc, nkb, nb,
-                                                                           store ? 1 : 0, err);
+    tc_update_kernel<MODE, BN><<<grid, TC_THREADS, TcTile<BN>::SMEM, st>>>(ma, mb, mc, (int)m, (int)nc, nkb, nb, err);
     FLG_LAUNCH_CHECK();
     return FLG_OK;
 }
 
 // The launch and the timeout check shared by both entry points below: C map, grid, flag.
 static int tc_run(const CUtensorMap &ma, const CUtensorMap &mb, float *C, int64_t ldc, int64_t m, int64_t nc,
-                  int64_t K, int mode, int bn, int sms, const TcBatch &bt, bool store, int *err, bool own_err,
+                  int64_t K, int mode, int bn, int sms, const TcBatch &bt, int *err, bool own_err,
                   cudaStream_t st) {
     const int nb = bt.count;
     CUtensorMap mc;
@@ -378,11 +374,11 @@ static int tc_run(const CUtensorMap &ma, const CUtensorMap &mb, float *C, int64_
     const int nkb = (int)(K / (mode == FLG_LU_TF32 ? 32 : 64));
     int rc;
     if (mode == FLG_LU_TF32)
-        rc = bn == 128 ? tc_launch<FLG_LU_TF32, 128>(ma, mb, mc, m, nc, nkb, nb, store, err, sms, st)
-                       : tc_launch<FLG_LU_TF32, 256>(ma, mb, mc, m, nc, nkb, nb, store, err, sms, st);
+        rc = bn == 128 ? tc_launch<FLG_LU_TF32, 128>(ma, mb, mc, m, nc, nkb, nb, err, sms, st)
+                       : tc_launch<FLG_LU_TF32, 256>(ma, mb, mc, m, nc, nkb, nb, err, sms, st);
     else
-        rc = bn == 128 ? tc_launch<FLG_LU_BF16, 128>(ma, mb, mc, m, nc, nkb, nb, store, err, sms, st)
-                       : tc_launch<FLG_LU_BF16, 256>(ma, mb, mc, m, nc, nkb, nb, store, err, sms, st);
+        rc = bn == 128 ? tc_launch<FLG_LU_BF16, 128>(ma, mb, mc, m, nc, nkb, nb, err, sms, st)
+                       : tc_launch<FLG_LU_BF16, 256>(ma, mb, mc, m, nc, nkb, nb, err, sms, st);
     FLG_TRY(rc);
     if (!own_err) return FLG_OK;
     int herr = 0;
@@ -411,7 +407,7 @@ static int tc_check_shape(int64_t m, int64_t nc, int64_t K, int tile, const TcBa
 // of bt.count systems, C, Lp and Ut of system z at + z * (bt.sC, bt.sL, bt.sU).
 int tc_update(float *C, int64_t ldc, const float *Lp, int64_t ldl, const float *Ut, int64_t ldu, int64_t m,
               int64_t nc, int64_t K, int mode, void *work, size_t work_bytes, cudaStream_t st, int *err_dev,
-              bool store, int tile, int max_ctas, const TcBatch &bt) {
+              int tile, int max_ctas, const TcBatch &bt) {
     FLG_REQUIRE(mode == FLG_LU_TF32 || mode == FLG_LU_BF16, "tensor-core mode must be TF32 or BF16");
     FLG_TRY(tc_check_shape(m, nc, K, tile, bt));
     const int nb = bt.count;
@@ -438,7 +434,7 @@ int tc_update(float *C, int64_t ldc, const float *Lp, int64_t ldl, const float *
         FLG_TRY(make_operand_map(&ma, La, m, K, K, mode, TC_BM, nb, m * K));
         FLG_TRY(make_operand_map(&mb, Ub, nc, K, K, mode, bn, nb, nc * K));
     }
-    return tc_run(ma, mb, C, ldc, m, nc, K, mode, bn, sms, bt, store, err, err_dev == nullptr, st);
+    return tc_run(ma, mb, C, ldc, m, nc, K, mode, bn, sms, bt, err, err_dev == nullptr, st);
 }
 
 // The BF16 update with operands already rounded to BF16 (K-major, row strides ldl / ldu
@@ -458,7 +454,7 @@ int tc_update_bf16(float *C, int64_t ldc, const void *La, int64_t ldl, const voi
     CUtensorMap ma, mb;
     FLG_TRY(make_operand_map(&ma, La, m, K, ldl, FLG_LU_BF16, TC_BM, nb, bt.sL));
     FLG_TRY(make_operand_map(&mb, Ub, nc, K, ldu, FLG_LU_BF16, bn, nb, bt.sU));
-    return tc_run(ma, mb, C, ldc, m, nc, K, FLG_LU_BF16, bn, sms, bt, false, err, err_dev == nullptr, st);
+    return tc_run(ma, mb, C, ldc, m, nc, K, FLG_LU_BF16, bn, sms, bt, err, err_dev == nullptr, st);
 }
 
 }  // namespace flg
@@ -473,5 +469,5 @@ extern "C" int flg_tc_rank_update(float *C, int64_t ldc, const float *A, int64_t
     FLG_REQUIRE(ldb == 128, "Bt must be compact (ldb == 128)");
     FLG_REQUIRE(lda >= 128 && ldc >= nc, "bad leading dimensions");
     return flg::tc_update(C, ldc, A, lda, Bt, 128, m, nc, 128, mode, work, work_bytes, flg::as_stream(stream), nullptr,
-                          false, 0, 0, flg::TcBatch{});
+                          0, 0, flg::TcBatch{});
 }
