@@ -36,7 +36,7 @@ def test_one_step_beyond_the_tolerance(lib):
     assert lib.ir_inner(1.0, 0.9) == lib.ir_inner(1.0, 1.0) == 1e-4
     assert not lib.ir_done(1.0, 1.1, 0) and not lib.ir_done(1.0, 1.1, 1)
     assert not lib.ir_done(1.0, 0.9, 0) and lib.ir_done(1.0, 0.9, 1)
-    assert not lib.ir_done(1.0, 0.03, 0) and lib.ir_done(1.0, 0.019, 0) and lib.ir_done(1.0, 0.0, 0)
+    assert not lib.ir_done(1.0, 0.031, 0) and lib.ir_done(1.0, 0.03, 0) and lib.ir_done(1.0, 0.0, 0)
 
 
 def test_degenerate_residuals(lib):
