@@ -1539,8 +1539,9 @@ extern "C" int flg_lu_factor_f64(int64_t n, double *A, int64_t ld, int32_t *ipiv
         const int64_t nc = n - c0;
         const int64_t nn = std::min<int64_t>(kPanel, nc);  // the next panel's columns first
         // where the substitution of all columns is a long launch (37 us from 2,432 columns on, 12 for the next
-        // panel's), the rest of them follows beside the panel: n = 4,608 15.26 -> 14.94 ms; at fewer columns
-        // the launch costs what it saves (2,304: 5.71, 5.82 ms)
+        // panel's), the rest of them follows beside the panel; at fewer columns the launch costs what it saves.
+        // Factorizations in ms without this / at any width: 2,432 5.96 / 6.02, 2,800 7.27 / 7.24, 3,200 8.77 / 8.58, 3,600
+        // 10.39 / 9.98, 4,608 14.68 / 14.11, 7,000 31.25 / 31.17
         const bool split = nc >= kTrsmWide * (int64_t)sm_count() && nc <= kClusterPanelRows;
         FLG_TRY(swap_trsm(A, ld, ipiv, k0, c0, split ? c0 + nn : n, sb.B, n, sb.eb, sb.mb, near, st));
         prof_begin(FLG_SLOT_LU_UPDATE, st);

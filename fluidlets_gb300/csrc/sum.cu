@@ -466,9 +466,10 @@ __global__ void __launch_bounds__(64) finalize_kernel(FinalArgs a) {
         for (int c = 0; c < OUTW; c++) u[c] += __shfl_xor_sync(0xffffffffu, u[c], o);
     if (i < a.M && l == 0) final_store(a, i, u);
 }
-// Eight lanes per target where there are many splits of few targets (4,099 targets, 30 splits: a call of
-// 1.29 ms with one lane, 1.26 with eight); more targets fill the chip by themselves, and 32 of them
-// per warp read whole sectors (32,768 targets, 19 splits: 1.24 ms with one lane, 1.26 with eight).
+// Eight lanes per target where there are many splits of few targets; more targets fill the chip by themselves, and
+// 32 of them per warp read whole sectors.  us of a sum over 1,000 sources with one lane / eight, Stokeslet and complex
+// Brinkman: 2,000 targets 96 / 74 and 359 / 313, 4,099: 124 / 112 and 577 / 554, 6,000: 156 / 150 and 764 / 754, 8,192: 204 /
+// 204 and 1,012 / 1,010, 10,000: 235 / 237 and 1,225 / 1,231, 16,000: 354 / 362 and 1,815 / 1,836.
 template <int OUTW>
 static void launch_finalize(const FinalArgs &a, cudaStream_t st) {
     if (a.S < 16 || a.M > 8192) finalize_kernel<OUTW, 1><<<(unsigned)ceil_div(a.M, 64), 64, 0, st>>>(a);
