@@ -10,8 +10,8 @@
 //
 //   x = 0, r = b, ||b||                              (prologue)
 //   WHILE the residual is above rtol ||b||:          (refinement steps)
-//     v0 = M^-1 r, beta = ||v0||, ptol = ir_inner_tolerance beta   (inner GMRES on M^-1 A d = M^-1 r)
-//     WHILE the inner residual estimate is above ptol and columns remain:
+//     v0 = M^-1 r, beta = ||v0||, ptol = kIrInner beta   (inner GMRES on M^-1 A d = M^-1 r)
+//     WHILE the inner residual estimate is above ir_inner_limit and columns remain:
 //       w = M^-1 (A32 v_k); two classical Gram-Schmidt passes; Givens update
 //     x += V y (upper-triangular least squares)
 //     r = b - K x (FP64), ||r||, stall and step-count checks
@@ -160,7 +160,7 @@ __global__ void ir_ctrl_init(IrState *S, double rtol, int m, int max_outer, cuda
 // start of an inner solve: beta = ||M^-1 r||, its tolerance, g = beta e1
 __global__ void ir_ctrl_inner_init(IrState *S, cudaGraphConditionalHandle h_inner) {
     S->beta = sqrt(fmax(S->dot, 0.0));
-    S->ptol = S->beta * ir_inner_tolerance(S->tol, S->rn);
+    S->ptol = S->beta * kIrInner;
     for (int q = 0; q <= S->m; q++) S->g[q] = 0.0;
     S->g[0] = S->beta;
     S->k = 0;
@@ -187,7 +187,7 @@ __device__ void ir_lartg(double f, double g, double &c, double &s, double &r) {
 }
 
 // after an Arnoldi step: the new Hessenberg column, the previous rotations applied, a new one
-// made, the residual estimate; the inner loop goes on while it exceeds ptol and columns remain
+// made, the residual estimate; the inner loop goes on while it exceeds its limit and columns remain
 __global__ void ir_ctrl_step(IrState *S, cudaGraphConditionalHandle h_inner) {
     const int col = S->k, m = S->m;
     double *hc = S->h + col * (m + 1);
@@ -216,7 +216,7 @@ __global__ void ir_ctrl_step(IrState *S, cudaGraphConditionalHandle h_inner) {
     S->presid = fabs(t);
     S->iters++;
     S->k = col + 1;
-    const bool more = S->presid > S->ptol && !S->breakdown && S->k < m;
+    const bool more = S->presid > ir_inner_limit(S->ptol, S->k) && !S->breakdown && S->k < m;
     cudaGraphSetConditional(h_inner, more ? 1u : 0u);
 }
 

@@ -160,6 +160,7 @@ struct Gmres {
     T *hdev = nullptr;     // 3 (m + 2) scalars
     int *flag = nullptr;
     int64_t nchunk = 0;
+    bool ir_steps = false;  // stop by ir_inner_limit (the steps of a dense refinement)
     // y = A v ; y = M^-1 v (optional)
     std::function<int(const T *, T *)> A, M;
 
@@ -358,7 +359,7 @@ struct Gmres {
             S_[col + 1] = t;
             presid = std::abs(t);
             iters++;
-            if (presid <= ptol || breakdown) break;
+            if (presid <= (ir_steps ? ir_inner_limit(ptol, col + 1) : ptol) || breakdown) break;
         }
         if (col == m) col = m - 1;
         // back substitution on the (col+1) x (col+1) upper triangle
@@ -651,8 +652,9 @@ extern "C" int flg_gmres_ir_dense(int64_t n, const double *A, int64_t ld, const 
     char *lw = ar.take<char>(lsb);
     float *xs = ar.take<float>(2 * n);
     FLG_REQUIRE(d && lw && xs, "workspace too small for GMRES-IR");
-    // outer residuals with the FP64 matrix; inner (preconditioned, ir_inner_tolerance) matvecs
+    // outer residuals with the FP64 matrix; inner (preconditioned, kIrInner) matvecs
     // with the FP32 copy when the caller provides one
+    gi.ir_steps = true;
     g.A = [&](const double *v, double *out) { return flg_gemv_f64(n, n, A, ld, v, out, st); };
     if (A32)
         gi.A = [&](const double *v, double *out) { return gemv_f32_presplit(n, n, A32, lda32, v, xs, out, st); };
@@ -684,7 +686,7 @@ extern "C" int flg_gmres_ir_dense(int64_t n, const double *A, int64_t ld, const 
         prev = rn;
         FLG_CUDA(cudaMemsetAsync(d, 0, sizeof(double) * n, st));
         double rin;
-        int s2 = gi.solve(g.r, d, ir_inner_tolerance(tol, rn), maxiter, *iters, rin, rn, true);
+        int s2 = gi.solve(g.r, d, kIrInner, maxiter, *iters, rin, rn, true);
         if (s2 != FLG_OK && s2 != FLG_ERR_NOT_CONVERGED) return s2;
         add_kernel<double><<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(x, d, n);
         FLG_LAUNCH_CHECK();

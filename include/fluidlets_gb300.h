@@ -319,8 +319,8 @@ int flg_gmres(int kind, double alpha_re, double alpha_im,
 
 /* Dense GMRES-IR: solves A x = b (n x n FP64 row-major, ld) to rtol with
  * FP64 residuals b - A x (FP64 GEMV), correcting with inner GMRES (tolerance
- * 1e-6, tighter in the last step; one step more where the residual ends above
- * 0.03 rtol) on the operator M^-1 A, M = the low-precision factors of
+ * 1e-4, 1e-6 to stop after one column; one step more where the residual ends
+ * above 0.05 rtol) on the operator M^-1 A, M = the low-precision factors of
  * flg_lu_factor_lowp (LU32, ld32, dinv).  The inner matvecs use A32 (an FP32
  * copy of A, leading dimension lda32) when it is not NULL, else A.  Real
  * only.  iters = total inner iterations, outer = refinement steps, resid =
