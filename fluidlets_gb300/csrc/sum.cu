@@ -1283,7 +1283,7 @@ void sum_layout(int kind, int64_t M, int64_t N, int nf, bool ck, int precision, 
     if (precision == FLG_PREC_FP64) {
         // splits down to 8 sources: a pair is a chain of several hundred clocks, so a small call's time is
         // the longest split (226 x 226: 112 us with whole tiles of 128, 9 us with 8); four waves
-        // of the four CTAs that fit an SM (4,099 x 2,500 complex: 1.20 ms a call, with eight 1.25, with two 1.23)
+        // of the four CTAs that fit an SM (4,099 x 2,500 complex: 0.93 ms a call, with six and eight 0.96, with three 0.93)
         split_plan(M, N, kF64Threads, kF64Tile, 8, 4, L.S, L.split_len);
     } else {
         split_plan(M, N, kF32Threads * far_tpt(kind, nf, ck), kF32Tile, kF32Tile, 4, L.S,
